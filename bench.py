@@ -142,17 +142,17 @@ def peaks():
 
 
 # ------------------------------------------------------------------------------------------ algorithmic counts
-# FP64 operations per cell of the cell kernels, counted from their source (csrc/q1.cu, csrc/q1_common.cuh):
-# one grad-u column = 30 (3 components x (2 bilinear lerps of 3 + final lerp and 1/h of 4)); det = 17; cofactor+det
-# = 35; curl = 3; sq_change = 20; compensated add = 8.  Barrier-active points add a few hundred more (not counted).
+# FP64 operations per cell of the cell kernels, counted from their source (csrc/q1.cu, csrc/q1_closed.cuh,
+# csrc/q1_common.cuh).  On the closed27 points: edges of one field 72, averages 120, det - 1 at 27 points 27 x 18,
+# curl coefficients 54; Legendre transform 27 x 6, weighted sums about 100.  At the Gauss points: one grad-u column = 30
+# (3 components x (2 bilinear lerps of 3 + final lerp and 1/h of 4)); det = 17; cofactor+det = 35; curl = 3.
+# Barrier-active points add a few hundred more (not counted).
 FLOP_PER_CELL = {
-    # edges 108 + reference sweep (45 columns + 27 x (det + curl)) 1890 + Gauss sweep2 (126 columns) 3780
-    # + 27 x (2 det + 2 curl + 4 stable changes + trial energy) 4833 + the trial's closed sweep (45 columns) 1350
-    # + 27 x det 459 (the base's closed sweep runs only in cells near the activation: not counted)
-    "cell_trial_kernel": 12420,
-    "cell_diff_kernel": 15006,
-    # edges 72 + ref sweep 1890 + Gauss sweep (45 columns) 1350 + 27 x 31 + closed sweep 1350 + 27 x det 459
-    "cell_energy_kernel": 5958,
+    # three fields x 732 + two residuals (subtract 27, transform 162, sums 100) + the curl sums 130
+    "cell_trial_kernel": 2904,
+    "cell_diff_kernel": 2850,
+    # two fields x 732 + one residual 289 + the curl sum 54
+    "cell_energy_kernel": 1807,
     # edges 72 + soft sweep2 3780 + 27 x 94 (cofactor, det, curls, fluxes) + adjoint scatter 693
     # + barrier sweep 1350 + 27 x det 459
     "cell_grad_kernel": 8892,
@@ -229,7 +229,7 @@ def kernel_counts(shape):
 STATE_DEPENDENT_KERNELS = ("prescreen_kernel", "fallback_grid_kernel", "classify_kernel", "jd_extension_kernel",
                            "jd_root_kernel", "cell_ggn_hvp_kernel", "cell_trial_barrier_kernel",
                            "cell_grad_barrier32_kernel", "cell_ggn_barrier32_kernel", "cell_grad_barrier_kernel",
-                           "cell_ggn_barrier_kernel", "cell_trial_diff_kernel")
+                           "cell_ggn_barrier_kernel", "cell_barrier_kernel")
 
 
 class Ranks:

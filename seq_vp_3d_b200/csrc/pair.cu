@@ -144,10 +144,6 @@ Q1Const make_const(const svp_grid *g, const svp_weights *w) {
     q.omega = (g->hx * g->hy) * g->hz;
     for (int p = 0; p < 27; p++) q.gw[p] = ((q.omega * w1[p % 3]) * w1[(p / 3) % 3]) * w1[p / 9];
     q.lam = w->lam; q.mu = w->mu; q.nu = w->nu;
-    for (int p = 0; p < 27; p++) {       // IEEE square roots: the values the device's sqrt gives
-        q.sqmu[p] = std::sqrt(q.mu * q.gw[p]);
-        q.sqnu[p] = std::sqrt(q.nu * q.gw[p]);
-    }
     for (int k = 0; k < 3; k++) {
         q.gnf[k] = (float)q.gn[k];
         q.gmf[k] = (float)q.gm[k];

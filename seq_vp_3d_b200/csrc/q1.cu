@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "pair.cuh"
+#include "q1_closed.cuh"
 
 namespace svp {
 namespace {
@@ -243,63 +244,108 @@ __device__ __forceinline__ void scatter_slice(const R *sl, int T, const C n[3], 
         }
 }
 
-// ============================================================================================== cell energy
-// Reference J and curl at the Gauss points of one cell into the thread's shared slice (4 values per point).
-__device__ __forceinline__ void reference_points(const double *__restrict__ uref, long long n0, const Q1Const &q,
-                                                 double *sl, int T) {
-    double Er[3][4][3];
-    load_edges(uref, n0, q, Er);
-    sweep<false>(Er, q, [&](int p, int, int, int, const double (&Vr)[3][3]) {
-        double Cr[3];
-        curl_of(Vr, Cr);
-        sl[(4 * p) * T] = det_only(Vr);
-        sl[(4 * p + 1) * T] = Cr[0];
-        sl[(4 * p + 2) * T] = Cr[1];
-        sl[(4 * p + 3) * T] = Cr[2];
-    });
-}
-
-// partial[block][0..2] = sum w (J - Jr)^2, sum w |C - Cr|^2, sum barrier; violations counted in *bad
-__global__ void __launch_bounds__(CS) cell_energy_kernel(Q1Const q, const double *__restrict__ u,
-                                                         const double *__restrict__ uref, dd *partial,
-                                                         unsigned long long *bad) {
+// ============================================================================================== cell energies
+// The JD and curl penalties of a state against u_ref (ENERGY) and their stable changes from a base (DIFF), one cell
+// per thread on its closed27 J (q1_closed.cuh): per cell sum w (J - Jr)^2 and sum w |C - Cr|^2, and the changes
+// d (2 r - d) in Legendre and Hadamard coefficients (r the state's residual, d the change from the base; the
+// difference of the squares without cancelling them).  Block sums in double-double; a cell's values do not depend on
+// which of the two parts is compiled in.
+//
+// Bound: FP64 issue.  About 2,000 FP64 instructions per cell with both parts (J of three fields at 27 points each 11
+// operations, edges and averages 162, two Legendre transforms 108); the Gauss27 form took 6,200.  The 27 J - 1, the
+// curl coefficients and the residual coefficients wait in the thread's shared slice (90 doubles: one access costs as
+// much as four FP64 instructions, so tables that are used at once stay in registers).  Trial on 256^3: 11.20 -> 3.04
+// ms per launch, FP64 pipe 64% busy; two warps per scheduler (255 registers) leave its dependency stalls.  Three warps
+// (168 registers, 800 bytes of spills) took 5.0 ms, loads of the next field before this field's points 3.36 ms.
+//
+// flags[c]: bit 0, some closed27 J of the state is not above the activation; bit 1, some of the base is not.
+// cell_barrier_kernel evaluates the barrier of those cells; elsewhere it and its change are zero.
+constexpr int kEnergySlots = 45, kDiffSlots = 90;
+template <bool ENERGY, bool DIFF>
+__global__ void __launch_bounds__(CS) cell_soft_kernel(Q1Const q, const double *__restrict__ ua,
+                                                       const double *__restrict__ ub,
+                                                       const double *__restrict__ uref, dd *pe, dd *pd,
+                                                       uint8_t *__restrict__ flags,
+                                                       uint8_t *__restrict__ trial_act) {
     extern __shared__ double smem[];
-    double *sl = smem + threadIdx.x;
+    double *sJ = smem + threadIdx.x;
     const int T = blockDim.x;
-    dd acc[3] = {{0., 0.}, {0., 0.}, {0., 0.}};
-    unsigned long long nbad = 0;
+    double *sC = sJ + 27 * T, *sR = sJ + 45 * T, *sX = sJ + 72 * T;
+    dd acc[2] = {{0., 0.}, {0., 0.}}, dif[2] = {{0., 0.}, {0., 0.}};
+    const double wj = .5 * q.mu * q.omega, wc = .5 * q.nu * q.omega, low = near_bound(q.act);
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
          c += (long long)gridDim.x * blockDim.x) {
-        long long n0 = cell_node0(c, q);
-        reference_points(uref, n0, q, sl, T);
-        double E[3][4][3];
-        load_edges(u, n0, q, E);
-        double sj = 0., sc = 0., sb = 0.;
-        sweep<false>(E, q, [&](int p, int, int, int, const double (&V)[3][3]) {
-            double C[3];
-            curl_of(V, C);
-            double dj = det_only(V) - sl[(4 * p) * T];
-            double c0 = C[0] - sl[(4 * p + 1) * T], c1 = C[1] - sl[(4 * p + 2) * T], c2 = C[2] - sl[(4 * p + 3) * T];
-            const double w = q.gw[p];
-            sj += w * dj * dj;
-            sc += w * (c0 * c0 + c1 * c1 + c2 * c2);
-        });
-        sweep<true>(E, q, [&](int, int, int, int, const double (&V)[3][3]) {
-            double J = det_only(V);
-            if (!(J > q.delta)) { nbad++; return; }
-            if (J < q.act) {
-                double b, b1, b2;
-                barrier_eval(J, q.act, q.delta, q.bw, b, b1, b2);
-                sb += b;
-            }
-        });
-        acc[0] = dd_add_d(acc[0], sj);
-        acc[1] = dd_add_d(acc[1], sc);
-        acc[2] = dd_add_d(acc[2], sb);
+        const long long n0 = cell_node0(c, q);
+        Columns C;
+        {
+            load_columns(uref, n0, q, C);
+            double k[18];
+            curl_coefficients(C, k);
+#pragma unroll
+            for (int i = 0; i < 18; i++) sC[i * T] = k[i];
+            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                 const double (&Z)[3]) { sJ[p * T] = det_minus_one(X, Y, Z); });
+        }
+        unsigned char flag = 0;
+        {
+            load_columns(ub, n0, q, C);
+            double k[18], r[27];
+            curl_coefficients(C, k);
+            const double s = curl_sum([&](int i, double &a) {
+                const double x = __dsub_rn(k[i], sC[i * T]);
+                a = __fma_rn(x, x, a);
+                if (DIFF) {
+                    sC[i * T] = k[i];
+                    sX[i * T] = x;
+                }
+            });
+            if (ENERGY) acc[1] = dd_add_d(acc[1], __dmul_rn(q.omega, s));
+            bool near = false;
+            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                 const double (&Z)[3]) {
+                const double J = det_minus_one(X, Y, Z);
+                near |= !(J >= low);
+                r[p] = __dsub_rn(J, sJ[p * T]);
+                if (DIFF) sJ[p * T] = J;
+            });
+            if (near) flag = 1;
+            legendre27(r);
+            if (ENERGY)
+                acc[0] = dd_add_d(acc[0], __dmul_rn(q.omega, legendre_sum([&](int i, double &a) {
+                                                        a = __fma_rn(r[i], r[i], a);
+                                                    })));
+            if (DIFF)
+#pragma unroll
+                for (int i = 0; i < 27; i++) sR[i * T] = r[i];
+        }
+        if (DIFF) {
+            load_columns(ua, n0, q, C);
+            double k[18], d[27];
+            curl_coefficients(C, k);
+            const double s = curl_sum([&](int i, double &a) {
+                const double x = __dsub_rn(sC[i * T], k[i]);
+                a = __fma_rn(x, __fma_rn(2., sX[i * T], -x), a);
+            });
+            dif[1] = dd_add_d(dif[1], __dmul_rn(wc, s));
+            bool near = false;
+            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                 const double (&Z)[3]) {
+                const double J = det_minus_one(X, Y, Z);
+                near |= !(J >= low);
+                d[p] = __dsub_rn(sJ[p * T], J);
+            });
+            if (near) flag |= 2;
+            legendre27(d);
+            dif[0] = dd_add_d(dif[0], __dmul_rn(wj, legendre_sum([&](int i, double &a) {
+                                                    a = __fma_rn(d[i], __fma_rn(2., sR[i * T], -d[i]), a);
+                                                })));
+        }
+        flags[c] = flag;
+        if (trial_act) trial_act[c] = 0;
     }
-    block_reduce_dd<3>(acc, partial);
-    for (int o = 16; o; o >>= 1) nbad += __shfl_xor_sync(0xFFFFFFFFu, nbad, o);
-    if ((threadIdx.x & 31) == 0 && nbad) atomicAdd(bad, nbad);
+    if (ENERGY) block_reduce_dd<2>(acc, pe);
+    if (ENERGY && DIFF) __syncthreads();     // the two reductions share block_reduce_dd's shared array
+    if (DIFF) block_reduce_dd<2>(dif, pd);
 }
 
 // Per-cell vertex values -> SoA locals L[(a * 3 + r) * ncell + c].
@@ -933,67 +979,18 @@ __global__ void __launch_bounds__(256) node_diff_kernel(Q1Const q, const double 
     block_reduce_dd<2>(acc, partial);
 }
 
-// Reference J and curl at the Gauss points go to the thread's shared slice first (108 values), so only the two
-// compared fields' edges are live in registers during the main pass.  Per-point changes are exact products
-// (sq_change) summed with a compensated (hi, lo) accumulator.
+// compensated (hi, lo) accumulation of t
 __device__ __forceinline__ void acc_add(dd &acc, dd t) {
     dd s = two_sum(acc.hi, t.hi);
     acc.hi = s.hi;
     acc.lo += s.lo + t.lo;
 }
-__global__ void __launch_bounds__(CS) cell_diff_kernel(Q1Const q, const double *__restrict__ ua,
-                                                       const double *__restrict__ ub,
-                                                       const double *__restrict__ uref, dd *partial,
-                                                       const uint8_t *__restrict__ act_a,
-                                                       const uint8_t *__restrict__ act_b,
-                                                       uint8_t *__restrict__ flags) {
-    extern __shared__ double smem[];
-    double *sl = smem + threadIdx.x;
-    const int T = blockDim.x;
-    dd acc[3] = {{0., 0.}, {0., 0.}, {0., 0.}};
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
-         c += (long long)gridDim.x * blockDim.x) {
-        long long n0 = cell_node0(c, q);
-        reference_points(uref, n0, q, sl, T);
-        double Ea[3][4][3], Eb[3][4][3];
-        load_edges(ua, n0, q, Ea);
-        load_edges(ub, n0, q, Eb);
-        sweep2<false>(Ea, Eb, q, [&](int p, int, int, int, const double (&Va)[3][3], const double (&Vb)[3][3]) {
-            double Ca[3], Cb[3];
-            const double jr = sl[(4 * p) * T];
-            const double smu = q.sqmu[p], snu = q.sqnu[p];
-            acc_add(acc[0], sq_change(smu * (det_only(Va) - jr), smu * (det_only(Vb) - jr)));
-            curl_of(Va, Ca);
-            curl_of(Vb, Cb);
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const double cr = sl[(4 * p + 1 + r) * T];
-                acc_add(acc[1], sq_change(snu * (Ca[r] - cr), snu * (Cb[r] - cr)));
-            }
-        });
-        double sb = 0.;
-        // with both masks, a cell inactive in both fields has no barrier difference at all; with flags, the cells
-        // that have one are handed to cell_trial_diff_kernel (the same per-cell value)
-        const bool needs = !(act_a && act_b && !act_a[c] && !act_b[c]);
-        if (flags)
-            flags[c] = needs ? 1 : 0;
-        else if (needs)
-            sweep2<true>(Ea, Eb, q, [&](int, int, int, int, const double (&Va)[3][3], const double (&Vb)[3][3]) {
-                double ja = det_only(Va), jb = det_only(Vb);
-                if (ja < q.act || jb < q.act) sb += barrier_difference(ja, jb, q.act, q.delta);
-            });
-        acc_add(acc[2], dd{q.bw * sb, 0.});
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++) acc[k] = two_sum(acc[k].hi, acc[k].lo);
-    block_reduce_dd<3>(acc, partial);
-}
 
 // ============================================================================================== line-search trial
-// A trial evaluated against its base in one node pass and one cell pass: the trial's warped image (and image
-// gradient), its energy sums exactly as node_energy_kernel / cell_energy_kernel form them, and the stable base ->
-// trial changes exactly as node_diff_kernel / cell_diff_kernel form them (same grids, same per-thread order, so the
-// results are bitwise those of the separate passes).
+// A trial evaluated against its base in one node pass and one cell pass (cell_soft_kernel, cell_barrier_kernel): the
+// trial's warped image (and image gradient), its energy sums exactly as node_energy_kernel and the energy-only cell
+// kernels form them, and the stable base -> trial changes exactly as node_diff_kernel and the difference-only cell
+// kernels form them (same grids, same per-thread order, so the results are bitwise those of the separate passes).
 template <bool GRAD>
 __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S, const double *__restrict__ ua,
                                                          const double *__restrict__ wa,
@@ -1036,117 +1033,67 @@ __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S,
     block_reduce_dd<2>(dif, pd);
 }
 
-// Barrier activity mask: act[c] = 1 when some closed27 J of cell c is below the activation; trial_act (optional)
-// receives the trial's mask, which later calls on that state use to skip barrier sweeps that contribute nothing.
-//
-// The closed27 part runs the trial's sweep alone first (its J values parked in the thread's slice, whose reference
-// values are dead after the Gauss sweep); the base's sweep and the barrier differences follow only where some point
-// of either state is below the activation: the trial's (just found) or the base's (base_act, its mask from its own
-// evaluation; NULL: unknown, always sweep).  Elsewhere every difference term is zero.  Same values in the same
-// order per accumulator as one two-field sweep.
-__global__ void __launch_bounds__(CS) cell_trial_kernel(Q1Const q, const double *__restrict__ ua,
-                                                        const double *__restrict__ ub,
-                                                        const double *__restrict__ uref, dd *pe, dd *pd,
-                                                        unsigned long long *bad, uint8_t *__restrict__ trial_act,
-                                                        const uint8_t *__restrict__ base_act,
-                                                        uint8_t *__restrict__ flags) {
-    extern __shared__ double smem[];
-    double *sl = smem + threadIdx.x;
-    const int T = blockDim.x;
-    dd acc[3] = {{0., 0.}, {0., 0.}, {0., 0.}}, dif[3] = {{0., 0.}, {0., 0.}, {0., 0.}};
-    unsigned long long nbad = 0;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
-         c += (long long)gridDim.x * blockDim.x) {
-        long long n0 = cell_node0(c, q);
-        reference_points(uref, n0, q, sl, T);
-        double Ea[3][4][3], Eb[3][4][3];
-        load_edges(ua, n0, q, Ea);
-        load_edges(ub, n0, q, Eb);
-        double sj = 0., sc = 0., sb = 0., sbd = 0.;
-        sweep2<false>(Ea, Eb, q, [&](int p, int, int, int, const double (&Va)[3][3], const double (&Vb)[3][3]) {
-            double Ca[3], Cb[3];
-            const double jr = sl[(4 * p) * T];
-            const double smu = q.sqmu[p], snu = q.sqnu[p];
-            const double jb = det_only(Vb);
-            acc_add(dif[0], sq_change(smu * (det_only(Va) - jr), smu * (jb - jr)));
-            curl_of(Va, Ca);
-            curl_of(Vb, Cb);
-            double cd[3];
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const double cr = sl[(4 * p + 1 + r) * T];
-                cd[r] = Cb[r] - cr;
-                acc_add(dif[1], sq_change(snu * (Ca[r] - cr), snu * cd[r]));
-            }
-            const double w = q.gw[p], dj = jb - jr;
-            sj += w * dj * dj;
-            sc += w * (cd[0] * cd[0] + cd[1] * cd[1] + cd[2] * cd[2]);
-        });
-        bool active = false;
-        sweep<true>(Eb, q, [&](int p, int, int, int, const double (&Vb)[3][3]) {
-            const double jb = det_only(Vb);
-            sl[p * T] = jb;
-            active |= jb < q.act;
-            if (!(jb > q.delta)) { nbad++; return; }
-            if (jb < q.act) {
-                double b, b1, b2;
-                barrier_eval(jb, q.act, q.delta, q.bw, b, b1, b2);
-                sb += b;
-            }
-        });
-        // the barrier differences of the cells where the trial or the base is active: here, or (flags) in
-        // cell_trial_diff_kernel over those cells alone
-        const bool needs = active || !base_act || base_act[c];
-        if (flags) {
-            flags[c] = needs ? 1 : 0;
-        } else if (needs) {
-            load_edges(ua, n0, q, Ea);
-            sweep<true>(Ea, q, [&](int p, int, int, int, const double (&Va)[3][3]) {
-                const double ja = det_only(Va), jb = sl[p * T];
-                if (ja < q.act || jb < q.act) sbd += barrier_difference(ja, jb, q.act, q.delta);
-            });
-        }
-        if (trial_act) trial_act[c] = active ? 1 : 0;
-        acc[0] = dd_add_d(acc[0], sj);
-        acc[1] = dd_add_d(acc[1], sc);
-        acc[2] = dd_add_d(acc[2], sb);
-        acc_add(dif[2], dd{q.bw * sbd, 0.});
-    }
-#pragma unroll
-    for (int k = 0; k < 3; k++) dif[k] = two_sum(dif[k].hi, dif[k].lo);
-    block_reduce_dd<3>(acc, pe);
-    __syncthreads();     // the two reductions share block_reduce_dd's shared array
-    block_reduce_dd<3>(dif, pd);
-    for (int o = 16; o; o >>= 1) nbad += __shfl_xor_sync(0xFFFFFFFFu, nbad, o);
-    if ((threadIdx.x & 31) == 0 && nbad) atomicAdd(bad, nbad);
-}
-
-// The float64 trial's barrier differences of the flagged cells (trial or base active), as cell_trial_kernel forms
-// them per cell: the trial's closed27 J from its edges, the base's, psi differences where either is below the
-// activation.  pd: per block, the barrier difference sum.
-__global__ void __launch_bounds__(CB) cell_trial_diff_kernel(Q1Const q, const double *__restrict__ ua,
-                                                             const double *__restrict__ ub,
-                                                             const uint8_t *__restrict__ flags, dd *pd) {
+// The barrier of the flagged cells (cell_soft_kernel's flags): the state's barrier sum, violations (J <= delta) and
+// activity mask (trial_act[c] = 1 when some closed27 J is below the activation), and with DIFF its stable change from
+// the base; the J are those of cell_soft_kernel.  Rolled loops over the 27 points keep the logarithms' code and
+// registers out of the soft kernel, and the queue hands them to full warps.
+template <bool ENERGY, bool DIFF>
+__global__ void __launch_bounds__(CB) cell_barrier_kernel(Q1Const q, const double *__restrict__ ua,
+                                                          const double *__restrict__ ub,
+                                                          const uint8_t *__restrict__ flags, dd *pe, dd *pd,
+                                                          unsigned long long *bad,
+                                                          uint8_t *__restrict__ trial_act) {
     extern __shared__ double smem[];
     __shared__ long long queue[CB / 32][64];
-    double *dsl = smem + threadIdx.x;
+    double *sb = smem + threadIdx.x;
     const int T = blockDim.x;
-    dd dif[1] = {{0., 0.}};
+    double *sa = sb + 27 * T;
+    dd acc[1] = {{0., 0.}}, dif[1] = {{0., 0.}};
+    unsigned long long nbad = 0;
     for_flagged_cells(q, flags, queue[threadIdx.x >> 5], [&](long long c, uint8_t) {
         const long long n0 = cell_node0(c, q);
-        double E[3][4][3];
-        load_edges(ub, n0, q, E);
-        sweep<true>(E, q, [&](int p, int, int, int, const double (&Vb)[3][3]) { dsl[p * T] = det_only(Vb); });
-        load_edges(ua, n0, q, E);
-        double sbd = 0.;
-        sweep<true>(E, q, [&](int p, int, int, int, const double (&Va)[3][3]) {
-            const double ja = det_only(Va), jb = dsl[p * T];
-            if (ja < q.act || jb < q.act) sbd += barrier_difference(ja, jb, q.act, q.delta);
+        Columns C;
+        load_columns(ub, n0, q, C);
+        closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
+            sb[p * T] = jacobian(det_minus_one(X, Y, Z));
         });
-        acc_add(dif[0], dd{q.bw * sbd, 0.});
+        if (ENERGY) {
+            double sum = 0.;
+            bool active = false;
+#pragma unroll 1
+            for (int p = 0; p < 27; p++) {
+                const double j = sb[p * T];
+                active |= j < q.act;
+                if (!(j > q.delta)) { nbad++; continue; }
+                if (j < q.act) {
+                    double b, b1, b2;
+                    barrier_eval(j, q.act, q.delta, q.bw, b, b1, b2);
+                    sum += b;
+                }
+            }
+            if (trial_act && active) trial_act[c] = 1;
+            acc[0] = dd_add_d(acc[0], sum);
+        }
+        if (DIFF) {
+            load_columns(ua, n0, q, C);
+            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                 const double (&Z)[3]) { sa[p * T] = jacobian(det_minus_one(X, Y, Z)); });
+            double sum = 0.;
+#pragma unroll 1
+            for (int p = 0; p < 27; p++) {
+                const double ja = sa[p * T], jb = sb[p * T];
+                if (ja < q.act || jb < q.act) sum += barrier_difference(ja, jb, q.act, q.delta);
+            }
+            dif[0] = dd_add_d(dif[0], __dmul_rn(q.bw, sum));
+        }
     });
-    dif[0] = two_sum(dif[0].hi, dif[0].lo);
-    block_reduce_dd<1>(dif, pd);
+    if (ENERGY) block_reduce_dd<1>(acc, pe);
+    if (ENERGY && DIFF) __syncthreads();     // the two reductions share block_reduce_dd's shared array
+    if (DIFF) block_reduce_dd<1>(dif, pd);
+    if (ENERGY) {
+        for (int o = 16; o; o >>= 1) nbad += __shfl_xor_sync(0xFFFFFFFFu, nbad, o);
+        if ((threadIdx.x & 31) == 0 && nbad) atomicAdd(bad, nbad);
+    }
 }
 
 // ============================================================================================== screened trial
@@ -1817,7 +1764,7 @@ unsigned slice_blocks(const svp_pair *p) { return blocks_for(p->q.ncell, CS, 2 *
 // dynamic shared memory of the slice kernels: k doubles per thread
 constexpr size_t slice_bytes(int k) { return sizeof(double) * (size_t)k * CS; }
 int allow_slices() {
-    // the 108-value slices are above the 48 KB default.  The attribute belongs to the device's context (the primary
+    // large slices are above the 48 KB default.  The attribute belongs to the device's context (the primary
     // context torch and this library share), so it is set on the first call per device, not on every launch: a
     // cudaFuncSetAttribute costs host time that the GPU then spends idle.
     static std::mutex mu;
@@ -1827,12 +1774,14 @@ int allow_slices() {
     SVP_REQUIRE(dev >= 0 && dev < 64, "allow_slices: device ordinal out of range");
     std::lock_guard<std::mutex> lock(mu);
     if (done[dev]) return SVP_OK;
-    SVP_CUDA(cudaFuncSetAttribute(cell_diff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)slice_bytes(108)));
-    SVP_CUDA(cudaFuncSetAttribute(cell_energy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)slice_bytes(108)));
-    SVP_CUDA(cudaFuncSetAttribute(cell_trial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)slice_bytes(108)));
+    SVP_CUDA(cudaFuncSetAttribute(cell_soft_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)slice_bytes(kDiffSlots)));
+    SVP_CUDA(cudaFuncSetAttribute(cell_soft_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)slice_bytes(kDiffSlots)));
+    SVP_CUDA(cudaFuncSetAttribute(cell_barrier_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(sizeof(double) * 54 * CB)));
+    SVP_CUDA(cudaFuncSetAttribute(cell_barrier_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)(sizeof(double) * 54 * CB)));
     SVP_CUDA(cudaFuncSetAttribute(cell_grad_barrier_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(sizeof(double) * 81 * CB)));
     done[dev] = true;
@@ -1904,19 +1853,30 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
                           int64_t *barrier_violations, void *stream) {
     SVP_REQUIRE(p && u && warped && terms5, "svp_energy: null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p);
-    int rc = pair_partials(p, (long long)nb * 2 + (long long)cb * 3, 1);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = barrier_blocks(p->q);
+    int rc = pair_partials(p, (long long)nb * 2 + (long long)cb * 2 + bb, 1);
     if (rc) return rc;
     if ((rc = allow_slices())) return rc;
+    if ((rc = pair_flags(p))) return rc;
     SVP_CUDA(cudaMemsetAsync(p->counter, 0, sizeof(long long) * 8, s));
     { svp::KernelTimer _t("node_energy_kernel", s); SVP_LAUNCH(node_energy_kernel<<<nb, 256, 0, s>>>(p->q, u, warped, p->fixed, p->u_ref, p->partial)); }
     SVP_LAUNCH_CHECK("node_energy_kernel");
-    dd *pc = p->partial + (long long)nb * 2;
-    { svp::KernelTimer _t("cell_energy_kernel", s); SVP_LAUNCH(cell_energy_kernel<<<cb, CS, slice_bytes(108), s>>>(p->q, u, p->u_ref, pc, (unsigned long long *)p->counter)); }
+    dd *pc = p->partial + (long long)nb * 2, *pb = pc + (long long)cb * 2;
+    {
+        svp::KernelTimer _t("cell_energy_kernel", s);
+        SVP_LAUNCH(cell_soft_kernel<true, false><<<cb, CS, slice_bytes(kEnergySlots), s>>>(
+            p->q, nullptr, u, p->u_ref, pc, nullptr, p->flags, nullptr));
+    }
+    {
+        svp::KernelTimer _t("cell_barrier_kernel", s);
+        SVP_LAUNCH(cell_barrier_kernel<true, false><<<bb, CB, sizeof(double) * 27 * CB, s>>>(
+            p->q, nullptr, u, p->flags, pb, nullptr, (unsigned long long *)p->counter, nullptr));
+    }
     SVP_LAUNCH_CHECK("cell_energy_kernel");
     double node2[2], cell3[3];
     SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(p->partial, nb, 2, p->result));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pc, cb, 3, p->result + 4));
+    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pc, cb, 2, p->result + 4));
+    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pb, bb, 1, p->result + 8));
     SVP_LAUNCH_CHECK("final_reduce_kernel");
     double tmp[10];
     long long bad = 0;
@@ -1940,32 +1900,31 @@ extern "C" int svp_energy_difference_masked(svp_pair *p, const double *base_u, c
                                             void *stream) {
     SVP_REQUIRE(p && base_u && base_warped && trial_u && trial_warped && diff2, "svp_energy_difference: null");
     cudaStream_t s = (cudaStream_t)stream;
+    // the cell kernels find the cells near the activation from the J they evaluate, so the masks save nothing here
+    (void)base_active;
+    (void)trial_active;
     unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = barrier_blocks(p->q);
-    int rc = pair_partials(p, (long long)nb * 2 + (long long)cb * 3 + bb, 1);
+    int rc = pair_partials(p, (long long)nb * 2 + (long long)cb * 2 + bb, 1);
     if (rc) return rc;
-    rc = allow_slices();
-    if (rc) return rc;
-    // with both states' masks, the barrier differences of the cells active in either run in cell_trial_diff_kernel
-    // over those cells alone (per cell the same value)
-    const bool apart = base_active && trial_active;
-    if (apart && (rc = pair_flags(p))) return rc;
+    if ((rc = allow_slices())) return rc;
+    if ((rc = pair_flags(p))) return rc;
     { svp::KernelTimer _t("node_diff_kernel", s); SVP_LAUNCH(node_diff_kernel<<<nb, 256, 0, s>>>(p->q, base_u, base_warped, trial_u, trial_warped, p->fixed, p->u_ref,
                                         p->partial)); }
-    dd *pc = p->partial + (long long)nb * 2, *pb = pc + (long long)cb * 3;
+    dd *pc = p->partial + (long long)nb * 2, *pb = pc + (long long)cb * 2;
     {
         svp::KernelTimer _t("cell_diff_kernel", s);
-        SVP_LAUNCH(cell_diff_kernel<<<cb, CS, slice_bytes(108), s>>>(p->q, base_u, trial_u, p->u_ref, pc, base_active,
-                                                                    trial_active, apart ? p->flags : nullptr));
+        SVP_LAUNCH(cell_soft_kernel<false, true><<<cb, CS, slice_bytes(kDiffSlots), s>>>(
+            p->q, base_u, trial_u, p->u_ref, nullptr, pc, p->flags, nullptr));
     }
-    if (apart) {
-        svp::KernelTimer _t("cell_trial_diff_kernel", s);
-        SVP_LAUNCH(cell_trial_diff_kernel<<<bb, CB, sizeof(double) * 27 * CB, s>>>(p->q, base_u, trial_u, p->flags,
-                                                                                 pb));
+    {
+        svp::KernelTimer _t("cell_barrier_kernel", s);
+        SVP_LAUNCH(cell_barrier_kernel<false, true><<<bb, CB, sizeof(double) * 54 * CB, s>>>(
+            p->q, base_u, trial_u, p->flags, nullptr, pb, nullptr, nullptr));
     }
     SVP_LAUNCH_CHECK("difference kernels");
     SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(p->partial, nb, 2, p->result));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pc, cb, 3, p->result + 4));
-    if (apart) SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pb, bb, 1, p->result + 8));
+    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pc, cb, 2, p->result + 4));
+    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pb, bb, 1, p->result + 8));
     SVP_LAUNCH_CHECK("final_reduce_kernel");
     double tmp[10];
     SVP_CUDA(cudaMemcpyAsync(tmp, p->result, sizeof tmp, cudaMemcpyDeviceToHost, s));
@@ -2065,7 +2024,7 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
     int rc = pair_partials(p, (long long)nb * 4 + (long long)cb * 10 + (long long)bb * 2, 1);
     if (rc) return rc;
     if ((rc = allow_slices())) return rc;
-    if (screened && (rc = pair_flags(p))) return rc;
+    if ((rc = pair_flags(p))) return rc;
     SVP_CUDA(cudaMemsetAsync(p->counter, 0, sizeof(long long) * 8, s));
     dd *pne = p->partial, *pnd = pne + (long long)nb * 2, *pce = pnd + (long long)nb * 2, *pcd = pce + (long long)cb * 3;
     dd *pcb = pcd + (long long)cb * 3, *pbe = pcb + (long long)cb * 4, *pbd = pbe + bb;
@@ -2090,38 +2049,24 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
         SVP_LAUNCH(cell_trial_barrier_kernel<<<bb, CB, sizeof(double) * 27 * CB, s>>>(
             p->q, base_u, trial_u, p->flags, pbe, pbd, (unsigned long long *)p->counter, trial_active, base_active));
     } else {
-        // with the base's mask, the barrier differences of the cells where the trial or the base is active run in
-        // cell_trial_diff_kernel over those cells alone (per cell the fused kernel's values)
-        const bool apart = base_active != nullptr;
-        if (apart && (rc = pair_flags(p))) return rc;
         {
             svp::KernelTimer _t("cell_trial_kernel", s);
-            SVP_LAUNCH(cell_trial_kernel<<<cb, CS, slice_bytes(108), s>>>(
-                p->q, base_u, trial_u, p->u_ref, pce, pcd, (unsigned long long *)p->counter, trial_active,
-                base_active, apart ? p->flags : nullptr));
+            SVP_LAUNCH(cell_soft_kernel<true, true><<<cb, CS, slice_bytes(kDiffSlots), s>>>(
+                p->q, base_u, trial_u, p->u_ref, pce, pcd, p->flags, trial_active));
         }
-        if (apart) {
-            svp::KernelTimer _t("cell_trial_diff_kernel", s);
-            SVP_LAUNCH(cell_trial_diff_kernel<<<bb, CB, sizeof(double) * 27 * CB, s>>>(p->q, base_u, trial_u,
-                                                                                     p->flags, pbd));
-        }
+        svp::KernelTimer _t("cell_barrier_kernel", s);
+        SVP_LAUNCH(cell_barrier_kernel<true, true><<<bb, CB, sizeof(double) * 54 * CB, s>>>(
+            p->q, base_u, trial_u, p->flags, pbe, pbd, (unsigned long long *)p->counter, trial_active));
     }
     SVP_LAUNCH_CHECK("cell_trial_kernel");
     SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pne, nb, 2, p->result));
     SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pnd, nb, 2, p->result + 10));
-    if (screened) {
-        // soft sums and differences from the float32 kernel, the barrier's from the float64 barrier kernel
-        SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pce, cb, 2, p->result + 4));
-        SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pbe, bb, 1, p->result + 8));
-        SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pcd, cb, 2, p->result + 14));
-        SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pbd, bb, 1, p->result + 18));
-        SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pcb, cb, 4, p->result + 20));
-    } else {
-        SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pce, cb, 3, p->result + 4));
-        SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pcd, cb, 3, p->result + 14));
-        // the barrier difference from its own kernel in place of the fused kernel's (zero) one
-        if (base_active) SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pbd, bb, 1, p->result + 18));
-    }
+    // soft sums and differences from the soft kernel, the barrier's from the barrier kernel
+    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pce, cb, 2, p->result + 4));
+    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pbe, bb, 1, p->result + 8));
+    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pcd, cb, 2, p->result + 14));
+    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pbd, bb, 1, p->result + 18));
+    if (screened) SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pcb, cb, 4, p->result + 20));
     SVP_LAUNCH_CHECK("final_reduce_kernel");
     double tmp[28];
     long long bad = 0;

@@ -12,7 +12,6 @@ struct Q1Const {
     double h[3], ih[3];            // spacing and fl(1/h) (cell_q1.py:126 divides +-1 by h)
     double gn[3], gm[3];           // Gauss nodes xi and 1 - xi (cell_q1.py:106)
     double gw[27];                 // Gauss27 weights omega*wx*wy*wz, p = 9 iz + 3 iy + ix (cell_q1.py:115)
-    double sqmu[27], sqnu[27];     // sqrt(mu gw[p]), sqrt(nu gw[p]) (stable differences of the Gauss terms)
     double omega;
     double lam, mu, nu, bw;        // weights; bw = kappa omega / 27 (problem.py:310)
     double act, delta;             // localized barrier activation a and delta
