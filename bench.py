@@ -153,9 +153,9 @@ FLOP_PER_CELL = {
     "cell_diff_kernel": 2850,
     # two fields x 732 + one residual 289 + the curl sum 54
     "cell_energy_kernel": 1807,
-    # edges 72 + soft sweep2 3780 + 27 x 94 (cofactor, det, curls, fluxes) + adjoint scatter 693
-    # + barrier sweep 1350 + 27 x det 459
-    "cell_grad_kernel": 8892,
+    # two fields x 732 + residuals 27 + mass matrices 270 + adjoint pass 27 x (6 + 36) + its averages 120 + scatter 108
+    # + curl adjoint 90
+    "cell_grad_kernel": 3213,
     # edges 36 + Gauss sweep 1350 + 27 x (cofactor 35 + 8 vertices x 30) + closed sweep 1350 + 27 x det 459
     # + the state-independent curl term 24
     "cell_ggn_diag_kernel": 10644,

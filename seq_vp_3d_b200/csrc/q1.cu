@@ -357,84 +357,182 @@ __device__ __forceinline__ void store_locals(R *__restrict__ L, long long c, lon
         for (int r = 0; r < 3; r++) L[(long long)(a * 3 + r) * ncell + c] = v[a][r];
 }
 
+// ============================================================================================== flagged cells
+// The plain form's barrier kernels: a block scans the flags of its cells (kScan groups of blockDim cells at a time,
+// groups dealt out over the grid), queues the flagged ones in cell order and hands up to blockDim of them to
+// body(n, queue).  Inside, the J of a cell belong to one thread and the n x 27 points are spread over the block: a
+// barrier point is a long dependency chain (a logarithm and a division), so a thread that walks the 27 points of
+// its cell leaves the SM idle (the trial's barrier on 48^3, 3.4% of its cells flagged: 37 us, spread 16 us; on 256^3
+// 606 -> 496 us).  The assignment is the same on every run, so the threads' sums are deterministic.
+constexpr int BT = 128;               // threads per block of these kernels
+constexpr int kScan = 4;
+template <class Body>
+__device__ __forceinline__ void for_flagged_blocks(const Q1Const &q, const uint8_t *__restrict__ flags,
+                                                   long long *queue, Body &&body) {
+    __shared__ int counts[kScan][BT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ngroup = (int)((q.ncell + BT - 1) / BT);
+    int n = 0;                         // queued cells, the same in every thread
+    for (int k = blockIdx.x; k < ngroup || n > 0;) {
+        while (n < BT && k < ngroup) {
+            unsigned m[kScan];
+#pragma unroll
+            for (int j = 0; j < kScan; j++) {
+                const long long c = (long long)(k + j * (int)gridDim.x) * BT + threadIdx.x;
+                m[j] = __ballot_sync(0xFFFFFFFFu, c < q.ncell && flags[c] != 0);
+                if (lane == 0) counts[j][warp] = __popc(m[j]);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < kScan; j++) {
+                int at = n;
+                for (int w = 0; w < BT / 32; w++) {
+                    if (w == warp && ((m[j] >> lane) & 1u))
+                        queue[at + __popc(m[j] & ((1u << lane) - 1u))] =
+                            (long long)(k + j * (int)gridDim.x) * BT + threadIdx.x;
+                    at += counts[j][w];
+                    if (w == BT / 32 - 1) n = at;
+                }
+            }
+            k += kScan * (int)gridDim.x;
+            __syncthreads();
+        }
+        const int take = n < BT ? n : BT;
+        if (take) body(take);
+        __syncthreads();
+        // at most kScan blocks of leftovers: move them to the front, one block at a time
+        for (int i = take; i < n; i += BT) {
+            const int at = i + threadIdx.x;
+            const long long c = at < n ? queue[at] : 0;
+            __syncthreads();
+            if (at < n) queue[at - take] = c;
+            __syncthreads();
+        }
+        n -= take;
+    }
+}
+constexpr int kBlockQueue = (kScan + 1) * BT;
+// Calls f(p, l) for the points p < 27 of the n queued cells, spread over the block (the cells rounded up to a power of
+// two, so a point's indices are a shift and a mask).
+template <class F>
+__device__ __forceinline__ void for_block_points(int n, F &&f) {
+    const int shift = 32 - __clz(n - 1), l = threadIdx.x & ((1 << shift) - 1);
+    if (l >= n) return;
+    for (int p = threadIdx.x >> shift; p < 27; p += BT >> shift) f(p, l);
+}
+unsigned flagged_blocks(const Q1Const &q) { return blocks_for(q.ncell, BT, 4); }
+
 // ============================================================================================== cell gradients
-// L1 = soft (JD, curl penalties scaled by mu_scale, nu_scale) + barrier; with split, L2 = barrier alone.
+// Vertex values of the soft penalties' gradient (mu_scale, nu_scale: 1 or 0), one cell per thread on its closed27 J
+// (q1_closed.cuh): the JD part's derivative by J at the 27 points is the 1D mass matrices applied to J - Jr, and one
+// adjoint pass of J carries it to the edge columns, where the curl part's Hadamard adjoint joins.  flags (when the
+// state has no mask): 1 for the cells with some closed27 J not above the activation, for cell_grad_barrier_kernel.
+//
+// Bound: FP64 issue (about 2,100 FP64 instructions per cell, the adjoint pass 27 x 24 of them; the Gauss27 form took
+// 4,500 and kept 81 flux sums in shared memory).  160x192x224: 3.06 -> 1.36 ms per launch.  The barrier's slopes stay
+// in their own kernel: evaluated here, on points packed over the warp, they cost 0.50 ms where that kernel takes 0.18
+// (a few warps per scheduler cannot hide their latency).
 __global__ void __launch_bounds__(CS) cell_grad_kernel(Q1Const q, const double *__restrict__ u,
                                                        const double *__restrict__ uref, double mu_scale,
-                                                       double nu_scale, bool barrier, bool split,
-                                                       double *__restrict__ L1, double *__restrict__ L2,
-                                                       const uint8_t *__restrict__ active) {
+                                                       double nu_scale, double *__restrict__ L1,
+                                                       uint8_t *__restrict__ flags) {
     extern __shared__ double smem[];
-    double *sl = smem + threadIdx.x;
+    double *sJ = smem + threadIdx.x;
     const int T = blockDim.x;
-    const double cn[3] = {0., .5, 1.}, cm[3] = {1., .5, 0.};
-    const double mu = q.mu * mu_scale, nu = q.nu * nu_scale;
+    double *sC = sJ + 27 * T;
+    // the mass matrices' 30 per axis and the quadrature's volume
+    const double wj = q.mu * mu_scale * q.omega * (1. / 27000.), wc = q.nu * nu_scale * q.omega;
+    const double low = near_bound(q.act);
+    const bool soft = mu_scale != 0. || nu_scale != 0.;     // neither: zeros, also where the field is not finite
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
          c += (long long)gridDim.x * blockDim.x) {
-        long long n0 = cell_node0(c, q);
-        double E[3][4][3], L[8][3];
-        load_edges(u, n0, q, E);
+        const long long n0 = cell_node0(c, q);
+        Columns C, G;
+        {
+            load_columns(uref, n0, q, C);
+            double k[18];
+            curl_coefficients(C, k);
 #pragma unroll
-        for (int a = 0; a < 8; a++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) L[a][r] = 0.;
-        if (mu != 0. || nu != 0.) {
-            double Er[3][4][3];
-            load_edges(uref, n0, q, Er);
-            zero_slice(sl, T, 81);
-            sweep2<false>(E, Er, q, [&](int p, int ix, int iy, int iz, const double (&V)[3][3],
-                                        const double (&Vr)[3][3]) {
-                double A[3][3], J, C[3], Cr[3];
-                cofactor_det(V, A, J);
-                double Jr = det_only(Vr);
-                curl_of(V, C);
-                curl_of(Vr, Cr);
-                const double gw = q.gw[p];
-                double jd = mu * gw * (J - Jr);
-                double k0 = nu * gw * (C[0] - Cr[0]), k1 = nu * gw * (C[1] - Cr[1]), k2 = nu * gw * (C[2] - Cr[2]);
-                double f[3][3];
-#pragma unroll
-                for (int r = 0; r < 3; r++)
-#pragma unroll
-                    for (int jj = 0; jj < 3; jj++) f[r][jj] = A[r][jj] * jd;
-                f[2][1] += k0; f[1][2] -= k0;
-                f[0][2] += k1; f[2][0] -= k1;
-                f[1][0] += k2; f[0][1] -= k2;
-                add_flux(sl, T, ix, iy, iz, f);
-            });
-            scatter_slice(sl, T, q.gn, q.gm, q.ih, L);
+            for (int i = 0; i < 18; i++) sC[i * T] = k[i];
+            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                 const double (&Z)[3]) { sJ[p * T] = det_minus_one(X, Y, Z); });
         }
-        bool any = false;
-        // cells whose closed27 J are all above the activation (the state's activity mask) have no barrier term
-        if (barrier && (!active || active[c])) {
-            zero_slice(sl, T, 81);
-            sweep<true>(E, q, [&](int, int ix, int iy, int iz, const double (&V)[3][3]) {
-                if (!(det_only(V) < q.act)) return;
-                double A[3][3], J, b, b1, b2;
-                cofactor_det(V, A, J);
-                barrier_eval(J, q.act, q.delta, q.bw, b, b1, b2);
-                double f[3][3];
+        load_columns(u, n0, q, C);
+        {
+            double k[18], r[27];
+            curl_coefficients(C, k);
 #pragma unroll
-                for (int r = 0; r < 3; r++)
-#pragma unroll
-                    for (int jj = 0; jj < 3; jj++) f[r][jj] = A[r][jj] * b1;
-                add_flux(sl, T, ix, iy, iz, f);
-                any = true;
+            for (int i = 0; i < 18; i++) sC[i * T] = __dsub_rn(k[i], sC[i * T]);
+            bool near = false;
+            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                 const double (&Z)[3]) {
+                const double J = det_minus_one(X, Y, Z);
+                near |= !(J >= low);
+                r[p] = __dsub_rn(J, sJ[p * T]);
             });
+            if (flags) flags[c] = near ? 1 : 0;
+            mass27(r);
+#pragma unroll
+            for (int p = 0; p < 27; p++) sJ[p * T] = wj * r[p];
         }
-        double Lb[8][3];
+        add_identity(C);
+        closed_adjoint(C, G, [&](int p) { return sJ[p * T]; });
+        {
+            double k[18];
 #pragma unroll
-        for (int a = 0; a < 8; a++)
+            for (int i = 0; i < 18; i++) k[i] = sC[i * T];
+            curl_adjoint(k, wc, G);
+        }
+        double L[8][3];
+        columns_to_vertices(G, q, L);
+        if (!soft) {
 #pragma unroll
-            for (int r = 0; r < 3; r++) Lb[a][r] = 0.;
-        if (any) scatter_slice(sl, T, cn, cm, q.ih, Lb);
+            for (int a = 0; a < 8; a++)
 #pragma unroll
-        for (int a = 0; a < 8; a++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) L[a][r] += Lb[a][r];
+                for (int r = 0; r < 3; r++) L[a][r] = 0.;
+        }
         store_locals(L1, c, q.ncell, L);
-        if (split) store_locals(L2, c, q.ncell, Lb);
     }
+}
+
+// The barrier's vertex values of the flagged cells (the state's mask, or the cells cell_grad_kernel flags): b'(J) at
+// the 27 points (zero above the activation) and the same adjoint pass; added to L1 and, with split, stored in L2 for
+// every flagged cell.
+__global__ void __launch_bounds__(BT) cell_grad_barrier_kernel(Q1Const q, const double *__restrict__ u,
+                                                               const uint8_t *__restrict__ flags, bool split,
+                                                               double *__restrict__ L1, double *__restrict__ L2) {
+    extern __shared__ double smem[];
+    __shared__ long long queue[kBlockQueue];
+    const BarrierRule rule = barrier_rule(q);
+    for_flagged_blocks(q, flags, queue, [&](int n) {
+        const bool mine = (int)threadIdx.x < n;
+        double *sl = smem + threadIdx.x;
+        const long long c = mine ? queue[threadIdx.x] : 0;
+        Columns C, G;
+        if (mine) {
+            load_columns(u, cell_node0(c, q), q, C);
+            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                 const double (&Z)[3]) { sl[p * BT] = jacobian(det_minus_one(X, Y, Z)); });
+        }
+        __syncthreads();
+        for_block_points(n, [&](int p, int l) {
+            const double J = smem[p * BT + l];
+            smem[p * BT + l] = J < q.act ? barrier_slope(J, rule) : 0.;
+        });
+        __syncthreads();
+        if (mine) {
+            load_columns(u, cell_node0(c, q), q, C);     // again: 36 columns do not wait in registers
+            add_identity(C);
+            closed_adjoint(C, G, [&](int p) { return sl[p * BT]; });
+            double Lb[8][3];
+            columns_to_vertices(G, q, Lb);
+#pragma unroll
+            for (int a = 0; a < 8; a++)
+#pragma unroll
+                for (int r = 0; r < 3; r++) L1[(size_t)(3 * a + r) * q.ncell + c] += Lb[a][r];
+            if (split) store_locals(L2, c, q.ncell, Lb);
+        }
+    });
 }
 
 // ============================================================================================== gather
@@ -444,10 +542,13 @@ struct GatherSpec {
     double *out[3];
 };
 
-// Free node (z, y, x): sum of the 8 cells' vertex values in fixed order a = 0..7, plus node terms.
-template <class LT>
+// Free node (z, y, x): sum of the 8 cells' vertex values in fixed order a = 0..7, plus node terms.  With TWO,
+// has2 marks the cells whose L2 values were written; the others' are zero (most cells have no barrier term: one byte
+// is read for 24).
+template <bool TWO, class LT>
 __global__ void __launch_bounds__(256) gather_kernel(Q1Const q, GatherSpec g, const LT *__restrict__ L1,
-                                                     const LT *__restrict__ L2, const double *__restrict__ u,
+                                                     const LT *__restrict__ L2,
+                                                     const uint8_t *__restrict__ has2, const double *__restrict__ u,
                                                      const double *__restrict__ uref,
                                                      const double *__restrict__ warped,
                                                      const double *__restrict__ fixed,
@@ -462,15 +563,27 @@ __global__ void __launch_bounds__(256) gather_kernel(Q1Const q, GatherSpec g, co
         double dimg = warped ? qw * (warped[node] - fixed[node]) : 0.;
         // the 8 cells' vertex values summed in the locals' type (float locals: one conversion per sum, not per term)
         LT t1[3] = {LT(0), LT(0), LT(0)}, t2[3] = {LT(0), LT(0), LT(0)};
+        long long cell[8];
+        uint8_t two[8], some = 0;
 #pragma unroll
         for (int a = 0; a < 8; a++) {
-            long long c = ((z - (a >> 2)) * q.cy + (y - ((a >> 1) & 1))) * q.cx + (x - (a & 1));
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                if (L1) t1[r] += L1[(long long)(a * 3 + r) * q.ncell + c];
-                if (L2) t2[r] += L2[(long long)(a * 3 + r) * q.ncell + c];
+            cell[a] = ((z - (a >> 2)) * q.cy + (y - ((a >> 1) & 1))) * q.cx + (x - (a & 1));
+            if (TWO) {
+                two[a] = has2[cell[a]];
+                some |= two[a];
             }
         }
+        if (L1)
+#pragma unroll
+            for (int a = 0; a < 8; a++)
+#pragma unroll
+                for (int r = 0; r < 3; r++) t1[r] += L1[(long long)(a * 3 + r) * q.ncell + cell[a]];
+        if (TWO && some)
+#pragma unroll
+            for (int a = 0; a < 8; a++)
+                if (two[a])
+#pragma unroll
+                    for (int r = 0; r < 3; r++) t2[r] += L2[(long long)(a * 3 + r) * q.ncell + cell[a]];
         const double s1[3] = {(double)t1[0], (double)t1[1], (double)t1[2]};
         const double s2[3] = {(double)t2[0], (double)t2[1], (double)t2[2]};
 #pragma unroll
@@ -735,12 +848,11 @@ __device__ __forceinline__ void load_edges_f32(const double *__restrict__ u, lon
 #pragma unroll
             for (int r = 0; r < 3; r++) E[j][e][r] = (float)E64[j][e][r];
 }
-// The soft part (JD, curl penalties) of the gradient locals; with split, L2 is zeroed for the barrier kernel.  flags
-// (when the state has no mask): 1 for the cells with some float32 closed27 J within the guard.
+// The soft part (JD, curl penalties) of the gradient locals.  flags (when the state has no mask): 1 for the cells with some float32 closed27 J within the guard.
 __global__ void __launch_bounds__(CS, 8) cell_grad32_kernel(Q1Const q, const double *__restrict__ u,
                                                          const double *__restrict__ uref, double mu_scale,
-                                                         double nu_scale, bool split, float *__restrict__ L1,
-                                                         float *__restrict__ L2, uint8_t *__restrict__ flags) {
+                                                         double nu_scale, float *__restrict__ L1,
+                                                         uint8_t *__restrict__ flags) {
     extern __shared__ float smemf[];
     float *sl = smemf + threadIdx.x;
     const int T = blockDim.x;
@@ -790,32 +902,21 @@ __global__ void __launch_bounds__(CS, 8) cell_grad32_kernel(Q1Const q, const dou
             flags[c] = near ? 1 : 0;
         }
         store_locals(L1, c, q.ncell, L);
-        if (split) {
-            float Z[8][3];
-#pragma unroll
-            for (int a = 0; a < 8; a++)
-#pragma unroll
-                for (int r = 0; r < 3; r++) Z[a][r] = 0.f;
-            store_locals(L2, c, q.ncell, Z);
-        }
     }
 }
 
 // The barrier's locals of the flagged cells in float64: the closed27 sweep from the float64 state, J, b' and the
-// cofactors exactly as the float64 kernel forms them, the flux rounded to the locals' type LT (float32 in the mixed
-// form, float64 in the plain one) and scattered as the soft kernel scatters its own; then added to the cell's locals
-// (L1 += Lb) and, for the outer triple, stored apart (L2).  In the plain form the values are those of the fused
-// float64 kernel (the same sweep of the same edges, the same add).
-template <class LT>
-__global__ void __launch_bounds__(CB) cell_grad_barrier_kernel(Q1Const q, const double *__restrict__ u,
+// cofactors in float64, the flux rounded to float32 and scattered as the soft kernel scatters its own; then added to
+// the cell's locals (L1 += Lb) and, for the outer triple, stored apart (L2, for every flagged cell).
+__global__ void __launch_bounds__(CB) cell_grad_barrier32_kernel(Q1Const q, const double *__restrict__ u,
                                                                const uint8_t *__restrict__ flags, bool split,
-                                                               LT *__restrict__ L1, LT *__restrict__ L2) {
-    extern __shared__ __align__(16) unsigned char smemb[];
+                                                               float *__restrict__ L1, float *__restrict__ L2) {
+    extern __shared__ float smemf[];
     __shared__ long long queue[CB / 32][64];
-    LT *sl = reinterpret_cast<LT *>(smemb) + threadIdx.x;
+    float *sl = smemf + threadIdx.x;
     const int T = blockDim.x;
-    const LT cn[3] = {LT(0), LT(.5), LT(1)}, cm[3] = {LT(1), LT(.5), LT(0)};
-    const LT ih[3] = {(LT)q.ih[0], (LT)q.ih[1], (LT)q.ih[2]};
+    const float cn[3] = {0.f, .5f, 1.f}, cm[3] = {1.f, .5f, 0.f};
+    const float ih[3] = {(float)q.ih[0], (float)q.ih[1], (float)q.ih[2]};
     for_flagged_cells(q, flags, queue[threadIdx.x >> 5], [&](long long c, uint8_t) {
         double E64[3][4][3];
         load_edges(u, cell_node0(c, q), q, E64);
@@ -826,25 +927,26 @@ __global__ void __launch_bounds__(CB) cell_grad_barrier_kernel(Q1Const q, const 
             double A[3][3], J, b, b1, b2;
             cofactor_det(V, A, J);
             barrier_eval(J, q.act, q.delta, q.bw, b, b1, b2);
-            LT f[3][3];
+            float f[3][3];
 #pragma unroll
             for (int r = 0; r < 3; r++)
 #pragma unroll
-                for (int jj = 0; jj < 3; jj++) f[r][jj] = (LT)(A[r][jj] * b1);
+                for (int jj = 0; jj < 3; jj++) f[r][jj] = (float)(A[r][jj] * b1);
             add_flux(sl, T, ix, iy, iz, f);
             any = true;
         });
-        if (!any) return;
-        LT Lb[8][3];
+        if (!any && !split) return;
+        float Lb[8][3];
 #pragma unroll
         for (int a = 0; a < 8; a++)
 #pragma unroll
-            for (int r = 0; r < 3; r++) Lb[a][r] = LT(0);
+            for (int r = 0; r < 3; r++) Lb[a][r] = 0.f;
         scatter_slice(sl, T, cn, cm, ih, Lb);
+        if (any)
 #pragma unroll
-        for (int a = 0; a < 8; a++)
+            for (int a = 0; a < 8; a++)
 #pragma unroll
-            for (int r = 0; r < 3; r++) L1[(size_t)(3 * a + r) * q.ncell + c] += Lb[a][r];
+                for (int r = 0; r < 3; r++) L1[(size_t)(3 * a + r) * q.ncell + c] += Lb[a][r];
         if (split) store_locals(L2, c, q.ncell, Lb);
     });
 }
@@ -1035,57 +1137,58 @@ __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S,
 
 // The barrier of the flagged cells (cell_soft_kernel's flags): the state's barrier sum, violations (J <= delta) and
 // activity mask (trial_act[c] = 1 when some closed27 J is below the activation), and with DIFF its stable change from
-// the base; the J are those of cell_soft_kernel.  Rolled loops over the 27 points keep the logarithms' code and
-// registers out of the soft kernel, and the queue hands them to full warps.
+// the base; the J are those of cell_soft_kernel.
 template <bool ENERGY, bool DIFF>
-__global__ void __launch_bounds__(CB) cell_barrier_kernel(Q1Const q, const double *__restrict__ ua,
+__global__ void __launch_bounds__(BT) cell_barrier_kernel(Q1Const q, const double *__restrict__ ua,
                                                           const double *__restrict__ ub,
                                                           const uint8_t *__restrict__ flags, dd *pe, dd *pd,
                                                           unsigned long long *bad,
                                                           uint8_t *__restrict__ trial_act) {
     extern __shared__ double smem[];
-    __shared__ long long queue[CB / 32][64];
-    double *sb = smem + threadIdx.x;
-    const int T = blockDim.x;
-    double *sa = sb + 27 * T;
+    __shared__ long long queue[kBlockQueue];
+    double *sb = smem, *sa = smem + 27 * BT;
     dd acc[1] = {{0., 0.}}, dif[1] = {{0., 0.}};
     unsigned long long nbad = 0;
-    for_flagged_cells(q, flags, queue[threadIdx.x >> 5], [&](long long c, uint8_t) {
-        const long long n0 = cell_node0(c, q);
-        Columns C;
-        load_columns(ub, n0, q, C);
-        closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
-            sb[p * T] = jacobian(det_minus_one(X, Y, Z));
+    const BarrierRule rule = barrier_rule(q);
+    for_flagged_blocks(q, flags, queue, [&](int n) {
+        if ((int)threadIdx.x < n) {
+            const long long n0 = cell_node0(queue[threadIdx.x], q);
+            Columns C;
+            load_columns(ub, n0, q, C);
+            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                 const double (&Z)[3]) {
+                sb[p * BT + threadIdx.x] = jacobian(det_minus_one(X, Y, Z));
+            });
+            if (DIFF) {
+                load_columns(ua, n0, q, C);
+                closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                     const double (&Z)[3]) {
+                    sa[p * BT + threadIdx.x] = jacobian(det_minus_one(X, Y, Z));
+                });
+            }
+        }
+        __syncthreads();
+        double sum = 0., change = 0.;
+        bool active = false;
+        int cell = 0;
+        for_block_points(n, [&](int p, int l) {
+            const double jb = sb[p * BT + l];
+            if (ENERGY) {
+                active |= jb < q.act;
+                cell = l;
+                if (!(jb > q.delta)) nbad++;
+                else if (jb < q.act) sum += barrier_value(jb, rule);
+            }
+            if (DIFF) {
+                const double ja = sa[p * BT + l];
+                if (ja < q.act || jb < q.act) change += barrier_change(ja, jb, rule);
+            }
         });
         if (ENERGY) {
-            double sum = 0.;
-            bool active = false;
-#pragma unroll 1
-            for (int p = 0; p < 27; p++) {
-                const double j = sb[p * T];
-                active |= j < q.act;
-                if (!(j > q.delta)) { nbad++; continue; }
-                if (j < q.act) {
-                    double b, b1, b2;
-                    barrier_eval(j, q.act, q.delta, q.bw, b, b1, b2);
-                    sum += b;
-                }
-            }
-            if (trial_act && active) trial_act[c] = 1;
+            if (trial_act && active) trial_act[queue[cell]] = 1;
             acc[0] = dd_add_d(acc[0], sum);
         }
-        if (DIFF) {
-            load_columns(ua, n0, q, C);
-            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
-                                 const double (&Z)[3]) { sa[p * T] = jacobian(det_minus_one(X, Y, Z)); });
-            double sum = 0.;
-#pragma unroll 1
-            for (int p = 0; p < 27; p++) {
-                const double ja = sa[p * T], jb = sb[p * T];
-                if (ja < q.act || jb < q.act) sum += barrier_difference(ja, jb, q.act, q.delta);
-            }
-            dif[0] = dd_add_d(dif[0], __dmul_rn(q.bw, sum));
-        }
+        if (DIFF) dif[0] = dd_add_d(dif[0], q.bw * change);
     });
     if (ENERGY) block_reduce_dd<1>(acc, pe);
     if (ENERGY && DIFF) __syncthreads();     // the two reductions share block_reduce_dd's shared array
@@ -1779,11 +1882,9 @@ int allow_slices() {
     SVP_CUDA(cudaFuncSetAttribute(cell_soft_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)slice_bytes(kDiffSlots)));
     SVP_CUDA(cudaFuncSetAttribute(cell_barrier_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(sizeof(double) * 54 * CB)));
+                                  (int)(sizeof(double) * 54 * BT)));
     SVP_CUDA(cudaFuncSetAttribute(cell_barrier_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(sizeof(double) * 54 * CB)));
-    SVP_CUDA(cudaFuncSetAttribute(cell_grad_barrier_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)(sizeof(double) * 81 * CB)));
+                                  (int)(sizeof(double) * 54 * BT)));
     done[dev] = true;
     return SVP_OK;
 }
@@ -1853,7 +1954,7 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
                           int64_t *barrier_violations, void *stream) {
     SVP_REQUIRE(p && u && warped && terms5, "svp_energy: null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = barrier_blocks(p->q);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
     int rc = pair_partials(p, (long long)nb * 2 + (long long)cb * 2 + bb, 1);
     if (rc) return rc;
     if ((rc = allow_slices())) return rc;
@@ -1869,7 +1970,7 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
     }
     {
         svp::KernelTimer _t("cell_barrier_kernel", s);
-        SVP_LAUNCH(cell_barrier_kernel<true, false><<<bb, CB, sizeof(double) * 27 * CB, s>>>(
+        SVP_LAUNCH(cell_barrier_kernel<true, false><<<bb, BT, sizeof(double) * 27 * BT, s>>>(
             p->q, nullptr, u, p->flags, pb, nullptr, (unsigned long long *)p->counter, nullptr));
     }
     SVP_LAUNCH_CHECK("cell_energy_kernel");
@@ -1903,7 +2004,7 @@ extern "C" int svp_energy_difference_masked(svp_pair *p, const double *base_u, c
     // the cell kernels find the cells near the activation from the J they evaluate, so the masks save nothing here
     (void)base_active;
     (void)trial_active;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = barrier_blocks(p->q);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
     int rc = pair_partials(p, (long long)nb * 2 + (long long)cb * 2 + bb, 1);
     if (rc) return rc;
     if ((rc = allow_slices())) return rc;
@@ -1918,7 +2019,7 @@ extern "C" int svp_energy_difference_masked(svp_pair *p, const double *base_u, c
     }
     {
         svp::KernelTimer _t("cell_barrier_kernel", s);
-        SVP_LAUNCH(cell_barrier_kernel<false, true><<<bb, CB, sizeof(double) * 54 * CB, s>>>(
+        SVP_LAUNCH(cell_barrier_kernel<false, true><<<bb, BT, sizeof(double) * 54 * BT, s>>>(
             p->q, base_u, trial_u, p->flags, nullptr, pb, nullptr, nullptr));
     }
     SVP_LAUNCH_CHECK("difference kernels");
@@ -2020,7 +2121,7 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
     SVP_REQUIRE(p && base_u && base_warped && trial_u && trial_warped && terms5 && diff2,
                 "svp_trial_energy: null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = barrier_blocks(p->q);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = screened ? barrier_blocks(p->q) : flagged_blocks(p->q);
     int rc = pair_partials(p, (long long)nb * 4 + (long long)cb * 10 + (long long)bb * 2, 1);
     if (rc) return rc;
     if ((rc = allow_slices())) return rc;
@@ -2055,7 +2156,7 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
                 p->q, base_u, trial_u, p->u_ref, pce, pcd, p->flags, trial_active));
         }
         svp::KernelTimer _t("cell_barrier_kernel", s);
-        SVP_LAUNCH(cell_barrier_kernel<true, true><<<bb, CB, sizeof(double) * 54 * CB, s>>>(
+        SVP_LAUNCH(cell_barrier_kernel<true, true><<<bb, BT, sizeof(double) * 54 * BT, s>>>(
             p->q, base_u, trial_u, p->flags, pbe, pbd, (unsigned long long *)p->counter, trial_active));
     }
     SVP_LAUNCH_CHECK("cell_trial_kernel");
@@ -2131,52 +2232,61 @@ extern "C" int svp_trial_energy(svp_pair *p, const double *base_u, const double 
 }
 
 template <class LT>
-static int run_gather(svp_pair *p, const GatherSpec &g, const LT *L1, const LT *L2, const double *u,
-                      const double *uref, const double *warped, const double *image_grad, cudaStream_t s) {
-    { svp::KernelTimer _t("gather_kernel", s); SVP_LAUNCH(gather_kernel<LT><<<node_blocks(p->q.nfree), 256, 0, s>>>(p->q, g, L1, L2, u, uref, warped, p->fixed, image_grad)); }
-    SVP_LAUNCH_CHECK("gather_kernel");
+static int run_gather(svp_pair *p, const GatherSpec &g, const LT *L1, const LT *L2, const uint8_t *has2,
+                      const double *u, const double *uref, const double *warped, const double *image_grad,
+                      cudaStream_t s) {
+    svp::KernelTimer _t("gather_kernel", s);
+    const unsigned nb = node_blocks(p->q.nfree);
+    if (L2)
+        SVP_LAUNCH((gather_kernel<true, LT><<<nb, 256, 0, s>>>(p->q, g, L1, L2, has2, u, uref, warped, p->fixed,
+                                                              image_grad)));
+    else
+        SVP_LAUNCH((gather_kernel<false, LT><<<nb, 256, 0, s>>>(p->q, g, L1, nullptr, nullptr, u, uref, warped,
+                                                               p->fixed, image_grad)));
     return SVP_OK;
 }
 
-// The plain form's gradient locals: with the state's activity mask, the soft float64 kernel and then the barrier
-// kernel over the active cells (the values of the fused kernel: the same sweep, the same add); without a mask the
-// fused kernel sweeps the barrier of every cell.
+// The plain form's gradient locals: the soft kernel, then the barrier kernel over the flagged cells (the state's mask,
+// or without one the cells the soft kernel flags).  *has2: the cells whose L2 values were written.
 static int grad64(svp_pair *p, const double *u, double mu_scale, double nu_scale, bool barrier, bool split,
-                  const uint8_t *active, cudaStream_t s) {
-    const bool apart = barrier && active;
+                  const uint8_t *active, const uint8_t **has2, cudaStream_t s) {
     int rc = allow_slices();
     if (rc) return rc;
+    if (barrier && !active && (rc = pair_flags(p))) return rc;
+    uint8_t *flags = barrier && !active ? p->flags : nullptr;
+    const uint8_t *marked = active ? active : flags;
     {
         svp::KernelTimer _t("cell_grad_kernel", s);
-        SVP_LAUNCH(cell_grad_kernel<<<slice_blocks(p), CS, slice_bytes(81), s>>>(
-            p->q, u, p->u_ref, mu_scale, nu_scale, barrier && !apart, split, p->loc1, split ? p->loc2 : nullptr,
-            active));
+        SVP_LAUNCH(cell_grad_kernel<<<slice_blocks(p), CS, slice_bytes(45), s>>>(p->q, u, p->u_ref, mu_scale,
+                                                                                nu_scale, p->loc1, flags));
     }
-    if (apart) {
+    if (barrier) {
         svp::KernelTimer _t("cell_grad_barrier_kernel", s);
-        SVP_LAUNCH(cell_grad_barrier_kernel<double><<<barrier_blocks(p->q), CB, sizeof(double) * 81 * CB, s>>>(
-            p->q, u, active, split, p->loc1, split ? p->loc2 : nullptr));
+        SVP_LAUNCH(cell_grad_barrier_kernel<<<flagged_blocks(p->q), BT, sizeof(double) * 27 * BT, s>>>(
+            p->q, u, marked, split, p->loc1, split ? p->loc2 : nullptr));
     }
+    *has2 = split ? marked : nullptr;
     return SVP_OK;
 }
 
 // The mixed form's gradient locals: the float32 soft kernel, then the float64 barrier kernel over the flagged cells
 // (the state's mask, or without one the cells the soft kernel flags from its float32 closed27 J).
 static int grad32(svp_pair *p, const double *u, double mu_scale, double nu_scale, bool barrier, bool split,
-                  const uint8_t *active, cudaStream_t s) {
+                  const uint8_t *active, const uint8_t **has2, cudaStream_t s) {
     int rc;
     if (barrier && !active && (rc = pair_flags(p))) return rc;
     uint8_t *flags = barrier && !active ? p->flags : nullptr;
     {
         svp::KernelTimer _t("cell_grad32_kernel", s);
         SVP_LAUNCH(cell_grad32_kernel<<<slice_blocks(p), CS, sizeof(float) * 81 * CS, s>>>(
-            p->q, u, p->u_ref, mu_scale, nu_scale, split, (float *)p->loc1, (float *)p->loc2, flags));
+            p->q, u, p->u_ref, mu_scale, nu_scale, (float *)p->loc1, flags));
     }
     if (barrier) {
         svp::KernelTimer _t("cell_grad_barrier32_kernel", s);
-        SVP_LAUNCH(cell_grad_barrier_kernel<float><<<barrier_blocks(p->q), CB, sizeof(float) * 81 * CB, s>>>(
+        SVP_LAUNCH(cell_grad_barrier32_kernel<<<barrier_blocks(p->q), CB, sizeof(float) * 81 * CB, s>>>(
             p->q, u, active ? active : flags, split, (float *)p->loc1, (float *)p->loc2));
     }
+    *has2 = split ? (active ? active : flags) : nullptr;
     return SVP_OK;
 }
 
@@ -2192,13 +2302,14 @@ extern "C" int svp_gradient_masked(svp_pair *p, const double *u, const double *w
     if (cellwork) {
         int rc = pair_locals(p, 1);
         if (rc) return rc;
+        const uint8_t *has2;
         if (mixed) {
             if ((rc = grad32(p, u, (terms & SVP_TERM_JD) ? 1. : 0., (terms & SVP_TERM_CURL) ? 1. : 0.,
-                             (terms & SVP_TERM_BARRIER) != 0, false, active, s)))
+                             (terms & SVP_TERM_BARRIER) != 0, false, active, &has2, s)))
                 return rc;
         } else {
             if ((rc = grad64(p, u, (terms & SVP_TERM_JD) ? 1. : 0., (terms & SVP_TERM_CURL) ? 1. : 0.,
-                             (terms & SVP_TERM_BARRIER) != 0, false, active, s)))
+                             (terms & SVP_TERM_BARRIER) != 0, false, active, &has2, s)))
                 return rc;
         }
         SVP_LAUNCH_CHECK("cell_grad_kernel");
@@ -2210,9 +2321,9 @@ extern "C" int svp_gradient_masked(svp_pair *p, const double *u, const double *w
     g.c1[0] = cellwork ? 1. : 0.;
     g.out[0] = out;
     if (mixed)
-        return run_gather<float>(p, g, cellwork ? (const float *)p->loc1 : nullptr, nullptr, u, p->u_ref,
+        return run_gather<float>(p, g, cellwork ? (const float *)p->loc1 : nullptr, nullptr, nullptr, u, p->u_ref,
                                  img ? warped : nullptr, img ? image_grad : nullptr, s);
-    return run_gather<double>(p, g, cellwork ? p->loc1 : nullptr, nullptr, u, p->u_ref, img ? warped : nullptr,
+    return run_gather<double>(p, g, cellwork ? p->loc1 : nullptr, nullptr, nullptr, u, p->u_ref, img ? warped : nullptr,
                               img ? image_grad : nullptr, s);
 }
 
@@ -2224,10 +2335,11 @@ extern "C" int svp_outer_gradients_masked(svp_pair *p, const double *u, const do
     int rc = pair_locals(p, 2);
     if (rc) return rc;
     const bool mixed = p->precision == SVP_PRECISION_MIXED;
+    const uint8_t *has2 = nullptr;
     if (mixed) {
-        if ((rc = grad32(p, u, 1., 1., true, true, active, s))) return rc;
+        if ((rc = grad32(p, u, 1., 1., true, true, active, &has2, s))) return rc;
     } else {
-        if ((rc = grad64(p, u, 1., 1., true, true, active, s))) return rc;
+        if ((rc = grad64(p, u, 1., 1., true, true, active, &has2, s))) return rc;
     }
     SVP_LAUNCH_CHECK("cell_grad_kernel");
     GatherSpec g{};
@@ -2236,8 +2348,8 @@ extern "C" int svp_outer_gradients_masked(svp_pair *p, const double *u, const do
     g.ci[0] = 1.; g.cp[0] = 0.; g.c1[0] = 0.; g.c2[0] = 1.; g.out[0] = gF;
     g.ci[1] = 1.; g.cp[1] = 0.; g.c1[1] = 0.; g.c2[1] = 0.; g.out[1] = gD;
     g.ci[2] = 1.; g.cp[2] = 1.; g.c1[2] = 1.; g.c2[2] = 0.; g.out[2] = gE;
-    if (mixed) return run_gather<float>(p, g, (const float *)p->loc1, (const float *)p->loc2, u, p->u_ref, warped, image_grad, s);
-    return run_gather<double>(p, g, p->loc1, p->loc2, u, p->u_ref, warped, image_grad, s);
+    if (mixed) return run_gather<float>(p, g, (const float *)p->loc1, (const float *)p->loc2, has2, u, p->u_ref, warped, image_grad, s);
+    return run_gather<double>(p, g, p->loc1, p->loc2, has2, u, p->u_ref, warped, image_grad, s);
 }
 
 extern "C" int svp_ggn_diagonal_masked(svp_pair *p, const double *u, const double *image_grad,

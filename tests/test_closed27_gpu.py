@@ -57,3 +57,25 @@ def test_energies_and_differences(problem):
     scale = np.array(Q.energy(OP, base, ob)[:5]) + ref      # a difference rounds relative to what it subtracts
     got = P.energy_difference(bd, wb, td, wt)
     assert abs(got[0] - dE) <= TOL * scale.sum() and abs(got[1] - dF) <= TOL * (scale[0] + scale[4])
+
+
+@pytest.mark.parametrize("term", ["total", "jd", "curl", "barrier", "outer"])
+def test_gradients(problem, term):
+    P, OP, bd, td, base, trial = problem
+    w, g = P.warp(bd, with_gradient=True)
+    ow, og = Q.warp(OP, base, True)
+    ref = Q.gradient(OP, base, ow, og, term)
+    got = P.gradient(bd, w, g, term).cpu().numpy()
+    assert np.linalg.norm(got - ref) <= TOL * np.linalg.norm(ref)
+
+
+def test_outer_gradients(problem):
+    P, OP, bd, td, base, trial = problem
+    w, g = P.warp(bd, with_gradient=True)
+    ow, og = Q.warp(OP, base, True)
+    active = P.trial_energy(td, P.warp(td)[0], bd)[5]
+    assert 0 < int(active.sum())
+    for mask in (None, active):
+        for got, term in zip(P.outer_gradients(bd, w, g, mask), ("outer", "image", "total")):
+            ref = Q.gradient(OP, base, ow, og, term)
+            assert np.linalg.norm(got.cpu().numpy() - ref) <= TOL * np.linalg.norm(ref)
