@@ -186,28 +186,151 @@ __device__ __forceinline__ bool hull_entry_v(const double v[8][3], int j, int r,
     return ok;
 }
 
+// One cell's margin in the reference's operation sequence; false where some interval was not finite.
 template <bool DIR>
-__global__ void __launch_bounds__(256) edge_hull_kernel(const double *__restrict__ u, CellGrid g, double delta,
+__device__ __noinline__ bool hull_margin_general(const double *__restrict__ u, long long base, const CellGrid &g,
+                                                 double delta, double *margin) {
+    double v[8][3];
+#pragma unroll
+    for (int a = 0; a < 8; a++)
+#pragma unroll
+        for (int r = 0; r < 3; r++) v[a][r] = __ldg(u + 3 * vnode(base, a, g.ny, g.nx) + r);
+    double fl[3][3], fh[3][3];
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+        for (int r = 0; r < 3; r++) ok &= hull_entry_v<DIR>(v, j, r, g.div, fl[r][j], fh[r][j]);
+    double jl, jh, ml, mh;
+    ok &= Idet<DIR>(fl, fh, jl, jh);
+    if constexpr (DIR) ok &= dsub(jl, jh, delta, delta, ml, mh);
+    else ok &= iout(rsub(jl, delta), rsub(jh, delta), ml, mh);
+    *margin = ml;
+    return ok;
+}
+
+// The same sequence for cells whose intervals all stay finite, which is checked once at the end:
+//  - the outward step of a finite x is one addition of the smallest subnormal rounded outward: x - 2^-1074 lies
+//    between x and its predecessor, so rounding down gives the predecessor (the integer steps and their selects
+//    took most of the general form's instructions); only the sign of a zero result can differ, and a zero's sign
+//    cannot reach a nonzero value through products, sums and steps, so it matters only for a margin that is zero;
+//  - with no NaN, minimum and maximum are one comparison each;
+//  - lo <= hi holds by monotone rounding; finiteness is the largest exponent seen.
+// Where a value was not finite or the margin is zero the general form decides.
+struct FiniteCheck {
+    int top = 0;
+    __device__ __forceinline__ void see(double lo, double hi) {
+        top = max(top, max(__double2hiint(lo) & 0x7FFFFFFF, __double2hiint(hi) & 0x7FFFFFFF));
+    }
+    __device__ __forceinline__ bool finite() const { return top < 0x7FF00000; }
+};
+__device__ __forceinline__ double min1(double a, double b) { return a <= b ? a : b; }
+__device__ __forceinline__ double max1(double a, double b) { return a >= b ? a : b; }
+__device__ __forceinline__ double out_down(double x) { return __dadd_rd(x, -4.9406564584124654e-324); }
+__device__ __forceinline__ double out_up(double x) { return __dadd_ru(x, 4.9406564584124654e-324); }
+template <bool DIR>
+__device__ __forceinline__ void Fadd(double al, double ah, double bl, double bh, double &rl, double &rh,
+                                     FiniteCheck &f) {
+    if constexpr (DIR) { rl = __dadd_rd(al, bl); rh = __dadd_ru(ah, bh); }
+    else { rl = out_down(radd(al, bl)); rh = out_up(radd(ah, bh)); }
+    f.see(rl, rh);
+}
+template <bool DIR>
+__device__ __forceinline__ void Fsub(double al, double ah, double bl, double bh, double &rl, double &rh,
+                                     FiniteCheck &f) {
+    Fadd<DIR>(al, ah, -bh, -bl, rl, rh, f);
+}
+template <bool DIR>
+__device__ __forceinline__ void Fmul(double al, double ah, double bl, double bh, double &rl, double &rh,
+                                     FiniteCheck &f) {
+    if constexpr (DIR) {
+        rl = min1(min1(__dmul_rd(al, bl), __dmul_rd(al, bh)), min1(__dmul_rd(ah, bl), __dmul_rd(ah, bh)));
+        rh = max1(max1(__dmul_ru(al, bl), __dmul_ru(al, bh)), max1(__dmul_ru(ah, bl), __dmul_ru(ah, bh)));
+    } else {
+        const double x = rmul(al, bl), y = rmul(al, bh), z = rmul(ah, bl), w = rmul(ah, bh);
+        rl = out_down(min1(min1(x, y), min1(z, w)));
+        rh = out_up(max1(max1(x, y), max1(z, w)));
+    }
+    f.see(rl, rh);
+}
+template <bool DIR>
+__device__ __forceinline__ double hull_margin_finite(const double (&v)[8][3], const AxisDiv &dv, double delta,
+                                                     bool &ok) {
+    FiniteCheck f;
+    // the vertices: a difference is NaN only where one of them is not finite (an infinite difference is a hull end)
+#pragma unroll
+    for (int a = 0; a < 8; a++)
+#pragma unroll
+        for (int r = 0; r < 3; r++) f.see(v[a][r], v[a][r]);
+    double fl[3][3], fh[3][3];
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            double lo, hi;
+            if constexpr (DIR) {
+                double l[4], h[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int a = edge_start(j, e), b = a | (1 << j);
+                    l[e] = __dsub_rd(v[b][r], v[a][r]);
+                    h[e] = __dsub_ru(v[b][r], v[a][r]);
+                }
+                lo = div_axis_rd(min1(min1(l[0], l[1]), min1(l[2], l[3])), dv, j);
+                hi = div_axis_ru(max1(max1(h[0], h[1]), max1(h[2], h[3])), dv, j);
+            } else {
+                double d[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int a = edge_start(j, e), b = a | (1 << j);
+                    d[e] = rsub(v[b][r], v[a][r]);
+                }
+                lo = out_down(div_axis(out_down(min1(min1(d[0], d[1]), min1(d[2], d[3]))), dv, j));
+                hi = out_up(div_axis(out_up(max1(max1(d[0], d[1]), max1(d[2], d[3]))), dv, j));
+            }
+            f.see(lo, hi);
+            const double id = r == j ? 1. : 0.;
+            Fadd<DIR>(lo, hi, id, id, fl[r][j], fh[r][j], f);
+        }
+    double p1l, p1h, p2l, p2h, al, ah, bl, bh, cl, ch, t1l, t1h, t2l, t2h, sl, sh, t3l, t3h, jl, jh, ml, mh;
+    Fmul<DIR>(fl[1][1], fh[1][1], fl[2][2], fh[2][2], p1l, p1h, f);
+    Fmul<DIR>(fl[1][2], fh[1][2], fl[2][1], fh[2][1], p2l, p2h, f);
+    Fsub<DIR>(p1l, p1h, p2l, p2h, al, ah, f);
+    Fmul<DIR>(fl[1][2], fh[1][2], fl[2][0], fh[2][0], p1l, p1h, f);
+    Fmul<DIR>(fl[1][0], fh[1][0], fl[2][2], fh[2][2], p2l, p2h, f);
+    Fsub<DIR>(p1l, p1h, p2l, p2h, bl, bh, f);
+    Fmul<DIR>(fl[1][0], fh[1][0], fl[2][1], fh[2][1], p1l, p1h, f);
+    Fmul<DIR>(fl[1][1], fh[1][1], fl[2][0], fh[2][0], p2l, p2h, f);
+    Fsub<DIR>(p1l, p1h, p2l, p2h, cl, ch, f);
+    Fmul<DIR>(fl[0][0], fh[0][0], al, ah, t1l, t1h, f);
+    Fmul<DIR>(fl[0][1], fh[0][1], bl, bh, t2l, t2h, f);
+    Fadd<DIR>(t1l, t1h, t2l, t2h, sl, sh, f);
+    Fmul<DIR>(fl[0][2], fh[0][2], cl, ch, t3l, t3h, f);
+    Fadd<DIR>(sl, sh, t3l, t3h, jl, jh, f);
+    Fsub<DIR>(jl, jh, delta, delta, ml, mh, f);
+    ok = f.finite() && ml != 0.;
+    return ml;
+}
+
+// Bound: FP64 issue.  About 320 FP64 instructions per cell (9 hull entries of 20, 9 interval products of 12), against
+// about 1,900 instructions of the general form, most of them integer steps and NaN-rule selects.  160x192x224: 928 ->
+// 231 us per launch (directed 424 us before).
+template <bool DIR>
+__global__ void __launch_bounds__(256, 2) edge_hull_kernel(const double *__restrict__ u, const __grid_constant__ CellGrid g,
+                                                           double delta,
                                                         double *__restrict__ margin, uint8_t *__restrict__ flag) {
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.ncell;
          c += (long long)gridDim.x * blockDim.x) {
-        long long base = cell_base(c, g);
+        const long long base = cell_base(c, g);
         double v[8][3];
 #pragma unroll
         for (int a = 0; a < 8; a++)
 #pragma unroll
             for (int r = 0; r < 3; r++) v[a][r] = __ldg(u + 3 * vnode(base, a, g.ny, g.nx) + r);
-        double fl[3][3], fh[3][3];
-        bool ok = true;
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) ok &= hull_entry_v<DIR>(v, j, r, g.div, fl[r][j], fh[r][j]);
-        double jl, jh, ml, mh;
-        ok &= Idet<DIR>(fl, fh, jl, jh);
-        if constexpr (DIR) ok &= dsub(jl, jh, delta, delta, ml, mh);
-        else ok &= iout(rsub(jl, delta), rsub(jh, delta), ml, mh);
-        margin[c] = ml;
+        bool ok;
+        double m = hull_margin_finite<DIR>(v, g.div, delta, ok);
+        if (!ok) ok = hull_margin_general<DIR>(u, base, g, delta, &m);
+        margin[c] = m;
         flag[c] = ok ? 0 : 1;
     }
 }
@@ -216,6 +339,8 @@ __global__ void __launch_bounds__(256) edge_hull_kernel(const double *__restrict
 struct PrescreenConst {
     double D[3 * 27 * 8];  // closed27 Q1 derivative table (3, 27, 8), passed by value (constant bank)
     double g12, g6, g3, sq27, eta;
+    double ih[3];          // fl(1 / h_j)
+    int shared;            // 1: 1 / h_j between 2^-100 and 2^100 (the shared form's range)
     int usable;            // 0: table not finite or has a subnormal entry -> every bound NaN
     int sparse;            // 1: every structurally vanishing entry (table_nonzero false) is exactly zero
 };
@@ -384,25 +509,205 @@ __device__ double prescreen_cell_sparse(const double *__restrict__ u, long long 
     return finite ? rsub(low, bound) : __longlong_as_double(0x7FF8000000000000LL);
 }
 
+// The same bound with the products and partial sums that the points share formed once.  A table entry is
+// +-(1/h_j) times 1, 1/2 or 1/4, so for |u| between 2^-900 and 2^900 (or zero) and 1/h_j between 2^-100 and 2^100 no
+// term or sum under- or overflows, scaling by a power of two commutes with every rounding, and an 8-term sum in vertex
+// order is 1, 1/2 or 1/4 of the sum of t_a = u_a / h_j over its 2, 4 or 8 vertices, whose leading terms the sums of
+// neighbouring points have in common: 72 products and 171 additions replace 875 and 875.  The magnitude sums are
+// needed for their maximum alone: the 2-term sums bound the 4- and 8-term averages except for rounding, so the
+// latter matter only where two neighbouring 2-term sums reach the maximum's leading 20 bits.  The caller then takes
+// the full form, as it does where |u| is outside the range (false is returned).  Otherwise the same bits.
+struct ColumnSums {
+    double c[4], m[4], mid;   // corners (0,0) (1,0) (0,1) (1,1) of the two other axes, mids, centre; grad entries
+};
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+    return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+}
+__device__ __forceinline__ unsigned long long max64(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
+// The column sums of axis J for one component: m[0] (1/2, 0), m[1] (1/2, 1), m[2] (0, 1/2), m[3] (1, 1/2).
+template <int J>
+__device__ __forceinline__ void column_sums(const double (&t)[8], ColumnSums &s) {
+    constexpr int b = 1 << J, lo = J == 0 ? 2 : 1, hi = J == 2 ? 2 : 4;    // this axis's bit, the two others'
+    const double e0 = rsub(t[b], t[0]), e1 = rsub(t[b + lo], t[lo]), e2 = rsub(t[b + hi], t[hi]),
+                 e3 = rsub(t[b + lo + hi], t[lo + hi]);
+    s.c[0] = e0; s.c[1] = e1; s.c[2] = e2; s.c[3] = e3;
+    double c0, c1, c2, c3, all;
+    if constexpr (J == 0) {          // signs - + - + - + - +
+        c0 = radd(rsub(e0, t[2]), t[3]);
+        c1 = radd(rsub(e2, t[6]), t[7]);
+        c2 = radd(rsub(e0, t[4]), t[5]);
+        c3 = radd(rsub(e1, t[6]), t[7]);
+        all = radd(rsub(radd(rsub(c0, t[4]), t[5]), t[6]), t[7]);
+    } else if constexpr (J == 1) {   // signs - - + + - - + +
+        c0 = radd(radd(-radd(t[0], t[1]), t[2]), t[3]);
+        c1 = radd(radd(-radd(t[4], t[5]), t[6]), t[7]);
+        c2 = radd(rsub(e0, t[4]), t[6]);
+        c3 = radd(rsub(e1, t[5]), t[7]);
+        all = radd(radd(rsub(rsub(c0, t[4]), t[5]), t[6]), t[7]);
+    } else {                         // signs - - - - + + + +
+        const double n01 = -radd(t[0], t[1]);
+        c0 = radd(radd(n01, t[4]), t[5]);
+        c1 = radd(radd(-radd(t[2], t[3]), t[6]), t[7]);
+        c2 = radd(radd(-radd(t[0], t[2]), t[4]), t[6]);
+        c3 = radd(radd(-radd(t[1], t[3]), t[5]), t[7]);
+        all = radd(radd(radd(radd(rsub(rsub(n01, t[2]), t[3]), t[4]), t[5]), t[6]), t[7]);
+    }
+    s.m[0] = c0; s.m[1] = c1; s.m[2] = c2; s.m[3] = c3;
+    s.mid = all;
+}
+// the magnitude sums' corners: the largest, and the largest of the smaller leading words of neighbouring pairs
+template <int J>
+__device__ __forceinline__ void magnitude_corners(const double (&t)[8], unsigned long long &sigma, int &pairs) {
+    constexpr int b = 1 << J, lo = J == 0 ? 2 : 1, hi = J == 2 ? 2 : 4;
+    const double m0 = radd(fabs(t[0]), fabs(t[b])), m1 = radd(fabs(t[lo]), fabs(t[b + lo])),
+                 m2 = radd(fabs(t[hi]), fabs(t[b + hi])), m3 = radd(fabs(t[lo + hi]), fabs(t[b + lo + hi]));
+    sigma = max64(max64(sigma, max64(abs_bits(m0), abs_bits(m1))), max64(abs_bits(m2), abs_bits(m3)));
+    const int h0 = __double2hiint(m0), h1 = __double2hiint(m1), h2 = __double2hiint(m2), h3 = __double2hiint(m3);
+    pairs = max(pairs, max(max(min(h0, h1), min(h2, h3)), max(min(h0, h2), min(h1, h3))));
+}
+// values at the 3 x 3 points of the two other axes, P[high][low], from the sums; the diagonal entries get the identity
+template <bool ID>
+__device__ __forceinline__ void point_values(const ColumnSums &s, double (&P)[3][3]) {
+    auto one = [](double x) { return ID ? radd(x, 1.) : x; };
+    // x / 2 and x / 4 are exact, so the fused form rounds the sum with the identity once, as radd does
+    auto half = [](double x) { return ID ? __fma_rn(.5, x, 1.) : rmul(.5, x); };
+    P[0][0] = one(s.c[0]); P[0][2] = one(s.c[1]); P[2][0] = one(s.c[2]); P[2][2] = one(s.c[3]);
+    P[0][1] = half(s.m[0]); P[2][1] = half(s.m[1]); P[1][0] = half(s.m[2]); P[1][2] = half(s.m[3]);
+    P[1][1] = ID ? __fma_rn(.25, s.mid, 1.) : rmul(.25, s.mid);
+}
+template <int J, int R>
+__device__ __forceinline__ void column_table(const double (&uv)[8][3], double ih, double (&P)[3][3],
+                                             unsigned long long &sigma, unsigned long long &phi, int &pairs) {
+    double t[8];
+#pragma unroll
+    for (int a = 0; a < 8; a++) t[a] = rmul(uv[a][R], ih);
+    magnitude_corners<J>(t, sigma, pairs);
+    ColumnSums s;
+    column_sums<J>(t, s);
+    point_values<J == R>(s, P);
+#pragma unroll
+    for (int i = 0; i < 9; i++) phi = max64(phi, abs_bits(P[i / 3][i % 3]));
+}
+// bs: the thread's slice (stride T): 27 point values, then the x and y columns' 54
+constexpr int kPrescreenSlots = 81;
+__device__ bool prescreen_cell_shared(const double *__restrict__ u, long long base, long long ny, long long nx,
+                                      const PrescreenConst &k, double *bs, int T, double &bound_out) {
+    double uv[8][3];
+    int least = 0x7FFFFFFF, most = 0;
+#pragma unroll
+    for (int a = 0; a < 8; a++) {
+        const long long off = (long long)(a >> 2) * ny * nx + (long long)((a >> 1) & 1) * nx + (a & 1);
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            uv[a][r] = __ldg(u + 3 * (base + off) + r);
+            const int h = __double2hiint(uv[a][r]) & 0x7FFFFFFF;
+            least = min(least, uv[a][r] == 0. ? 0x7FFFFFFF : h);
+            most = max(most, h);
+        }
+    }
+    if (least < ((1023 - 900) << 20) || most >= ((1023 + 900) << 20)) return false;
+    unsigned long long sigma = 0, phi = 0, big = 0;
+    int pairs = 0;
+    double *X = bs + 27 * T, *Y = bs + 54 * T;     // X[(iz, iy)][r], Y[(iz, ix)][r]
+    double Z[3][3][3];                             // [r][iy][ix]
+    {
+        double P[3][3];
+#define SVP_STORE_TABLE(TAB, R)                                                              \
+    _Pragma("unroll") for (int i = 0; i < 9; i++) TAB[(3 * i + R) * T] = P[i / 3][i % 3];
+        column_table<0, 0>(uv, k.ih[0], P, sigma, phi, pairs); SVP_STORE_TABLE(X, 0)
+        column_table<0, 1>(uv, k.ih[0], P, sigma, phi, pairs); SVP_STORE_TABLE(X, 1)
+        column_table<0, 2>(uv, k.ih[0], P, sigma, phi, pairs); SVP_STORE_TABLE(X, 2)
+        column_table<1, 0>(uv, k.ih[1], P, sigma, phi, pairs); SVP_STORE_TABLE(Y, 0)
+        column_table<1, 1>(uv, k.ih[1], P, sigma, phi, pairs); SVP_STORE_TABLE(Y, 1)
+        column_table<1, 2>(uv, k.ih[1], P, sigma, phi, pairs); SVP_STORE_TABLE(Y, 2)
+#undef SVP_STORE_TABLE
+        column_table<2, 0>(uv, k.ih[2], Z[0], sigma, phi, pairs);
+        column_table<2, 1>(uv, k.ih[2], Z[1], sigma, phi, pairs);
+        column_table<2, 2>(uv, k.ih[2], Z[2], sigma, phi, pairs);
+    }
+    if (pairs >= (int)(sigma >> 32) - 1) return false;
+    double b[27];
+#pragma unroll
+    for (int iz = 0; iz < 3; iz++) {
+        double Yp[3][3];
+#pragma unroll
+        for (int i = 0; i < 9; i++) Yp[i / 3][i % 3] = Y[(9 * iz + i) * T];
+#pragma unroll
+        for (int iy = 0; iy < 3; iy++) {
+            const double x0 = X[(9 * iz + 3 * iy) * T], x1 = X[(9 * iz + 3 * iy + 1) * T],
+                         x2 = X[(9 * iz + 3 * iy + 2) * T];
+#pragma unroll
+            for (int ix = 0; ix < 3; ix++) {
+                const double y0 = Yp[ix][0], y1 = Yp[ix][1], y2 = Yp[ix][2];
+                const double z0 = Z[0][iy][ix], z1 = Z[1][iy][ix], z2 = Z[2][iy][ix];
+                const double t0 = rmul(x0, rsub(rmul(y1, z2), rmul(z1, y2)));
+                const double t1 = rmul(y0, rsub(rmul(z1, x2), rmul(x1, z2)));
+                const double t2 = rmul(z0, rsub(rmul(x1, y2), rmul(y1, x2)));
+                const double v = radd(radd(t0, t1), t2);
+                b[9 * iz + 3 * iy + ix] = v;
+                big = max64(big, abs_bits(v));
+            }
+        }
+    }
+    // the middle entry of each line -> 2 b_m - (b_l + b_r) / 2: both products exact, one rounding either way
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+        const int stride = s == 0 ? 1 : (s == 1 ? 3 : 9);
+#pragma unroll
+        for (int p = 0; p < 27; p++)
+            if ((p / stride) % 3 == 1) b[p] = rsub(rmul(2., b[p]), rmul(.5, radd(b[p - stride], b[p + stride])));
+    }
+    const double sg = __longlong_as_double((long long)sigma), ph = __longlong_as_double((long long)phi),
+                 bg = __longlong_as_double((long long)big);
+    double e = radd(rmul(k.g12, radd(sg, ph)), k.eta);
+    double P = radd(ph, e);
+    double inner = radd(radd(rmul(rmul(3., P), P), rmul(rmul(3., P), e)), rmul(e, e));
+    double ej = radd(rmul(rmul(k.sq27, e), inner), rmul(rmul(rmul(rmul(6., k.g6), P), P), P));
+    double bound = radd(rmul(1.01, radd(rmul(27., ej), rmul(rmul(135., k.g3), bg))), k.eta);
+    double low = b[0];
+    int top = __double2hiint(bound) & 0x7FFFFFFF;
+#pragma unroll
+    for (int p = 0; p < 27; p++) {
+        top = max(top, __double2hiint(b[p]) & 0x7FFFFFFF);
+        if (p) low = b[p] < low ? b[p] : low;
+    }
+    bound_out = top < 0x7FF00000 ? rsub(low, bound) : __longlong_as_double(0x7FF8000000000000LL);
+    return true;
+}
+__device__ __noinline__ double prescreen_cell_full(const double *__restrict__ u, long long base, long long ny,
+                                                   long long nx, const PrescreenConst &k, double *bs, int T) {
+    return prescreen_cell_sparse(u, base, ny, nx, k, bs, T);
+}
+
+// Bound: FP64 issue (about 950 FP64 instructions per cell in the shared form, 2,900 in the full one).  2.37 M cells of
+// 160x192x224: 880 -> 265 us per launch.
+constexpr int PT = 64;      // threads per block
 template <bool SPARSE>
-__global__ void __launch_bounds__(128) prescreen_kernel(const double *__restrict__ u, CellGrid g,
-                                                        const long long *__restrict__ cells, long long n,
-                                                        const PrescreenConst k, double *__restrict__ out) {
-    __shared__ double slice[27 * 128];
+__global__ void __launch_bounds__(PT) prescreen_kernel(const double *__restrict__ u, CellGrid g,
+                                                       const long long *__restrict__ cells, long long n,
+                                                       const __grid_constant__ PrescreenConst k,
+                                                       double *__restrict__ out) {
+    extern __shared__ double slice[];
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
         const long long base = cell_base(cells[i], g);
-        out[i] = !k.usable ? __longlong_as_double(0x7FF8000000000000LL)
-                 : SPARSE  ? prescreen_cell_sparse(u, base, g.ny, g.nx, k, slice + threadIdx.x, blockDim.x)
-                           : prescreen_cell(u, base, g.ny, g.nx, k);
+        double *bs = slice + threadIdx.x;
+        double low;
+        if (!k.usable) low = __longlong_as_double(0x7FF8000000000000LL);
+        else if (!SPARSE) low = prescreen_cell(u, base, g.ny, g.nx, k);
+        else if (!k.shared || !prescreen_cell_shared(u, base, g.ny, g.nx, k, bs, PT, low))
+            low = prescreen_cell_full(u, base, g.ny, g.nx, k, bs, PT);
+        out[i] = low;
     }
 }
-void launch_prescreen(const double *u, const CellGrid &g, const long long *cells, long long n,
-                      const PrescreenConst &k, double *out, cudaStream_t s) {
+int launch_prescreen(const double *u, const CellGrid &g, const long long *cells, long long n,
+                     const PrescreenConst &k, double *out, cudaStream_t s) {
+    constexpr int slots = sizeof(double) * kPrescreenSlots * PT;
     if (k.sparse)
-        prescreen_kernel<true><<<blocks_for(n, 128, 8), 128, 0, s>>>(u, g, cells, n, k, out);
+        SVP_LAUNCH(prescreen_kernel<true><<<blocks_for(n, PT, 16), PT, slots, s>>>(u, g, cells, n, k, out));
     else
-        prescreen_kernel<false><<<blocks_for(n, 128, 8), 128, 0, s>>>(u, g, cells, n, k, out);
+        SVP_LAUNCH(prescreen_kernel<false><<<blocks_for(n, PT, 16), PT, 0, s>>>(u, g, cells, n, k, out));
+    return SVP_OK;
 }
 
 // ============================================================================================== 3a. fallback arrays
@@ -1044,6 +1349,11 @@ PrescreenConst prescreen_const(const double h[3]) {
     k.g12 = gamma(12); k.g6 = gamma(6); k.g3 = gamma(3);
     k.sq27 = 5.196152422706633;
     k.eta = 1e-290;
+    k.shared = 1;
+    for (int j = 0; j < 3; j++) {
+        k.ih[j] = 1. / h[j];
+        if (!(k.ih[j] > 0x1p-100 && k.ih[j] < 0x1p100)) k.shared = 0;
+    }
     k.usable = 1;
     k.sparse = 1;
     for (int i = 0; i < 3 * 27 * 8; i++) {
@@ -1086,9 +1396,7 @@ extern "C" int svp_prescreen_lower_bounds(const svp_grid *g, const double *u, co
     SVP_REQUIRE(u && cells && out, "svp_prescreen_lower_bounds: null pointer");
     CellGrid cg = cell_grid(g);
     PrescreenConst k = prescreen_const(cg.h);
-    { svp::KernelTimer _t("prescreen_kernel", (cudaStream_t)stream); SVP_LAUNCH(launch_prescreen(u, cg, (const long long *)cells, n, k, out, (cudaStream_t)stream)); }
-    SVP_LAUNCH_CHECK("prescreen_kernel");
-    return SVP_OK;
+    { svp::KernelTimer _t("prescreen_kernel", (cudaStream_t)stream); return launch_prescreen(u, cg, (const long long *)cells, n, k, out, (cudaStream_t)stream); }
 }
 
 static int fallback_arrays(const double *vertices, int64_t n, const double *spacing3, double delta, double *p_lo,
@@ -1409,8 +1717,9 @@ extern "C" int svp_certify_map(svp_certifier *c, const double *u, svp_cert_resul
     const long long *list2 = c->list1;
     const bool staged = n1 != 0;   // a later stage updates acc; with no flagged cell the copy above is final
     if (c->cfg.prescreen && n1) {
-        { svp::KernelTimer _t("prescreen_kernel", s); SVP_LAUNCH(launch_prescreen(u, c->cg, c->list1, n1, c->pk, c->lower, s)); }
-        SVP_LAUNCH_CHECK("prescreen_kernel");
+        int rc1;
+        { svp::KernelTimer _t("prescreen_kernel", s); rc1 = launch_prescreen(u, c->cg, c->list1, n1, c->pk, c->lower, s); }
+        if (rc1) return rc1;
         SVP_LAUNCH(prescreen_stage_kernel<<<blocks_for(n1, 256, 8), 256, 0, s>>>(c->lower, n1, delta, c->sel, c->acc));
         SVP_LAUNCH_CHECK("prescreen stage");
         rc = select_flagged<true>(c, c->list1, c->sel, c->list2, c->counts + 1, n1, s);
