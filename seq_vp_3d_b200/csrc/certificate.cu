@@ -683,22 +683,25 @@ __device__ __noinline__ double prescreen_cell_full(const double *__restrict__ u,
 // 160x192x224: 880 -> 265 us per launch.
 constexpr int PT = 64;      // threads per block
 template <bool SPARSE>
-__global__ void __launch_bounds__(PT) prescreen_kernel(const double *__restrict__ u, CellGrid g,
+__device__ __forceinline__ double prescreen_bound(const double *__restrict__ u, const CellGrid &g, long long c,
+                                                  const PrescreenConst &k, double *bs) {
+    if (!k.usable) return __longlong_as_double(0x7FF8000000000000LL);
+    const long long base = cell_base(c, g);
+    double low;
+    if (!SPARSE) return prescreen_cell(u, base, g.ny, g.nx, k);
+    if (k.shared && prescreen_cell_shared(u, base, g.ny, g.nx, k, bs, PT, low)) return low;
+    return prescreen_cell_full(u, base, g.ny, g.nx, k, bs, PT);
+}
+template <bool SPARSE>
+__global__ void __launch_bounds__(PT) prescreen_kernel(const double *__restrict__ u,
+                                                       const __grid_constant__ CellGrid g,
                                                        const long long *__restrict__ cells, long long n,
                                                        const __grid_constant__ PrescreenConst k,
                                                        double *__restrict__ out) {
     extern __shared__ double slice[];
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        const long long base = cell_base(cells[i], g);
-        double *bs = slice + threadIdx.x;
-        double low;
-        if (!k.usable) low = __longlong_as_double(0x7FF8000000000000LL);
-        else if (!SPARSE) low = prescreen_cell(u, base, g.ny, g.nx, k);
-        else if (!k.shared || !prescreen_cell_shared(u, base, g.ny, g.nx, k, bs, PT, low))
-            low = prescreen_cell_full(u, base, g.ny, g.nx, k, bs, PT);
-        out[i] = low;
-    }
+         i += (long long)gridDim.x * blockDim.x)
+        out[i] = prescreen_bound<SPARSE>(u, g, cells[i], k, slice + threadIdx.x);
 }
 int launch_prescreen(const double *u, const CellGrid &g, const long long *cells, long long n,
                      const PrescreenConst &k, double *out, cudaStream_t s) {
@@ -1133,46 +1136,56 @@ struct Accum {
     unsigned long long nonfinite, boundary, invalid;   // pre-checks (nodes)
     unsigned long long fast, prescreened, unknown, bad, boxes_extra, fallback_ok_cells;
     long long lowest_key, sampled_key, max_depth, witness_cell;
-    int any_margin, arith, has_witness, pad;
+    int any_margin, arith, has_witness, flagged;       // flagged: some hull enclosure was not finite
+    unsigned long long list1, list2;                   // entries of the hull's and the prescreen's lists
     double witness[3];
 };
 
-// Sampling-domain and boundary checks per node (interpolation.py:43 check_map_domain, validation zero_boundary).
+// Sampling-domain and boundary checks of a node (interpolation.py:43 check_map_domain, validation zero_boundary).
+struct NodeChecks {
+    unsigned nonfinite = 0, boundary = 0, invalid = 0;
+    __device__ __forceinline__ void see(const double (&q)[3], long long x, long long y, long long z,
+                                        const CellGrid &g, const double (&org)[3]) {
+        const long long idx[3] = {x, y, z}, len[3] = {g.nx, g.ny, g.nz};
+        const bool face = z == 0 || z == g.nz - 1 || y == 0 || y == g.ny - 1 || x == 0 || x == g.nx - 1;
+        bool bad = false;
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const double lo = org[j], hi = radd(org[j], rmul(g.h[j], (double)(len[j] - 1)));
+            const double value = radd(q[j], radd(org[j], rmul(g.h[j], (double)idx[j])));
+            if (!finite64(value) || value < lo || value > hi) bad = true;
+            if (!face && (value <= lo || value >= hi)) bad = true;
+        }
+        nonfinite += !(finite64(q[0]) && finite64(q[1]) && finite64(q[2]));
+        boundary += face && (q[0] != 0 || q[1] != 0 || q[2] != 0);
+        invalid += bad;
+    }
+    __device__ __forceinline__ void add_to(Accum *acc) {
+        for (int o = 16; o; o >>= 1) {
+            nonfinite += __shfl_xor_sync(0xFFFFFFFFu, nonfinite, o);
+            boundary += __shfl_xor_sync(0xFFFFFFFFu, boundary, o);
+            invalid += __shfl_xor_sync(0xFFFFFFFFu, invalid, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            if (nonfinite) atomicAdd(&acc->nonfinite, (unsigned long long)nonfinite);
+            if (boundary) atomicAdd(&acc->boundary, (unsigned long long)boundary);
+            if (invalid) atomicAdd(&acc->invalid, (unsigned long long)invalid);
+        }
+    }
+};
 __global__ void precheck_kernel(const double *__restrict__ u, CellGrid g, double x0, double y0, double z0,
                                 Accum *acc) {
-    unsigned long long nf = 0, nb = 0, ni = 0;
-    long long nn = g.nx * g.ny * g.nz;
+    NodeChecks checks;
+    const long long nn = g.nx * g.ny * g.nz;
     const double org[3] = {x0, y0, z0};
-    const long long len[3] = {g.nx, g.ny, g.nz};
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nn;
          i += (long long)gridDim.x * blockDim.x) {
-        long long x = i % g.nx, y = (i / g.nx) % g.ny, z = i / (g.nx * g.ny);
-        long long idx[3] = {x, y, z};
-        double q[3] = {u[3 * i], u[3 * i + 1], u[3 * i + 2]};
-        bool nonfin = !(finite64(q[0]) && finite64(q[1]) && finite64(q[2]));
-        bool face = z == 0 || z == g.nz - 1 || y == 0 || y == g.ny - 1 || x == 0 || x == g.nx - 1;
-        bool interior = !face;
-        bool bad = false;
-        for (int j = 0; j < 3; j++) {
-            double lo = org[j], hi = radd(org[j], rmul(g.h[j], (double)(len[j] - 1)));
-            double value = radd(q[j], radd(org[j], rmul(g.h[j], (double)idx[j])));
-            if (!finite64(value) || value < lo || value > hi) bad = true;
-            if (interior && (value <= lo || value >= hi)) bad = true;
-        }
-        nf += nonfin;
-        nb += face && (q[0] != 0 || q[1] != 0 || q[2] != 0);
-        ni += bad;
+        long long x, y, z;
+        unflatten3(i, g.nx, g.ny, x, y, z);
+        const double q[3] = {u[3 * i], u[3 * i + 1], u[3 * i + 2]};
+        checks.see(q, x, y, z, g, org);
     }
-    for (int o = 16; o; o >>= 1) {
-        nf += __shfl_xor_sync(0xFFFFFFFFu, nf, o);
-        nb += __shfl_xor_sync(0xFFFFFFFFu, nb, o);
-        ni += __shfl_xor_sync(0xFFFFFFFFu, ni, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (nf) atomicAdd(&acc->nonfinite, nf);
-        if (nb) atomicAdd(&acc->boundary, nb);
-        if (ni) atomicAdd(&acc->invalid, ni);
-    }
+    checks.add_to(acc);
 }
 
 __global__ void tile_flag_kernel(const uint8_t *__restrict__ flag, long long ncell, long long tile,
@@ -1187,6 +1200,107 @@ __device__ __forceinline__ void warp_min_key(long long &k) {
         long long y = __shfl_xor_sync(0xFFFFFFFFu, k, o);
         k = y < k ? y : k;
     }
+}
+
+// Appends cells to a list in global memory through the warp's shared buffer: a full buffer costs one atomic, so the
+// counter's address is touched once per kListBuffer - 32 entries.  The order of the list is the order of arrival; each
+// listed cell is then evaluated by itself and the record takes sums, minima and the lowest witness.
+constexpr int kListBuffer = 256;
+struct WarpList {
+    long long *buffer, *out;
+    unsigned long long *count;
+    int n = 0;
+    __device__ WarpList(long long *b, long long *o, unsigned long long *c) : buffer(b), out(o), count(c) {}
+    __device__ __forceinline__ void flush() {
+        const int lane = threadIdx.x & 31;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(count, (unsigned long long)n);
+        at = __shfl_sync(0xFFFFFFFFu, at, 0);
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) out[at + i] = buffer[i];
+        __syncwarp();
+        n = 0;
+    }
+    __device__ __forceinline__ void push(bool on, long long c) {     // all lanes of the warp
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, on);
+        if (on) buffer[n + __popc(m & ((1u << (threadIdx.x & 31)) - 1u))] = c;
+        n += __popc(m);
+        if (n > kListBuffer - 32) flush();
+    }
+    __device__ __forceinline__ void finish() {
+        if (n) flush();
+    }
+};
+// count and lowest margin of the cells a stage proves
+struct Proven {
+    unsigned n = 0;
+    long long key = kKeyPosInf;
+    __device__ __forceinline__ void see(double margin) {
+        n++;
+        const long long k = order_key(margin);
+        key = k < key ? k : key;
+    }
+    __device__ __forceinline__ void add_to(Accum *acc, unsigned long long *count) {
+        for (int o = 16; o; o >>= 1) n += __shfl_xor_sync(0xFFFFFFFFu, n, o);
+        warp_min_key(key);
+        if ((threadIdx.x & 31) == 0 && n) {
+            atomicAdd(count, (unsigned long long)n);
+            atomicMin(&acc->lowest_key, key);
+            acc->any_margin = 1;
+        }
+    }
+};
+
+// The first stage of certify_map in one pass over the cells: the node checks (a cell checks its lower corner, the last
+// cell of an axis its upper one too), the edge-hull margin, the proven cells' count and lowest margin, and the list of
+// the others.  acc->flagged where some enclosure was not finite: the tile rule then needs every margin, and the host
+// takes the staged form (margins, tile flags, selection) instead.
+// Bound: FP64 issue (edge_hull_kernel's, plus 25 for the checks); 24 B/node read, 8 B per listed cell written.  The
+// staged form took five kernels here and read the field twice and margins, flags and selection once more:
+// 160x192x224 404 us of kernels against 317 us, 32^3 19 us in eleven launches and
+// copies against 8 us.
+template <bool DIR>
+__global__ void __launch_bounds__(256, 2) hull_list_kernel(const double *__restrict__ u,
+                                                           const __grid_constant__ CellGrid g, double x0, double y0,
+                                                           double z0, double delta, long long *__restrict__ list,
+                                                           Accum *acc) {
+    __shared__ long long buffer[8][kListBuffer];
+    const double org[3] = {x0, y0, z0};
+    NodeChecks checks;
+    Proven proven;
+    WarpList todo(buffer[threadIdx.x >> 5], list, &acc->list1);
+    bool flagged = false;
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (long long w = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); w < g.ncell; w += step) {
+        const long long c = w + (threadIdx.x & 31);
+        bool unproven = false;
+        if (c < g.ncell) {
+            long long x, y, z;
+            unflatten3(c, g.cx, g.cy, x, y, z);
+            const long long base = (z * g.ny + y) * g.nx + x;
+            double v[8][3];
+#pragma unroll
+            for (int a = 0; a < 8; a++)
+#pragma unroll
+                for (int r = 0; r < 3; r++) v[a][r] = __ldg(u + 3 * vnode(base, a, g.ny, g.nx) + r);
+            const bool last[3] = {x == g.cx - 1, y == g.cy - 1, z == g.cz - 1};
+#pragma unroll
+            for (int a = 0; a < 8; a++)
+                if ((!(a & 1) || last[0]) && (!(a & 2) || last[1]) && (!(a & 4) || last[2]))
+                    checks.see(v[a], x + (a & 1), y + ((a >> 1) & 1), z + (a >> 2), g, org);
+            bool ok;
+            double m = hull_margin_finite<DIR>(v, g.div, delta, ok);
+            if (!ok) ok = hull_margin_general<DIR>(u, base, g, delta, &m);
+            flagged |= !ok;
+            unproven = !(m > 0);
+            if (!unproven) proven.see(m);
+        }
+        todo.push(unproven, c);
+    }
+    todo.finish();
+    checks.add_to(acc);
+    proven.add_to(acc, &acc->fast);
+    if (flagged) acc->flagged = 1;
 }
 
 // hull-proven cells: margin > 0 in an unflagged tile; sel[c] = 1 marks the rest (prescreen/fallback candidates)
@@ -1238,6 +1352,46 @@ __global__ void prescreen_stage_kernel(const double *__restrict__ lower, long lo
         atomicMin(&acc->lowest_key, key);
         acc->any_margin = 1;
     }
+}
+
+// The prescreen of the hull's list with its decision: proven cells counted, the others listed.  Runs behind
+// hull_list_kernel without the host knowing the list's length.
+template <bool SPARSE>
+__global__ void __launch_bounds__(PT) prescreen_list_kernel(const double *__restrict__ u,
+                                                            const __grid_constant__ CellGrid g,
+                                                            const long long *__restrict__ cells,
+                                                            const __grid_constant__ PrescreenConst k, double delta,
+                                                            long long *__restrict__ list, Accum *acc) {
+    extern __shared__ double slice[];
+    __shared__ long long buffer[PT / 32][kListBuffer];
+    const long long n = (long long)acc->list1, step = (long long)gridDim.x * blockDim.x;
+    Proven proven;
+    WarpList todo(buffer[threadIdx.x >> 5], list, &acc->list2);
+    for (long long w = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); w < n; w += step) {
+        const long long i = w + (threadIdx.x & 31);
+        bool unproven = false;
+        long long c = 0;
+        if (i < n) {
+            c = cells[i];
+            const double low = prescreen_bound<SPARSE>(u, g, c, k, slice + threadIdx.x);
+            const double m = delta == 0. ? low : step_down(rsub(low, delta));
+            unproven = !(m > 0);
+            if (!unproven) proven.see(m);
+        }
+        todo.push(unproven, c);
+    }
+    todo.finish();
+    proven.add_to(acc, &acc->prescreened);
+}
+int launch_prescreen_list(const double *u, const CellGrid &g, const long long *cells, const PrescreenConst &k,
+                          double delta, long long *list, Accum *acc, cudaStream_t s) {
+    constexpr int slots = sizeof(double) * kPrescreenSlots * PT;
+    const unsigned nb = blocks_for(g.ncell, PT, 8);
+    if (k.sparse)
+        SVP_LAUNCH(prescreen_list_kernel<true><<<nb, PT, slots, s>>>(u, g, cells, k, delta, list, acc));
+    else
+        SVP_LAUNCH(prescreen_list_kernel<false><<<nb, PT, 0, s>>>(u, g, cells, k, delta, list, acc));
+    return SVP_OK;
 }
 
 __global__ void job_fail_kernel(const long long *__restrict__ cells, const uint8_t *__restrict__ ok, long long n,
@@ -1495,7 +1649,7 @@ struct svp_certifier {
     uint8_t *flag = nullptr, *sel = nullptr;
     int *tile_bad = nullptr, *tile_fail = nullptr;
     long long *list1 = nullptr, *list2 = nullptr, *list3 = nullptr, *counts = nullptr;
-    svp::Accum *acc = nullptr;
+    svp::Accum *acc = nullptr, *host = nullptr;   // device counts, pinned host copy
     long long *sel_cnt = nullptr;    // per-block flag counts of the stage-list compaction
     size_t sel_bytes = 0;
     // fallback workspace (grows on demand)
@@ -1602,6 +1756,21 @@ int select_flagged(svp_certifier *c, const long long *list, const uint8_t *flags
     return SVP_OK;
 }
 
+// The counts on the host, through the handle's pinned buffer (a copy to pageable memory is staged by the driver).
+int read_accum(svp_certifier *c, Accum *acc, cudaStream_t s) {
+    SVP_CUDA(cudaMemcpyAsync(c->host, c->acc, sizeof(Accum), cudaMemcpyDeviceToHost, s));
+    SVP_CUDA(cudaStreamSynchronize(s));
+    *acc = *c->host;
+    return SVP_OK;
+}
+// The staged form's per-cell arrays, allocated when it is first taken.
+int ensure_staged(svp_certifier *c) {
+    if (!c->margin) SVP_CUDA(cudaMalloc((void **)&c->margin, sizeof(double) * c->ncell));
+    if (!c->lower) SVP_CUDA(cudaMalloc((void **)&c->lower, sizeof(double) * c->ncell));
+    if (!c->flag) SVP_CUDA(cudaMalloc((void **)&c->flag, c->ncell));
+    return SVP_OK;
+}
+
 }  // namespace
 }  // namespace svp
 
@@ -1631,9 +1800,6 @@ extern "C" int svp_certifier_create(const svp_grid *g, const svp_cert_config *cf
         return cuda_fail(e, what);
     };
     cudaError_t e;
-    if ((e = cudaMalloc((void **)&c->margin, sizeof(double) * c->ncell)) != cudaSuccess) return bail(e, "margin");
-    if ((e = cudaMalloc((void **)&c->lower, sizeof(double) * c->ncell)) != cudaSuccess) return bail(e, "lower");
-    if ((e = cudaMalloc((void **)&c->flag, c->ncell)) != cudaSuccess) return bail(e, "flag");
     if ((e = cudaMalloc((void **)&c->sel, c->ncell)) != cudaSuccess) return bail(e, "sel");
     if ((e = cudaMalloc((void **)&c->tile_bad, sizeof(int) * c->ntiles)) != cudaSuccess) return bail(e, "tiles");
     if ((e = cudaMalloc((void **)&c->tile_fail, sizeof(int) * c->ntiles)) != cudaSuccess) return bail(e, "tiles");
@@ -1642,6 +1808,7 @@ extern "C" int svp_certifier_create(const svp_grid *g, const svp_cert_config *cf
     if ((e = cudaMalloc((void **)&c->list3, sizeof(long long) * c->ncell)) != cudaSuccess) return bail(e, "list3");
     if ((e = cudaMalloc((void **)&c->counts, sizeof(long long) * 4)) != cudaSuccess) return bail(e, "counts");
     if ((e = cudaMalloc((void **)&c->acc, sizeof(Accum))) != cudaSuccess) return bail(e, "accum");
+    if ((e = cudaMallocHost((void **)&c->host, sizeof(Accum))) != cudaSuccess) return bail(e, "accum host");
     c->heap_slots = cfg->max_boxes + 2;
     c->heap_warps = (long long)kSMs * 8;
     if ((e = cudaMalloc((void **)&c->heap, warp_scratch_bytes(c->heap_slots) * c->heap_warps)) != cudaSuccess)
@@ -1654,7 +1821,7 @@ extern "C" int svp_certifier_destroy(svp_certifier *c) {
     if (!c) return SVP_OK;
     cudaFree(c->margin); cudaFree(c->lower); cudaFree(c->flag); cudaFree(c->sel);
     cudaFree(c->tile_bad); cudaFree(c->tile_fail); cudaFree(c->list1); cudaFree(c->list2); cudaFree(c->list3);
-    cudaFree(c->counts); cudaFree(c->acc); cudaFree(c->sel_cnt); cudaFree(c->fb); cudaFree(c->fb_ok);
+    cudaFree(c->counts); cudaFree(c->acc); cudaFreeHost(c->host); cudaFree(c->sel_cnt); cudaFree(c->fb); cudaFree(c->fb_ok);
     cudaFree(c->verdicts); cudaFree(c->heap);
     delete c;
     return SVP_OK;
@@ -1678,58 +1845,81 @@ extern "C" int svp_certify_map(svp_certifier *c, const double *u, svp_cert_resul
     out->min_jd_lower_bound = out->min_margin_lower_bound = out->sampled_min_jd = nan;
     out->witness_point[0] = out->witness_point[1] = out->witness_point[2] = nan;
 
-    SVP_LAUNCH(accum_init_kernel<<<1, 1, 0, s>>>(c->acc));
-    { svp::KernelTimer _t("precheck_kernel", s); SVP_LAUNCH(precheck_kernel<<<blocks_for(n_nodes(&c->grid), 256, 8), 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0,
-                                                                            c->grid.z0, c->acc)); }
-    SVP_LAUNCH_CHECK("precheck_kernel");
-    SVP_CUDA(cudaMemsetAsync(c->tile_fail, 0, sizeof(int) * c->ntiles, s));
+    Accum acc;
+    long long n2 = 0;
+    const long long *list2 = nullptr;
+    int rc = SVP_OK;
+    bool staged = !hull;
     if (hull) {
+        SVP_LAUNCH(accum_init_kernel<<<1, 1, 0, s>>>(c->acc));
         {
             svp::KernelTimer _t("edge_hull_kernel", s);
+            const unsigned nb = blocks_for(n, 256, 8);
+            if (directed)
+                SVP_LAUNCH(hull_list_kernel<true><<<nb, 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0, c->grid.z0, delta,
+                                                                   c->list1, c->acc));
+            else
+                SVP_LAUNCH(hull_list_kernel<false><<<nb, 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0, c->grid.z0,
+                                                                    delta, c->list1, c->acc));
+        }
+        if (c->cfg.prescreen) {
+            svp::KernelTimer _t("prescreen_kernel", s);
+            if ((rc = launch_prescreen_list(u, c->cg, c->list1, c->pk, delta, c->list2, c->acc, s))) return rc;
+        }
+        if ((rc = read_accum(c, &acc, s))) return rc;
+    } else {
+        SVP_LAUNCH(accum_init_kernel<<<1, 1, 0, s>>>(c->acc));
+        SVP_LAUNCH(precheck_kernel<<<blocks_for(n_nodes(&c->grid), 256, 8), 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0,
+                                                                                      c->grid.z0, c->acc));
+        if ((rc = read_accum(c, &acc, s))) return rc;
+    }
+    // early returns, in certify_map's order (feasibility.py:412-428)
+    if (acc.nonfinite) { out->reason = R_NONFINITE; return SVP_OK; }
+    if (acc.boundary) { out->status = ST_INFEASIBLE; out->reason = R_BOUNDARY; return SVP_OK; }
+    if (acc.invalid) { out->status = ST_INFEASIBLE; out->reason = R_DOMAIN; return SVP_OK; }
+    if (hull && !acc.flagged) {
+        n2 = (long long)(c->cfg.prescreen ? acc.list2 : acc.list1);
+        list2 = c->cfg.prescreen ? c->list2 : c->list1;
+    } else {
+        // The staged form: without the preproof (feasibility.py:447-491) every cell goes to the fallback; with it and
+        // an enclosure that was not finite, every cell of that enclosure's tile does (feasibility.py:650).
+        staged = true;
+        SVP_LAUNCH(accum_init_kernel<<<1, 1, 0, s>>>(c->acc));
+        if ((rc = ensure_staged(c))) return rc;
+        SVP_CUDA(cudaMemsetAsync(c->tile_bad, hull ? 0 : 1, sizeof(int) * c->ntiles, s));
+        if (hull) {
             if (directed)
                 SVP_LAUNCH(edge_hull_kernel<true><<<blocks_for(n, 256, 8), 256, 0, s>>>(u, c->cg, delta, c->margin,
                                                                                       c->flag));
             else
                 SVP_LAUNCH(edge_hull_kernel<false><<<blocks_for(n, 256, 8), 256, 0, s>>>(u, c->cg, delta, c->margin,
                                                                                        c->flag));
+            SVP_LAUNCH(tile_flag_kernel<<<blocks_for(n, 256, 8), 256, 0, s>>>(c->flag, n, tile, c->tile_bad));
         }
-        SVP_LAUNCH_CHECK("edge_hull_kernel");
-        SVP_CUDA(cudaMemsetAsync(c->tile_bad, 0, sizeof(int) * c->ntiles, s));
-        SVP_LAUNCH(tile_flag_kernel<<<blocks_for(n, 256, 8), 256, 0, s>>>(c->flag, n, tile, c->tile_bad));
-    } else {
-        // the whole-cell Bernstein execution (feasibility.py:447-491): no preproof, every cell to the fallback
-        SVP_CUDA(cudaMemsetAsync(c->tile_bad, 1, sizeof(int) * c->ntiles, s));
-    }
-    SVP_LAUNCH(hull_stage_kernel<<<blocks_for(n, 256, 8), 256, 0, s>>>(c->margin, c->tile_bad, n, tile, c->sel, c->acc));
-    SVP_LAUNCH_CHECK("hull stage");
-    int rc = select_flagged<false>(c, nullptr, c->sel, c->list1, c->counts, n, s);
-    if (rc) return rc;
-    Accum acc;
-    long long counts[4];
-    SVP_CUDA(cudaMemcpyAsync(&acc, c->acc, sizeof acc, cudaMemcpyDeviceToHost, s));
-    SVP_CUDA(cudaMemcpyAsync(counts, c->counts, sizeof(long long), cudaMemcpyDeviceToHost, s));
-    SVP_CUDA(cudaStreamSynchronize(s));
-    // early returns, in certify_map's order (feasibility.py:412-428)
-    if (acc.nonfinite) { out->reason = R_NONFINITE; return SVP_OK; }
-    if (acc.boundary) { out->status = ST_INFEASIBLE; out->reason = R_BOUNDARY; return SVP_OK; }
-    if (acc.invalid) { out->status = ST_INFEASIBLE; out->reason = R_DOMAIN; return SVP_OK; }
-    long long n1 = counts[0], n2 = n1;
-    const long long *list2 = c->list1;
-    const bool staged = n1 != 0;   // a later stage updates acc; with no flagged cell the copy above is final
-    if (c->cfg.prescreen && n1) {
-        int rc1;
-        { svp::KernelTimer _t("prescreen_kernel", s); rc1 = launch_prescreen(u, c->cg, c->list1, n1, c->pk, c->lower, s); }
-        if (rc1) return rc1;
-        SVP_LAUNCH(prescreen_stage_kernel<<<blocks_for(n1, 256, 8), 256, 0, s>>>(c->lower, n1, delta, c->sel, c->acc));
-        SVP_LAUNCH_CHECK("prescreen stage");
-        rc = select_flagged<true>(c, c->list1, c->sel, c->list2, c->counts + 1, n1, s);
-        if (rc) return rc;
-        SVP_CUDA(cudaMemcpyAsync(&n2, c->counts + 1, sizeof(long long), cudaMemcpyDeviceToHost, s));
+        SVP_LAUNCH(hull_stage_kernel<<<blocks_for(n, 256, 8), 256, 0, s>>>(c->margin, c->tile_bad, n, tile, c->sel,
+                                                                         c->acc));
+        if ((rc = select_flagged<false>(c, nullptr, c->sel, c->list1, c->counts, n, s))) return rc;
+        long long n1 = 0;
+        SVP_CUDA(cudaMemcpyAsync(&n1, c->counts, sizeof n1, cudaMemcpyDeviceToHost, s));
         SVP_CUDA(cudaStreamSynchronize(s));
-        list2 = c->list2;
+        n2 = n1;
+        list2 = c->list1;
+        if (c->cfg.prescreen && n1) {
+            {
+                svp::KernelTimer _t("prescreen_kernel", s);
+                if ((rc = launch_prescreen(u, c->cg, c->list1, n1, c->pk, c->lower, s))) return rc;
+            }
+            SVP_LAUNCH(prescreen_stage_kernel<<<blocks_for(n1, 256, 8), 256, 0, s>>>(c->lower, n1, delta, c->sel,
+                                                                                   c->acc));
+            if ((rc = select_flagged<true>(c, c->list1, c->sel, c->list2, c->counts + 1, n1, s))) return rc;
+            SVP_CUDA(cudaMemcpyAsync(&n2, c->counts + 1, sizeof(long long), cudaMemcpyDeviceToHost, s));
+            SVP_CUDA(cudaStreamSynchronize(s));
+            list2 = c->list2;
+        }
     }
     long long n3 = 0;
     if (n2) {
+        SVP_CUDA(cudaMemsetAsync(c->tile_fail, 0, sizeof(int) * c->ntiles, s));
         rc = ensure_fallback(c, n2);
         if (rc) return rc;
         double *fb = c->fb, *plo = fb, *phi = fb + 27 * n2, *clo = fb + 2 * 27 * n2, *chi = fb + 3 * 27 * n2,
@@ -1765,10 +1955,8 @@ extern "C" int svp_certify_map(svp_certifier *c, const double *u, svp_cert_resul
             SVP_LAUNCH_CHECK("verdict stage");
         }
     }
-    if (staged) {
-        SVP_CUDA(cudaMemcpyAsync(&acc, c->acc, sizeof acc, cudaMemcpyDeviceToHost, s));
-        SVP_CUDA(cudaStreamSynchronize(s));
-    }
+    // a later stage updated the counts; otherwise the copy above is final
+    if ((staged || n2) && (rc = read_accum(c, &acc, s))) return rc;
     // the record (feasibility.py:755-771)
     long long fallback = n2;
     long long unknown = (long long)acc.unknown, bad = (long long)acc.bad;
