@@ -159,7 +159,8 @@ FLOP_PER_CELL = {
     # edges 36 + Gauss sweep 1350 + 27 x (cofactor 35 + 8 vertices x 30) + closed sweep 1350 + 27 x det 459
     # + the state-independent curl term 24
     "cell_ggn_diag_kernel": 10644,
-    "cell_min_jd_kernel": 2009,
+    # one field 678 + 12 edge quadratics 120 + Bernstein 27 x 4 + minima 54
+    "cell_min_jd_kernel": 960,
 }
 FP64_PEAK_TFLOPS = 148 * 64 * 2 * 1.965e9 / 1e12     # nominal: 148 SMs x 64 FP64 FMA/clk x 2 x 1965 MHz
 # float32 operations per cell of the mixed form's cell kernels (the float64 barrier of the flagged cells runs in its

@@ -1370,6 +1370,8 @@ __global__ void __launch_bounds__(CB) cell_trial_barrier_kernel(Q1Const q, const
 // ============================================================================================== node JD measure
 // ext_act > 0 (T69/T73): cells whose closed27 Bernstein coefficients allow a value below min(m_c, ext_act) are
 // appended to cand (order of arrival; each is then estimated independently, so the order does not matter).
+// Bound: FP64 issue, about 600 FP64 instructions per cell (closed27 J 459, 12 edge quadratics); 160x192x224: 1.00 ->
+// 0.49 ms per launch (the edge and Bernstein loops unrolled on registers: 0.86 -> 0.49).
 __global__ void __launch_bounds__(CS) cell_min_jd_kernel(Q1Const q, const double *__restrict__ u,
                                                          double *__restrict__ m, double ext_act,
                                                          unsigned long long *__restrict__ ncand,
@@ -1379,49 +1381,45 @@ __global__ void __launch_bounds__(CS) cell_min_jd_kernel(Q1Const q, const double
     const int T = blockDim.x;
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
          c += (long long)gridDim.x * blockDim.x) {
-        double E[3][4][3];
-        load_edges(u, cell_node0(c, q), q, E);
+        Columns C;
+        load_columns(u, cell_node0(c, q), q, C);
         double mn = __longlong_as_double(0x7FF0000000000000LL);
-        sweep<true>(E, q, [&](int p, int, int, int, const double (&V)[3][3]) {
-            double j = det_only(V);
+        closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
+            const double j = jacobian(det_minus_one(X, Y, Z));
             J[p * T] = j;
             mn = fmin(mn, j);
         });
+        double j[27];
+#pragma unroll
+        for (int p = 0; p < 27; p++) j[p] = J[p * T];
         // exact interior minima of the edge quadratics through t = 0, 1/2, 1 (solvers/jd_affine.py:24)
-#pragma unroll 1
+#pragma unroll
         for (int e = 0; e < 12; e++) {
-            int f0, st;
-            if (e < 4) {            // x edges: iz, iy in {0, 2}
-                f0 = 9 * ((e >> 1) * 2) + 3 * ((e & 1) * 2); st = 1;
-            } else if (e < 8) {     // y edges: iz, ix in {0, 2}
-                int k = e - 4;
-                f0 = 9 * ((k >> 1) * 2) + (k & 1) * 2; st = 3;
-            } else {                // z edges: iy, ix in {0, 2}
-                int k = e - 8;
-                f0 = 3 * ((k >> 1) * 2) + (k & 1) * 2; st = 9;
-            }
-            double j0 = J[f0 * T], j1 = J[(f0 + st) * T], j2 = J[(f0 + 2 * st) * T];
-            double a = 2 * (j0 - 2 * j1 + j2);
-            double b = -3 * j0 + 4 * j1 - j2;
+            // x edges: iz, iy in {0, 2}; y edges: iz, ix; z edges: iy, ix
+            const int k = e & 3, st = e < 4 ? 1 : (e < 8 ? 3 : 9);
+            const int f0 = e < 4 ? 9 * ((k >> 1) * 2) + 3 * ((k & 1) * 2)
+                                 : (e < 8 ? 9 * ((k >> 1) * 2) + (k & 1) * 2 : 3 * ((k >> 1) * 2) + (k & 1) * 2);
+            const double j0 = j[f0], j1 = j[f0 + st], j2 = j[f0 + 2 * st];
+            const double a = 2 * (j0 - 2 * j1 + j2);
+            const double b = -3 * j0 + 4 * j1 - j2;
             if (a > 0 && b < 0 && -b < 2 * a) mn = fmin(mn, j0 - b * b / (4 * a));
         }
         m[c] = mn;
         if (ext_act > 0.) {
-            // closed27 values -> Bernstein coefficients in place: per axis x, y, z the middle entry becomes
-            // 2 b - (a + c) / 2 (bernstein_barrier.py:26 to_bernstein)
-#pragma unroll 1
+            // closed27 values -> Bernstein coefficients: per axis x, y, z the middle entry becomes 2 b - (a + c) / 2
+            // (bernstein_barrier.py:26 to_bernstein)
+#pragma unroll
             for (int axis = 0; axis < 3; axis++) {
                 const int st = axis == 0 ? 1 : (axis == 1 ? 3 : 9);
-#pragma unroll 1
+#pragma unroll
                 for (int l = 0; l < 9; l++) {
                     const int o = axis == 0 ? 3 * l : (axis == 1 ? (l / 3) * 9 + (l % 3) : l);
-                    const double v0 = J[o * T], v1 = J[(o + st) * T], v2 = J[(o + 2 * st) * T];
-                    J[(o + st) * T] = 2. * v1 - .5 * (v0 + v2);
+                    j[o + st] = 2. * j[o + st] - .5 * (j[o] + j[o + 2 * st]);
                 }
             }
-            double bmin = J[0];
-#pragma unroll 1
-            for (int k = 1; k < 27; k++) bmin = fmin(bmin, J[k * T]);
+            double bmin = j[0];
+#pragma unroll
+            for (int k = 1; k < 27; k++) bmin = fmin(bmin, j[k]);
             if (bmin < fmin(mn, ext_act)) cand[atomicAdd(ncand, 1ull)] = c;
         }
     }
