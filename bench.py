@@ -156,9 +156,8 @@ FLOP_PER_CELL = {
     # two fields x 732 + residuals 27 + mass matrices 270 + adjoint pass 27 x (6 + 36) + its averages 120 + scatter 108
     # + curl adjoint 90
     "cell_grad_kernel": 3213,
-    # edges 36 + Gauss sweep 1350 + 27 x (cofactor 35 + 8 vertices x 30) + closed sweep 1350 + 27 x det 459
-    # + the state-independent curl term 24
-    "cell_ggn_diag_kernel": 10644,
+    # edges 84 + columns 27 x 14 + 27 x (3 rows x (9 + 3 + 8 + 4 + 16 + 16) + 4) + the state-independent curl term 24
+    "cell_ggn_diag_kernel": 5130,
     # one field 678 + 12 edge quadratics 120 + Bernstein 27 x 4 + minima 54
     "cell_min_jd_kernel": 960,
 }

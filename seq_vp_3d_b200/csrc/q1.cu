@@ -599,66 +599,104 @@ __global__ void __launch_bounds__(256) gather_kernel(Q1Const q, GatherSpec g, co
 }
 
 // ============================================================================================== GGN
-// Per-cell diagonal contributions: sum_p w (mu lj^2 + nu cs) + sum_closed27 b'' lc^2, lj = sum_j A_rj D_jpa.
-template <bool CLOSED>
-__device__ __forceinline__ void point_D(const Q1Const &q, int ix, int iy, int iz, int a, double D[3]) {
-    const int bx = a & 1, by = (a >> 1) & 1, bz = (a >> 2) & 1;
-    const double fx = bx ? rule_n<CLOSED>(q, ix) : rule_m<CLOSED>(q, ix);
-    const double fy = by ? rule_n<CLOSED>(q, iy) : rule_m<CLOSED>(q, iy);
-    const double fz = bz ? rule_n<CLOSED>(q, iz) : rule_m<CLOSED>(q, iz);
-    D[0] = (bx ? q.ih[0] : -q.ih[0]) * fy * fz;
-    D[1] = (by ? q.ih[1] : -q.ih[1]) * fx * fz;
-    D[2] = (bz ? q.ih[2] : -q.ih[2]) * fx * fy;
+// Per-cell diagonal contributions sum_p w_p l_a,r(p)^2 with l = sum_j A_rj D_j(p, a), A the cofactors of F.  D_j is
+// +-1/h_j times the two other coordinates' linear shape values f, so with P, Q, R = the weighted A_r0, A_r1, A_r2 the
+// eight vertices' l are +-f_y f_z P + f_x (+-f_z Q +- f_y R): 28 operations per point and row for all eight, where
+// forming each vertex's D and dot product took 100.  The rule's columns are linear interpolations per plane and row.
+// weight(p, ix, iy, iz): the factor of l (SQUARED: of l^2).
+template <bool CLOSED, bool SQUARED, class Weight>
+__device__ __forceinline__ void ggn_points(const Columns &C, const Q1Const &q, Weight &&weight, double (&out)[8][3]) {
+    const double n[3] = {rule_n<CLOSED>(q, 0), rule_n<CLOSED>(q, 1), rule_n<CLOSED>(q, 2)};
+    const double m[3] = {rule_m<CLOSED>(q, 0), rule_m<CLOSED>(q, 1), rule_m<CLOSED>(q, 2)};
+#pragma unroll 1
+    for (int iz = 0; iz < 3; iz++) {
+        const double nz = rule_n<CLOSED>(q, iz), mz = rule_m<CLOSED>(q, iz);
+        double X[3][3], Y[3][3];
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            const double x0 = fma(nz, C.X[2][r] - C.X[0][r], C.X[0][r]), x1 = fma(nz, C.X[3][r] - C.X[1][r], C.X[1][r]);
+            const double y0 = fma(nz, C.Y[2][r] - C.Y[0][r], C.Y[0][r]), y1 = fma(nz, C.Y[3][r] - C.Y[1][r], C.Y[1][r]);
+            const double dx = x1 - x0, dy = y1 - y0;
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                X[i][r] = fma(n[i], dx, x0);
+                Y[i][r] = fma(n[i], dy, y0);
+            }
+        }
+#pragma unroll
+        for (int iy = 0; iy < 3; iy++) {
+            double z0[3], dz[3];
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                z0[r] = fma(n[iy], C.Z[2][r] - C.Z[0][r], C.Z[0][r]);
+                dz[r] = fma(n[iy], C.Z[3][r] - C.Z[1][r], C.Z[1][r]) - z0[r];
+            }
+#pragma unroll
+            for (int ix = 0; ix < 3; ix++) {
+                const double s = weight(9 * iz + 3 * iy + ix, ix, iy, iz);
+                double F[3][3];      // rows of F
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    F[r][0] = X[iy][r];
+                    F[r][1] = Y[ix][r];
+                    F[r][2] = fma(n[ix], dz[r], z0[r]);
+                }
+                const double k0 = SQUARED ? q.ih[0] : s * q.ih[0], k1 = SQUARED ? q.ih[1] : s * q.ih[1],
+                             k2 = SQUARED ? q.ih[2] : s * q.ih[2];
+                const double fy[2] = {m[iy], n[iy]}, fz[2] = {mz, nz};
+                const double fyz[2][2] = {{fy[0] * fz[0], fy[0] * fz[1]}, {fy[1] * fz[0], fy[1] * fz[1]}};
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    const int j = (r + 1) % 3, k = (r + 2) % 3;
+                    const double P = k0 * (F[j][1] * F[k][2] - F[j][2] * F[k][1]);
+                    const double Q = k1 * (F[j][2] * F[k][0] - F[j][0] * F[k][2]);
+                    const double R = k2 * (F[j][0] * F[k][1] - F[j][1] * F[k][0]);
+                    const double Qz[2] = {fz[0] * Q, fz[1] * Q}, Ry[2] = {fy[0] * R, fy[1] * R};
+#pragma unroll
+                    for (int bz = 0; bz < 2; bz++)
+#pragma unroll
+                        for (int by = 0; by < 2; by++) {
+                            const double t1 = fyz[by][bz] * P;
+                            const double t2 = (by ? Qz[bz] : -Qz[bz]) + (bz ? Ry[by] : -Ry[by]);
+                            const double l0 = fma(m[ix], t2, -t1), l1 = fma(n[ix], t2, t1);
+                            double &o0 = out[2 * by + 4 * bz][r], &o1 = out[1 + 2 * by + 4 * bz][r];
+                            o0 = fma(SQUARED ? s * l0 : l0, l0, o0);
+                            o1 = fma(SQUARED ? s * l1 : l1, l1, o1);
+                        }
+                }
+            }
+        }
+    }
 }
 
-__global__ void __launch_bounds__(CT) cell_ggn_diag_kernel(Q1Const q, const double *__restrict__ u,
-                                                           double *__restrict__ L,
-                                                           const uint8_t *__restrict__ active, bool barrier) {
+// The JD part at the Gauss points (weights w mu) plus the state-independent curl part q.ggn_curl.  flags (when the
+// state has no mask): 1 for the cells with some closed27 J not above the activation.
+// Bound: FP64 issue, about 3,300 FP64 instructions per cell (5,600 with a D per vertex): 128x144x128 0.78 -> 0.47
+// ms per launch.
+__global__ void __launch_bounds__(CS) cell_ggn_diag_kernel(Q1Const q, const double *__restrict__ u,
+                                                           double *__restrict__ L, uint8_t *__restrict__ flags) {
+    const double root = sqrt(q.mu * q.omega), low = near_bound(q.act);
+    constexpr double side = 0.52704627669472988, centre = 2. / 3.;     // sqrt(5 / 18), sqrt(4 / 9)
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
          c += (long long)gridDim.x * blockDim.x) {
-        double E[3][4][3], out[8][3];
-        load_edges(u, cell_node0(c, q), q, E);
+        Columns C;
+        load_columns(u, cell_node0(c, q), q, C);
+        if (flags) {
+            bool near = false;
+            closed_points(C, [&](int, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
+                near |= !(det_minus_one(X, Y, Z) >= low);
+            });
+            flags[c] = near ? 1 : 0;
+        }
+        add_identity(C);
+        double out[8][3];
 #pragma unroll
         for (int a = 0; a < 8; a++)
 #pragma unroll
-            for (int r = 0; r < 3; r++) out[a][r] = 0.;
-        // JD part per Gauss point; the curl part is the state-independent q.ggn_curl
-        sweep<false>(E, q, [&](int p, int ix, int iy, int iz, const double (&V)[3][3]) {
-            double A[3][3], J;
-            cofactor_det(V, A, J);
-            const double gmu = q.gw[p] * q.mu;
-#pragma unroll
-            for (int a = 0; a < 8; a++) {
-                double D[3];
-                point_D<false>(q, ix, iy, iz, a, D);
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    double lj = A[r][0] * D[0] + A[r][1] * D[1] + A[r][2] * D[2];
-                    out[a][r] += gmu * (lj * lj);
-                }
-            }
-        });
-#pragma unroll
-        for (int a = 0; a < 8; a++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) out[a][r] += q.ggn_curl[3 * a + r];
-        if (barrier && (!active || active[c]))
-        sweep<true>(E, q, [&](int, int ix, int iy, int iz, const double (&V)[3][3]) {
-            if (!(det_only(V) < q.act)) return;
-            double A[3][3], J, b, b1, b2;
-            cofactor_det(V, A, J);
-            barrier_eval(J, q.act, q.delta, q.bw, b, b1, b2);
-#pragma unroll
-            for (int a = 0; a < 8; a++) {
-                double D[3];
-                point_D<true>(q, ix, iy, iz, a, D);
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    double lc = A[r][0] * D[0] + A[r][1] * D[1] + A[r][2] * D[2];
-                    out[a][r] += b2 * lc * lc;
-                }
-            }
-        });
+            for (int r = 0; r < 3; r++) out[a][r] = q.ggn_curl[3 * a + r];
+        ggn_points<false, false>(C, q, [&](int, int ix, int iy, int iz) {
+            return root * (iz == 1 ? centre : side) * ((iy == 1 ? centre : side) * (ix == 1 ? centre : side));
+        }, out);
         store_locals(L, c, q.ncell, out);
     }
 }
@@ -999,18 +1037,27 @@ __global__ void __launch_bounds__(CT, 4) cell_ggn_diag32_kernel(Q1Const q, const
     }
 }
 
+template <bool CLOSED>
+__device__ __forceinline__ void point_D(const Q1Const &q, int ix, int iy, int iz, int a, double D[3]) {
+    const int bx = a & 1, by = (a >> 1) & 1, bz = (a >> 2) & 1;
+    const double fx = bx ? rule_n<CLOSED>(q, ix) : rule_m<CLOSED>(q, ix);
+    const double fy = by ? rule_n<CLOSED>(q, iy) : rule_m<CLOSED>(q, iy);
+    const double fz = bz ? rule_n<CLOSED>(q, iz) : rule_m<CLOSED>(q, iz);
+    D[0] = (bx ? q.ih[0] : -q.ih[0]) * fy * fz;
+    D[1] = (by ? q.ih[1] : -q.ih[1]) * fx * fz;
+    D[2] = (bz ? q.ih[2] : -q.ih[2]) * fx * fy;
+}
+
 // The barrier curvature b'' lc^2 of the flagged cells in float64 (J, b'' and the cofactors lc from the float64
-// state), rounded to the locals' type LT and added point by point in sweep order to the cell's locals (in the plain
-// form the additions of the fused float64 kernel).
-template <class LT>
-__global__ void __launch_bounds__(CB) cell_ggn_barrier_kernel(Q1Const q, const double *__restrict__ u,
+// state), rounded to float32 and added point by point in sweep order to the cell's locals.
+__global__ void __launch_bounds__(CB) cell_ggn_barrier32_kernel(Q1Const q, const double *__restrict__ u,
                                                               const uint8_t *__restrict__ flags,
-                                                              LT *__restrict__ L) {
+                                                              float *__restrict__ L) {
     __shared__ long long queue[CB / 32][64];
     for_flagged_cells(q, flags, queue[threadIdx.x >> 5], [&](long long c, uint8_t) {
         double E64[3][4][3];
         load_edges(u, cell_node0(c, q), q, E64);
-        LT out[8][3];
+        float out[8][3];
 #pragma unroll
         for (int a = 0; a < 8; a++)
 #pragma unroll
@@ -1029,12 +1076,53 @@ __global__ void __launch_bounds__(CB) cell_ggn_barrier_kernel(Q1Const q, const d
 #pragma unroll
                 for (int r = 0; r < 3; r++) {
                     double lc = A[r][0] * D[0] + A[r][1] * D[1] + A[r][2] * D[2];
-                    if constexpr (sizeof(LT) == 8) out[a][r] += b2 * lc * lc;   // the fused kernel's expression
-                    else out[a][r] += (LT)(b2 * lc * lc);
+                    out[a][r] += (float)(b2 * lc * lc);
                 }
             }
         });
         if (any) store_locals(L, c, q.ncell, out);
+    });
+}
+
+// The plain form's barrier curvature of the flagged cells: b'' at the 27 points spread over the block, then each
+// cell's squares by its own thread, added to its locals.
+__global__ void __launch_bounds__(BT) cell_ggn_barrier_kernel(Q1Const q, const double *__restrict__ u,
+                                                              const uint8_t *__restrict__ flags,
+                                                              double *__restrict__ L) {
+    extern __shared__ double smem[];
+    __shared__ long long queue[kBlockQueue];
+    for_flagged_blocks(q, flags, queue, [&](int n) {
+        const bool mine = (int)threadIdx.x < n;
+        const long long c = mine ? queue[threadIdx.x] : 0;
+        Columns C;
+        if (mine) {
+            load_columns(u, cell_node0(c, q), q, C);
+            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
+                                 const double (&Z)[3]) {
+                smem[p * BT + threadIdx.x] = jacobian(det_minus_one(X, Y, Z));
+            });
+        }
+        __syncthreads();
+        for_block_points(n, [&](int p, int l) {
+            const double J = smem[p * BT + l];
+            double b, b1, b2 = 0.;
+            if (J < q.act) barrier_eval(J, q.act, q.delta, q.bw, b, b1, b2);
+            smem[p * BT + l] = b2;
+        });
+        __syncthreads();
+        if (mine) {
+            add_identity(C);
+            double out[8][3];
+#pragma unroll
+            for (int a = 0; a < 8; a++)
+#pragma unroll
+                for (int r = 0; r < 3; r++) out[a][r] = 0.;
+            ggn_points<true, true>(C, q, [&](int p, int, int, int) { return smem[p * BT + threadIdx.x]; }, out);
+#pragma unroll
+            for (int a = 0; a < 8; a++)
+#pragma unroll
+                for (int r = 0; r < 3; r++) L[(size_t)(3 * a + r) * q.ncell + c] += out[a][r];
+        }
     });
 }
 
@@ -2365,19 +2453,21 @@ extern "C" int svp_ggn_diagonal_masked(svp_pair *p, const double *u, const doubl
         }
         {
             svp::KernelTimer _t("cell_ggn_barrier32_kernel", s);
-            SVP_LAUNCH(cell_ggn_barrier_kernel<float><<<barrier_blocks(p->q), CB, 0, s>>>(
+            SVP_LAUNCH(cell_ggn_barrier32_kernel<<<barrier_blocks(p->q), CB, 0, s>>>(
                 p->q, u, active ? active : p->flags, (float *)p->loc1));
         }
         SVP_LAUNCH(ggn_node_kernel<float><<<node_blocks(p->q.nfree), 256, 0, s>>>(p->q, (const float *)p->loc1, image_grad, nullptr, out));
     } else {
-        // with the state's mask, the barrier curvature of the active cells in its own kernel (the same values)
+        if (!active && (rc = pair_flags(p))) return rc;
         {
             svp::KernelTimer _t("cell_ggn_diag_kernel", s);
-            SVP_LAUNCH(cell_ggn_diag_kernel<<<cell_blocks(p), CT, 0, s>>>(p->q, u, p->loc1, active, active == nullptr));
+            SVP_LAUNCH(cell_ggn_diag_kernel<<<slice_blocks(p), CS, 0, s>>>(p->q, u, p->loc1,
+                                                                         active ? nullptr : p->flags));
         }
-        if (active) {
+        {
             svp::KernelTimer _t("cell_ggn_barrier_kernel", s);
-            SVP_LAUNCH(cell_ggn_barrier_kernel<double><<<barrier_blocks(p->q), CB, 0, s>>>(p->q, u, active, p->loc1));
+            SVP_LAUNCH(cell_ggn_barrier_kernel<<<flagged_blocks(p->q), BT, sizeof(double) * 27 * BT, s>>>(
+                p->q, u, active ? active : p->flags, p->loc1));
         }
         SVP_LAUNCH(ggn_node_kernel<double><<<node_blocks(p->q.nfree), 256, 0, s>>>(p->q, p->loc1, image_grad, nullptr, out));
     }

@@ -79,3 +79,14 @@ def test_outer_gradients(problem):
         for got, term in zip(P.outer_gradients(bd, w, g, mask), ("outer", "image", "total")):
             ref = Q.gradient(OP, base, ow, og, term)
             assert np.linalg.norm(got.cpu().numpy() - ref) <= TOL * np.linalg.norm(ref)
+
+
+def test_ggn_diagonal(problem):
+    P, OP, bd, td, base, trial = problem
+    _, g = P.warp(bd, with_gradient=True)
+    _, og = Q.warp(OP, base, True)
+    active = P.trial_energy(td, P.warp(td)[0], bd)[5]
+    ref = Q.ggn_diagonal(OP, base, og)
+    for mask in (None, active):
+        got = P.ggn_diagonal(bd, g, mask).cpu().numpy()
+        assert np.linalg.norm(got - ref) <= TOL * np.linalg.norm(ref)
