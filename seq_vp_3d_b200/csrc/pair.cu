@@ -188,7 +188,7 @@ extern "C" int svp_pair_destroy(svp_pair *p) {
     for (int k = 0; k < 3; k++) {
         cudaFree(p->knots[k]); cudaFree(p->spline_rcp[k]); cudaFree(p->dst_half[k]); cudaFree(p->dst_pad[k]); cudaFree(p->dst_tf32[k]);
     }
-    cudaFree(p->loc1); cudaFree(p->loc2); cudaFree(p->cellbuf); cudaFree(p->partial); cudaFree(p->result);
+    cudaFree(p->loc1); cudaFree(p->loc2); cudaFree(p->cellbuf); cudaFree(p->partial); cudaFreeHost(p->host);
     cudaFree(p->counter); cudaFree(p->cand); cudaFree(p->flags); cudaFree(p->dst_tmp); cudaFree(p->den);
     delete p;
     return SVP_OK;
@@ -220,8 +220,10 @@ extern "C" int svp_pair_create(const svp_grid *g, const svp_weights *w, const do
     if ((e = cudaMalloc((void **)&p->u_ref, sizeof(double) * 3 * nn)) != cudaSuccess) return bail(cuda_fail(e, "uref"));
     if ((e = cudaMalloc((void **)&p->cellbuf, sizeof(double) * p->q.ncell)) != cudaSuccess)
         return bail(cuda_fail(e, "cellbuf"));
-    if ((e = cudaMalloc((void **)&p->result, sizeof(double) * 64)) != cudaSuccess) return bail(cuda_fail(e, "result"));
+    if ((e = cudaMallocHost((void **)&p->host, sizeof(double) * 64)) != cudaSuccess) return bail(cuda_fail(e, "results"));
     if ((e = cudaMalloc((void **)&p->counter, sizeof(long long) * 8)) != cudaSuccess)
+        return bail(cuda_fail(e, "counter"));
+    if ((e = cudaMemsetAsync(p->counter, 0, sizeof(long long) * 8, s)) != cudaSuccess)
         return bail(cuda_fail(e, "counter"));
     if ((e = cudaMemcpyAsync(p->fixed, fixed, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
         return bail(cuda_fail(e, "fixed copy"));

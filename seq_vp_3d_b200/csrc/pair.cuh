@@ -18,7 +18,7 @@ struct svp_pair {
     double *cellbuf = nullptr;                // (ncell)
     svp::dd *partial = nullptr;               // block partial sums
     long long partial_cap = 0;                // in dd entries
-    double *result = nullptr;                 // small device result area (64 doubles)
+    double *host = nullptr;                   // pinned results that kernels write (64 doubles)
     long long *counter = nullptr;             // small device counters (8)
     long long *cand = nullptr;                // candidate cells of the T69/T73 node JD extension (ncell)
     uint8_t *flags = nullptr;                 // (ncell) cells the float32 cell kernels hand to the float64 barrier

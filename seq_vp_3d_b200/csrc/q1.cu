@@ -1918,20 +1918,44 @@ __global__ void __launch_bounds__(256) pg_scale_kernel(Q1Const q, const double *
 }
 
 // ============================================================================================== final reduction
-__global__ void final_reduce_kernel(const dd *__restrict__ partial, long long blocks, int K, double *out) {
-    // one block; thread t reduces blocks t, t + 256, ... in order, then a fixed tree
+// All block sums of one evaluation in one launch, one block per sum: thread t adds blocks t, t + 256, ... in order, then
+// a fixed tree.  The results go straight to the pair's pinned host buffer, with the violation count (which is zeroed
+// for the next evaluation), so the evaluation ends with a wait and no copy.  A trial took six of these launches, a
+// memset and two copies to pageable memory: on 48^3 about 60 of its 161 us.
+struct ReduceSpec {
+    static constexpr int kMost = 8;
+    const dd *src[kMost];
+    long long blocks[kMost];
+    int K[kMost], out[kMost], n = 0, sums = 0;
+    unsigned long long *bad = nullptr;
+    void add(const dd *partial, long long count, int k, int at) {
+        src[n] = partial; blocks[n] = count; K[n] = k; out[n] = at;
+        n++;
+        sums += k;
+    }
+};
+constexpr int kBadSlot = 62;      // of the 64 result slots: the violation count's bits
+__global__ void __launch_bounds__(256) reduce_results_kernel(const __grid_constant__ ReduceSpec r, double *out) {
     __shared__ dd sh[256];
-    for (int k = 0; k < K; k++) {
-        dd acc = {0., 0.};
-        for (long long b = threadIdx.x; b < blocks; b += blockDim.x) acc = dd_add(acc, partial[b * K + k]);
-        sh[threadIdx.x] = acc;
+    int i = 0, k = blockIdx.x;
+    while (k >= r.K[i]) k -= r.K[i++];
+    const dd *partial = r.src[i];
+    const int K = r.K[i];
+    dd acc = {0., 0.};
+    for (long long b = threadIdx.x; b < r.blocks[i]; b += blockDim.x) acc = dd_add(acc, partial[b * K + k]);
+    sh[threadIdx.x] = acc;
+    __syncthreads();
+    for (int s = blockDim.x / 2; s; s >>= 1) {
+        if ((int)threadIdx.x < s) sh[threadIdx.x] = dd_add(sh[threadIdx.x], sh[threadIdx.x + s]);
         __syncthreads();
-        for (int s = blockDim.x / 2; s; s >>= 1) {
-            if ((int)threadIdx.x < s) sh[threadIdx.x] = dd_add(sh[threadIdx.x], sh[threadIdx.x + s]);
-            __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        out[r.out[i] + 2 * k] = sh[0].hi;
+        out[r.out[i] + 2 * k + 1] = sh[0].lo;
+        if (blockIdx.x == 0 && r.bad) {
+            out[kBadSlot] = __longlong_as_double((long long)*r.bad);
+            *r.bad = 0;
         }
-        if (threadIdx.x == 0) { out[2 * k] = sh[0].hi; out[2 * k + 1] = sh[0].lo; }
-        __syncthreads();
     }
 }
 
@@ -1975,6 +1999,19 @@ int allow_slices() {
     return SVP_OK;
 }
 unsigned node_blocks(long long n) { return blocks_for(n, 256, 8); }
+
+// The evaluations' violation counter: its own word, zero between evaluations.
+unsigned long long *violations(svp_pair *p) { return (unsigned long long *)(p->counter + 6); }
+int reduce_results(svp_pair *p, const ReduceSpec &r, cudaStream_t s) {
+    SVP_LAUNCH(reduce_results_kernel<<<(unsigned)r.sums, 256, 0, s>>>(r, p->host));
+    SVP_CUDA(cudaStreamSynchronize(s));
+    return SVP_OK;
+}
+long long violation_count(const svp_pair *p) {
+    long long n;
+    memcpy(&n, &p->host[kBadSlot], sizeof n);
+    return n;
+}
 
 }  // namespace
 
@@ -2045,7 +2082,6 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
     if (rc) return rc;
     if ((rc = allow_slices())) return rc;
     if ((rc = pair_flags(p))) return rc;
-    SVP_CUDA(cudaMemsetAsync(p->counter, 0, sizeof(long long) * 8, s));
     { svp::KernelTimer _t("node_energy_kernel", s); SVP_LAUNCH(node_energy_kernel<<<nb, 256, 0, s>>>(p->q, u, warped, p->fixed, p->u_ref, p->partial)); }
     SVP_LAUNCH_CHECK("node_energy_kernel");
     dd *pc = p->partial + (long long)nb * 2, *pb = pc + (long long)cb * 2;
@@ -2057,19 +2093,18 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
     {
         svp::KernelTimer _t("cell_barrier_kernel", s);
         SVP_LAUNCH(cell_barrier_kernel<true, false><<<bb, BT, sizeof(double) * 27 * BT, s>>>(
-            p->q, nullptr, u, p->flags, pb, nullptr, (unsigned long long *)p->counter, nullptr));
+            p->q, nullptr, u, p->flags, pb, nullptr, violations(p), nullptr));
     }
     SVP_LAUNCH_CHECK("cell_energy_kernel");
     double node2[2], cell3[3];
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(p->partial, nb, 2, p->result));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pc, cb, 2, p->result + 4));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pb, bb, 1, p->result + 8));
-    SVP_LAUNCH_CHECK("final_reduce_kernel");
-    double tmp[10];
-    long long bad = 0;
-    SVP_CUDA(cudaMemcpyAsync(tmp, p->result, sizeof tmp, cudaMemcpyDeviceToHost, s));
-    SVP_CUDA(cudaMemcpyAsync(&bad, p->counter, sizeof bad, cudaMemcpyDeviceToHost, s));
-    SVP_CUDA(cudaStreamSynchronize(s));
+    ReduceSpec red;
+    red.add(p->partial, nb, 2, 0);
+    red.add(pc, cb, 2, 4);
+    red.add(pb, bb, 1, 8);
+    red.bad = violations(p);
+    if ((rc = reduce_results(p, red, s))) return rc;
+    const double *tmp = p->host;
+    const long long bad = violation_count(p);
     for (int k = 0; k < 2; k++) node2[k] = tmp[2 * k] + tmp[2 * k + 1];
     for (int k = 0; k < 3; k++) cell3[k] = tmp[4 + 2 * k] + tmp[4 + 2 * k + 1];
     terms5[0] = .5 * node2[0];
@@ -2109,13 +2144,12 @@ extern "C" int svp_energy_difference_masked(svp_pair *p, const double *base_u, c
             p->q, base_u, trial_u, p->flags, nullptr, pb, nullptr, nullptr));
     }
     SVP_LAUNCH_CHECK("difference kernels");
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(p->partial, nb, 2, p->result));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pc, cb, 2, p->result + 4));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pb, bb, 1, p->result + 8));
-    SVP_LAUNCH_CHECK("final_reduce_kernel");
-    double tmp[10];
-    SVP_CUDA(cudaMemcpyAsync(tmp, p->result, sizeof tmp, cudaMemcpyDeviceToHost, s));
-    SVP_CUDA(cudaStreamSynchronize(s));
+    ReduceSpec red;
+    red.add(p->partial, nb, 2, 0);
+    red.add(pc, cb, 2, 4);
+    red.add(pb, bb, 1, 8);
+    if ((rc = reduce_results(p, red, s))) return rc;
+    const double *tmp = p->host;
     // E = image + proximity + jd + curl + barrier; F = image + barrier (sums of double-double pieces)
     double img = tmp[0] + tmp[1], prox = tmp[2] + tmp[3];
     double jd = tmp[4] + tmp[5], curl = tmp[6] + tmp[7], bar = tmp[8] + tmp[9];
@@ -2161,7 +2195,6 @@ extern "C" int svp_energy_difference_screened(svp_pair *p, const double *base_u,
     if (rc) return rc;
     if ((rc = allow_slices())) return rc;
     if ((rc = pair_flags(p))) return rc;
-    SVP_CUDA(cudaMemsetAsync(p->counter, 0, sizeof(long long) * 8, s));
     dd *pn = p->partial, *pce = pn + (long long)nb * 2, *pcd = pce + (long long)cb * 2, *pcb = pcd + (long long)cb * 2;
     dd *pbe = pcb + (long long)cb * 4, *pbd = pbe + bb;
     {
@@ -2177,18 +2210,18 @@ extern "C" int svp_energy_difference_screened(svp_pair *p, const double *base_u,
     {
         svp::KernelTimer _t("cell_trial_barrier_kernel", s);
         SVP_LAUNCH(cell_trial_barrier_kernel<<<bb, CB, sizeof(double) * 27 * CB, s>>>(
-            p->q, base_u, trial_u, p->flags, pbe, pbd, (unsigned long long *)p->counter, nullptr, base_active));
+            p->q, base_u, trial_u, p->flags, pbe, pbd, violations(p), nullptr, base_active));
     }
     SVP_LAUNCH_CHECK("screened difference kernels");
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pn, nb, 2, p->result));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pcd, cb, 2, p->result + 4));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pbd, bb, 1, p->result + 8));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pce, cb, 2, p->result + 10));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pcb, cb, 4, p->result + 14));
-    SVP_LAUNCH_CHECK("final_reduce_kernel");
-    double tmp[22];
-    SVP_CUDA(cudaMemcpyAsync(tmp, p->result, sizeof tmp, cudaMemcpyDeviceToHost, s));
-    SVP_CUDA(cudaStreamSynchronize(s));
+    ReduceSpec red;
+    red.add(pn, nb, 2, 0);
+    red.add(pcd, cb, 2, 4);
+    red.add(pbd, bb, 1, 8);
+    red.add(pce, cb, 2, 10);
+    red.add(pcb, cb, 4, 14);
+    red.bad = violations(p);
+    if ((rc = reduce_results(p, red, s))) return rc;
+    const double *tmp = p->host;
     // E = image + proximity + jd + curl + barrier; F = image + barrier, as svp_energy_difference combines them
     double img = tmp[0] + tmp[1], prox = tmp[2] + tmp[3];
     double jd = tmp[4] + tmp[5], curl = tmp[6] + tmp[7], bar = tmp[8] + tmp[9];
@@ -2212,7 +2245,6 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
     if (rc) return rc;
     if ((rc = allow_slices())) return rc;
     if ((rc = pair_flags(p))) return rc;
-    SVP_CUDA(cudaMemsetAsync(p->counter, 0, sizeof(long long) * 8, s));
     dd *pne = p->partial, *pnd = pne + (long long)nb * 2, *pce = pnd + (long long)nb * 2, *pcd = pce + (long long)cb * 3;
     dd *pcb = pcd + (long long)cb * 3, *pbe = pcb + (long long)cb * 4, *pbd = pbe + bb;
     SplineRef S = spline_ref(p);
@@ -2234,7 +2266,7 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
         }
         svp::KernelTimer _t("cell_trial_barrier_kernel", s);
         SVP_LAUNCH(cell_trial_barrier_kernel<<<bb, CB, sizeof(double) * 27 * CB, s>>>(
-            p->q, base_u, trial_u, p->flags, pbe, pbd, (unsigned long long *)p->counter, trial_active, base_active));
+            p->q, base_u, trial_u, p->flags, pbe, pbd, violations(p), trial_active, base_active));
     } else {
         {
             svp::KernelTimer _t("cell_trial_kernel", s);
@@ -2243,23 +2275,22 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
         }
         svp::KernelTimer _t("cell_barrier_kernel", s);
         SVP_LAUNCH(cell_barrier_kernel<true, true><<<bb, BT, sizeof(double) * 54 * BT, s>>>(
-            p->q, base_u, trial_u, p->flags, pbe, pbd, (unsigned long long *)p->counter, trial_active));
+            p->q, base_u, trial_u, p->flags, pbe, pbd, violations(p), trial_active));
     }
     SVP_LAUNCH_CHECK("cell_trial_kernel");
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pne, nb, 2, p->result));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pnd, nb, 2, p->result + 10));
     // soft sums and differences from the soft kernel, the barrier's from the barrier kernel
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pce, cb, 2, p->result + 4));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pbe, bb, 1, p->result + 8));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pcd, cb, 2, p->result + 14));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pbd, bb, 1, p->result + 18));
-    if (screened) SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(pcb, cb, 4, p->result + 20));
-    SVP_LAUNCH_CHECK("final_reduce_kernel");
-    double tmp[28];
-    long long bad = 0;
-    SVP_CUDA(cudaMemcpyAsync(tmp, p->result, sizeof(double) * (screened ? 28 : 20), cudaMemcpyDeviceToHost, s));
-    SVP_CUDA(cudaMemcpyAsync(&bad, p->counter, sizeof bad, cudaMemcpyDeviceToHost, s));
-    SVP_CUDA(cudaStreamSynchronize(s));
+    ReduceSpec red;
+    red.add(pne, nb, 2, 0);
+    red.add(pce, cb, 2, 4);
+    red.add(pbe, bb, 1, 8);
+    red.add(pnd, nb, 2, 10);
+    red.add(pcd, cb, 2, 14);
+    red.add(pbd, bb, 1, 18);
+    if (screened) red.add(pcb, cb, 4, 20);
+    red.bad = violations(p);
+    if ((rc = reduce_results(p, red, s))) return rc;
+    const double *tmp = p->host;
+    const long long bad = violation_count(p);
     // energy terms exactly as svp_energy
     double node2[2], cell3[3];
     for (int k = 0; k < 2; k++) node2[k] = tmp[2 * k] + tmp[2 * k + 1];
@@ -2566,11 +2597,11 @@ extern "C" int svp_image_shift(svp_pair *p, const double *image_grad, double fac
     int rc = pair_partials(p, nb, 1);
     if (rc) return rc;
     SVP_LAUNCH(shift_kernel<<<nb, 256, 0, s>>>(p->q, image_grad, p->partial));
-    SVP_LAUNCH(final_reduce_kernel<<<1, 256, 0, s>>>(p->partial, nb, 1, p->result));
     SVP_LAUNCH_CHECK("shift kernels");
-    double tmp[2];
-    SVP_CUDA(cudaMemcpyAsync(tmp, p->result, sizeof tmp, cudaMemcpyDeviceToHost, s));
-    SVP_CUDA(cudaStreamSynchronize(s));
+    ReduceSpec red;
+    red.add(p->partial, nb, 1, 0);
+    if ((rc = reduce_results(p, red, s))) return rc;
+    const double *tmp = p->host;
     *alpha = factor * ((tmp[0] + tmp[1]) / (double)p->q.nfree) / 3;
     return SVP_OK;
 }

@@ -144,20 +144,20 @@ __global__ void __launch_bounds__(256) step_dots_kernel(const double *__restrict
     block_reduce_dd<K>(acc, partial);
 }
 
-__global__ void multi_final_kernel(const dd *__restrict__ partial, long long blocks, int K, double *out) {
+// one block per sum (the K sums of one block one after another took 10 us for K = 6)
+__global__ void __launch_bounds__(256) multi_final_kernel(const dd *__restrict__ partial, long long blocks, int K,
+                                                          double *out) {
     __shared__ dd sh[256];
-    for (int k = 0; k < K; k++) {
-        dd acc = {0., 0.};
-        for (long long b = threadIdx.x; b < blocks; b += blockDim.x) acc = dd_add(acc, partial[b * K + k]);
-        sh[threadIdx.x] = acc;
-        __syncthreads();
-        for (int s = blockDim.x / 2; s; s >>= 1) {
-            if ((int)threadIdx.x < s) sh[threadIdx.x] = dd_add(sh[threadIdx.x], sh[threadIdx.x + s]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[k] = sh[0].hi + sh[0].lo;
+    const int k = blockIdx.x;
+    dd acc = {0., 0.};
+    for (long long b = threadIdx.x; b < blocks; b += blockDim.x) acc = dd_add(acc, partial[b * K + k]);
+    sh[threadIdx.x] = acc;
+    __syncthreads();
+    for (int s = blockDim.x / 2; s; s >>= 1) {
+        if ((int)threadIdx.x < s) sh[threadIdx.x] = dd_add(sh[threadIdx.x], sh[threadIdx.x + s]);
         __syncthreads();
     }
+    if (threadIdx.x == 0) out[k] = sh[0].hi + sh[0].lo;
 }
 
 // max |a - b| and max |b| as order keys of non-negative values; a NaN maps above +inf (propagates)
@@ -260,7 +260,7 @@ extern "C" int svp_bb2_dots_dev(const double *theta, const double *theta_old, co
     dd *part = nullptr;
     SVP_CUDA(scratch_alloc((void **)&part, sizeof(dd) * 4 * nb, s));
     SVP_LAUNCH_KEEP(bb2_kernel<<<nb, 256, 0, s>>>(theta, theta_old, g, g_old, p_old, pvec, n, part));
-    SVP_LAUNCH_KEEP(multi_final_kernel<<<1, 256, 0, s>>>(part, nb, 4, out4_dev));
+    SVP_LAUNCH_KEEP(multi_final_kernel<<<4, 256, 0, s>>>(part, nb, 4, out4_dev));
     cudaError_t le = cudaGetLastError();
     cudaError_t fe = scratch_free(part, s);
     if (le != cudaSuccess) return cuda_fail(le, "bb2 kernels");
@@ -282,7 +282,7 @@ extern "C" int svp_step_dots_dev(const double *g, const double *pvec, const doub
         SVP_LAUNCH_KEEP(step_dots_kernel<6><<<nb, 256, 0, s>>>(g, pvec, theta, theta_old, g_old, p_old, n, part));
     else
         SVP_LAUNCH_KEEP(step_dots_kernel<2><<<nb, 256, 0, s>>>(g, pvec, nullptr, nullptr, nullptr, nullptr, n, part));
-    SVP_LAUNCH_KEEP(multi_final_kernel<<<1, 256, 0, s>>>(part, nb, K, out_dev));
+    SVP_LAUNCH_KEEP(multi_final_kernel<<<K, 256, 0, s>>>(part, nb, K, out_dev));
     cudaError_t le = cudaGetLastError();
     cudaError_t fe = scratch_free(part, s);
     if (le != cudaSuccess) return cuda_fail(le, "step dots kernels");
@@ -335,7 +335,7 @@ extern "C" int svp_bb2_dots(const double *theta, const double *theta_old, const 
     SVP_CUDA(scratch_alloc((void **)&part, sizeof(dd) * 4 * nb + 4 * sizeof(double), s));
     double *res = (double *)(part + 4 * nb);
     SVP_LAUNCH_KEEP(bb2_kernel<<<nb, 256, 0, s>>>(theta, theta_old, g, g_old, p_old, pvec, n, part));
-    SVP_LAUNCH_KEEP(multi_final_kernel<<<1, 256, 0, s>>>(part, nb, 4, res));
+    SVP_LAUNCH_KEEP(multi_final_kernel<<<4, 256, 0, s>>>(part, nb, 4, res));
     cudaError_t le = cudaGetLastError();
     double host[4];
     cudaError_t ce = cudaMemcpyAsync(host, res, sizeof host, cudaMemcpyDeviceToHost, s);
