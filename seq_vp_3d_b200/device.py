@@ -14,8 +14,12 @@ def require_cuda():
 
 
 def stream_ptr(stream=None):
-    s = torch.cuda.current_stream() if stream is None else stream
-    return ctypes.c_void_p(s.cuda_stream)
+    """cudaStream_t of a torch stream (default: the calling thread's current stream on its current device).  The raw
+    query costs 0.3 us where torch.cuda.current_stream() builds a Stream object in 5 us, and a registration step asks
+    about 13 times."""
+    if stream is None:
+        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return ctypes.c_void_p(stream.cuda_stream)
 
 
 def ptr(t):

@@ -242,6 +242,7 @@ class Scalars:
     def __init__(self, n=16, device="cuda"):
         self.dev = torch.zeros(n, dtype=torch.float64, device=device)
         self.host = torch.zeros(n, dtype=torch.float64).pin_memory()
+        self._done = torch.cuda.Event()
 
     def slot(self, k):
         return ctypes.c_void_p(self.dev.data_ptr() + 8 * k)
@@ -269,11 +270,13 @@ class Scalars:
     def copy_async(self, stream=None):
         """Start the copy of every slot to the host; values() waits for it (usually already done by then, when a
         later call synchronized the stream)."""
-        s = torch.cuda.current_stream() if stream is None else stream
-        with torch.cuda.stream(s):
+        if stream is None:
             self.host.copy_(self.dev, non_blocking=True)
-            self._done = torch.cuda.Event()
-            self._done.record(s)
+            self._done.record()
+        else:
+            with torch.cuda.stream(stream):
+                self.host.copy_(self.dev, non_blocking=True)
+                self._done.record(stream)
 
     def values(self):
         self._done.synchronize()
@@ -281,8 +284,5 @@ class Scalars:
 
     def fetch(self, stream=None):
         """Copy every slot to the host and wait; returns a numpy copy."""
-        s = torch.cuda.current_stream() if stream is None else stream
-        with torch.cuda.stream(s):
-            self.host.copy_(self.dev, non_blocking=True)
-        s.synchronize()
-        return self.host.numpy().copy()
+        self.copy_async(stream)
+        return self.values()
