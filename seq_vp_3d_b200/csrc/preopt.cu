@@ -11,6 +11,7 @@
 // lr m^ / (sqrt(v^) + eps); the step is scaled so that its largest entry is at most `cap` voxels; u -= step; then
 // optionally u = Gaussian(sigma_field) * u.  Everything stays on the device; the cap's scale is computed there.
 #include <cmath>
+#include <utility>
 #include <vector>
 
 #include "svp_common.cuh"
@@ -35,9 +36,19 @@ __device__ __forceinline__ float node_u(const float *__restrict__ u, int c, int 
     return u[interior_index(c, z, y, x, D, H, W)];
 }
 
+// flat index -> (x, y, z) over rows of nx and planes of ny; z counts on over stacked components
+struct Index3 {
+    int x, y, z;
+};
+__device__ __forceinline__ Index3 index3(long long i, int nx, int ny) {
+    long long x, y, z;
+    unflatten3(i, nx, ny, x, y, z);
+    return {(int)x, (int)y, (int)z};
+}
+
 // float block reduction of K sums (fixed order) -> partial[block * K + k]
 template <int K>
-__device__ void block_sum_f(float (&v)[K], float *partial) {
+__device__ void block_sum_f(float (&v)[K], float *partial, int block) {
     __shared__ float sh[PT / 32][K];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -51,7 +62,7 @@ __device__ void block_sum_f(float (&v)[K], float *partial) {
     if (threadIdx.x < K) {
         float s = 0.f;
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += sh[w][threadIdx.x];
-        partial[(size_t)blockIdx.x * K + threadIdx.x] = s;
+        partial[(size_t)block * K + threadIdx.x] = s;
     }
 }
 
@@ -70,13 +81,14 @@ __device__ __forceinline__ float sample_coord(float xi, float u, int n, float &c
 }
 
 // residual r = T(x + u) - F at every node; data gradient r dT/di chi on interior nodes into grad; sums 1/2 r^2
-__global__ void __launch_bounds__(PT) pre_data_kernel(const float *__restrict__ F, const float *__restrict__ M,
-                                                      int D, int H, int W, const float *__restrict__ u,
-                                                      float *__restrict__ grad, float *partial) {
+__device__ __forceinline__ void pre_data(const float *__restrict__ F, const float *__restrict__ M, int D, int H, int W,
+                                         const float *__restrict__ u, float *__restrict__ grad, float *partial,
+                                         int block, int blocks) {
     float acc[1] = {0.f};
     const long long n = (long long)D * H * W;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((long long)W * H));
+    for (long long i = block * (long long)PT + threadIdx.x; i < n; i += (long long)blocks * PT) {
+        const Index3 p = index3(i, W, H);
+        const int x = p.x, y = p.y, z = p.z;
         float cx, cy, cz;
         const float ix = sample_coord((float)x, node_u(u, 0, z, y, x, D, H, W), W, cx);
         const float iy = sample_coord((float)y, node_u(u, 1, z, y, x, D, H, W), H, cy);
@@ -121,21 +133,21 @@ __global__ void __launch_bounds__(PT) pre_data_kernel(const float *__restrict__ 
             grad[interior_index(2, z, y, x, D, H, W)] = r * dtz * cz;
         }
     }
-    block_sum_f<1>(acc, partial);
+    block_sum_f<1>(acc, partial, block);
 }
 
 // ---------------------------------------------------------------------------------------------- cell terms
 // Per cell: cell-centre F, det, curl, geometry and floor energies, and G_cd = dE_cell / d(voxel derivative of u_c
 // along d) (preopt_grad.py:103 cell_geometry), stored SoA G[(3 c + d) * ncell + cell]; min det reduced.
-__global__ void __launch_bounds__(PT) pre_cell_kernel(int D, int H, int W, float r01, float r02, float r10,
-                                                      float r12, float r20, float r21, float mu, float kappa,
-                                                      float j0, const float *__restrict__ u, float *__restrict__ G,
-                                                      float *partial) {
+__device__ __forceinline__ void pre_cell(int D, int H, int W, float r01, float r02, float r10, float r12, float r20,
+                                         float r21, float mu, float kappa, float j0, const float *__restrict__ u,
+                                         float *__restrict__ G, float *partial, int block, int blocks) {
     float acc[3] = {0.f, 0.f, 0.f};     // geometry, floor, -min det (as max of -det)
     float mndet = __int_as_float(0x7F800000);
     const long long cx = W - 1, cy = H - 1, cz = D - 1, ncell = cx * cy * cz;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < ncell; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % cx), y = (int)((i / cx) % cy), z = (int)(i / (cx * cy));
+    for (long long i = block * (long long)PT + threadIdx.x; i < ncell; i += (long long)blocks * PT) {
+        const Index3 at = index3(i, (int)cx, (int)cy);
+        const int x = at.x, y = at.y, z = at.z;
         float v[3][2][2][2];
 #pragma unroll
         for (int c = 0; c < 3; c++)
@@ -191,23 +203,23 @@ __global__ void __launch_bounds__(PT) pre_cell_kernel(int D, int H, int W, float
 #pragma unroll
     for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, o));
     if ((threadIdx.x & 31) == 0) shm[threadIdx.x >> 5] = mx;
-    block_sum_f<2>(s2, partial);         // contains a __syncthreads
+    block_sum_f<2>(s2, partial, block);         // contains a __syncthreads
     if (threadIdx.x == 0) {
         float m = shm[0];
         for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmaxf(m, shm[w]);
-        partial[(size_t)gridDim.x * 2 + blockIdx.x] = m;
+        partial[(size_t)blocks * 2 + block] = m;
     }
 }
 
 // seven-point Laplacian (physical) of u, times h_c, on interior nodes (zero faces); sums 1/2 lap^2
-__global__ void __launch_bounds__(PT) pre_lap_kernel(int D, int H, int W, float ihx2, float ihy2, float ihz2,
-                                                     float hx, float hy, float hz, const float *__restrict__ u,
-                                                     float *__restrict__ lap, float *partial) {
+__device__ __forceinline__ void pre_lap(int D, int H, int W, float ihx2, float ihy2, float ihz2, float hx, float hy,
+                                        float hz, const float *__restrict__ u, float *__restrict__ lap, float *partial,
+                                        int block, int blocks) {
     float acc[1] = {0.f};
     const long long n = 3LL * (D - 2) * (H - 2) * (W - 2);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % (W - 2)) + 1, y = (int)((i / (W - 2)) % (H - 2)) + 1;
-        const int z = (int)((i / ((long long)(W - 2) * (H - 2))) % (D - 2)) + 1, c = (int)(i / ((long long)(W - 2) * (H - 2) * (D - 2)));
+    for (long long i = block * (long long)PT + threadIdx.x; i < n; i += (long long)blocks * PT) {
+        const Index3 p = index3(i, W - 2, H - 2);
+        const int x = p.x + 1, y = p.y + 1, z = p.z % (D - 2) + 1, c = p.z / (D - 2);
         const float ui = u[i];
         const float lz = (node_u(u, c, z + 1, y, x, D, H, W) - 2.f * ui + node_u(u, c, z - 1, y, x, D, H, W)) * ihz2;
         const float ly = (node_u(u, c, z, y + 1, x, D, H, W) - 2.f * ui + node_u(u, c, z, y - 1, x, D, H, W)) * ihy2;
@@ -216,7 +228,27 @@ __global__ void __launch_bounds__(PT) pre_lap_kernel(int D, int H, int W, float 
         lap[i] = l;
         acc[0] += .5f * l * l;
     }
-    block_sum_f<1>(acc, partial);
+    block_sum_f<1>(acc, partial, block);
+}
+
+// The data term, the cell terms and the Laplacian read u and write arrays of their own, so they run as one launch:
+// blocks 0 .. bd - 1, the next bc, the next bl (each part's own grid, so its block sums are those of a launch by
+// itself).  On the pyramid's coarse levels each part alone leaves most of the SMs idle.
+struct PreTerms {
+    const float *F, *M, *u;
+    int D, H, W, bd, bc, bl;
+    float r01, r02, r10, r12, r20, r21, mu, kappa, j0, ihx2, ihy2, ihz2, hx, hy, hz;
+    float *grad, *G, *lap, *pd, *pc, *pl;
+};
+__global__ void __launch_bounds__(PT) pre_terms_kernel(const __grid_constant__ PreTerms a) {
+    const int b = blockIdx.x;
+    if (b < a.bd)
+        pre_data(a.F, a.M, a.D, a.H, a.W, a.u, a.grad, a.pd, b, a.bd);
+    else if (b < a.bd + a.bc)
+        pre_cell(a.D, a.H, a.W, a.r01, a.r02, a.r10, a.r12, a.r20, a.r21, a.mu, a.kappa, a.j0, a.u, a.G, a.pc, b - a.bd,
+                 a.bc);
+    else
+        pre_lap(a.D, a.H, a.W, a.ihx2, a.ihy2, a.ihz2, a.hx, a.hy, a.hz, a.u, a.lap, a.pl, b - a.bd - a.bc, a.bl);
 }
 
 // interior-node gradient: data part (already in grad) + the 8 cells' G (+-1/4 per axis) + alpha h_c Delta_h lap
@@ -227,8 +259,8 @@ __global__ void __launch_bounds__(PT) pre_node_kernel(int D, int H, int W, const
     const long long n = 3LL * (D - 2) * (H - 2) * (W - 2);
     const long long cx = W - 1, cy = H - 1, ncell = cx * cy * (D - 1);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(i % (W - 2)) + 1, y = (int)((i / (W - 2)) % (H - 2)) + 1;
-        const int z = (int)((i / ((long long)(W - 2) * (H - 2))) % (D - 2)) + 1, c = (int)(i / ((long long)(W - 2) * (H - 2) * (D - 2)));
+        const Index3 p = index3(i, W - 2, H - 2);
+        const int x = p.x + 1, y = p.y + 1, z = p.z % (D - 2) + 1, c = p.z / (D - 2);
         float g = 0.f;
 #pragma unroll
         for (int a = 0; a < 8; a++) {
@@ -269,17 +301,103 @@ __global__ void __launch_bounds__(PT) gauss_axis_kernel(const float *__restrict_
         for (int j = -r; j <= r; j++) {
             int q = pos + j;
             q = q < 0 ? 0 : (q > len - 1 ? len - 1 : q);
-            s += k[j + r] * in[base + (long long)q * st];
+            s = __fmaf_rn(k[j + r], in[base + (long long)q * st], s);
         }
         out[i] = s;
     }
 }
 
-// Adam moments and step (the update itself waits for the largest entry): step into `step`, block maxima of |step|
+// The three axes (z, then y, then x) in one pass for radii R up to 3.  A warp row is 32 wide with its halo, so a block's
+// tile is (32 - 2R) x (16 - 2R) x 8: a thread filters its z column from registers as it is loaded, then its y column
+// from shared memory, then x.  Indexes are clamped to the array as they are loaded (a clamped row's filtered value is
+// the filtered clamped row, so the padding is that of the separate passes), and each value goes through the same
+// products and sums in the same order as three gauss_axis_kernel passes, so the bits are theirs.  UPDATE: the input is
+// in[i] - step[i] scale, formed as it is loaded.
+// Bound: L2 and launches.  The smoothings of a four-level 96^3 pyramid's 260 iterations: 12.5 ms in 1,560 passes, 3.6
+// ms in 520 of these.
+constexpr int GZ = 8;
+// scale = 1 if largest <= cap else cap / largest (double, then float as PyTorch's float32 scalar)
+__device__ __forceinline__ float cap_scale(const unsigned *largest_bits, double cap) {
+    const double largest = (double)__uint_as_float(*largest_bits);
+    return (float)(largest <= cap ? 1. : cap / largest);
+}
+template <int R, bool UPDATE>
+__global__ void __launch_bounds__(PT) gauss3_kernel(const float *__restrict__ in, const float *__restrict__ step,
+                                                    const unsigned *__restrict__ largest, double cap,
+                                                    float *__restrict__ out, int d0, int d1, int d2,
+                                                    const float *__restrict__ taps, int tx, int ty, int tz) {
+    constexpr int GX = 32 - 2 * R, GY = 16 - 2 * R, N = 2 * R + 1;
+    __shared__ float B[GZ][16][32], C[GZ][GY][32 + 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float k[N];
+#pragma unroll
+    for (int j = 0; j < N; j++) k[j] = taps[j];
+    const float scale = UPDATE ? cap_scale(largest, cap) : 1.f;
+    int t = blockIdx.x;
+    const int bx = t % tx * GX; t /= tx;
+    const int by = t % ty * GY; t /= ty;
+    const int bz = t % tz * GZ, c = t / tz;
+    const long long plane = (long long)d1 * d2, base = (long long)c * d0 * plane;
+    const int x = min(max(bx + lane - R, 0), d2 - 1);
+#pragma unroll
+    for (int iy = warp; iy < 16; iy += PT / 32) {
+        const long long col = base + (long long)min(max(by + iy - R, 0), d1 - 1) * d2 + x;
+        float v[GZ + 2 * R];
+#pragma unroll
+        for (int i = 0; i < GZ + 2 * R; i++) {
+            const long long at = col + min(max(bz + i - R, 0), d0 - 1) * plane;
+            v[i] = UPDATE ? __fmaf_rn(-step[at], scale, in[at]) : in[at];
+        }
+#pragma unroll
+        for (int i = 0; i < GZ; i++) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < N; j++) s = __fmaf_rn(k[j], v[i + j], s);
+            B[i][iy][lane] = s;
+        }
+    }
+    __syncthreads();
+    {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = B[warp][i][lane];
+#pragma unroll
+        for (int i = 0; i < GY; i++) {
+            float s = 0.f;
+#pragma unroll
+            for (int j = 0; j < N; j++) s = __fmaf_rn(k[j], v[i + j], s);
+            C[warp][i][lane] = s;
+        }
+    }
+    __syncwarp();            // the x pass reads the warp's own plane
+    const int z = bz + warp;
+    if (z >= d0 || lane >= GX || bx + lane >= d2) return;
+#pragma unroll
+    for (int i = 0; i < GY; i++) {
+        if (by + i >= d1) break;
+        float s = 0.f;
+#pragma unroll
+        for (int j = 0; j < N; j++) s = __fmaf_rn(k[j], C[warp][i][lane + j], s);
+        out[base + z * plane + (long long)(by + i) * d2 + bx + lane] = s;
+    }
+}
+static_assert(GZ == PT / 32, "one z plane per warp in the y and x passes");
+template <bool UPDATE>
+void launch_gauss3(int r, const float *in, const float *step, const unsigned *largest, double cap, float *out, int d0,
+                   int d1, int d2, const float *taps, cudaStream_t s) {
+    const int tx = (d2 + 31 - 2 * r) / (32 - 2 * r), ty = (d1 + 15 - 2 * r) / (16 - 2 * r), tz = (d0 + GZ - 1) / GZ;
+    const unsigned tiles = (unsigned)(3LL * tx * ty * tz);
+    if (r == 1) SVP_LAUNCH_KEEP(gauss3_kernel<1, UPDATE><<<tiles, PT, 0, s>>>(in, step, largest, cap, out, d0, d1, d2, taps, tx, ty, tz));
+    else if (r == 2) SVP_LAUNCH_KEEP(gauss3_kernel<2, UPDATE><<<tiles, PT, 0, s>>>(in, step, largest, cap, out, d0, d1, d2, taps, tx, ty, tz));
+    else SVP_LAUNCH_KEEP(gauss3_kernel<3, UPDATE><<<tiles, PT, 0, s>>>(in, step, largest, cap, out, d0, d1, d2, taps, tx, ty, tz));
+}
+
+// Adam moments and step (the update itself waits for the largest entry): step into `step`, the bits of the largest
+// |step| (ordered as integers) into *largest, which starts at zero
 __global__ void __launch_bounds__(PT) adam_kernel(long long n, const float *__restrict__ g, float *__restrict__ m,
                                                   float *__restrict__ v, float b1, float ob1, float b2, float ob2,
                                                   float lr, float rc1, float rc2, float eps, float *__restrict__ step,
-                                                  float *partial) {
+                                                  unsigned *largest) {
     float mx = 0.f;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float gi = g[i];
@@ -297,36 +415,18 @@ __global__ void __launch_bounds__(PT) adam_kernel(long long n, const float *__re
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = mx;
     __syncthreads();
     if (threadIdx.x == 0) {
-        float r = sh[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) r = fmaxf(r, sh[w]);
-        partial[blockIdx.x] = r;
+        for (int w = 1; w < (int)(blockDim.x >> 5); w++) mx = fmaxf(mx, sh[w]);
+        atomicMax(largest, __float_as_uint(mx));
     }
 }
 
-// scale = 1 if largest <= cap else cap / largest (double, then float as PyTorch's float32 scalar); counts cap hits
-__global__ void cap_kernel(const float *partial, int blocks, double cap, float *scale, unsigned long long *hits) {
-    __shared__ float sh[PT];
-    float m = 0.f;
-    for (int b = threadIdx.x; b < blocks; b += blockDim.x) m = fmaxf(m, partial[b]);
-    sh[threadIdx.x] = m;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s; s >>= 1) {
-        if ((int)threadIdx.x < s) sh[threadIdx.x] = fmaxf(sh[threadIdx.x], sh[threadIdx.x + s]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const double largest = (double)sh[0];
-        const double sc = largest <= cap ? 1. : cap / largest;
-        *scale = (float)sc;
-        if (sc < 1.) *hits += 1;
-    }
-}
-
+// u -= step * scale, for a field that is not smoothed or whose radius the fused pass does not take
 __global__ void __launch_bounds__(PT) update_kernel(long long n, const float *__restrict__ step,
-                                                    const float *__restrict__ scale, float *__restrict__ u) {
-    const float s = *scale;
+                                                    const unsigned *__restrict__ largest, double cap,
+                                                    float *__restrict__ u) {
+    const float s = cap_scale(largest, cap);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        u[i] = u[i] - step[i] * s;
+        u[i] = __fmaf_rn(-step[i], s, u[i]);
 }
 
 // terms[it * 6 + k] = data, geometry, floor, curvature, min det, total (from the block partials of one iteration)
@@ -411,7 +511,8 @@ struct PreWork {
     unsigned bd = 0, bc = 0, bl = 0;
 };
 
-// one evaluation of the pre-objective's gradient (and its terms into terms_dev[6], device)
+// one evaluation of the pre-objective's gradient (and, with terms_dev, its six terms there: one thread's sums in block
+// order, 35 us, so an iteration whose terms nobody sees leaves them out)
 int pre_gradient(const float *F, const float *M, int D, int H, int W, const double h[3], const float *u, double mu,
                  double alpha, double kappa, double j0, float *grad, float *terms_dev, PreWork &w, cudaStream_t s) {
     const long long nn = (long long)D * H * W, nc = (long long)(D - 1) * (H - 1) * (W - 1);
@@ -420,11 +521,18 @@ int pre_gradient(const float *F, const float *M, int D, int H, int W, const doub
     const float r01 = (float)(h[0] / h[1]), r02 = (float)(h[0] / h[2]), r10 = (float)(h[1] / h[0]);
     const float r12 = (float)(h[1] / h[2]), r20 = (float)(h[2] / h[0]), r21 = (float)(h[2] / h[1]);
     const float ihx2 = (float)(1. / (h[0] * h[0])), ihy2 = (float)(1. / (h[1] * h[1])), ihz2 = (float)(1. / (h[2] * h[2]));
-    { svp::KernelTimer _t("pre_data_kernel", s); SVP_LAUNCH(pre_data_kernel<<<w.bd, PT, 0, s>>>(F, M, D, H, W, u, grad, pd)); }
-    { svp::KernelTimer _t("pre_cell_kernel", s); SVP_LAUNCH(pre_cell_kernel<<<w.bc, PT, 0, s>>>(D, H, W, r01, r02, r10, r12, r20, r21, (float)mu, (float)kappa, (float)j0, u, w.G, pc)); }
-    if (alpha > 0) SVP_LAUNCH(pre_lap_kernel<<<w.bl, PT, 0, s>>>(D, H, W, ihx2, ihy2, ihz2, (float)h[0], (float)h[1], (float)h[2], u, w.lap, pl));
+    PreTerms t;
+    t.F = F; t.M = M; t.u = u;
+    t.D = D; t.H = H; t.W = W; t.bd = (int)w.bd; t.bc = (int)w.bc; t.bl = alpha > 0 ? (int)w.bl : 0;
+    t.r01 = r01; t.r02 = r02; t.r10 = r10; t.r12 = r12; t.r20 = r20; t.r21 = r21;
+    t.mu = (float)mu; t.kappa = (float)kappa; t.j0 = (float)j0;
+    t.ihx2 = ihx2; t.ihy2 = ihy2; t.ihz2 = ihz2; t.hx = (float)h[0]; t.hy = (float)h[1]; t.hz = (float)h[2];
+    t.grad = grad; t.G = w.G; t.lap = w.lap; t.pd = pd; t.pc = pc; t.pl = pl;
+    { svp::KernelTimer _t("pre_terms_kernel", s); SVP_LAUNCH(pre_terms_kernel<<<(unsigned)(t.bd + t.bc + t.bl), PT, 0, s>>>(t)); }
     { svp::KernelTimer _t("pre_node_kernel", s); SVP_LAUNCH(pre_node_kernel<<<grid_for(ni), PT, 0, s>>>(D, H, W, w.G, w.lap, (float)alpha, ihx2, ihy2, ihz2, (float)h[0], (float)h[1], (float)h[2], grad)); }
-    SVP_LAUNCH(terms_kernel<<<1, 1, 0, s>>>(pd, w.bd, pc, w.bc, pl, alpha > 0 ? w.bl : 0, (float)mu, (float)kappa, (float)alpha, terms_dev));
+    if (terms_dev)
+        SVP_LAUNCH(terms_kernel<<<1, 1, 0, s>>>(pd, w.bd, pc, w.bc, pl, alpha > 0 ? w.bl : 0, (float)mu, (float)kappa,
+                                                (float)alpha, terms_dev));
     SVP_LAUNCH_CHECK("pre-objective gradient");
     (void)nn; (void)nc;
     return SVP_OK;
@@ -494,16 +602,15 @@ extern "C" int svp_pre_level(const float *fixed, const float *moving, int32_t D,
     PreWork w;
     int rc = pre_alloc(D, H, W, w, s);
     if (rc) return rc;
-    float *grad = nullptr, *tmp = nullptr, *step = nullptr, *taps = nullptr, *scale = nullptr, *terms = nullptr;
-    float *apart = nullptr;
-    unsigned long long *hits = nullptr;
+    float *grad = nullptr, *tmp = nullptr, *aux = nullptr, *step = nullptr, *taps = nullptr, *terms = nullptr;
+    unsigned *largest = nullptr;         // per iteration, the bits of the largest |step|
     const unsigned ab = grid_for(ni);
     std::vector<float> kg = gauss_taps(prm->sigma_grad > 0 ? prm->sigma_grad : 1.);
     std::vector<float> kf = gauss_taps(prm->sigma_field > 0 ? prm->sigma_field : 1.);
     const int rg = (int)(kg.size() / 2), rf = (int)(kf.size() / 2);
     auto bail = [&](int code) {
-        for (void *p : {(void *)grad, (void *)tmp, (void *)step, (void *)taps, (void *)scale, (void *)terms,
-                        (void *)apart, (void *)hits})
+        for (void *p : {(void *)grad, (void *)tmp, (void *)aux, (void *)step, (void *)taps, (void *)terms,
+                        (void *)largest})
             if (p) scratch_free(p, s);
         pre_free(w, s);
         return code;
@@ -511,49 +618,67 @@ extern "C" int svp_pre_level(const float *fixed, const float *moving, int32_t D,
     if (scratch_alloc((void **)&grad, sizeof(float) * ni, s) || scratch_alloc((void **)&tmp, sizeof(float) * ni, s) ||
         scratch_alloc((void **)&step, sizeof(float) * ni, s) ||
         scratch_alloc((void **)&taps, sizeof(float) * (kg.size() + kf.size()), s) ||
-        scratch_alloc((void **)&scale, sizeof(float), s) ||
-        scratch_alloc((void **)&terms, sizeof(float) * 12, s) || scratch_alloc((void **)&apart, sizeof(float) * ab, s) ||
-        scratch_alloc((void **)&hits, sizeof(unsigned long long), s))
+        scratch_alloc((void **)&aux, sizeof(float) * ni, s) ||
+        scratch_alloc((void **)&terms, sizeof(float) * 12, s) || 
+        scratch_alloc((void **)&largest, sizeof(unsigned) * (iterations + 1), s))
         return bail(fail(SVP_ENOMEM, "svp_pre_level: scratch"));
     if (cudaMemcpyAsync(taps, kg.data(), sizeof(float) * kg.size(), cudaMemcpyHostToDevice, s) ||
         cudaMemcpyAsync(taps + kg.size(), kf.data(), sizeof(float) * kf.size(), cudaMemcpyHostToDevice, s) ||
-        cudaMemsetAsync(hits, 0, sizeof(unsigned long long), s) || cudaMemsetAsync(terms, 0, sizeof(float) * 12, s))
+        cudaMemsetAsync(largest, 0, sizeof(unsigned) * (iterations + 1), s) || cudaMemsetAsync(terms, 0, sizeof(float) * 12, s))
         return bail(fail(SVP_ECUDA, "svp_pre_level: setup copies"));
     const int dz = D - 2, dy = H - 2, dx = W - 2;
-    auto smooth = [&](float *x, const float *k, int r) -> int {
-        // z, then y, then x; x -> tmp -> x -> tmp -> ... ending in x
+    auto smooth = [&](float *x, const float *k, int r) {
+        // z, then y, then x; x -> tmp -> step (free here) -> x
         SVP_LAUNCH_KEEP(gauss_axis_kernel<<<grid_for(ni), PT, 0, s>>>(x, tmp, dz, dy, dx, 0, k, r));
         SVP_LAUNCH_KEEP(gauss_axis_kernel<<<grid_for(ni), PT, 0, s>>>(tmp, step, dz, dy, dx, 1, k, r));
         SVP_LAUNCH_KEEP(gauss_axis_kernel<<<grid_for(ni), PT, 0, s>>>(step, x, dz, dy, dx, 2, k, r));
-        return SVP_OK;
     };
+    constexpr int kFused = 3;            // the largest radius of the fused smoothing
+    float *u = u_int, *other = aux;      // the fused field pass goes from one to the other
     for (int it = 0; it < iterations; it++) {
-        float *tdev = terms + (it == 0 ? 0 : 6);
-        if ((rc = pre_gradient(fixed, moving, D, H, W, h, u_int, prm->mu, prm->alpha, prm->kappa, prm->j0, grad, tdev,
-                               w, s)))
+        // the record has the first and the last iteration's terms
+        float *tdev = it == 0 ? terms : (it == iterations - 1 ? terms + 6 : nullptr);
+        if ((rc = pre_gradient(fixed, moving, D, H, W, h, u, prm->mu, prm->alpha, prm->kappa, prm->j0, grad, tdev, w, s)))
             return bail(rc);
-        if (prm->sigma_grad > 0) smooth(grad, taps, rg);
+        float *g = grad;
+        if (prm->sigma_grad > 0) {
+            if (rg <= kFused) {
+                launch_gauss3<false>(rg, grad, nullptr, nullptr, 0., tmp, dz, dy, dx, taps, s);
+                g = tmp;
+            } else {
+                smooth(grad, taps, rg);
+            }
+        }
         const int t = first_iteration + it + 1;
         // PyTorch divides by the float bias corrections as a multiplication by their float32 reciprocals
         const float rc1 = 1.f / (float)(1. - std::pow(prm->beta1, t));
         const float rc2 = 1.f / (float)(1. - std::pow(prm->beta2, t));
-        { svp::KernelTimer _t("adam_kernel", s); SVP_LAUNCH_KEEP(adam_kernel<<<ab, PT, 0, s>>>(ni, grad, m, v, (float)prm->beta1, (float)(1. - prm->beta1), (float)prm->beta2, (float)(1. - prm->beta2), (float)prm->lr, rc1, rc2, (float)prm->eps, step, apart)); }
-        SVP_LAUNCH_KEEP(cap_kernel<<<1, PT, 0, s>>>(apart, (int)ab, prm->cap, scale, hits));
-        SVP_LAUNCH_KEEP(update_kernel<<<ab, PT, 0, s>>>(ni, step, scale, u_int));
-        if (prm->sigma_field > 0) smooth(u_int, taps + kg.size(), rf);
+        { svp::KernelTimer _t("adam_kernel", s); SVP_LAUNCH_KEEP(adam_kernel<<<ab, PT, 0, s>>>(ni, g, m, v, (float)prm->beta1, (float)(1. - prm->beta1), (float)prm->beta2, (float)(1. - prm->beta2), (float)prm->lr, rc1, rc2, (float)prm->eps, step, largest + it)); }
+        if (prm->sigma_field > 0 && rf <= kFused) {
+            launch_gauss3<true>(rf, u, step, largest + it, prm->cap, other, dz, dy, dx, taps + kg.size(), s);
+            std::swap(u, other);
+        } else {
+            SVP_LAUNCH_KEEP(update_kernel<<<ab, PT, 0, s>>>(ni, step, largest + it, prm->cap, u));
+            if (prm->sigma_field > 0) smooth(u, taps + kg.size(), rf);
+        }
         cudaError_t le = cudaGetLastError();
         if (le != cudaSuccess) return bail(cuda_fail(le, "pre-optimizer iteration"));
     }
-    unsigned long long h_hits = 0;
+    if (u != u_int && cudaMemcpyAsync(u_int, u, sizeof(float) * ni, cudaMemcpyDeviceToDevice, s))
+        return bail(fail(SVP_ECUDA, "svp_pre_level: field copy"));
+    std::vector<float> most((size_t)iterations + 1);
     float th[12];
     if (cudaMemcpyAsync(th, terms, sizeof th, cudaMemcpyDeviceToHost, s) ||
-        cudaMemcpyAsync(&h_hits, hits, sizeof h_hits, cudaMemcpyDeviceToHost, s))
+        cudaMemcpyAsync(most.data(), largest, sizeof(float) * most.size(), cudaMemcpyDeviceToHost, s))
         return bail(fail(SVP_ECUDA, "svp_pre_level: result copies"));
     rc = bail(SVP_OK);
     SVP_CUDA(cudaStreamSynchronize(s));
     if (terms_first) for (int k = 0; k < 6; k++) terms_first[k] = th[k];
     if (terms_last) for (int k = 0; k < 6; k++) terms_last[k] = iterations > 1 ? th[6 + k] : th[k];
-    if (cap_hits) *cap_hits = (int64_t)h_hits;
+    if (cap_hits) {
+        *cap_hits = 0;
+        for (float x : most) *cap_hits += (double)x > prm->cap;     // the iterations whose step was scaled
+    }
     return rc;
 }
 
