@@ -927,51 +927,54 @@ static std::vector<double> cached_dst1_half(int n) {
     return H;
 }
 
-int pair_dst_setup(svp_pair *p) {
+void pair_dst_carve(svp_pair *p, SlabCursor &c) {
     const long long f[3] = {p->q.fx, p->q.fy, p->q.fz};
     for (int k = 0; k < 3; k++) {
-        std::vector<double> H = cached_dst1_half((int)f[k]);
-        SVP_CUDA(cudaMalloc((void **)&p->dst_half[k], sizeof(double) * H.size()));
-        SVP_CUDA(cudaMemcpy(p->dst_half[k], H.data(), sizeof(double) * H.size(), cudaMemcpyHostToDevice));
-        {
-            int kg[2], ipad[2], kpad[2];
-            const long long words = pad_geometry(k, (int)f[k], kg, ipad, kpad) / 2;
-            SVP_CUDA(cudaMalloc((void **)&p->dst_pad[k], sizeof(double) * words));
-            const PadF64 T = pad_f64(p->dst_pad[k], k, (int)f[k]);
-            for (int g = 0; g < 2; g++) {
-                pad_half_kernel<<<blocks_for((long long)ipad[g] * kpad[g], 256, 4), 256>>>(
-                    p->dst_half[k], kg[g], g ? (long long)kg[0] * kg[0] : 0, k != 0, ipad[g], kpad[g],
-                    const_cast<double *>(T.h[g]));
-                SVP_CUDA(cudaGetLastError());
-            }
-            SVP_CUDA(cudaStreamSynchronize(0));
-        }
-        // the mixed form's matrices: rounded once to float32, then split into TF32 parts on the device (the same
-        // cvt.rna the passes use for their staged operands)
-        std::vector<float> H32(H.begin(), H.end());
-        float *h32 = nullptr;
-        SVP_CUDA(cudaMalloc((void **)&h32, sizeof(float) * H32.size()));
-        cudaError_t e = cudaMemcpy(h32, H32.data(), sizeof(float) * H32.size(), cudaMemcpyHostToDevice);
         int kg[2], ipad[2], kpad[2];
         const long long words = pad_geometry(k, (int)f[k], kg, ipad, kpad);
-        if (e == cudaSuccess) e = cudaMalloc((void **)&p->dst_tf32[k], sizeof(unsigned) * words);
-        if (e == cudaSuccess) {
-            const PadTf32 T = pad_tf32(p->dst_tf32[k], k, (int)f[k]);
-            for (int g = 0; g < 2 && e == cudaSuccess; g++) {
-                const long long src = g ? (long long)kg[0] * kg[0] : 0;
-                split_pad_kernel<<<blocks_for((long long)ipad[g] * kpad[g], 256, 4), 256>>>(
-                    h32, kg[g], src, k != 0, ipad[g], kpad[g], const_cast<unsigned *>(T.b[g]),
-                    const_cast<unsigned *>(T.s[g]));
-                e = cudaGetLastError();
-            }
-        }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-        cudaFree(h32);
-        if (e != cudaSuccess) return cuda_fail(e, "dst tf32 split");
+        c.take(p->dst_pad[k], (size_t)words / 2);
+        c.take(p->dst_tf32[k], (size_t)words);
+    }
+    c.take(p->dst_tmp, (size_t)(2 * 3 * p->q.nfree));
+    c.take(p->den, (size_t)p->q.nfree);
+}
+
+// Fills the padded matrices: the folded half matrices of the three axes, and their values rounded once to float32, go
+// up in one copy each and are laid out (and split into TF32 parts with the cvt.rna of the passes) on the device.
+int pair_dst_setup(svp_pair *p, cudaStream_t s) {
+    const long long f[3] = {p->q.fx, p->q.fy, p->q.fz};
+    std::vector<double> all;
+    size_t off[3];
+    for (int k = 0; k < 3; k++) {
+        const std::vector<double> H = cached_dst1_half((int)f[k]);
+        off[k] = all.size();
+        all.insert(all.end(), H.begin(), H.end());
         p->dst_n[k] = (int)f[k];
     }
-    SVP_CUDA(cudaMalloc((void **)&p->dst_tmp, sizeof(double) * 2 * 3 * p->q.nfree));
-    SVP_CUDA(cudaMalloc((void **)&p->den, sizeof(double) * p->q.nfree));
+    const std::vector<float> all32(all.begin(), all.end());
+    double *h = nullptr;
+    SVP_CUDA(scratch_alloc((void **)&h, (sizeof(double) + sizeof(float)) * all.size(), s));
+    float *h32 = reinterpret_cast<float *>(h + all.size());
+    cudaError_t e = cudaMemcpyAsync(h, all.data(), sizeof(double) * all.size(), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(h32, all32.data(), sizeof(float) * all32.size(), cudaMemcpyHostToDevice, s);
+    for (int k = 0; k < 3 && e == cudaSuccess; k++) {
+        const PadF64 D = pad_f64(p->dst_pad[k], k, (int)f[k]);
+        const PadTf32 T = pad_tf32(p->dst_tf32[k], k, (int)f[k]);
+        for (int g = 0; g < 2; g++) {
+            const unsigned nb = blocks_for((long long)D.ipad[g] * D.kpad[g], 256, 4);
+            const long long src = (long long)off[k] + (g ? (long long)D.kg[0] * D.kg[0] : 0);
+            pad_half_kernel<<<nb, 256, 0, s>>>(h, D.kg[g], src, k != 0, D.ipad[g], D.kpad[g],
+                                               const_cast<double *>(D.h[g]));
+            split_pad_kernel<<<nb, 256, 0, s>>>(h32, D.kg[g], src, k != 0, D.ipad[g], D.kpad[g],
+                                                const_cast<unsigned *>(T.b[g]), const_cast<unsigned *>(T.s[g]));
+        }
+        e = cudaGetLastError();
+    }
+    const cudaError_t fe = scratch_free(h, s), se = cudaStreamSynchronize(s);   // the host copies must outlive theirs
+    if (e != cudaSuccess) return cuda_fail(e, "DST matrices");
+    if (fe != cudaSuccess) return cuda_fail(fe, "DST matrices free");
+    if (se != cudaSuccess) return cuda_fail(se, "DST matrices");
     return SVP_OK;
 }
 

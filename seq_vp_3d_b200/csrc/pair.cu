@@ -12,7 +12,6 @@
 namespace svp {
 int apply_axis(const double *M, int axis, long long batch, long long n2, long long n1, long long n0,
                const double *in, double *out, cudaStream_t s);
-int pair_dst_setup(svp_pair *p);
 
 namespace {
 
@@ -184,12 +183,7 @@ using namespace svp;
 
 extern "C" int svp_pair_destroy(svp_pair *p) {
     if (!p) return SVP_OK;
-    cudaFree(p->fixed); cudaFree(p->coeff); cudaFree(p->u_ref);
-    for (int k = 0; k < 3; k++) {
-        cudaFree(p->knots[k]); cudaFree(p->spline_rcp[k]); cudaFree(p->dst_half[k]); cudaFree(p->dst_pad[k]); cudaFree(p->dst_tf32[k]);
-    }
-    cudaFree(p->loc1); cudaFree(p->loc2); cudaFree(p->cellbuf); cudaFree(p->partial); cudaFreeHost(p->host);
-    cudaFree(p->counter); cudaFree(p->cand); cudaFree(p->flags); cudaFree(p->dst_tmp); cudaFree(p->den);
+    cudaFree(p->slab); cudaFree(p->loc1); cudaFree(p->loc2); cudaFree(p->cand); cudaFreeHost(p->host);
     delete p;
     return SVP_OK;
 }
@@ -215,14 +209,27 @@ extern "C" int svp_pair_create(const svp_grid *g, const svp_weights *w, const do
         return rc;
     };
     cudaError_t e;
-    if ((e = cudaMalloc((void **)&p->fixed, sizeof(double) * nn)) != cudaSuccess) return bail(cuda_fail(e, "fixed"));
-    if ((e = cudaMalloc((void **)&p->coeff, sizeof(double) * nn)) != cudaSuccess) return bail(cuda_fail(e, "coeff"));
-    if ((e = cudaMalloc((void **)&p->u_ref, sizeof(double) * 3 * nn)) != cudaSuccess) return bail(cuda_fail(e, "uref"));
-    if ((e = cudaMalloc((void **)&p->cellbuf, sizeof(double) * p->q.ncell)) != cudaSuccess)
-        return bail(cuda_fail(e, "cellbuf"));
+    const long long len[3] = {g->nx, g->ny, g->nz};
+    const double org[3] = {g->x0, g->y0, g->z0}, h[3] = {g->hx, g->hy, g->hz};
+    // carve the slab: a first pass counts, the second hands out the pieces
+    for (int pass = 0; pass < 2; pass++) {
+        SlabCursor c{p->slab};
+        c.take(p->fixed, (size_t)nn);
+        c.take(p->coeff, (size_t)nn);
+        c.take(p->u_ref, (size_t)(3 * nn));
+        c.take(p->cellbuf, (size_t)p->q.ncell);
+        c.take(p->counter, 8);
+        c.take(p->partial, (size_t)pair_partial_count(p->q));
+        c.take(p->flags, (size_t)p->q.ncell);
+        for (int k = 0; k < 3; k++) {
+            c.take(p->knots[k], (size_t)(len[k] + 4));
+            c.take(p->spline_rcp[k], (size_t)(14 * len[k]));
+        }
+        pair_dst_carve(p, c);
+        if (pass == 0 && (e = cudaMalloc((void **)&p->slab, c.used)) != cudaSuccess)
+            return bail(cuda_fail(e, "pair arrays"));
+    }
     if ((e = cudaMallocHost((void **)&p->host, sizeof(double) * 64)) != cudaSuccess) return bail(cuda_fail(e, "results"));
-    if ((e = cudaMalloc((void **)&p->counter, sizeof(long long) * 8)) != cudaSuccess)
-        return bail(cuda_fail(e, "counter"));
     if ((e = cudaMemsetAsync(p->counter, 0, sizeof(long long) * 8, s)) != cudaSuccess)
         return bail(cuda_fail(e, "counter"));
     if ((e = cudaMemcpyAsync(p->fixed, fixed, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
@@ -230,22 +237,17 @@ extern "C" int svp_pair_create(const svp_grid *g, const svp_weights *w, const do
     if ((e = cudaMemcpyAsync(p->u_ref, u_ref, sizeof(double) * 3 * nn, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
         return bail(cuda_fail(e, "u_ref copy"));
     // knots and spline coefficients: prefilter z, then y, then x (the reference's axis order)
-    const long long len[3] = {g->nx, g->ny, g->nz};
-    const double org[3] = {g->x0, g->y0, g->z0}, h[3] = {g->hx, g->hy, g->hz};
-    std::vector<double> inv[3];
+    std::vector<double> inv[3], t[3], rcp[3];
     for (int k = 0; k < 3; k++) {
         std::vector<double> x((size_t)len[k]);
         for (long long i = 0; i < len[k]; i++) x[(size_t)i] = org[k] + h[k] * (double)i;
-        std::vector<double> t = not_a_knot(x);
-        if ((e = cudaMalloc((void **)&p->knots[k], sizeof(double) * t.size())) != cudaSuccess)
-            return bail(cuda_fail(e, "knots"));
-        if ((e = cudaMemcpy(p->knots[k], t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice)) != cudaSuccess)
-            return bail(cuda_fail(e, "knots copy"));
-        std::vector<double> rcp = spline_reciprocals(t, len[k]);
-        if ((e = cudaMalloc((void **)&p->spline_rcp[k], sizeof(double) * rcp.size())) != cudaSuccess)
-            return bail(cuda_fail(e, "spline reciprocals"));
-        if ((e = cudaMemcpy(p->spline_rcp[k], rcp.data(), sizeof(double) * rcp.size(), cudaMemcpyHostToDevice)) !=
+        t[k] = not_a_knot(x);
+        if ((e = cudaMemcpyAsync(p->knots[k], t[k].data(), sizeof(double) * t[k].size(), cudaMemcpyHostToDevice, s)) !=
             cudaSuccess)
+            return bail(cuda_fail(e, "knots copy"));
+        rcp[k] = spline_reciprocals(t[k], len[k]);
+        if ((e = cudaMemcpyAsync(p->spline_rcp[k], rcp[k].data(), sizeof(double) * rcp[k].size(),
+                                 cudaMemcpyHostToDevice, s)) != cudaSuccess)
             return bail(cuda_fail(e, "spline reciprocals copy"));
         inv[k] = cached_inverse_collocation(x);
     }
@@ -274,7 +276,7 @@ extern "C" int svp_pair_create(const svp_grid *g, const svp_weights *w, const do
     if (tmp) scratch_free(tmp, s);
     cudaStreamSynchronize(s);      // the host matrices above must outlive their copies
     if (rc) return bail(rc);
-    if ((rc = pair_dst_setup(p))) return bail(rc);
+    if ((rc = pair_dst_setup(p, s))) return bail(rc);
     *out = p;
     return SVP_OK;
 }

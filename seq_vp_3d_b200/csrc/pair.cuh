@@ -7,6 +7,9 @@ struct svp_pair {
     svp_weights w;
     svp::Q1Const q;
     int device = 0;
+    // one allocation for everything whose size the grid fixes (the arrays below except loc1, loc2, cand): a
+    // registration allocates and frees 5 blocks instead of 30
+    char *slab = nullptr;
     // images and spline
     double *fixed = nullptr;      // (nz, ny, nx)
     double *coeff = nullptr;      // (nz, ny, nx) not-a-knot cubic coefficients
@@ -17,14 +20,13 @@ struct svp_pair {
     double *loc1 = nullptr, *loc2 = nullptr;  // (24, ncell) per-cell vertex values (SoA)
     double *cellbuf = nullptr;                // (ncell)
     svp::dd *partial = nullptr;               // block partial sums
-    long long partial_cap = 0;                // in dd entries
     double *host = nullptr;                   // pinned results that kernels write (64 doubles)
     long long *counter = nullptr;             // small device counters (8)
     long long *cand = nullptr;                // candidate cells of the T69/T73 node JD extension (ncell)
     uint8_t *flags = nullptr;                 // (ncell) cells the float32 cell kernels hand to the float64 barrier
     // DST-I Poisson metric
-    double *dst_half[3] = {nullptr, nullptr, nullptr};  // folded orthonormal DST-I half matrices, x, y, z
-    double *dst_pad[3] = {nullptr, nullptr, nullptr};   // the same zero-padded to the passes' tiles (PadF64)
+    // folded orthonormal DST-I half matrices, x, y, z, zero-padded to the passes' tiles (PadF64)
+    double *dst_pad[3] = {nullptr, nullptr, nullptr};
     int dst_n[3] = {0, 0, 0};                               // their transform lengths (free nodes per axis)
     // the same rounded to float32 for the mixed form, as TF32 parts: big parts of H0^T, H1^T, then the small parts
     unsigned *dst_tf32[3] = {nullptr, nullptr, nullptr};
@@ -36,7 +38,19 @@ struct svp_pair {
 };
 
 namespace svp {
-int pair_partials(svp_pair *p, long long blocks, int k);
 int pair_locals(svp_pair *p, int n);
-int pair_flags(svp_pair *p);
+// block sums (double-double) of the largest evaluation of a grid
+long long pair_partial_count(const Q1Const &q);
+// consecutive 256-byte aligned pieces of the slab; with a null base only the size is counted
+struct SlabCursor {
+    char *base;
+    size_t used = 0;
+    template <class T>
+    void take(T *&ptr, size_t count) {
+        if (base) ptr = reinterpret_cast<T *>(base + used);
+        used += (sizeof(T) * count + 255) / 256 * 256;
+    }
+};
+void pair_dst_carve(svp_pair *p, SlabCursor &c);
+int pair_dst_setup(svp_pair *p, cudaStream_t s);
 }  // namespace svp

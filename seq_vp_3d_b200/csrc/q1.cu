@@ -1973,7 +1973,8 @@ SplineRef spline_ref(const svp_pair *p) {
 }
 
 unsigned cell_blocks(const svp_pair *p) { return blocks_for(p->q.ncell, CT, CELL_PER_SM); }
-unsigned slice_blocks(const svp_pair *p) { return blocks_for(p->q.ncell, CS, 2 * CELL_PER_SM); }
+unsigned slice_blocks(const Q1Const &q) { return blocks_for(q.ncell, CS, 2 * CELL_PER_SM); }
+unsigned slice_blocks(const svp_pair *p) { return slice_blocks(p->q); }
 // dynamic shared memory of the slice kernels: k doubles per thread
 constexpr size_t slice_bytes(int k) { return sizeof(double) * (size_t)k * CS; }
 int allow_slices() {
@@ -2015,26 +2016,16 @@ long long violation_count(const svp_pair *p) {
 
 }  // namespace
 
-int pair_partials(svp_pair *p, long long blocks, int k) {
-    long long need = blocks * k;
-    if (need <= p->partial_cap) return SVP_OK;
-    cudaFree(p->partial);
-    p->partial = nullptr;
-    p->partial_cap = 0;
-    SVP_CUDA(cudaMalloc((void **)&p->partial, sizeof(dd) * need));
-    p->partial_cap = need;
-    return SVP_OK;
+long long pair_partial_count(const Q1Const &q) {
+    const long long nb = node_blocks(q.nnode), cb = slice_blocks(q);
+    const long long bb = barrier_blocks(q) > flagged_blocks(q) ? barrier_blocks(q) : flagged_blocks(q);
+    return nb * 4 + cb * 10 + bb * 2;       // the screened trial's sums
 }
 
 int pair_locals(svp_pair *p, int n) {
     size_t bytes = sizeof(double) * 24 * (size_t)p->q.ncell;
     if (n >= 1 && !p->loc1) SVP_CUDA(cudaMalloc((void **)&p->loc1, bytes));
     if (n >= 2 && !p->loc2) SVP_CUDA(cudaMalloc((void **)&p->loc2, bytes));
-    return SVP_OK;
-}
-
-int pair_flags(svp_pair *p) {
-    if (!p->flags) SVP_CUDA(cudaMalloc((void **)&p->flags, (size_t)p->q.ncell));
     return SVP_OK;
 }
 
@@ -2078,10 +2069,8 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
     SVP_REQUIRE(p && u && warped && terms5, "svp_energy: null argument");
     cudaStream_t s = (cudaStream_t)stream;
     unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
-    int rc = pair_partials(p, (long long)nb * 2 + (long long)cb * 2 + bb, 1);
+    int rc = allow_slices();
     if (rc) return rc;
-    if ((rc = allow_slices())) return rc;
-    if ((rc = pair_flags(p))) return rc;
     { svp::KernelTimer _t("node_energy_kernel", s); SVP_LAUNCH(node_energy_kernel<<<nb, 256, 0, s>>>(p->q, u, warped, p->fixed, p->u_ref, p->partial)); }
     SVP_LAUNCH_CHECK("node_energy_kernel");
     dd *pc = p->partial + (long long)nb * 2, *pb = pc + (long long)cb * 2;
@@ -2126,10 +2115,8 @@ extern "C" int svp_energy_difference_masked(svp_pair *p, const double *base_u, c
     (void)base_active;
     (void)trial_active;
     unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
-    int rc = pair_partials(p, (long long)nb * 2 + (long long)cb * 2 + bb, 1);
+    int rc = allow_slices();
     if (rc) return rc;
-    if ((rc = allow_slices())) return rc;
-    if ((rc = pair_flags(p))) return rc;
     { svp::KernelTimer _t("node_diff_kernel", s); SVP_LAUNCH(node_diff_kernel<<<nb, 256, 0, s>>>(p->q, base_u, base_warped, trial_u, trial_warped, p->fixed, p->u_ref,
                                         p->partial)); }
     dd *pc = p->partial + (long long)nb * 2, *pb = pc + (long long)cb * 2;
@@ -2191,10 +2178,8 @@ extern "C" int svp_energy_difference_screened(svp_pair *p, const double *base_u,
                 "svp_energy_difference_screened: null argument");
     cudaStream_t s = (cudaStream_t)stream;
     unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = barrier_blocks(p->q);
-    int rc = pair_partials(p, (long long)nb * 2 + (long long)cb * 8 + (long long)bb * 2, 1);
+    int rc = allow_slices();
     if (rc) return rc;
-    if ((rc = allow_slices())) return rc;
-    if ((rc = pair_flags(p))) return rc;
     dd *pn = p->partial, *pce = pn + (long long)nb * 2, *pcd = pce + (long long)cb * 2, *pcb = pcd + (long long)cb * 2;
     dd *pbe = pcb + (long long)cb * 4, *pbd = pbe + bb;
     {
@@ -2241,10 +2226,8 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
                 "svp_trial_energy: null argument");
     cudaStream_t s = (cudaStream_t)stream;
     unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = screened ? barrier_blocks(p->q) : flagged_blocks(p->q);
-    int rc = pair_partials(p, (long long)nb * 4 + (long long)cb * 10 + (long long)bb * 2, 1);
+    int rc = allow_slices();
     if (rc) return rc;
-    if ((rc = allow_slices())) return rc;
-    if ((rc = pair_flags(p))) return rc;
     dd *pne = p->partial, *pnd = pne + (long long)nb * 2, *pce = pnd + (long long)nb * 2, *pcd = pce + (long long)cb * 3;
     dd *pcb = pcd + (long long)cb * 3, *pbe = pcb + (long long)cb * 4, *pbd = pbe + bb;
     SplineRef S = spline_ref(p);
@@ -2369,7 +2352,6 @@ static int grad64(svp_pair *p, const double *u, double mu_scale, double nu_scale
                   const uint8_t *active, const uint8_t **has2, cudaStream_t s) {
     int rc = allow_slices();
     if (rc) return rc;
-    if (barrier && !active && (rc = pair_flags(p))) return rc;
     uint8_t *flags = barrier && !active ? p->flags : nullptr;
     const uint8_t *marked = active ? active : flags;
     {
@@ -2390,8 +2372,6 @@ static int grad64(svp_pair *p, const double *u, double mu_scale, double nu_scale
 // (the state's mask, or without one the cells the soft kernel flags from its float32 closed27 J).
 static int grad32(svp_pair *p, const double *u, double mu_scale, double nu_scale, bool barrier, bool split,
                   const uint8_t *active, const uint8_t **has2, cudaStream_t s) {
-    int rc;
-    if (barrier && !active && (rc = pair_flags(p))) return rc;
     uint8_t *flags = barrier && !active ? p->flags : nullptr;
     {
         svp::KernelTimer _t("cell_grad32_kernel", s);
@@ -2476,7 +2456,6 @@ extern "C" int svp_ggn_diagonal_masked(svp_pair *p, const double *u, const doubl
     int rc = pair_locals(p, 1);
     if (rc) return rc;
     if (p->precision == SVP_PRECISION_MIXED) {
-        if (!active && (rc = pair_flags(p))) return rc;
         {
             svp::KernelTimer _t("cell_ggn_diag32_kernel", s);
             SVP_LAUNCH(cell_ggn_diag32_kernel<<<cell_blocks(p), CT, 0, s>>>(p->q, u, (float *)p->loc1,
@@ -2489,7 +2468,6 @@ extern "C" int svp_ggn_diagonal_masked(svp_pair *p, const double *u, const doubl
         }
         SVP_LAUNCH(ggn_node_kernel<float><<<node_blocks(p->q.nfree), 256, 0, s>>>(p->q, (const float *)p->loc1, image_grad, nullptr, out));
     } else {
-        if (!active && (rc = pair_flags(p))) return rc;
         {
             svp::KernelTimer _t("cell_ggn_diag_kernel", s);
             SVP_LAUNCH(cell_ggn_diag_kernel<<<slice_blocks(p), CS, 0, s>>>(p->q, u, p->loc1,
@@ -2594,13 +2572,12 @@ extern "C" int svp_image_shift(svp_pair *p, const double *image_grad, double fac
     SVP_REQUIRE(p && image_grad && alpha, "svp_image_shift: null argument");
     cudaStream_t s = (cudaStream_t)stream;
     unsigned nb = node_blocks(p->q.nfree);
-    int rc = pair_partials(p, nb, 1);
-    if (rc) return rc;
     SVP_LAUNCH(shift_kernel<<<nb, 256, 0, s>>>(p->q, image_grad, p->partial));
     SVP_LAUNCH_CHECK("shift kernels");
     ReduceSpec red;
     red.add(p->partial, nb, 1, 0);
-    if ((rc = reduce_results(p, red, s))) return rc;
+    int rc = reduce_results(p, red, s);
+    if (rc) return rc;
     const double *tmp = p->host;
     *alpha = factor * ((tmp[0] + tmp[1]) / (double)p->q.nfree) / 3;
     return SVP_OK;
