@@ -90,3 +90,21 @@ def test_ggn_diagonal(problem):
     for mask in (None, active):
         got = P.ggn_diagonal(bd, g, mask).cpu().numpy()
         assert np.linalg.norm(got - ref) <= TOL * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("term", ["total", "jd", "curl"])
+def test_mixed_gradients(problem, term):
+    """The float32 soft gradient on the same grids against the float64 one: within 1e-4 (J and curl of the two fields
+    round at 1e-7 to 2e-7 each, the residuals between them are no smaller than 4e-3)."""
+    P, OP, bd, td, base, trial = problem
+    w, g = P.warp(bd, with_gradient=True)
+    ref = P.gradient(bd, w, g, term)
+    P.precision = "mixed"
+    from seq_vp_3d_b200 import _lib
+    _lib.call("svp_pair_set_precision", P._h, 1)
+    try:
+        got = P.gradient(bd, w, g, term)
+    finally:
+        _lib.call("svp_pair_set_precision", P._h, 0)
+        P.precision = "plain"
+    assert float((got - ref).norm()) <= 1e-4 * float(ref.norm())
