@@ -25,26 +25,18 @@ std::vector<double> not_a_knot(const std::vector<double> &x) {
     return t;
 }
 
-// The reciprocals cubic_basis multiplies by, per span s in [3, n-1] (row s of 14): the Cox-de Boor denominators
-// t[s+r+1] - t[s+1-d+r] for d = 1..3, r < d (6), then for each basis function k = 0..3 of the span the two derivative
-// denominators a = t[i+3] - t[i], b = t[i+4] - t[i+1] with i = s - 3 + k (1 where a difference is zero, the
-// reference's guard).  Rows below 3 are unused (zero).
+// The reciprocals cubic_basis multiplies by, per span s in [3, n-1] (row s of 6): the Cox-de Boor denominators
+// t[s+r+1] - t[s+1-d+r] for d = 1..3, r < d.  Those of d = 3 are also the derivative's denominators t[i+4] - t[i+1]
+// and t[i+3] - t[i] of the span's basis functions.  Rows below 3 are unused (zero).
 std::vector<double> spline_reciprocals(const std::vector<double> &t, long long n) {
-    std::vector<double> R((size_t)n * 14, 0.);
+    std::vector<double> R((size_t)n * 6, 0.);
     for (long long s = 3; s <= n - 1; s++) {
-        double *row = R.data() + 14 * s;
-        int k = 0;
+        double *row = R.data() + 6 * s;
         for (int d = 1; d <= 3; d++)
             for (int r = 0; r < d; r++) {
                 double len = t[(size_t)(s + r + 1)] - t[(size_t)(s + 1 - d + r)];
-                row[k++] = len != 0. ? 1. / len : 0.;
+                *row++ = len != 0. ? 1. / len : 0.;
             }
-        for (int b = 0; b < 4; b++) {
-            long long i = s - 3 + b;
-            double a = t[(size_t)(i + 3)] - t[(size_t)i], bb = t[(size_t)(i + 4)] - t[(size_t)(i + 1)];
-            row[6 + 2 * b] = 1. / (a != 0. ? a : 1.);
-            row[7 + 2 * b] = 1. / (bb != 0. ? bb : 1.);
-        }
     }
     return R;
 }
@@ -223,7 +215,7 @@ extern "C" int svp_pair_create(const svp_grid *g, const svp_weights *w, const do
         c.take(p->flags, (size_t)p->q.ncell);
         for (int k = 0; k < 3; k++) {
             c.take(p->knots[k], (size_t)(len[k] + 4));
-            c.take(p->spline_rcp[k], (size_t)(14 * len[k]));
+            c.take(p->spline_rcp[k], (size_t)(6 * len[k]));
         }
         pair_dst_carve(p, c);
         if (pass == 0 && (e = cudaMalloc((void **)&p->slab, c.used)) != cudaSuccess)

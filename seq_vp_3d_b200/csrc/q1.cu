@@ -24,7 +24,7 @@ constexpr int CELL_PER_SM = 8;
 struct SplineRef {
     const double *c;
     const double *t[3];    // x, y, z knots
-    const double *rcp[3];  // per span, the reciprocals of the knot differences cubic_basis divides by (14 per span)
+    const double *rcp[3];  // per span, the reciprocals of the knot differences cubic_basis divides by (6 per span)
     long long n[3];        // nx, ny, nz coefficients per axis
     double x0[3], ih[3];
 };
@@ -42,11 +42,14 @@ __device__ __forceinline__ int find_span(const double *__restrict__ t, long long
 
 // backends/spline.py:12 cubic_basis: Cox-de Boor values and derivatives of the 4 B-splines on the span.  The
 // denominators are knot differences (right + left = t[s+r+1] - t[s+1-d+r] up to rounding), so their reciprocals are
-// tabled per span and the 14 divisions per axis become multiplies (a relative change of one rounding, inside the
-// float64 contract's 1e-12).
+// tabled per span and the divisions become multiplies (a relative change of one rounding, inside the float64
+// contract's 1e-12).  The derivative's denominators are those of degree 3, so 6 reciprocals do, read as 3 pairs: a
+// warp's lanes stand on 32 x spans, and each load of the x row touches every line of the 32 rows.
 __device__ __forceinline__ void cubic_basis(const double *__restrict__ t, const double *__restrict__ rcp, int s,
                                             double x, double B[4], double dB[4]) {
-    const double *R = rcp + 14 * (long long)s;
+    const double2 *R2 = reinterpret_cast<const double2 *>(rcp + 6 * (long long)s);
+    const double2 r01 = __ldg(R2), r23 = __ldg(R2 + 1), r45 = __ldg(R2 + 2);
+    const double R[6] = {r01.x, r01.y, r23.x, r23.y, r45.x, r45.y};
     double b[4] = {1., 0., 0., 0.}, q[3];
 #pragma unroll
     for (int degree = 1; degree <= 3; degree++) {
@@ -56,7 +59,7 @@ __device__ __forceinline__ void cubic_basis(const double *__restrict__ t, const 
         for (int r = 0; r < degree; r++) {
             double right = __ldg(t + s + r + 1) - x;
             double left = x - __ldg(t + s + 1 - degree + r);
-            double temp = b[r] * __ldg(R + (degree - 1) * degree / 2 + r);
+            double temp = b[r] * R[(degree - 1) * degree / 2 + r];
             nb[r] = saved + right * temp;
             saved = left * temp;
         }
@@ -66,11 +69,16 @@ __device__ __forceinline__ void cubic_basis(const double *__restrict__ t, const 
         if (degree == 2) { q[0] = b[0]; q[1] = b[1]; q[2] = b[2]; }
     }
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        double left = k == 0 ? 0. : q[k - 1], right = k == 3 ? 0. : q[k];
-        dB[k] = 3. * left * __ldg(R + 6 + 2 * k) - 3. * right * __ldg(R + 7 + 2 * k);
-        B[k] = b[k];
-    }
+    for (int k = 0; k < 4; k++) B[k] = b[k];
+    const double d0 = 3. * q[0] * R[3], d1 = 3. * q[1] * R[4], d2 = 3. * q[2] * R[5];
+    dB[0] = -d0;
+    dB[1] = d0 - d1;
+    dB[2] = d1 - d2;
+    dB[3] = d2;
+}
+
+__device__ __forceinline__ void prefetch_l1(const void *p) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
 
 // value and (optionally) xyz gradient at physical point (x, y, z)
@@ -79,20 +87,28 @@ __device__ __forceinline__ double spline_eval(const SplineRef &S, double px, dou
     int sx = find_span(S.t[0], S.n[0], px, S.x0[0], S.ih[0]);
     int sy = find_span(S.t[1], S.n[1], py, S.x0[1], S.ih[1]);
     int sz = find_span(S.t[2], S.n[2], pz, S.x0[2], S.ih[2]);
+    const long long nx = S.n[0], plane = S.n[1] * nx;
+    const double *c = S.c + (long long)(sz - 3) * plane + (long long)(sy - 3) * nx + (sx - 3);
+    // the first plane's 16 coefficients are on their way while the bases are formed, then a plane ahead
+    double f[16];
+    auto fetch = [&](const double *p) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) f[4 * j + k] = __ldg(p + j * nx + k);
+    };
+    fetch(c);
     double bx[4], dx[4], by[4], dy[4], bz[4], dz[4];
     cubic_basis(S.t[0], S.rcp[0], sx, px, bx, dx);
     cubic_basis(S.t[1], S.rcp[1], sy, py, by, dy);
     cubic_basis(S.t[2], S.rcp[2], sz, pz, bz, dz);
-    const long long nx = S.n[0], ny = S.n[1];
-    const double *c = S.c + ((long long)(sz - 3) * ny + (sy - 3)) * nx + (sx - 3);
     double val = 0., gx = 0., gy = 0., gz = 0.;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         double pv = 0., px_ = 0., py_ = 0.;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const double *row = c + ((long long)i * ny + j) * nx;
-            double c0 = __ldg(row), c1 = __ldg(row + 1), c2 = __ldg(row + 2), c3 = __ldg(row + 3);
+            const double c0 = f[4 * j], c1 = f[4 * j + 1], c2 = f[4 * j + 2], c3 = f[4 * j + 3];
             double rv = c0 * bx[0] + c1 * bx[1] + c2 * bx[2] + c3 * bx[3];
             pv += by[j] * rv;
             if (GRAD) {
@@ -101,6 +117,7 @@ __device__ __forceinline__ double spline_eval(const SplineRef &S, double px, dou
                 py_ += dy[j] * rv;
             }
         }
+        if (i < 3) fetch(c + (i + 1) * plane);
         val += bz[i] * pv;
         if (GRAD) {
             gx += bz[i] * px_;
@@ -1309,6 +1326,9 @@ __device__ __forceinline__ void acc_add(dd &acc, dd t) {
 // trial's warped image (and image gradient), its energy sums exactly as node_energy_kernel and the energy-only cell
 // kernels form them, and the stable base -> trial changes exactly as node_diff_kernel and the difference-only cell
 // kernels form them (same grids, same per-thread order, so the results are bitwise those of the separate passes).
+// Bound by the latency of its scattered loads (16 warps per SM at 128 registers; 85 registers spill and lose).  At
+// 256^3: 1441 us; 1401 with a plane of coefficients fetched ahead, 1329 with the L1 prefetches, 1240 with 6 reciprocals
+// per axis read as pairs in place of 14 single ones.  its 16 doubles a node at 6.55 TB/s would take 328 us.
 template <bool GRAD>
 __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S, const double *__restrict__ ua,
                                                          const double *__restrict__ wa,
@@ -1321,6 +1341,13 @@ __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S,
          i += (long long)gridDim.x * blockDim.x) {
         long long x, y, z;
         unflatten3(i, q.nx, q.ny, x, y, z);
+        // the operands read after the spline, and the next node's displacement, on their way to L1 meanwhile: no register
+        const long long next = i + (long long)gridDim.x * blockDim.x;
+        prefetch_l1(wa + i);
+        prefetch_l1(fixed + i);
+        prefetch_l1(uref + 3 * i);
+        prefetch_l1(ua + 3 * i);
+        if (next < q.nnode) prefetch_l1(ub + 3 * next);
         double ux = ub[3 * i], uy = ub[3 * i + 1], uz = ub[3 * i + 2];
         double px = (q.x0[0] + q.h[0] * (double)x) + ux;
         double py = (q.x0[1] + q.h[1] * (double)y) + uy;
