@@ -70,10 +70,12 @@ __device__ __forceinline__ void cubic_basis(const double *__restrict__ t, const 
     }
 #pragma unroll
     for (int k = 0; k < 4; k++) B[k] = b[k];
+    // 3 q_(k-1) R - 3 q_k R, the first product fused: the mixed form rounds the image gradient to float32, where a change
+    // of the last float64 bit can show as one of the last float32 bit
     const double d0 = 3. * q[0] * R[3], d1 = 3. * q[1] * R[4], d2 = 3. * q[2] * R[5];
     dB[0] = -d0;
-    dB[1] = d0 - d1;
-    dB[2] = d1 - d2;
+    dB[1] = fma(3. * q[0], R[3], -d1);
+    dB[2] = fma(3. * q[1], R[4], -d2);
     dB[3] = d2;
 }
 
