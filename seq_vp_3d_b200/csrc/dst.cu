@@ -119,21 +119,30 @@ __global__ void __launch_bounds__(256) gemm_right_kernel(const double *__restric
 // output rows of one parity need only half the columns, against the folded input u_k = x_k + x_(n-1-k) (even i;
 // u_mid = x_mid when n is odd) or v_k = x_k - x_(n-1-k) (odd i): half the FLOPs of the dense product.  The folded
 // half matrices are stored per parity, H0 (ceil(n/2) x ceil(n/2)) then H1 (floor(n/2) x floor(n/2)), row-major.
-// FP64 tensor-core product D = A B + D on one 8x8x4 tile (mma.sync m8n8k4 f64): lane (g = lane / 4, t = lane % 4)
-// holds A[g][t], B[t][g] and D[g][2t], D[g][2t + 1].  FP64 has no tcgen05 kind on sm_100a; this is B200's FP64
-// tensor path, one instruction per 256 fused multiply-adds.
-__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-                 : "+d"(d[0]), "+d"(d[1])
-                 : "d"(a), "d"(b));
-}
-
-// The mixed form's passes: float32 operands on the tensor cores as 3xTF32 (mma.sync m16n8k8 .tf32, float32
-// accumulate).  Each operand x splits into big = tf32(x) and small = tf32(x - big); the product sums
-// small*big + big*small + big*big, which keeps float32-level accuracy (the small*small term is below float32
-// rounding).  Fragment layout of m16n8k8 (lane: gid = lane / 4, tig = lane % 4): A a0 = A[gid][tig],
-// a1 = A[gid + 8][tig], a2 = A[gid][tig + 4], a3 = A[gid + 8][tig + 4]; B b0 = B[tig][gid], b1 = B[tig + 4][gid];
-// D d0, d1 = D[gid][2 tig + {0, 1}], d2, d3 = D[gid + 8][2 tig + {0, 1}].
+//
+// One kernel does a pass along any axis, D = H F with H a half matrix (m16 row tiles) and F the folded field, [k][col].
+// A block takes QC columns and up to 8 row tiles of BOTH parities: the raw pair (x_k, x_(n-1-k)) is loaded once, and
+// its sum and its difference are staged side by side for the warps of parity 0 and 1.  The half matrices are laid out
+// once per grid in the order in which the lanes of an mma read them, so a warp loads its fragments of H with two
+// 16-byte loads per tile and 8 k through L1, and only the field goes through shared memory.  The columns of all
+// batches are one flattened range: a short x axis leaves no part-filled tile per (batch, z).  The result returns
+// through shared memory, so that both parities of a line and QC columns (x pass: whole rows) are stored together and
+// the epilogue's operands are read along lines.  Every output is accumulated in k order, so the values do not depend
+// on the tiling.
+//
+// Bound by the FP64 tensor pipe (float64: half busy, the rest is the latency of the field's loads and the phases
+// around the products) and by instruction issue (3xTF32).  Blocks of 4 warps, 4 per SM, cover each other's phases
+// better than 2 of 8 warps (1278 against 1350 us for the six float64 passes on 224 x 192 x 160, 367 against 377 us for
+// the six mixed ones on 119 x 165 x 141).  Against 128 x 64 (x: 64 or 128 x 16 ceil(k0 / 16)) tiles per parity with
+// both operands staged through shared memory: six passes 1584 -> 1235 us float64, 672 -> 354 us mixed; the operations
+// of the float64 passes (11.4 G fused multiply-adds) take 614 us at 18.6 T/s, the bytes of the mixed ones 60 us.
+//
+// Float64: mma.sync m16n8k8 f64 (FP64 has no tcgen05 kind on sm_100a; this is B200's FP64 tensor path).  Mixed form:
+// float32 operands as 3xTF32 (mma.sync m16n8k8 .tf32, float32 accumulate): each operand x splits into big = tf32(x)
+// and small = tf32(x - big); the product sums small*big + big*small + big*big, which keeps float32-level accuracy (the
+// small*small term is below float32 rounding).  Fragments of m16n8k8, both types (lane: gid = lane / 4, tig = lane %
+// 4): a0 = A[gid][tig], a1 = A[gid + 8][tig], a2 = A[gid][tig + 4], a3 = A[gid + 8][tig + 4]; b0 = B[tig][gid],
+// b1 = B[tig + 4][gid]; d0, d1 = D[gid][2 tig + {0, 1}], d2, d3 = D[gid + 8][2 tig + {0, 1}].
 __device__ __forceinline__ unsigned tf32_of(float x) {
     unsigned r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
@@ -143,259 +152,201 @@ __device__ __forceinline__ void tf32_split(float x, unsigned &big, unsigned &sma
     big = tf32_of(x);
     small = tf32_of(x - __uint_as_float(big));
 }
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint4 &a, unsigned b0, unsigned b1) {
     asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
                  "{%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+                 : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_f64(double (&d)[4], const double2 &a01, const double2 &a23, const double2 &b) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+                 : "d"(a01.x), "d"(a01.y), "d"(a23.x), "d"(a23.y), "d"(b.x), "d"(b.y));
 }
 
-// One K block of the folded operand: the raw pair (x_k, x_(n-1-k)) of each of a thread's entries is fetched into
-// registers one block ahead (the loads fly while the previous block's products run) and folded when it is stored
-// to shared memory.  fold = x_k (middle row of odd n), x_k + x_m (parity 0) or x_k - x_m (parity 1), formed in
-// float64 (with the optional pre-scale) and rounded once to the pass's type; entries outside the operand are +0.
+// A 16-byte cell holds what one lane needs of an operand for a pair (k, k + 4): both values (float64), or the big and
+// small part of each (3xTF32).  H: per parity, tile and 8 k, two cells per lane (float64: a0 a1, a2 a3; 3xTF32: the
+// four big parts, the four small parts); F: one cell per (k % 4, column).
+constexpr int QK = 16;                                             // K block: two mma steps
+constexpr int DT = 128;                                            // threads: parity x two row warps
+constexpr int kLines = 8;                                          // lines of the epilogue in flight per thread
+template <class TC> constexpr int kNC = sizeof(TC) == 8 ? 2 : 4;   // n8 tiles per warp
+template <class TC> constexpr int kQC = 8 * kNC<TC>;               // columns per block
+
+struct DstFrag {
+    const uint4 *h[2];       // per parity
+    int n, kg[2];            // axis length, rows per parity
+    int k8, mt, tiles;       // mma steps along K, m16 tiles per block (<= 8) and blocks along the rows
+};
+// The rows of parity 0 are split evenly: 16 ceil(k0 / 16) rows leave at most 15 + 16 (tiles - 1) rows of padding.
+inline DstFrag frag_geometry(int n) {
+    DstFrag F;
+    F.h[0] = F.h[1] = nullptr;
+    F.n = n;
+    F.kg[0] = (n + 1) / 2;
+    F.kg[1] = n / 2;
+    F.k8 = (F.kg[0] + 7) / 8;
+    const int m16 = (F.kg[0] + 15) / 16;
+    F.tiles = (m16 + 7) / 8;
+    F.mt = (m16 + F.tiles - 1) / F.tiles;
+    return F;
+}
+inline size_t frag_cells(const DstFrag &F) { return (size_t)F.tiles * F.mt * F.k8 * 64; }   // per parity
+inline DstFrag frag_of(const void *t, int n) {
+    DstFrag F = frag_geometry(n);
+    F.h[0] = reinterpret_cast<const uint4 *>(t);
+    F.h[1] = F.h[0] + frag_cells(F);
+    return F;
+}
+
+// h: H0 (k0 x k0) then H1 (k1 x k1), row-major; out: the cells of parity g (src = offset of H_g), zeros outside H_g
 template <class TC>
-__device__ __forceinline__ TC fold_value(double xa, double xb, bool mid, int g) {
-    return (TC)(mid ? xa : (g ? xa - xb : xa + xb));
-}
-
-// ---------------------------------------------------------------------------------------- mixed form (3xTF32)
-// The float32 passes keep each operand as its two TF32 parts in shared memory: the half matrices are split once per
-// grid into zero-padded tiles (split_pad_kernel), the folded fields once when a K block is staged, so a fragment is
-// loaded, never split, and the staging loads need no bounds checks on the matrix side.  A block computes a 128-row x
-// 64-column (left pass) or 128-row x 16 NT-column (right pass) output tile with 8 warps of 32 x 32 (32 x 8 NT), each
-// K block of 16 staged twice-buffered through registers.  Every output is accumulated in k order, three mma per k8
-// step (small x big, big x small, big x big), so any tiling gives the same bits.
-constexpr int QR = 128, QK = 16;           // output rows per block, K block
-constexpr int QC = 64;                     // output columns per block of the left pass
-constexpr int QPA = QR + 8, QPB = QC + 8;  // left pass: [k][row] and [k][col] rows padded to 8 mod 32 words
-constexpr int QPK = QK + 4;                // right pass: [row][k] rows padded to 4 mod 32 words
-
-struct PadTf32 {
-    const unsigned *b[2], *s[2];   // per parity: big / small parts, zero-padded to kpad x ipad (left) or ipad x kpad
-    int n, kg[2], ipad[2], kpad[2];
-};
-
-// h: H0 (k0 x k0) then H1 (k1 x k1), row-major float32.  out, per parity g: big parts then small parts of H_g in the
-// pass's layout, kmajor: T[k][a] = H_g[a][k] (kpad x ipad), else T[a][k] = H_g[a][k] (ipad x kpad), zeros outside.
-__global__ void split_pad_kernel(const float *__restrict__ h, int kg, long long src, int kmajor, int ipad, int kpad,
-                                 unsigned *__restrict__ big, unsigned *__restrict__ small) {
-    const long long total = (long long)ipad * kpad;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+__global__ void frag_kernel(const TC *__restrict__ h, int kg, long long src, long long cells, int k8,
+                            uint4 *__restrict__ out) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < cells;
          e += (long long)gridDim.x * blockDim.x) {
-        const int a = kmajor ? (int)(e % ipad) : (int)(e / kpad), k = kmajor ? (int)(e / ipad) : (int)(e % kpad);
-        unsigned b = 0u, s = 0u;
-        if (a < kg && k < kg) tf32_split(h[src + (long long)a * kg + k], b, s);
-        big[e] = b;
-        small[e] = s;
+        const int lane = (int)(e & 31), half = (int)(e >> 5) & 1, gid = lane >> 2, tig = lane & 3;
+        const int step = (int)((e >> 6) % k8), tile = (int)((e >> 6) / k8);
+        TC a[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int i = 16 * tile + gid + 8 * (j & 1), k = 8 * step + tig + 4 * (j >> 1);
+            a[j] = (i < kg && k < kg) ? h[src + (long long)i * kg + k] : TC(0);
+        }
+        if constexpr (sizeof(TC) == 8) {
+            reinterpret_cast<double2 *>(out)[e] = half ? make_double2(a[2], a[3]) : make_double2(a[0], a[1]);
+        } else {
+            unsigned big[4], small[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) tf32_split(a[j], big[j], small[j]);
+            out[e] = half ? make_uint4(small[0], small[1], small[2], small[3])
+                          : make_uint4(big[0], big[1], big[2], big[3]);
+        }
     }
 }
 
-template <class TI>
-__device__ __forceinline__ float fold_tf32(TI xa, TI xb, bool mid, int g) {
-    // formed in the input type and rounded once: a float32 sum or difference is the rounded exact value either way
-    return (float)(mid ? xa : (g ? xa - xb : xa + xb));
+// Half a cell of a folded value; formed in the input type and rounded once to the pass's type.
+template <class TC, class TI>
+__device__ __forceinline__ uint2 fold_half(TI v) {
+    uint2 h;
+    if constexpr (sizeof(TC) == 8) {
+        const double d = (double)v;
+        h = *reinterpret_cast<const uint2 *>(&d);
+    } else {
+        tf32_split((float)v, h.x, h.y);
+    }
+    return h;
 }
 
-// Left pass along y or z: C[b][2i + g][w] = sum_k H_g[i][k] fold_g(X)[b][k][w] (rows of length W, stride ldx, batch
-// stride bs).  EPI 1 divides by den[index within the batch] (den is one component's array: the z pass's batch stride
-// is its length), EPI 2 multiplies by sign * post[flat] (the operation order of the separate elementwise passes).
-// 3xTF32: A = H_g^T tile [k][row], B = the folded field [k][col].
-template <int EPI, class TI, class TO>
-__global__ void __launch_bounds__(256) dst_left_tf32_kernel(PadTf32 D, const TI *__restrict__ X, long long W,
-                                                            long long ldx, long long bs, TO *__restrict__ C,
-                                                            const double *__restrict__ den,
-                                                            const double *__restrict__ post, double sign) {
-    extern __shared__ __align__(16) unsigned qsm[];
-    unsigned(*sAb)[QK][QPA] = reinterpret_cast<unsigned(*)[QK][QPA]>(qsm);
-    unsigned(*sAs)[QK][QPA] = reinterpret_cast<unsigned(*)[QK][QPA]>(qsm + 2 * QK * QPA);
-    unsigned(*sBb)[QK][QPB] = reinterpret_cast<unsigned(*)[QK][QPB]>(qsm + 4 * QK * QPA);
-    unsigned(*sBs)[QK][QPB] = reinterpret_cast<unsigned(*)[QK][QPB]>(qsm + 4 * QK * QPA + 2 * QK * QPB);
+// Row strides of the returned tile: [line][column] (left passes; a lane writes two columns at once) and
+// [row][position] (x pass).
+template <class TC> constexpr int kTileCol = kQC<TC> + 4;
+inline __host__ __device__ int tile_row(int mt) { return 32 * mt + 1; }
+template <class TC> constexpr int kStep = 4 * (kQC<TC> + 2) + 1;   // cells of one staged mma step, see dst_pass_kernel
+template <class TC>
+size_t dst_smem(bool x, int mt) {
+    const size_t stage = sizeof(uint4) * 2 * 2 * 2 * kStep<TC>;
+    const size_t tile = sizeof(TC) * (x ? (size_t)kQC<TC> * tile_row(mt) : (size_t)32 * mt * kTileCol<TC>);
+    return stage > tile ? stage : tile;
+}
+
+// address of flattened column col at k = 0 (ncol < 2^32)
+__device__ __forceinline__ long long flat_base(long long col, int W, long long bs) {
+    const unsigned b = (unsigned)col / (unsigned)W;
+    return (long long)b * bs + ((unsigned)col - b * (unsigned)W);
+}
+__device__ __forceinline__ void prefetch_l2(const void *p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+// XP (x pass): columns are the R rows of length n, C[r][2i + g] = sum_k fold_g(pre X)[r][k] H_g[i][k], pre an optional
+// scale applied first.  Else (y, z): C[b][2i + g][w] = sum_k H_g[i][k] fold_g(X)[b][k][w], rows of length W, stride
+// ldx = W, batch stride bs, ncol = batches * W; EPI 1 divides by den[index within the batch] (den is one component's
+// array: the z pass's batch stride is its length), EPI 2 multiplies by sign * post[flat].
+// MW: m16 tiles per warp, two row warps per parity (the second one has mt - MW).
+template <bool XP, bool PRE, int MW, int EPI, class TC, class TI, class TO>
+__global__ void __launch_bounds__(DT, 512 / DT) dst_pass_kernel(DstFrag D, const TI *__restrict__ X, long long ncol,
+                                                                int W, long long bs, TO *__restrict__ C,
+                                                                const double *__restrict__ pre,
+                                                                const double *__restrict__ den,
+                                                                const double *__restrict__ post, double sign) {
+    constexpr bool F64 = sizeof(TC) == 8;
+    constexpr int NC = kNC<TC>, QC = kQC<TC>, PC = QC + 2;
+    constexpr int NE = QK * QC / DT;   // entries (k, column) of a K block a thread stages
+    extern __shared__ __align__(16) unsigned char dsm[];
+    // [buffer][parity][step], cell (k % 4, column) at PC (k % 4) + column: the 8 lanes of a 16-byte fragment load (4 k,
+    // 2 columns) and the 16 lanes of an x pass's 8-byte store (16 k of a column) fall in distinct banks
+    uint4(*sF)[2][2][kStep<TC>] = reinterpret_cast<uint4(*)[2][2][kStep<TC>]>(dsm);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
-    const int wm = warp >> 1, wn = warp & 1;
-    const int t0 = D.ipad[0] / QR;
-    const int g = (int)blockIdx.x < t0 ? 0 : 1;
-    const int rows = g ? D.kg[1] : D.kg[0], K = rows, ip = g ? D.ipad[1] : D.ipad[0];
-    const int i0 = ((int)blockIdx.x - (g ? t0 : 0)) * QR;
-    const unsigned *Hb = g ? D.b[1] : D.b[0], *Hs = g ? D.s[1] : D.s[0];
-    const long long w0 = (long long)blockIdx.y * QC;
-    const TI *Xb = X + (long long)blockIdx.z * bs;
-    float facc[2][4][4];
+    // both parities' second row warps would share schedulers if they had the same place: they swap
+    const int g = warp >> 1, wm = (warp & 1) ^ g;
+    const int tile = (int)(blockIdx.x % (unsigned)D.tiles);
+    const long long c0 = (long long)(blockIdx.x / (unsigned)D.tiles) * QC;
+    const int n = D.n, K = D.kg[0], k1 = D.kg[1], mine = wm ? D.mt - MW : MW;   // MW or MW - 1 tiles
+    const bool full = mine == MW;
+    const uint4 *H = (g ? D.h[1] : D.h[0]) + (long long)(tile * D.mt + wm * MW) * D.k8 * 64 + lane;
+    TC acc[MW][NC][4];
 #pragma unroll
-    for (int a = 0; a < 2; a++)
+    for (int m = 0; m < MW; m++)
 #pragma unroll
-        for (int c = 0; c < 4; c++)
+        for (int c = 0; c < NC; c++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) facc[a][c][e] = 0.f;
-    // staging: the matrix block (16 x 128 words per part) as two uint4 per thread, the field block (16 rows x 64
-    // columns, each with its mirror row) as two column pairs per thread
-    const int hr = threadIdx.x >> 5, hc = (threadIdx.x & 31) * 4;
-    const int xr = threadIdx.x >> 5, xc = (threadIdx.x & 31) * 2;
-    const bool ok0 = w0 + xc < W, ok1 = w0 + xc + 1 < W;
-    uint4 hb[2], hs[2];
-    TI xa[2][2], xb[2][2];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int t = 0; t < 2; t++) {
-            const long long hk = (long long)(k0 + hr + 8 * t) * ip + i0 + hc;
-            hb[t] = *reinterpret_cast<const uint4 *>(Hb + hk);
-            hs[t] = *reinterpret_cast<const uint4 *>(Hs + hk);
-            const int k = k0 + xr + 8 * t;
-            const bool ok = k < K;
-            const TI *ra = Xb + (long long)k * ldx + w0 + xc, *rb = Xb + (long long)(D.n - 1 - k) * ldx + w0 + xc;
-            xa[t][0] = ok && ok0 ? ra[0] : TI(0);
-            xa[t][1] = ok && ok1 ? ra[1] : TI(0);
-            xb[t][0] = ok && ok0 ? rb[0] : TI(0);
-            xb[t][1] = ok && ok1 ? rb[1] : TI(0);
-        }
-    };
-    auto stash = [&](int buf, int k0) {
-#pragma unroll
-        for (int t = 0; t < 2; t++) {
-            *reinterpret_cast<uint4 *>(&sAb[buf][hr + 8 * t][hc]) = hb[t];
-            *reinterpret_cast<uint4 *>(&sAs[buf][hr + 8 * t][hc]) = hs[t];
-            const int k = k0 + xr + 8 * t;
-            const bool mid = k == D.n - 1 - k;
-            unsigned b0, s0, b1, s1;
-            tf32_split(fold_tf32<TI>(xa[t][0], xb[t][0], mid, g), b0, s0);
-            tf32_split(fold_tf32<TI>(xa[t][1], xb[t][1], mid, g), b1, s1);
-            *reinterpret_cast<uint2 *>(&sBb[buf][xr + 8 * t][xc]) = make_uint2(b0, b1);
-            *reinterpret_cast<uint2 *>(&sBs[buf][xr + 8 * t][xc]) = make_uint2(s0, s1);
-        }
-    };
-    fetch(0);
-    stash(0, 0);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = 0; k0 < K; k0 += QK) {
-        const bool more = k0 + QK < K;
-        if (more) fetch(k0 + QK);
-#pragma unroll
-        for (int kb = 0; kb < QK; kb += 8) {
-            unsigned ab[2][4], as[2][4];
-#pragma unroll
-            for (int a = 0; a < 2; a++) {
-                const int r = wm * 32 + a * 16 + gid;
-                ab[a][0] = sAb[buf][kb + tig][r];
-                ab[a][1] = sAb[buf][kb + tig][r + 8];
-                ab[a][2] = sAb[buf][kb + tig + 4][r];
-                ab[a][3] = sAb[buf][kb + tig + 4][r + 8];
-                as[a][0] = sAs[buf][kb + tig][r];
-                as[a][1] = sAs[buf][kb + tig][r + 8];
-                as[a][2] = sAs[buf][kb + tig + 4][r];
-                as[a][3] = sAs[buf][kb + tig + 4][r + 8];
-            }
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int col = wn * 32 + 8 * c + gid;
-                const unsigned b0b = sBb[buf][kb + tig][col], b0s = sBs[buf][kb + tig][col];
-                const unsigned b1b = sBb[buf][kb + tig + 4][col], b1s = sBs[buf][kb + tig + 4][col];
-#pragma unroll
-                for (int a = 0; a < 2; a++) {
-                    mma_tf32(facc[a][c], as[a], b0b, b1b);
-                    mma_tf32(facc[a][c], ab[a], b0s, b1s);
-                    mma_tf32(facc[a][c], ab[a], b0b, b1b);
+            for (int e = 0; e < 4; e++) acc[m][c][e] = TC(0);
+    // staging: of a K block's 16 k, y and z passes give a thread one column (lanes along the columns), the x pass one k
+    // (16 lanes along a row)
+    constexpr int KE = XP ? 0 : DT / QC, CE = XP ? DT / 16 : 0;      // entry e: k + KE e, column + CE e
+    const int fk = XP ? (int)threadIdx.x & 15 : (int)threadIdx.x / QC;
+    const int fc = XP ? (int)threadIdx.x >> 4 : (int)threadIdx.x % QC;
+    const long long ks = XP ? 1 : W;
+    const TI *fx = X + (XP ? (c0 + fc) * n : (c0 + fc < ncol ? flat_base(c0 + fc, W, bs) : 0));
+    // Float64: the field of the block that will take this one's place (512 / DT per SM) is brought to L2, up to two
+    // lines per k, or the rows of the x pass: 1278 -> 1241 us for the six passes above; the 3xTF32 passes, bound by
+    // issue, lose by it (367 -> 371 us, 64.6 -> 65.6 ms for a solve on 224 x 192 x 160).
+    if (F64) {
+        const long long cn = c0 + 148LL * (512 / DT) * QC / D.tiles;
+        if (cn + QC <= ncol) {
+            if (XP) {
+                for (int o = threadIdx.x * 16; o < QC * n; o += DT * 16) {   // 16 doubles to a line
+                    prefetch_l2(X + cn * n + o);
+                    if (PRE) prefetch_l2(pre + cn * n + o);
                 }
-            }
-        }
-        if (more) stash(buf ^ 1, k0 + QK);
-        __syncthreads();
-        buf ^= 1;
-    }
-    const long long cb = (long long)blockIdx.z * bs;
-#pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const int ii = i0 + wm * 32 + a * 16 + gid + 8 * (e >> 1);
-                const long long w = w0 + wn * 32 + 8 * c + 2 * tig + (e & 1);
-                if (ii >= rows || w >= W) continue;
-                const long long io = (long long)(2 * ii + g) * ldx + w, o = cb + io;
-                double v = (double)facc[a][c][e];
-                if (EPI == 1) v = v / den[io];
-                if (EPI == 2) v = sign * (post[o] * v);
-                C[o] = (TO)v;
-            }
-}
-
-// Right pass along x over contiguous rows of length n: C[r][2i + g] = sum_k fold_g(pre X)[r][k] H_g[i][k], pre an
-// optional scale applied first.  3xTF32: A = the folded rows [row][k],
-// B = H_g tile [col][k] with 16 NT columns (NT n8 tiles per warp along the 2 column warps).
-template <int NT, class TI, class TO>
-__global__ void __launch_bounds__(256) dst_right_tf32_kernel(PadTf32 D, const TI *__restrict__ X, long long R,
-                                                             const double *__restrict__ pre, TO *__restrict__ C) {
-    constexpr int QN = 16 * NT;
-    extern __shared__ __align__(16) unsigned qsm[];
-    unsigned(*sAb)[QR][QPK] = reinterpret_cast<unsigned(*)[QR][QPK]>(qsm);
-    unsigned(*sAs)[QR][QPK] = reinterpret_cast<unsigned(*)[QR][QPK]>(qsm + 2 * QR * QPK);
-    unsigned(*sBb)[QN][QPK] = reinterpret_cast<unsigned(*)[QN][QPK]>(qsm + 4 * QR * QPK);
-    unsigned(*sBs)[QN][QPK] = reinterpret_cast<unsigned(*)[QN][QPK]>(qsm + 4 * QR * QPK + 2 * QN * QPK);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
-    const int wm = warp >> 1, wn = warp & 1;
-    const int t0 = D.ipad[0] / QN;
-    const int g = (int)blockIdx.x < t0 ? 0 : 1;
-    const int cols = g ? D.kg[1] : D.kg[0], K = cols, kp = g ? D.kpad[1] : D.kpad[0];
-    const int i0 = ((int)blockIdx.x - (g ? t0 : 0)) * QN;
-    const unsigned *Hb = g ? D.b[1] : D.b[0], *Hs = g ? D.s[1] : D.s[0];
-    const long long r0 = (long long)blockIdx.y * QR;
-    const int n = D.n;
-    float facc[2][NT][4];
-#pragma unroll
-    for (int a = 0; a < 2; a++)
-#pragma unroll
-        for (int c = 0; c < NT; c++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) facc[a][c][e] = 0.f;
-    // staging: the field block (128 rows x 16 k, each with its mirror) as 8 entries per thread, 16 consecutive k of
-    // a row per half warp; the matrix block (16 NT rows x 16 k per part) as uint4 along k
-    const int xk = threadIdx.x & 15, xr = threadIdx.x >> 4;
-    constexpr int HV = QN * QK / 4, HT = (HV + 255) / 256;
-    TI xa[8], xb[8];
-    uint4 hb[HT], hs[HT];
-    auto fetch = [&](int k0) {
-        const int k = k0 + xk;
-#pragma unroll
-        for (int t = 0; t < 8; t++) {
-            const long long r = r0 + xr + 16 * t;
-            const bool ok = r < R && k < K;
-            const long long a = r * n + k, m = r * n + (n - 1 - k);
-            if (pre) {
-                xa[t] = ok ? (TI)(pre[a] * (double)X[a]) : TI(0);
-                xb[t] = ok ? (TI)(pre[m] * (double)X[m]) : TI(0);
             } else {
-                xa[t] = ok ? X[a] : TI(0);
-                xb[t] = ok ? X[m] : TI(0);
+                const TI *q = X + flat_base(cn + (threadIdx.x & 1) * (QC / 2), W, bs);
+                for (int k = threadIdx.x >> 1; k < n; k += DT / 2) prefetch_l2(q + (long long)k * W);
             }
         }
+    }
+    const double *fp = PRE ? pre + (c0 + fc) * n : nullptr;
+    TI xa[NE], xb[NE];
+    double pa[PRE ? NE : 1], pb[PRE ? NE : 1];
+    auto fetch = [&](int k0) {
 #pragma unroll
-        for (int t = 0; t < HT; t++) {
-            const int v = threadIdx.x + 256 * t;
-            if (v < HV) {
-                const long long hk = (long long)(i0 + v / (QK / 4)) * kp + k0 + (v % (QK / 4)) * 4;
-                hb[t] = *reinterpret_cast<const uint4 *>(Hb + hk);
-                hs[t] = *reinterpret_cast<const uint4 *>(Hs + hk);
+        for (int e = 0; e < NE; e++) {
+            const int k = k0 + fk + KE * e;
+            const bool ok = c0 + fc + CE * e < ncol && k < K;
+            const long long o = (long long)CE * e * n, a = o + k * ks, b = o + (n - 1 - k) * ks;
+            xa[e] = ok ? fx[a] : TI(0);
+            xb[e] = ok ? fx[b] : TI(0);
+            if (PRE) {
+                pa[e] = ok ? fp[a] : 0.;
+                pb[e] = ok ? fp[b] : 0.;
             }
         }
     };
     auto stash = [&](int buf, int k0) {
-        const int k = k0 + xk;
-        const bool mid = k == n - 1 - k;
 #pragma unroll
-        for (int t = 0; t < 8; t++) {
-            unsigned b, s;
-            tf32_split(fold_tf32<TI>(xa[t], xb[t], mid, g), b, s);
-            sAb[buf][xr + 16 * t][xk] = b;
-            sAs[buf][xr + 16 * t][xk] = s;
-        }
-#pragma unroll
-        for (int t = 0; t < HT; t++) {
-            const int v = threadIdx.x + 256 * t;
-            if (v < HV) {
-                *reinterpret_cast<uint4 *>(&sBb[buf][v / (QK / 4)][(v % (QK / 4)) * 4]) = hb[t];
-                *reinterpret_cast<uint4 *>(&sBs[buf][v / (QK / 4)][(v % (QK / 4)) * 4]) = hs[t];
+        for (int e = 0; e < NE; e++) {
+            const int kl = fk + KE * e, k = k0 + kl;
+            if (PRE) {
+                xa[e] = (TI)(pa[e] * (double)xa[e]);
+                xb[e] = (TI)(pb[e] * (double)xb[e]);
             }
+            const TI u = k == n - 1 - k ? xa[e] : xa[e] + xb[e];   // the middle of an odd axis has no mirror
+            const TI v = k < k1 ? xa[e] - xb[e] : TI(0);
+            const int at = 2 * ((kl & 3) * PC + fc + CE * e) + ((kl >> 2) & 1);
+            reinterpret_cast<uint2 *>(sF[buf][0][kl >> 3])[at] = fold_half<TC, TI>(u);
+            reinterpret_cast<uint2 *>(sF[buf][1][kl >> 3])[at] = fold_half<TC, TI>(v);
         }
     };
     fetch(0);
@@ -406,30 +357,34 @@ __global__ void __launch_bounds__(256) dst_right_tf32_kernel(PadTf32 D, const TI
         const bool more = k0 + QK < K;
         if (more) fetch(k0 + QK);
 #pragma unroll
-        for (int kb = 0; kb < QK; kb += 8) {
-            unsigned ab[2][4], as[2][4];
+        for (int st = 0; st < 2; st++) {
+            const int step = k0 / 8 + st;
+            if (step < D.k8) {
+                uint4 f[NC];
 #pragma unroll
-            for (int a = 0; a < 2; a++) {
-                const int r = wm * 32 + a * 16 + gid;
-                ab[a][0] = sAb[buf][r][kb + tig];
-                ab[a][1] = sAb[buf][r + 8][kb + tig];
-                ab[a][2] = sAb[buf][r][kb + tig + 4];
-                ab[a][3] = sAb[buf][r + 8][kb + tig + 4];
-                as[a][0] = sAs[buf][r][kb + tig];
-                as[a][1] = sAs[buf][r + 8][kb + tig];
-                as[a][2] = sAs[buf][r][kb + tig + 4];
-                as[a][3] = sAs[buf][r + 8][kb + tig + 4];
-            }
+                for (int c = 0; c < NC; c++) f[c] = sF[buf][g][st][tig * PC + 8 * c + gid];
 #pragma unroll
-            for (int c = 0; c < NT; c++) {
-                const int col = wn * 8 * NT + 8 * c + gid;
-                const unsigned b0b = sBb[buf][col][kb + tig], b0s = sBs[buf][col][kb + tig];
-                const unsigned b1b = sBb[buf][col][kb + tig + 4], b1s = sBs[buf][col][kb + tig + 4];
+                for (int m = 0; m < MW; m++) {
+                    if (m < MW - 1 || full) {
+                        const uint4 *hm = H + (m * D.k8 + step) * 64;
+                        const uint4 h0 = __ldg(hm), h1 = __ldg(hm + 32);
 #pragma unroll
-                for (int a = 0; a < 2; a++) {
-                    mma_tf32(facc[a][c], as[a], b0b, b1b);
-                    mma_tf32(facc[a][c], ab[a], b0s, b1s);
-                    mma_tf32(facc[a][c], ab[a], b0b, b1b);
+                        for (int c = 0; c < NC; c++) {
+                            if constexpr (F64) {
+                                mma_f64(acc[m][c], *reinterpret_cast<const double2 *>(&h0),
+                                        *reinterpret_cast<const double2 *>(&h1),
+                                        *reinterpret_cast<const double2 *>(&f[c]));
+                            } else if constexpr (XP) {   // field small x H big, field big x H small, big x big
+                                mma_tf32(acc[m][c], h0, f[c].y, f[c].w);
+                                mma_tf32(acc[m][c], h1, f[c].x, f[c].z);
+                                mma_tf32(acc[m][c], h0, f[c].x, f[c].z);
+                            } else {                     // H small x field big, H big x field small, big x big
+                                mma_tf32(acc[m][c], h1, f[c].x, f[c].z);
+                                mma_tf32(acc[m][c], h0, f[c].y, f[c].w);
+                                mma_tf32(acc[m][c], h0, f[c].x, f[c].z);
+                            }
+                        }
+                    }
                 }
             }
         }
@@ -437,358 +392,96 @@ __global__ void __launch_bounds__(256) dst_right_tf32_kernel(PadTf32 D, const TI
         __syncthreads();
         buf ^= 1;
     }
+    // the tile returns through shared memory (the last barrier above also ends the reads of the staged field)
+    TC *out = reinterpret_cast<TC *>(dsm);
+    const int lines = 32 * D.mt, px = tile_row(D.mt);
 #pragma unroll
-    for (int a = 0; a < 2; a++)
+    for (int m = 0; m < MW; m++) {
+        if (m < mine) {
 #pragma unroll
-        for (int c = 0; c < NT; c++)
+            for (int c = 0; c < NC; c++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const long long r = r0 + wm * 32 + a * 16 + gid + 8 * (e >> 1);
-                const int ii = i0 + wn * 8 * NT + 8 * c + 2 * tig + (e & 1);
-                if (r < R && ii < cols) C[r * n + 2 * ii + g] = (TO)facc[a][c][e];
-            }
-}
-
-// right-pass column tile: 16 NT columns with NT = ceil(k0 / 16) in 3..8 (one tile per parity up to 128 columns)
-inline int right_nt(int k0) {
-    const int nt = (k0 + 15) / 16;
-    return nt < 3 ? 3 : (nt > 8 ? 8 : nt);
-}
-inline size_t left_tf32_smem() { return sizeof(unsigned) * 4 * QK * (QPA + QPB); }
-inline size_t right_tf32_smem(int nt) { return sizeof(unsigned) * 4 * QPK * (QR + 16 * nt); }
-
-// Padded TF32 tiles of one axis: the right pass (x) stores H_g row-major padded to column tiles of its width, the left
-// passes (y, z) H_g^T padded to 128-row tiles; K is padded to the K block.  Buffer: big g0, big g1, small g0, small g1.
-inline long long pad_geometry(int axis, int n, int kg[2], int ipad[2], int kpad[2]) {
-    kg[0] = (n + 1) / 2;
-    kg[1] = n / 2;
-    const int tile = axis == 0 ? 16 * right_nt(kg[0]) : QR;
-    for (int g = 0; g < 2; g++) {
-        ipad[g] = (kg[g] + tile - 1) / tile * tile;
-        kpad[g] = (kg[g] + QK - 1) / QK * QK;
+                for (int e = 0; e < 4; e++) {
+                    const int line = 2 * (16 * (wm * MW + m) + gid + 8 * (e >> 1)) + g;
+                    const int cc = 8 * c + 2 * tig + (e & 1);
+                    out[XP ? cc * px + line : line * kTileCol<TC> + cc] = acc[m][c][e];
+                }
+        }
     }
-    return 2LL * ((long long)ipad[0] * kpad[0] + (long long)ipad[1] * kpad[1]);
-}
-inline PadTf32 pad_tf32(const unsigned *t, int axis, int n) {
-    PadTf32 T;
-    T.n = n;
-    pad_geometry(axis, n, T.kg, T.ipad, T.kpad);
-    const long long a0 = (long long)T.ipad[0] * T.kpad[0], a1 = (long long)T.ipad[1] * T.kpad[1];
-    T.b[0] = t;
-    T.b[1] = t + a0;
-    T.s[0] = t + a0 + a1;
-    T.s[1] = t + 2 * a0 + a1;
-    return T;
+    __syncthreads();
+    const int l0 = tile * lines, left = n - l0 < lines ? n - l0 : lines;
+    if (XP) {
+        for (int r = warp; r < QC && c0 + r < ncol; r += DT / 32) {
+            TO *row = C + (c0 + r) * n + l0;
+#pragma unroll 4
+            for (int j = lane; j < left; j += 32) row[j] = (TO)out[r * px + j];
+        }
+    } else {
+        constexpr int LC = QC < 32 ? QC : 32, LR = DT / LC;   // threads along a line, lines at a time
+        const int l2 = (int)threadIdx.x / LC;
+#pragma unroll
+        for (int h = 0; h < QC / LC; h++) {
+            const int cc = (int)threadIdx.x % LC + LC * h;
+            const long long oc = c0 + cc;
+            if (oc >= ncol) continue;
+            const long long cb = (long long)((unsigned)oc / (unsigned)W) * bs;
+            const int w = (int)((unsigned)oc % (unsigned)W);
+            // the operands of kLines lines are loaded together, then used: a load and a divide per line in turn would
+            // add up their latencies (float64 z passes of the solve above 392 -> 296 us)
+            for (int l1 = l2; l1 < left; l1 += LR * kLines) {
+                double op[kLines];
+#pragma unroll
+                for (int j = 0; j < kLines; j++) {
+                    const int line = l1 + LR * j;
+                    const long long io = (long long)(l0 + line) * W + w;
+                    if (EPI) op[j] = line < left ? (EPI == 1 ? den[io] : post[cb + io]) : 1.;
+                }
+#pragma unroll
+                for (int j = 0; j < kLines; j++) {
+                    const int line = l1 + LR * j;
+                    if (line >= left) break;
+                    double v = (double)out[line * kTileCol<TC> + cc];
+                    if (EPI == 1) v = v / op[j];
+                    if (EPI == 2) v = sign * (op[j] * v);
+                    C[cb + (long long)(l0 + line) * W + w] = (TO)v;
+                }
+            }
+        }
+    }
 }
 
-// the TF32 passes' shared memory is above the 48 KB default: set once per device (see allow_slices in q1.cu)
-template <int NT>
-int allow_right_tf32() {
-    SVP_CUDA(cudaFuncSetAttribute(dst_right_tf32_kernel<NT, double, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)right_tf32_smem(NT)));
-    SVP_CUDA(cudaFuncSetAttribute(dst_right_tf32_kernel<NT, float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)right_tf32_smem(NT)));
-    return SVP_OK;
-}
-int allow_tf32() {
+// the passes' shared memory may lie above the 48 KB default: set once per kernel and device (see allow_slices in q1.cu)
+template <bool XP, bool PRE, int MW, int EPI, class TC, class TI, class TO>
+int launch_dst(const DstFrag &F, const TI *in, long long ncol, int W, long long bs, TO *out, const double *pre,
+               const double *den, const double *post, double sign, cudaStream_t s) {
     static std::mutex mu;
     static bool done[64] = {};
     int dev = 0;
     SVP_CUDA(cudaGetDevice(&dev));
-    SVP_REQUIRE(dev >= 0 && dev < 64, "allow_tf32: device ordinal out of range");
-    std::lock_guard<std::mutex> lock(mu);
-    if (done[dev]) return SVP_OK;
-    const int ls = (int)left_tf32_smem();
-    SVP_CUDA(cudaFuncSetAttribute(dst_left_tf32_kernel<0, float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, ls));
-    SVP_CUDA(cudaFuncSetAttribute(dst_left_tf32_kernel<1, float, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, ls));
-    SVP_CUDA(cudaFuncSetAttribute(dst_left_tf32_kernel<0, float, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, ls));
-    SVP_CUDA(cudaFuncSetAttribute(dst_left_tf32_kernel<2, float, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, ls));
-    int rc;
-    if ((rc = allow_right_tf32<3>()) || (rc = allow_right_tf32<4>()) || (rc = allow_right_tf32<5>()) ||
-        (rc = allow_right_tf32<6>()) || (rc = allow_right_tf32<7>()) || (rc = allow_right_tf32<8>()))
-        return rc;
-    done[dev] = true;
+    SVP_REQUIRE(dev >= 0 && dev < 64, "launch_dst: device ordinal out of range");
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!done[dev]) {
+            SVP_CUDA(cudaFuncSetAttribute(dst_pass_kernel<XP, PRE, MW, EPI, TC, TI, TO>,
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dst_smem<TC>(XP, 2 * MW)));
+            done[dev] = true;
+        }
+    }
+    const long long blocks = div_up(ncol, kQC<TC>) * F.tiles;
+    SVP_REQUIRE(blocks <= 0x7fffffffLL && ncol <= 0xffffffffLL, "dst pass: grid too large");
+    SVP_LAUNCH((dst_pass_kernel<XP, PRE, MW, EPI, TC, TI, TO><<<(unsigned)blocks, DT, dst_smem<TC>(XP, F.mt), s>>>(
+        F, in, ncol, W, bs, out, pre, den, post, sign)));
     return SVP_OK;
 }
-template <class TI, class TO>
-int launch_right_tf32(int nt, dim3 grid, const PadTf32 &T, const TI *in, long long R, const double *pre, TO *out,
-                      cudaStream_t s) {
-    const size_t sm = right_tf32_smem(nt);
-    switch (nt) {
-        case 3: SVP_LAUNCH((dst_right_tf32_kernel<3, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        case 4: SVP_LAUNCH((dst_right_tf32_kernel<4, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        case 5: SVP_LAUNCH((dst_right_tf32_kernel<5, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        case 6: SVP_LAUNCH((dst_right_tf32_kernel<6, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        case 7: SVP_LAUNCH((dst_right_tf32_kernel<7, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        default: SVP_LAUNCH((dst_right_tf32_kernel<8, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
+template <bool XP, bool PRE, int EPI, class TC, class TI, class TO>
+int launch_dst_rows(const DstFrag &F, const TI *in, long long ncol, int W, long long bs, TO *out,
+                    const double *pre, const double *den, const double *post, double sign, cudaStream_t s) {
+    switch ((F.mt + 1) / 2) {
+        case 1: return launch_dst<XP, PRE, 1, EPI, TC, TI, TO>(F, in, ncol, W, bs, out, pre, den, post, sign, s);
+        case 2: return launch_dst<XP, PRE, 2, EPI, TC, TI, TO>(F, in, ncol, W, bs, out, pre, den, post, sign, s);
+        case 3: return launch_dst<XP, PRE, 3, EPI, TC, TI, TO>(F, in, ncol, W, bs, out, pre, den, post, sign, s);
+        default: return launch_dst<XP, PRE, 4, EPI, TC, TI, TO>(F, in, ncol, W, bs, out, pre, den, post, sign, s);
     }
-    return SVP_OK;
-}
-
-// ------------------------------------------------------------------------------- plain form (FP64 DMMA), tiled
-// The float64 passes with the tiling of the 3xTF32 ones: zero-padded half matrices (pad_half_kernel, the same
-// geometry), a 128 x 64 (left) or 64 x 16 NT (right) output tile per block, 8 warps of 32 x 32 (16 x 8 NT) = 4 x 4
-// (2 x NT) DMMA 8x8x4 tiles, K blocks of 16 staged twice-buffered through registers.  Rows of the staged blocks are
-// padded to 4 mod 16 doubles, so the 64-bit fragment loads of each half warp fall in distinct bank pairs.  Every
-// output is the DMMA sequence over k in order (kb = 0, 4, 8, ...), the accumulation of a plain 8x8x4 tiling, so the
-// values do not depend on the tile shape.
-constexpr int DPB = QC + 4, DPK = QK + 4;
-
-struct PadF64 {
-    const double *h[2];   // per parity, zero-padded to kpad x ipad (left, k-major) or ipad x kpad (right)
-    int n, kg[2], ipad[2], kpad[2];
-};
-
-__global__ void pad_half_kernel(const double *__restrict__ h, int kg, long long src, int kmajor, int ipad, int kpad,
-                                double *__restrict__ out) {
-    const long long total = (long long)ipad * kpad;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        const int a = kmajor ? (int)(e % ipad) : (int)(e / kpad), k = kmajor ? (int)(e / ipad) : (int)(e % kpad);
-        out[e] = (a < kg && k < kg) ? h[src + (long long)a * kg + k] : 0.;
-    }
-}
-
-// MR m8 row tiles per warp: a block covers 32 MR rows (4 row warps) x 64 columns (2 column warps).
-template <int MR, int EPI, class TI, class TO>
-__global__ void __launch_bounds__(256) dst_left_dmma_kernel(PadF64 D, const TI *__restrict__ X, long long W,
-                                                            long long ldx, long long bs, TO *__restrict__ C,
-                                                            const double *__restrict__ den,
-                                                            const double *__restrict__ post, double sign) {
-    constexpr int RB = 32 * MR, PA = RB + 4;
-    extern __shared__ __align__(16) double dsm[];
-    double(*sA)[QK][PA] = reinterpret_cast<double(*)[QK][PA]>(dsm);
-    double(*sB)[QK][DPB] = reinterpret_cast<double(*)[QK][DPB]>(dsm + 2 * QK * PA);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
-    const int wm = warp >> 1, wn = warp & 1;
-    const int t0 = D.ipad[0] / RB;
-    const int g = (int)blockIdx.x < t0 ? 0 : 1;
-    const int rows = g ? D.kg[1] : D.kg[0], K = rows, ip = g ? D.ipad[1] : D.ipad[0];
-    const int i0 = ((int)blockIdx.x - (g ? t0 : 0)) * RB;
-    const double *H = g ? D.h[1] : D.h[0];
-    const long long w0 = (long long)blockIdx.y * QC;
-    const TI *Xb = X + (long long)blockIdx.z * bs;
-    double dacc[MR][4][2];
-#pragma unroll
-    for (int a = 0; a < MR; a++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) dacc[a][c][0] = dacc[a][c][1] = 0.;
-    // staging: the matrix block (16 x 32 MR) as MR double2 per thread (16 MR per row), the field block (16 x 64,
-    // with mirrors) as four entries per thread
-    const int xr = threadIdx.x >> 6, xc = threadIdx.x & 63;
-    const bool okw = w0 + xc < W;
-    double2 hv[MR];
-    TI xa[4], xb[4];
-    auto fetch = [&](int k0) {
-#pragma unroll
-        for (int t = 0; t < MR; t++) {
-            const int v = threadIdx.x + 256 * t;
-            hv[t] = *reinterpret_cast<const double2 *>(H + (long long)(k0 + v / (16 * MR)) * ip + i0 +
-                                                       (v % (16 * MR)) * 2);
-        }
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-            const int k = k0 + xr + 4 * t;
-            const bool ok = okw && k < K;
-            xa[t] = ok ? Xb[(long long)k * ldx + w0 + xc] : TI(0);
-            xb[t] = ok ? Xb[(long long)(D.n - 1 - k) * ldx + w0 + xc] : TI(0);
-        }
-    };
-    auto stash = [&](int buf, int k0) {
-#pragma unroll
-        for (int t = 0; t < MR; t++) {
-            const int v = threadIdx.x + 256 * t;
-            *reinterpret_cast<double2 *>(&sA[buf][v / (16 * MR)][(v % (16 * MR)) * 2]) = hv[t];
-        }
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-            const int k = k0 + xr + 4 * t;
-            sB[buf][xr + 4 * t][xc] = fold_value<double>((double)xa[t], (double)xb[t], k == D.n - 1 - k, g);
-        }
-    };
-    fetch(0);
-    stash(0, 0);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = 0; k0 < K; k0 += QK) {
-        const bool more = k0 + QK < K;
-        if (more) fetch(k0 + QK);
-#pragma unroll
-        for (int kb = 0; kb < QK; kb += 4) {
-            double a[MR], x[4];
-#pragma unroll
-            for (int m = 0; m < MR; m++) a[m] = sA[buf][kb + tig][wm * 8 * MR + 8 * m + gid];
-#pragma unroll
-            for (int c = 0; c < 4; c++) x[c] = sB[buf][kb + tig][wn * 32 + 8 * c + gid];
-#pragma unroll
-            for (int m = 0; m < MR; m++)
-#pragma unroll
-                for (int c = 0; c < 4; c++) dmma_8x8x4(dacc[m][c], a[m], x[c]);
-        }
-        if (more) stash(buf ^ 1, k0 + QK);
-        __syncthreads();
-        buf ^= 1;
-    }
-    const long long cb = (long long)blockIdx.z * bs;
-#pragma unroll
-    for (int m = 0; m < MR; m++)
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int ii = i0 + wm * 8 * MR + 8 * m + gid;
-                const long long w = w0 + wn * 32 + 8 * c + 2 * tig + e;
-                if (ii >= rows || w >= W) continue;
-                const long long io = (long long)(2 * ii + g) * ldx + w, o = cb + io;
-                double v = dacc[m][c][e];
-                if (EPI == 1) v = v / den[io];
-                if (EPI == 2) v = sign * (post[o] * v);
-                C[o] = (TO)v;
-            }
-}
-
-// MR m8 row tiles per warp: a block covers 32 MR rows (4 row warps) x 16 NT columns (2 column warps).
-template <int MR, int NT, class TI, class TO>
-__global__ void __launch_bounds__(256) dst_right_dmma_kernel(PadF64 D, const TI *__restrict__ X, long long R,
-                                                             const double *__restrict__ pre, TO *__restrict__ C) {
-    constexpr int QN = 16 * NT, RB = 32 * MR, XT = RB / 16;
-    extern __shared__ __align__(16) double dsm[];
-    double(*sA)[RB][DPK] = reinterpret_cast<double(*)[RB][DPK]>(dsm);
-    double(*sB)[QN][DPK] = reinterpret_cast<double(*)[QN][DPK]>(dsm + 2 * RB * DPK);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
-    const int wm = warp >> 1, wn = warp & 1;
-    const int t0 = D.ipad[0] / QN;
-    const int g = (int)blockIdx.x < t0 ? 0 : 1;
-    const int cols = g ? D.kg[1] : D.kg[0], K = cols, kp = g ? D.kpad[1] : D.kpad[0];
-    const int i0 = ((int)blockIdx.x - (g ? t0 : 0)) * QN;
-    const double *H = g ? D.h[1] : D.h[0];
-    const long long r0 = (long long)blockIdx.y * RB;
-    const int n = D.n;
-    double dacc[MR][NT][2];
-#pragma unroll
-    for (int a = 0; a < MR; a++)
-#pragma unroll
-        for (int c = 0; c < NT; c++) dacc[a][c][0] = dacc[a][c][1] = 0.;
-    const int xk = threadIdx.x & 15, xr = threadIdx.x >> 4;
-    constexpr int HV = QN * QK / 2, HT = (HV + 255) / 256;
-    double xa[XT], xb[XT];
-    double2 hv[HT];
-    auto fetch = [&](int k0) {
-        const int k = k0 + xk;
-#pragma unroll
-        for (int t = 0; t < XT; t++) {
-            const long long r = r0 + xr + 16 * t;
-            const bool ok = r < R && k < K;
-            const long long a = r * n + k, m = r * n + (n - 1 - k);
-            xa[t] = ok ? (pre ? pre[a] * (double)X[a] : (double)X[a]) : 0.;
-            xb[t] = ok ? (pre ? pre[m] * (double)X[m] : (double)X[m]) : 0.;
-        }
-#pragma unroll
-        for (int t = 0; t < HT; t++) {
-            const int v = threadIdx.x + 256 * t;
-            if (v < HV)
-                hv[t] = *reinterpret_cast<const double2 *>(H + (long long)(i0 + v / (QK / 2)) * kp + k0 +
-                                                           (v % (QK / 2)) * 2);
-        }
-    };
-    auto stash = [&](int buf, int k0) {
-        const int k = k0 + xk;
-        const bool mid = k == n - 1 - k;
-#pragma unroll
-        for (int t = 0; t < XT; t++) sA[buf][xr + 16 * t][xk] = fold_value<double>(xa[t], xb[t], mid, g);
-#pragma unroll
-        for (int t = 0; t < HT; t++) {
-            const int v = threadIdx.x + 256 * t;
-            if (v < HV) *reinterpret_cast<double2 *>(&sB[buf][v / (QK / 2)][(v % (QK / 2)) * 2]) = hv[t];
-        }
-    };
-    fetch(0);
-    stash(0, 0);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = 0; k0 < K; k0 += QK) {
-        const bool more = k0 + QK < K;
-        if (more) fetch(k0 + QK);
-#pragma unroll
-        for (int kb = 0; kb < QK; kb += 4) {
-            double a[MR], x[NT];
-#pragma unroll
-            for (int m = 0; m < MR; m++) a[m] = sA[buf][wm * 8 * MR + 8 * m + gid][kb + tig];
-#pragma unroll
-            for (int c = 0; c < NT; c++) x[c] = sB[buf][wn * 8 * NT + 8 * c + gid][kb + tig];
-#pragma unroll
-            for (int m = 0; m < MR; m++)
-#pragma unroll
-                for (int c = 0; c < NT; c++) dmma_8x8x4(dacc[m][c], a[m], x[c]);
-        }
-        if (more) stash(buf ^ 1, k0 + QK);
-        __syncthreads();
-        buf ^= 1;
-    }
-#pragma unroll
-    for (int m = 0; m < MR; m++)
-#pragma unroll
-        for (int c = 0; c < NT; c++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const long long r = r0 + wm * 8 * MR + 8 * m + gid;
-                const int ii = i0 + wn * 8 * NT + 8 * c + 2 * tig + e;
-                if (r < R && ii < cols) C[r * n + 2 * ii + g] = (TO)dacc[m][c][e];
-            }
-}
-
-// the left float64 passes: DML m8 row tiles per warp (blocks of 32 DML rows)
-constexpr int DML = 4;
-inline size_t left_dmma_smem() { return sizeof(double) * 2 * QK * (32 * DML + 4 + DPB); }
-// the right float64 pass: 64-row blocks (2 m8 tiles per warp) keep two 256-thread blocks resident per SM
-constexpr int DMR = 2;
-inline size_t right_dmma_smem(int nt) { return sizeof(double) * 2 * DPK * (32 * DMR + 16 * nt); }
-inline PadF64 pad_f64(const double *t, int axis, int n) {
-    PadF64 T;
-    T.n = n;
-    pad_geometry(axis, n, T.kg, T.ipad, T.kpad);
-    T.h[0] = t;
-    T.h[1] = t + (long long)T.ipad[0] * T.kpad[0];
-    return T;
-}
-template <int NT>
-int allow_right_dmma() {
-    SVP_CUDA(cudaFuncSetAttribute(dst_right_dmma_kernel<DMR, NT, double, double>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)right_dmma_smem(NT)));
-    return SVP_OK;
-}
-int allow_dmma() {
-    static std::mutex mu;
-    static bool done[64] = {};
-    int dev = 0;
-    SVP_CUDA(cudaGetDevice(&dev));
-    SVP_REQUIRE(dev >= 0 && dev < 64, "allow_dmma: device ordinal out of range");
-    std::lock_guard<std::mutex> lock(mu);
-    if (done[dev]) return SVP_OK;
-    const int ls = (int)left_dmma_smem();
-    SVP_CUDA(cudaFuncSetAttribute(dst_left_dmma_kernel<DML, 0, double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, ls));
-    SVP_CUDA(cudaFuncSetAttribute(dst_left_dmma_kernel<DML, 1, double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, ls));
-    SVP_CUDA(cudaFuncSetAttribute(dst_left_dmma_kernel<DML, 2, double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, ls));
-    int rc;
-    if ((rc = allow_right_dmma<3>()) || (rc = allow_right_dmma<4>()) || (rc = allow_right_dmma<5>()) ||
-        (rc = allow_right_dmma<6>()) || (rc = allow_right_dmma<7>()) || (rc = allow_right_dmma<8>()))
-        return rc;
-    done[dev] = true;
-    return SVP_OK;
-}
-template <class TI, class TO>
-int launch_right_dmma(int nt, dim3 grid, const PadF64 &T, const TI *in, long long R, const double *pre, TO *out,
-                      cudaStream_t s) {
-    const size_t sm = right_dmma_smem(nt);
-    switch (nt) {
-        case 3: SVP_LAUNCH((dst_right_dmma_kernel<DMR, 3, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        case 4: SVP_LAUNCH((dst_right_dmma_kernel<DMR, 4, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        case 5: SVP_LAUNCH((dst_right_dmma_kernel<DMR, 5, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        case 6: SVP_LAUNCH((dst_right_dmma_kernel<DMR, 6, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        case 7: SVP_LAUNCH((dst_right_dmma_kernel<DMR, 7, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-        default: SVP_LAUNCH((dst_right_dmma_kernel<DMR, 8, TI, TO><<<grid, 256, sm, s>>>(T, in, R, pre, out))); break;
-    }
-    return SVP_OK;
 }
 
 __global__ void scale_kernel(const double *__restrict__ x, const double *__restrict__ s, double sign, long long n,
@@ -834,52 +527,46 @@ int apply_axis(const double *M, int axis, long long batch, long long n2, long lo
 
 std::vector<double> dst1_matrix(int n);
 
-// One DST-I pass along `axis` of (3, n2, n1, n0) fields with the folded half matrices; see dst_left_tf32_kernel for
-// pre / EPI.
+// One DST-I pass along `axis` of (3, n2, n1, n0) fields with the folded half matrices; see dst_pass_kernel for pre,
+// the epilogues and sign.
 template <class TC, class TI, class TO>
 static int dst_pass(const svp_pair *p, int axis, const TI *in, TO *out, const double *pre, int epi, double sign,
                     const double *post, cudaStream_t s) {
     const long long n0 = p->q.fx, n1 = p->q.fy, n2 = p->q.fz;
-    const int n = p->dst_n[axis], k0 = (n + 1) / 2;
-    constexpr bool kDouble = sizeof(TC) == 8;
-    PadF64 D = pad_f64(p->dst_pad[axis], axis, n);
-    PadTf32 T = pad_tf32(p->dst_tf32[axis], axis, n);
-    {
-        int rc = kDouble ? allow_dmma() : allow_tf32();
-        if (rc) return rc;
-    }
+    const DstFrag F = frag_of(sizeof(TC) == 8 ? (const void *)p->dst_f64[axis] : (const void *)p->dst_tf32[axis],
+                              p->dst_n[axis]);
+    int rc;
     if (axis == 0) {
         SVP_REQUIRE(epi == 0, "dst_pass: x pass has no epilogue");
-        long long R = 3 * n2 * n1;
+        const long long R = 3 * n2 * n1;
         svp::KernelTimer _t("dst_right_kernel", s);
-        // the column tiles of one row block lead the grid: the blocks that share rows run together (L2 reuse)
-        const int nt = right_nt(k0);
-        dim3 grid((unsigned)((T.ipad[0] + T.ipad[1]) / (16 * nt)), (unsigned)div_up(R, kDouble ? 32 * DMR : QR));
-        int rc;
-        if constexpr (kDouble) rc = launch_right_dmma<TI, TO>(nt, grid, D, in, R, pre, out, s);
-        else rc = launch_right_tf32<TI, TO>(nt, grid, T, in, R, pre, out, s);
-        if (rc) return rc;
+        rc = SVP_OK;
+        if constexpr (sizeof(TO) == sizeof(TC))   // the x pass returns its own type
+            rc = pre ? launch_dst_rows<true, true, 0, TC, TI, TO>(F, in, R, 1, 0, out, pre, nullptr, nullptr, 1., s)
+                     : launch_dst_rows<true, false, 0, TC, TI, TO>(F, in, R, 1, 0, out, pre, nullptr, nullptr, 1., s);
     } else {
         SVP_REQUIRE(!pre, "dst_pass: pre-scale only on the x pass");
         SVP_REQUIRE(epi != 1 || axis == 2, "dst_pass: the 1/den epilogue rides in the z pass (batch stride = nfree)");
-        long long W = axis == 1 ? n0 : n1 * n0;
-        long long ldx = W, bs = axis == 1 ? n1 * n0 : n2 * n1 * n0;
-        // the row tiles of both parities lead the grid: the blocks that read the same field columns run together
-        dim3 qgrid((unsigned)((T.ipad[0] + T.ipad[1]) / QR), (unsigned)div_up(W, QC), (unsigned)(axis == 1 ? 3 * n2 : 3));
+        const long long W = axis == 1 ? n0 : n1 * n0, bs = axis == 1 ? n1 * n0 : n2 * n1 * n0;
+        const long long ncol = (axis == 1 ? 3 * n2 : 3) * W;
+        SVP_REQUIRE(W <= 0x7fffffffLL, "dst_pass: plane too large");
         svp::KernelTimer _t("dst_left_kernel", s);
-        if constexpr (kDouble) {
-            const size_t ds = left_dmma_smem();
-            dim3 dgrid((unsigned)((D.ipad[0] + D.ipad[1]) / (32 * DML)), qgrid.y, qgrid.z);
-            if (epi == 0) SVP_LAUNCH((dst_left_dmma_kernel<DML, 0, TI, TO><<<dgrid, 256, ds, s>>>(D, in, W, ldx, bs, out, nullptr, nullptr, 1.)));
-            else if (epi == 1) SVP_LAUNCH((dst_left_dmma_kernel<DML, 1, TI, TO><<<dgrid, 256, ds, s>>>(D, in, W, ldx, bs, out, p->den, nullptr, 1.)));
-            else SVP_LAUNCH((dst_left_dmma_kernel<DML, 2, TI, TO><<<dgrid, 256, ds, s>>>(D, in, W, ldx, bs, out, nullptr, post, sign)));
-        } else {
-            const size_t qs = left_tf32_smem();
-            if (epi == 0) SVP_LAUNCH((dst_left_tf32_kernel<0, TI, TO><<<qgrid, 256, qs, s>>>(T, in, W, ldx, bs, out, nullptr, nullptr, 1.)));
-            else if (epi == 1) SVP_LAUNCH((dst_left_tf32_kernel<1, TI, TO><<<qgrid, 256, qs, s>>>(T, in, W, ldx, bs, out, p->den, nullptr, 1.)));
-            else SVP_LAUNCH((dst_left_tf32_kernel<2, TI, TO><<<qgrid, 256, qs, s>>>(T, in, W, ldx, bs, out, nullptr, post, sign)));
+        rc = SVP_OK;
+        if constexpr (sizeof(TI) == sizeof(TC)) {
+            if (epi == 0)
+                rc = launch_dst_rows<false, false, 0, TC, TI, TO>(F, in, ncol, (int)W, bs, out, nullptr,
+                                                           nullptr, nullptr, 1., s);
+            if constexpr (sizeof(TO) == sizeof(TC))
+                if (epi == 1)
+                    rc = launch_dst_rows<false, false, 1, TC, TI, TO>(F, in, ncol, (int)W, bs, out, nullptr,
+                                                               p->den, nullptr, 1., s);
+            if constexpr (sizeof(TO) == 8)
+                if (epi == 2)
+                    rc = launch_dst_rows<false, false, 2, TC, TI, TO>(F, in, ncol, (int)W, bs, out, nullptr,
+                                                               nullptr, post, sign, s);
         }
     }
+    if (rc) return rc;
     SVP_LAUNCH_CHECK("dst pass");
     return SVP_OK;
 }
@@ -930,16 +617,15 @@ static std::vector<double> cached_dst1_half(int n) {
 void pair_dst_carve(svp_pair *p, SlabCursor &c) {
     const long long f[3] = {p->q.fx, p->q.fy, p->q.fz};
     for (int k = 0; k < 3; k++) {
-        int kg[2], ipad[2], kpad[2];
-        const long long words = pad_geometry(k, (int)f[k], kg, ipad, kpad);
-        c.take(p->dst_pad[k], (size_t)words / 2);
-        c.take(p->dst_tf32[k], (size_t)words);
+        const size_t cells = 2 * frag_cells(frag_geometry((int)f[k]));
+        c.take(p->dst_f64[k], 2 * cells);
+        c.take(p->dst_tf32[k], 4 * cells);
     }
     c.take(p->dst_tmp, (size_t)(2 * 3 * p->q.nfree));
     c.take(p->den, (size_t)p->q.nfree);
 }
 
-// Fills the padded matrices: the folded half matrices of the three axes, and their values rounded once to float32, go
+// Fills the fragment cells: the folded half matrices of the three axes, and their values rounded once to float32, go
 // up in one copy each and are laid out (and split into TF32 parts with the cvt.rna of the passes) on the device.
 int pair_dst_setup(svp_pair *p, cudaStream_t s) {
     const long long f[3] = {p->q.fx, p->q.fy, p->q.fz};
@@ -959,15 +645,13 @@ int pair_dst_setup(svp_pair *p, cudaStream_t s) {
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(h32, all32.data(), sizeof(float) * all32.size(), cudaMemcpyHostToDevice, s);
     for (int k = 0; k < 3 && e == cudaSuccess; k++) {
-        const PadF64 D = pad_f64(p->dst_pad[k], k, (int)f[k]);
-        const PadTf32 T = pad_tf32(p->dst_tf32[k], k, (int)f[k]);
+        const DstFrag D = frag_of(p->dst_f64[k], (int)f[k]), T = frag_of(p->dst_tf32[k], (int)f[k]);
+        const long long cells = (long long)frag_cells(D);
         for (int g = 0; g < 2; g++) {
-            const unsigned nb = blocks_for((long long)D.ipad[g] * D.kpad[g], 256, 4);
+            const unsigned nb = blocks_for(cells, 256, 4);
             const long long src = (long long)off[k] + (g ? (long long)D.kg[0] * D.kg[0] : 0);
-            pad_half_kernel<<<nb, 256, 0, s>>>(h, D.kg[g], src, k != 0, D.ipad[g], D.kpad[g],
-                                               const_cast<double *>(D.h[g]));
-            split_pad_kernel<<<nb, 256, 0, s>>>(h32, D.kg[g], src, k != 0, D.ipad[g], D.kpad[g],
-                                                const_cast<unsigned *>(T.b[g]), const_cast<unsigned *>(T.s[g]));
+            frag_kernel<double><<<nb, 256, 0, s>>>(h, D.kg[g], src, cells, D.k8, const_cast<uint4 *>(D.h[g]));
+            frag_kernel<float><<<nb, 256, 0, s>>>(h32, D.kg[g], src, cells, T.k8, const_cast<uint4 *>(T.h[g]));
         }
         e = cudaGetLastError();
     }

@@ -25,10 +25,10 @@ struct svp_pair {
     long long *cand = nullptr;                // candidate cells of the T69/T73 node JD extension (ncell)
     uint8_t *flags = nullptr;                 // (ncell) cells the float32 cell kernels hand to the float64 barrier
     // DST-I Poisson metric
-    // folded orthonormal DST-I half matrices, x, y, z, zero-padded to the passes' tiles (PadF64)
-    double *dst_pad[3] = {nullptr, nullptr, nullptr};
+    // folded orthonormal DST-I half matrices, x, y, z, zero-padded and in the mma's fragment order (DstFrag)
+    double *dst_f64[3] = {nullptr, nullptr, nullptr};
     int dst_n[3] = {0, 0, 0};                               // their transform lengths (free nodes per axis)
-    // the same rounded to float32 for the mixed form, as TF32 parts: big parts of H0^T, H1^T, then the small parts
+    // the same rounded to float32 for the mixed form, as TF32 parts (big cells, small cells)
     unsigned *dst_tf32[3] = {nullptr, nullptr, nullptr};
     int precision = 0;                                      // SVP_PRECISION_PLAIN or SVP_PRECISION_MIXED
     double *dst_tmp = nullptr;                          // 2 * 3 * nfree scratch
