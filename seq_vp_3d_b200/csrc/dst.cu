@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(256) gemm_right_kernel(const double *__restric
 // around the products) and by instruction issue (3xTF32).  Blocks of 4 warps, 4 per SM, cover each other's phases
 // better than 2 of 8 warps (1278 against 1350 us for the six float64 passes on 224 x 192 x 160, 367 against 377 us for
 // the six mixed ones on 119 x 165 x 141).  Against 128 x 64 (x: 64 or 128 x 16 ceil(k0 / 16)) tiles per parity with
-// both operands staged through shared memory: six passes 1584 -> 1235 us float64, 672 -> 354 us mixed; the operations
+// both operands staged through shared memory: six passes 1584 -> 1205 us float64, 672 -> 344 us mixed; the operations
 // of the float64 passes (11.4 G fused multiply-adds) take 614 us at 18.6 T/s, the bytes of the mixed ones 60 us.
 //
 // Float64: mma.sync m16n8k8 f64 (FP64 has no tcgen05 kind on sm_100a; this is B200's FP64 tensor path).  Mixed form:
@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(DT, 512 / DT) dst_pass_kernel(DstFrag D, const
     const int fk = XP ? (int)threadIdx.x & 15 : (int)threadIdx.x / QC;
     const int fc = XP ? (int)threadIdx.x >> 4 : (int)threadIdx.x % QC;
     const long long ks = XP ? 1 : W;
+    const unsigned last = (unsigned)(n - 1) * (unsigned)W;
     const TI *fx = X + (XP ? (c0 + fc) * n : (c0 + fc < ncol ? flat_base(c0 + fc, W, bs) : 0));
     // Float64: the field of the block that will take this one's place (512 / DT per SM) is brought to L2, up to two
     // lines per k, or the rows of the x pass: 1278 -> 1241 us for the six passes above; the 3xTF32 passes, bound by
@@ -326,8 +327,14 @@ __global__ void __launch_bounds__(DT, 512 / DT) dst_pass_kernel(DstFrag D, const
             const int k = k0 + fk + KE * e;
             const bool ok = c0 + fc + CE * e < ncol && k < K;
             const long long o = (long long)CE * e * n, a = o + k * ks, b = o + (n - 1 - k) * ks;
-            xa[e] = ok ? fx[a] : TI(0);
-            xb[e] = ok ? fx[b] : TI(0);
+            if (XP || EPI) {
+                xa[e] = ok ? fx[a] : TI(0);
+                xb[e] = ok ? fx[b] : TI(0);
+            } else {   // y pass: 32-bit offsets 177 -> 165 us float64, 111 -> 105 mixed; the z passes lose (58 -> 65 us)
+                const unsigned at = (unsigned)k * (unsigned)W;
+                xa[e] = ok ? fx[at] : TI(0);
+                xb[e] = ok ? fx[last - at] : TI(0);
+            }
             if (PRE) {
                 pa[e] = ok ? fp[a] : 0.;
                 pb[e] = ok ? fp[b] : 0.;
@@ -549,7 +556,7 @@ static int dst_pass(const svp_pair *p, int axis, const TI *in, TO *out, const do
         SVP_REQUIRE(epi != 1 || axis == 2, "dst_pass: the 1/den epilogue rides in the z pass (batch stride = nfree)");
         const long long W = axis == 1 ? n0 : n1 * n0, bs = axis == 1 ? n1 * n0 : n2 * n1 * n0;
         const long long ncol = (axis == 1 ? 3 * n2 : 3) * W;
-        SVP_REQUIRE(W <= 0x7fffffffLL, "dst_pass: plane too large");
+        SVP_REQUIRE(p->q.nfree <= 0x7fffffffLL, "dst_pass: more than 2^31 - 1 free nodes");
         svp::KernelTimer _t("dst_left_kernel", s);
         rc = SVP_OK;
         if constexpr (sizeof(TI) == sizeof(TC)) {
