@@ -2093,22 +2093,14 @@ struct ReduceSpec {
 };
 constexpr int kBadSlot = 62;      // of the 64 result slots: the violation count's bits
 __global__ void __launch_bounds__(256) reduce_results_kernel(const __grid_constant__ ReduceSpec r, double *out) {
-    __shared__ dd sh[256];
     int i = 0, k = blockIdx.x;
     while (k >= r.K[i]) k -= r.K[i++];
     const dd *partial = r.src[i];
     const int K = r.K[i];
-    dd acc = {0., 0.};
-    for (long long b = threadIdx.x; b < r.blocks[i]; b += blockDim.x) acc = dd_add(acc, partial[b * K + k]);
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s; s >>= 1) {
-        if ((int)threadIdx.x < s) sh[threadIdx.x] = dd_add(sh[threadIdx.x], sh[threadIdx.x + s]);
-        __syncthreads();
-    }
+    const dd sum = sum_partials(partial, r.blocks[i], K, k);
     if (threadIdx.x == 0) {
-        out[r.out[i] + 2 * k] = sh[0].hi;
-        out[r.out[i] + 2 * k + 1] = sh[0].lo;
+        out[r.out[i] + 2 * k] = sum.hi;
+        out[r.out[i] + 2 * k + 1] = sum.lo;
         if (blockIdx.x == 0 && r.bad) {
             out[kBadSlot] = __longlong_as_double((long long)*r.bad);
             *r.bad = 0;

@@ -55,29 +55,81 @@ __device__ __forceinline__ dd dd_shfl_xor(dd a, int o) {
     return {__shfl_xor_sync(0xFFFFFFFFu, a.hi, o), __shfl_xor_sync(0xFFFFFFFFu, a.lo, o)};
 }
 
-// Block reduction of K double-double accumulators, fixed tree order; thread 0 writes partial[blockIdx][k].
+// Sums of K double-doubles over a warp, lanes 16, 8, 4, 2, 1 apart.  While a lane holds several values it keeps half of
+// them and sends the others to its partner, so 6 values take 8 additions per lane in place of 30 (each is 20 float64
+// operations: at one element per thread they are the kernel).  dd_add is symmetric, so every value has the bits of
+// adding it in all lanes.  Value `first` is in acc[0] of the one lane that returns
+// true for it.
+template <int K>
+__device__ __forceinline__ bool warp_reduce_dd(dd (&acc)[K], int &first) {
+    const int lane = threadIdx.x & 31;
+    int count = K, same = 0;      // values of this lane (`have` at most); lane bits over which the sums are equal
+    first = 0;
+#pragma unroll
+    for (int o = 16, have = K; o; o >>= 1) {
+        const int low = (have + 1) / 2;
+        if (have > 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int k = 0; k < K; k++)
+                if (k < low) {
+                    const dd upper = k + low < have ? acc[(k + low) % K] : dd{0., 0.};
+                    const dd got = dd_shfl_xor(up ? acc[k] : upper, o);
+                    acc[k] = dd_add(up ? upper : acc[k], got);
+                }
+            first += up ? low : 0;
+            count = up ? count - low : (count < low ? count : low);
+        } else {
+            acc[0] = dd_add(acc[0], dd_shfl_xor(acc[0], o));
+            same |= o;
+        }
+        have = low;
+    }
+    return count > 0 && !(lane & same);
+}
+
+// Block reduction of K double-double accumulators, fixed tree order: value k of block b to partial[b][k].
 template <int K>
 __device__ void block_reduce_dd(dd (&acc)[K], dd *partial) {
     __shared__ dd sh[32][K];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; k++)
-#pragma unroll
-        for (int o = 16; o; o >>= 1) acc[k] = dd_add(acc[k], dd_shfl_xor(acc[k], o));
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < K; k++) sh[warp][k] = acc[k];
+    int first;
+    if (warp_reduce_dd<K>(acc, first)) sh[warp][first] = acc[0];
     __syncthreads();
     if (warp == 0) {
         const int nw = blockDim.x >> 5;
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-            dd v = lane < nw ? sh[lane][k] : dd{0., 0.};
-#pragma unroll
-            for (int o = 16; o; o >>= 1) v = dd_add(v, dd_shfl_xor(v, o));
-            if (lane == 0) partial[(size_t)blockIdx.x * K + k] = v;
-        }
+        for (int k = 0; k < K; k++) acc[k] = lane < nw ? sh[lane][k] : dd{0., 0.};
+        if (warp_reduce_dd<K>(acc, first)) partial[(size_t)blockIdx.x * K + first] = acc[0];
     }
+}
+
+// One of K interleaved block sums, added up by a block of 256: thread t takes blocks t, t + 256, ... in order (four
+// loads in flight), then a fixed tree, whose last 32 values need no barrier.  Thread 0 returns the sum.
+__device__ __forceinline__ dd sum_partials(const dd *__restrict__ partial, long long blocks, int K, int k) {
+    __shared__ dd sh[256];
+    const int t = threadIdx.x;
+    dd acc = {0., 0.};
+    for (long long b = t; b < blocks; b += 1024) {
+        dd v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = b + 256 * j < blocks ? partial[(b + 256 * j) * K + k] : dd{0., 0.};
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (b + 256 * j < blocks) acc = dd_add(acc, v[j]);
+    }
+    sh[t] = acc;
+    __syncthreads();
+    if (t < 128) sh[t] = acc = dd_add(acc, sh[t + 128]);
+    __syncthreads();
+    if (t < 64) sh[t] = acc = dd_add(acc, sh[t + 64]);
+    __syncthreads();
+    if (t < 32) {
+        acc = dd_add(acc, sh[t + 32]);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) acc = dd_add(acc, dd_shfl_xor(acc, o));
+    }
+    return acc;
 }
 
 // ------------------------------------------------------------------------------------------- cell geometry

@@ -17,17 +17,9 @@ __global__ void __launch_bounds__(256) dot_kernel(const double *__restrict__ a, 
     block_reduce_dd<1>(acc, partial);
 }
 
-__global__ void dot_final_kernel(const dd *__restrict__ partial, long long blocks, double *out) {
-    __shared__ dd sh[256];
-    dd acc = {0., 0.};
-    for (long long b = threadIdx.x; b < blocks; b += blockDim.x) acc = dd_add(acc, partial[b]);
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s; s >>= 1) {
-        if ((int)threadIdx.x < s) sh[threadIdx.x] = dd_add(sh[threadIdx.x], sh[threadIdx.x + s]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[0] = sh[0].hi + sh[0].lo;
+__global__ void __launch_bounds__(256) dot_final_kernel(const dd *__restrict__ partial, long long blocks, double *out) {
+    const dd sum = sum_partials(partial, blocks, 1, 0);
+    if (threadIdx.x == 0) out[0] = sum.hi + sum.lo;
 }
 
 // y = fl(x + fl(tau * p)): the trial step's two roundings (no FMA), as base.theta + tau * direction
@@ -147,17 +139,8 @@ __global__ void __launch_bounds__(256) step_dots_kernel(const double *__restrict
 // one block per sum (the K sums of one block one after another took 10 us for K = 6)
 __global__ void __launch_bounds__(256) multi_final_kernel(const dd *__restrict__ partial, long long blocks, int K,
                                                           double *out) {
-    __shared__ dd sh[256];
-    const int k = blockIdx.x;
-    dd acc = {0., 0.};
-    for (long long b = threadIdx.x; b < blocks; b += blockDim.x) acc = dd_add(acc, partial[b * K + k]);
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s; s >>= 1) {
-        if ((int)threadIdx.x < s) sh[threadIdx.x] = dd_add(sh[threadIdx.x], sh[threadIdx.x + s]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[k] = sh[0].hi + sh[0].lo;
+    const dd sum = sum_partials(partial, blocks, K, blockIdx.x);
+    if (threadIdx.x == 0) out[blockIdx.x] = sum.hi + sum.lo;
 }
 
 // max |a - b| and max |b| as order keys of non-negative values; a NaN maps above +inf (propagates)
