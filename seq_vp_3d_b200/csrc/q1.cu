@@ -70,8 +70,8 @@ __device__ __forceinline__ void cubic_basis(const double *__restrict__ t, const 
     }
 #pragma unroll
     for (int k = 0; k < 4; k++) B[k] = b[k];
-    // 3 q_(k-1) R - 3 q_k R, the first product fused: the mixed form rounds the image gradient to float32, where a change
-    // of the last float64 bit can show as one of the last float32 bit
+    // 3 q_(k-1) R - 3 q_k R, the first product fused: the mixed form rounds the image gradient to float32, where a
+    // change of the last float64 bit can show as one of the last float32 bit
     const double d0 = 3. * q[0] * R[3], d1 = 3. * q[1] * R[4], d2 = 3. * q[2] * R[5];
     dB[0] = -d0;
     dB[1] = fma(3. * q[0], R[3], -d1);
@@ -1282,6 +1282,32 @@ __device__ __forceinline__ dd sq_change(double a, double b) {
     return {p.hi * .5, p.lo * .5};
 }
 
+// node_weight halves omega once per face that the node lies on: four values, whose roots the stable differences scale
+// by.  A block forms them once: two roots per node were 75 of warp_trial_kernel's 1211 us at 256^3.
+struct NodeScale {
+    double w[4], sq[4], sl[4];    // weight, sqrt(weight), sqrt(lambda weight) on 0..3 faces
+};
+__device__ __forceinline__ void node_scale(const Q1Const &q, NodeScale &t) {
+    if (threadIdx.x < 4) {
+        double w = q.omega;
+        for (int m = 0; m < (int)threadIdx.x; m++) w *= .5;
+        t.w[threadIdx.x] = w;
+        t.sq[threadIdx.x] = sqrt(w);
+        t.sl[threadIdx.x] = sqrt(q.lam * w);
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ int node_faces(long long x, long long y, long long z, const Q1Const &q) {
+    return (x == 0 || x == q.nx - 1) + (y == 0 || y == q.ny - 1) + (z == 0 || z == q.nz - 1);
+}
+
+// compensated (hi, lo) accumulation of t
+__device__ __forceinline__ void acc_add(dd &acc, dd t) {
+    dd s = two_sum(acc.hi, t.hi);
+    acc.hi = s.hi;
+    acc.lo += s.lo + t.lo;
+}
+
 // energy_comparison.py:14-62 localized branch (double precision), unweighted
 __device__ __forceinline__ double barrier_difference(double ja, double jb, double act, double d) {
     double a = ja < act ? ja : act, b = jb < act ? jb : act;
@@ -1300,27 +1326,24 @@ __global__ void __launch_bounds__(256) node_diff_kernel(Q1Const q, const double 
                                                         const double *__restrict__ wb,
                                                         const double *__restrict__ fixed,
                                                         const double *__restrict__ uref, dd *partial) {
+    __shared__ NodeScale scale;
+    node_scale(q, scale);
     dd acc[2] = {{0., 0.}, {0., 0.}};
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < q.nnode;
          i += (long long)gridDim.x * blockDim.x) {
         long long x, y, z;
         unflatten3(i, q.nx, q.ny, x, y, z);
-        double qw = node_weight(x, y, z, q);
-        double sq = sqrt(qw), sl = sqrt(q.lam * qw);
-        acc[0] = dd_add(acc[0], sq_change(sq * (wa[i] - fixed[i]), sq * (wb[i] - fixed[i])));
+        const int m = node_faces(x, y, z, q);
+        const double sq = scale.sq[m], sl = scale.sl[m];
+        acc_add(acc[0], sq_change(sq * (wa[i] - fixed[i]), sq * (wb[i] - fixed[i])));
 #pragma unroll
         for (int r = 0; r < 3; r++)
-            acc[1] = dd_add(acc[1], sq_change(sl * (ua[3 * i + r] - uref[3 * i + r]),
-                                              sl * (ub[3 * i + r] - uref[3 * i + r])));
+            acc_add(acc[1], sq_change(sl * (ua[3 * i + r] - uref[3 * i + r]),
+                                  sl * (ub[3 * i + r] - uref[3 * i + r])));
     }
+#pragma unroll
+    for (int k = 0; k < 2; k++) acc[k] = two_sum(acc[k].hi, acc[k].lo);
     block_reduce_dd<2>(acc, partial);
-}
-
-// compensated (hi, lo) accumulation of t
-__device__ __forceinline__ void acc_add(dd &acc, dd t) {
-    dd s = two_sum(acc.hi, t.hi);
-    acc.hi = s.hi;
-    acc.lo += s.lo + t.lo;
 }
 
 // ============================================================================================== line-search trial
@@ -1328,9 +1351,11 @@ __device__ __forceinline__ void acc_add(dd &acc, dd t) {
 // trial's warped image (and image gradient), its energy sums exactly as node_energy_kernel and the energy-only cell
 // kernels form them, and the stable base -> trial changes exactly as node_diff_kernel and the difference-only cell
 // kernels form them (same grids, same per-thread order, so the results are bitwise those of the separate passes).
-// Bound by the latency of its scattered loads (16 warps per SM at 128 registers; 85 registers spill and lose).  At
-// 256^3: 1441 us; 1401 with a plane of coefficients fetched ahead, 1329 with the L1 prefetches, 1240 with 6 reciprocals
-// per axis read as pairs in place of 14 single ones.  its 16 doubles a node at 6.55 TB/s would take 328 us.
+// Bound by the latency of its scattered loads (16 warps per SM at 128 registers; 85 registers spill and lose) and the
+// float64 work between them.  At 256^3: 1441 us; 1401 with a plane of coefficients fetched ahead, 1329 with the L1
+// prefetches, 1240 with 6 reciprocals per axis read as pairs in place of 14 single ones, 1211 with the differences
+// accumulated in 8 operations for 20, 1136 with the weights' roots from a table.  Its 16 doubles a node at 6.55 TB/s
+// would take 328 us.
 template <bool GRAD>
 __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S, const double *__restrict__ ua,
                                                          const double *__restrict__ wa,
@@ -1338,6 +1363,8 @@ __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S,
                                                          const double *__restrict__ fixed,
                                                          const double *__restrict__ uref, double *__restrict__ wb,
                                                          double *__restrict__ image_grad, dd *pe, dd *pd) {
+    __shared__ NodeScale scale;
+    node_scale(q, scale);
     dd acc[2] = {{0., 0.}, {0., 0.}}, dif[2] = {{0., 0.}, {0., 0.}};
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < q.nnode;
          i += (long long)gridDim.x * blockDim.x) {
@@ -1362,19 +1389,22 @@ __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S,
             image_grad[3 * i + 1] = g[1];
             image_grad[3 * i + 2] = g[2];
         }
-        double qw = node_weight(x, y, z, q);
+        const int m = node_faces(x, y, z, q);
+        const double qw = scale.w[m];
         double f = fixed[i];
         double d = w - f;
         double r0 = uref[3 * i], r1 = uref[3 * i + 1], r2 = uref[3 * i + 2];
         double e0 = ux - r0, e1 = uy - r1, e2 = uz - r2;
         acc[0] = dd_add_d(acc[0], qw * d * d);
         acc[1] = dd_add_d(acc[1], qw * (e0 * e0 + e1 * e1 + e2 * e2));
-        double sq = sqrt(qw), sl = sqrt(q.lam * qw);
-        dif[0] = dd_add(dif[0], sq_change(sq * (wa[i] - f), sq * d));
-        dif[1] = dd_add(dif[1], sq_change(sl * (ua[3 * i] - r0), sl * e0));
-        dif[1] = dd_add(dif[1], sq_change(sl * (ua[3 * i + 1] - r1), sl * e1));
-        dif[1] = dd_add(dif[1], sq_change(sl * (ua[3 * i + 2] - r2), sl * e2));
+        const double sq = scale.sq[m], sl = scale.sl[m];
+        acc_add(dif[0], sq_change(sq * (wa[i] - f), sq * d));
+        acc_add(dif[1], sq_change(sl * (ua[3 * i] - r0), sl * e0));
+        acc_add(dif[1], sq_change(sl * (ua[3 * i + 1] - r1), sl * e1));
+        acc_add(dif[1], sq_change(sl * (ua[3 * i + 2] - r2), sl * e2));
     }
+#pragma unroll
+    for (int k = 0; k < 2; k++) dif[k] = two_sum(dif[k].hi, dif[k].lo);
     block_reduce_dd<2>(acc, pe);
     __syncthreads();     // the two reductions share block_reduce_dd's shared array
     block_reduce_dd<2>(dif, pd);
