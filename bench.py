@@ -169,20 +169,22 @@ FLOP32_PER_CELL = {
     # (squares, stable change, magnitudes) + 8 weighted sums) 2700 + the trial's closed sweep 1350 + 27 x det 459
     # (the base's closed sweep runs only where the base may be active: not counted)
     "cell_trial32_kernel": 10287,
-    # edges 72 + soft sweep2 3780 + 27 x 94 (cofactor, det, curls, fluxes) + adjoint scatter 693
-    "cell_grad32_kernel": 7083,
+    # edges 72 + two fields x (interpolants 162, values 540, curls 162) + 27 x det 459 + 27 x 71 (cofactor, det, fluxes,
+    # sums) + adjoint scatter 693
+    "cell_grad32_kernel": 4869,
     # edges 36 + Gauss sweep 1350 + 27 x (cofactor 35 + 8 vertices x 30) + the curl constants 24
     "cell_ggn_diag32_kernel": 8835,
 }
 FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12    # nominal: 148 SMs x 128 FP32 FMA/clk x 2 x 1965 MHz
-# DRAM bytes (read + write) per cell measured by ncu on the 160x192x96 pair (2,885,055 cells; profiles/
-# traffic_cell_trial_edge_hull_warp_160x192x96.md); scaled to a launch by the cells it processes (traffic grows with
-# the cell count: every launch streams its fields once, plus neighbour re-reads of the same order)
-TRAFFIC_PER_CELL = {"cell_trial_kernel": (325667584 + 1371392) / 2885055,
-                    # full size, 160x192x224 (6,772,287 cells; profiles/cell_kernels_head_pair_160x192x224.md)
+# DRAM bytes (read + write) per cell measured by ncu on a 160^3 grid (4,019,679 cells; profiles/
+# trial_certify_gradient_dst_160.md); scaled to a launch by the cells it processes (traffic grows with the cell count:
+# every launch streams its fields once, plus neighbour re-reads of the same order)
+TRAFFIC_PER_CELL = {"cell_trial_kernel": (481246976 + 7654144) / 4019679,
+                    # 160x192x224 (6,772,287 cells; profiles/cell_kernels_head_pair_160x192x224.md)
                     "cell_trial32_kernel": (813766656 + 19263232) / 6772287,
-                    "edge_hull_kernel": (74312512 + 8776576) / 2885055,
-                    "warp_trial_kernel_grad": (312493568 + 74758400) / 2885055}
+                    "cell_grad32_kernel": (325485312 + 340621568) / 4019679,
+                    "edge_hull_kernel": (106352896 + 8323072) / 4019679,
+                    "warp_trial_kernel_grad": (426808576 + 114931712) / 4019679}
 
 
 def kernel_counts(shape):
@@ -197,7 +199,7 @@ def kernel_counts(shape):
     return {
         # base u, trial u, u_ref: 24 B/node each
         "cell_trial_kernel": (3 * 24 * nn, c("cell_trial_kernel")),
-        # the mixed form's screened trial: the same fields in, float32 sweeps; the barrier flags and the mask out
+        # the screened entry point's trial: the same fields in, float32 sweeps; the barrier flags and the mask out
         "cell_trial32_kernel": (3 * 24 * nn + 2 * nc, None),
         "cell_diff_kernel": (3 * 24 * nn, c("cell_diff_kernel")),
         "cell_energy_kernel": (2 * 24 * nn, c("cell_energy_kernel")),
@@ -515,8 +517,8 @@ def parity_leg(grid, fixed, moving, weights, u_dev, planes):
                                                                    r.min_jd_lower_bound is not None and
                                                                    rd.min_jd_lower_bound >= r.min_jd_lower_bound))
     mixed["note"] = ("float32 gradient / GGN diagonal / DST-I against the float64 path on the final state; the "
-                     "energies of record are float64 in both forms (energy_terms_rel); the mixed form screens its E "
-                     "differences in float32 and retakes them in float64 near every decision (result.screen)")
+                     "energies of record are float64 in both forms (energy_terms_rel); its trials and E "
+                     "differences are float64 too, so nothing is screened (result.screen)")
     out["mixed_form_errors"] = mixed
     del pair, mp, warped, image_grad, g_dev
     # DST-I apply at full size

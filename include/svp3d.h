@@ -257,7 +257,7 @@ int svp_trial_energy_active(svp_pair *p, const double *base_u, const double *bas
                             void *stream);
 
 /* svp_trial_energy_active with the JD and curl penalties of the trial and of its differences evaluated in float32
- * (the mixed form's float32 energy screen; the reference screens trial energies in float32 in its default execution,
+ * (a screen for hosts that take one; the reference screens trial energies in float32 in its default execution,
  * backends/accelerated.py:66-77).  The node terms (image, proximity), the barrier violations and the activity mask
  * are those of svp_trial_energy_active bit for bit, the localized barrier and its difference equal within rounding
  * (a cell with some float32 closed27 J within 1e-3 of the activation takes the float64 closed27 sweep); terms5[2..3]

@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(256) gemm_right_kernel(const double *__restric
 // better than 2 of 8 warps (1278 against 1350 us for the six float64 passes on 224 x 192 x 160, 367 against 377 us for
 // the six mixed ones on 119 x 165 x 141).  Against 128 x 64 (x: 64 or 128 x 16 ceil(k0 / 16)) tiles per parity with
 // both operands staged through shared memory: six passes 1584 -> 1205 us float64, 672 -> 344 us mixed; the operations
-// of the float64 passes (11.4 G fused multiply-adds) take 614 us at 18.6 T/s, the bytes of the mixed ones 60 us.
+// of the float64 passes (11.4 G fused multiply-adds) take 614 us at 18.6 T/s, the right-hand side, scale and result of
+// the mixed ones 29 us.
 //
 // Float64: mma.sync m16n8k8 f64 (FP64 has no tcgen05 kind on sm_100a; this is B200's FP64 tensor path).  Mixed form:
 // float32 operands as 3xTF32 (mma.sync m16n8k8 .tf32, float32 accumulate): each operand x splits into big = tf32(x)

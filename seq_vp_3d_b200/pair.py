@@ -104,7 +104,7 @@ class DevicePair:
         return d[0], d[1]
 
     def energy_difference_screened(self, base_u, base_w, trial_u, trial_w, base_active=None, stream=None):
-        """energy_difference with the JD/curl penalty differences in float32 (the mixed form's screen): (dE, dF,
+        """energy_difference with the JD/curl penalty differences in float32 (for hosts that screen): (dE, dF,
         band), dE within band of the float64 difference, dF the float64 call's value."""
         d = (ctypes.c_double * 2)()
         band = ctypes.c_double()
@@ -131,7 +131,7 @@ class DevicePair:
         return w, g, np.array(t[:]), int(bad.value), (d[0], d[1]), act
 
     def trial_energy_screened(self, base_u, base_w, trial_u, with_gradient=True, base_active=None, stream=None):
-        """trial_energy with the JD/curl penalties in float32 (the mixed form's energy screen): the same tuple plus
+        """trial_energy with the JD/curl penalties in float32 (for hosts that screen energies): the same tuple plus
         the error estimate of the E difference (the node terms, the barrier and F are the float64 call's bits)."""
         w = self.node()
         g = self.node(3) if with_gradient else None
