@@ -277,7 +277,7 @@ __device__ __forceinline__ void scatter_slice(const R *sl, int T, const C n[3], 
 // ms per launch, FP64 pipe 64% busy; two warps per scheduler (255 registers) leave its dependency stalls.  Three warps
 // (168 registers, 800 bytes of spills) took 5.0 ms, loads of the next field before this field's points 3.36 ms.
 //
-// flags[c]: bit 0, some closed27 J of the state is not above the activation; bit 1, some of the base is not.
+// flags[c]: bit 0, some closed27 J of the state may be below the activation; bit 1, some of the base may be.
 // cell_barrier_kernel evaluates the barrier of those cells; elsewhere it and its change are zero.
 constexpr int kEnergySlots = 45, kDiffSlots = 90;
 template <bool ENERGY, bool DIFF>
@@ -445,7 +445,7 @@ unsigned flagged_blocks(const Q1Const &q) { return blocks_for(q.ncell, BT, 4); }
 // Vertex values of the soft penalties' gradient (mu_scale, nu_scale: 1 or 0), one cell per thread on its closed27 J
 // (q1_closed.cuh): the JD part's derivative by J at the 27 points is the 1D mass matrices applied to J - Jr, and one
 // adjoint pass of J carries it to the edge columns, where the curl part's Hadamard adjoint joins.  flags (when the
-// state has no mask): 1 for the cells with some closed27 J not above the activation, for cell_grad_barrier_kernel.
+// state has no mask): 1 for the cells with some closed27 J that may be below the activation, for cell_grad_barrier_kernel.
 //
 // Bound: FP64 issue (about 2,100 FP64 instructions per cell, the adjoint pass 27 x 24 of them; the Gauss27 form took
 // 4,500 and kept 81 flux sums in shared memory).  160x192x224: 3.06 -> 1.36 ms per launch.  The barrier's slopes stay
@@ -530,8 +530,7 @@ __global__ void __launch_bounds__(BT) cell_grad_barrier_kernel(Q1Const q, const 
         Columns C, G;
         if (mine) {
             load_columns(u, cell_node0(c, q), q, C);
-            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
-                                 const double (&Z)[3]) { sl[p * BT] = jacobian(det_minus_one(X, Y, Z)); });
+            closed_jacobians(C, [&](int p, double J) { sl[p * BT] = J; });
         }
         __syncthreads();
         for_block_points(n, [&](int p, int l) {
@@ -693,7 +692,7 @@ __device__ __forceinline__ void ggn_points(const Columns &C, const Q1Const &q, W
 }
 
 // The JD part at the Gauss points (weights w mu) plus the state-independent curl part q.ggn_curl.  flags (when the
-// state has no mask): 1 for the cells with some closed27 J not above the activation.
+// state has no mask): 1 for the cells with some closed27 J that may be below the activation.
 // Bound: FP64 issue, about 3,300 FP64 instructions per cell (5,600 with a D per vertex): 128x144x128 0.78 -> 0.47
 // ms per launch.
 __global__ void __launch_bounds__(CS) cell_ggn_diag_kernel(Q1Const q, const double *__restrict__ u,
@@ -1248,10 +1247,7 @@ __global__ void __launch_bounds__(BT) cell_ggn_barrier_kernel(Q1Const q, const d
         Columns C;
         if (mine) {
             load_columns(u, cell_node0(c, q), q, C);
-            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
-                                 const double (&Z)[3]) {
-                smem[p * BT + threadIdx.x] = jacobian(det_minus_one(X, Y, Z));
-            });
+            closed_jacobians(C, [&](int p, double J) { smem[p * BT + threadIdx.x] = J; });
         }
         __syncthreads();
         for_block_points(n, [&](int p, int l) {
@@ -1262,7 +1258,6 @@ __global__ void __launch_bounds__(BT) cell_ggn_barrier_kernel(Q1Const q, const d
         });
         __syncthreads();
         if (mine) {
-            add_identity(C);
             double out[8][3];
 #pragma unroll
             for (int a = 0; a < 8; a++)
@@ -1416,7 +1411,7 @@ __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S,
 
 // The barrier of the flagged cells (cell_soft_kernel's flags): the state's barrier sum, violations (J <= delta) and
 // activity mask (trial_act[c] = 1 when some closed27 J is below the activation), and with DIFF its stable change from
-// the base; the J are those of cell_soft_kernel.
+// the base.
 template <bool ENERGY, bool DIFF>
 __global__ void __launch_bounds__(BT) cell_barrier_kernel(Q1Const q, const double *__restrict__ ua,
                                                           const double *__restrict__ ub,
@@ -1434,16 +1429,10 @@ __global__ void __launch_bounds__(BT) cell_barrier_kernel(Q1Const q, const doubl
             const long long n0 = cell_node0(queue[threadIdx.x], q);
             Columns C;
             load_columns(ub, n0, q, C);
-            closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
-                                 const double (&Z)[3]) {
-                sb[p * BT + threadIdx.x] = jacobian(det_minus_one(X, Y, Z));
-            });
+            closed_jacobians(C, [&](int p, double J) { sb[p * BT + threadIdx.x] = J; });
             if (DIFF) {
                 load_columns(ua, n0, q, C);
-                closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
-                                     const double (&Z)[3]) {
-                    sa[p * BT + threadIdx.x] = jacobian(det_minus_one(X, Y, Z));
-                });
+                closed_jacobians(C, [&](int p, double J) { sa[p * BT + threadIdx.x] = J; });
             }
         }
         __syncthreads();
@@ -1649,9 +1638,10 @@ __global__ void __launch_bounds__(CB) cell_trial_barrier_kernel(Q1Const q, const
 // ============================================================================================== node JD measure
 // ext_act > 0 (T69/T73): cells whose closed27 Bernstein coefficients allow a value below min(m_c, ext_act) are
 // appended to cand (order of arrival; each is then estimated independently, so the order does not matter).
-// Bound: FP64 issue, about 600 FP64 instructions per cell (closed27 J 459, 12 edge quadratics); 160x192x224: 1.00 ->
-// 0.49 ms per launch (the edge and Bernstein loops unrolled on registers: 0.86 -> 0.49).
-__global__ void __launch_bounds__(CS) cell_min_jd_kernel(Q1Const q, const double *__restrict__ u,
+// Bound: FP64 issue, about 560 FP64 instructions per cell (closed27 J 243 and their columns 204, 12 edge quadratics);
+// 160x192x224: 1.00 -> 0.49 ms per launch (the edge and Bernstein loops unrolled on registers: 0.86 -> 0.49).  Six
+// blocks per SM: the compiler's 190 registers allow five (metric call on 128x144x128 1050 against 1025 us).
+__global__ void __launch_bounds__(CS, 6) cell_min_jd_kernel(Q1Const q, const double *__restrict__ u,
                                                          double *__restrict__ m, double ext_act,
                                                          unsigned long long *__restrict__ ncand,
                                                          long long *__restrict__ cand) {
@@ -1663,8 +1653,7 @@ __global__ void __launch_bounds__(CS) cell_min_jd_kernel(Q1Const q, const double
         Columns C;
         load_columns(u, cell_node0(c, q), q, C);
         double mn = __longlong_as_double(0x7FF0000000000000LL);
-        closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
-            const double j = jacobian(det_minus_one(X, Y, Z));
+        closed_jacobians(C, [&](int p, double j) {
             J[p * T] = j;
             mn = fmin(mn, j);
         });

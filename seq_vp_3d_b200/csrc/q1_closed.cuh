@@ -8,12 +8,14 @@
 //    powers that (J - Jr)^2 has) equal the integrals of the interpolating quadratics: diagonal sums in the Legendre
 //    basis, or the tensor product of the 1D mass matrix [4 2 -1; 2 16 2; -1 2 4] / 30;
 //  - the curl penalty is a sum of squares of 18 Hadamard coefficients of edge differences.
-// The localized barrier is defined on the closed27 points, so its J are the same values.  Every sum equals the
-// Gauss27 form's in exact arithmetic.  J - 1 is formed from grad u without adding the identity first, so a residual
-// J - Jr rounds relative to |grad u| and not to 1: against 80-bit sums the JD penalty and its changes are 1.5 to 9
-// times closer than the Gauss27 form with F = I + grad u (which 27 independent point errors average), at 2 of 11
-// operations per point.  The operations are explicit round-to-nearest intrinsics: each kernel that evaluates a cell
-// gets the same bits.
+// The localized barrier and the node measure are defined on the closed27 points.  Every sum equals the Gauss27 form's in
+// exact arithmetic.  J is formed in two ways, each where it is the closer one:
+//  - for a residual J - Jr, J - 1 from grad u without adding the identity first: it rounds relative to |grad u| and not
+//    to 1.  Against 80-bit sums the JD penalty and its changes are 1.5 to 9 times closer than the Gauss27 form with F =
+//    I + grad u (which 27 independent point errors average), at 2 of 11 operations per point;
+//  - for J itself, the determinant of F = I + grad u: its products keep a small J's relative accuracy (5e-16 at J = 1e-6,
+//    where 1 + (J - 1) has 6e-11 and the barrier's slope and curvature go like 1/J and 1/J^2), at 9 operations per point.
+// The operations are explicit round-to-nearest intrinsics: each kernel that evaluates a cell gets the same bits.
 #pragma once
 #include "q1_common.cuh"
 
@@ -81,10 +83,33 @@ __device__ __forceinline__ double det_minus_one(const double (&x)[3], const doub
     const double c2 = __fma_rn(-y[1], z[0], __fma_rn(y[0], z[1], -z[0]));
     return __fma_rn(x[2], c2, __fma_rn(x[1], c1, __fma_rn(x[0], k, __dadd_rn(x[0], k))));
 }
-// J of a point from J - 1, and the bound on J - 1 below which J may be below the activation a (J - 1 >= a - 1
-// + one rounding of J implies J >= a)
-__device__ __forceinline__ double jacobian(double jm) { return __dadd_rn(1., jm); }
-__device__ __forceinline__ double near_bound(double a) { return __dadd_rn(__dsub_rn(a, 1.), 4.440892098500626e-16); }
+// The bound on J - 1 below which J may be below the activation a.  The two forms of J differ by some 20 roundings of
+// products of three column entries, less than 2^-30 for entries up to 100.
+__device__ __forceinline__ double near_bound(double a) { return __dadd_rn(__dsub_rn(a, 1.), 0x1p-30); }
+
+// Adds the identity: columns of F from those of grad u.
+__device__ __forceinline__ void add_identity(Columns &C) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        C.X[e][0] = __dadd_rn(C.X[e][0], 1.);
+        C.Y[e][1] = __dadd_rn(C.Y[e][1], 1.);
+        C.Z[e][2] = __dadd_rn(C.Z[e][2], 1.);
+    }
+}
+// J = x . (y x z) for the columns of F at a point
+__device__ __forceinline__ double det_columns(const double (&x)[3], const double (&y)[3], const double (&z)[3]) {
+    const double c0 = __fma_rn(y[1], z[2], -__dmul_rn(y[2], z[1])), c1 = __fma_rn(y[2], z[0], -__dmul_rn(y[0], z[2])),
+                 c2 = __fma_rn(y[0], z[1], -__dmul_rn(y[1], z[0]));
+    return __fma_rn(x[2], c2, __fma_rn(x[1], c1, __dmul_rn(x[0], c0)));
+}
+// Turns the columns of grad u into those of F and visits the closed27 J: body(p, J).
+template <class Body>
+__device__ __forceinline__ void closed_jacobians(Columns &C, Body &&body) {
+    add_identity(C);
+    closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
+        body(p, det_columns(X, Y, Z));
+    });
+}
 
 // ------------------------------------------------------------------------------------------- JD penalty
 // Values at (0, 1/2, 1) -> Legendre coefficients of the interpolating quadratic, per axis and in place: (a, b, c) ->
@@ -238,15 +263,6 @@ __device__ __forceinline__ void column_plane_adjoint(const double (&S)[3][3], in
             E[t][r] += a;
             E[t + 1][r] += b;
         }
-    }
-}
-// Adds the identity: columns of F from those of grad u.
-__device__ __forceinline__ void add_identity(Columns &C) {
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-        C.X[e][0] += 1.;
-        C.Y[e][1] += 1.;
-        C.Z[e][2] += 1.;
     }
 }
 // G = sum_p g(p) dJ_p / d(edge columns) for columns C of F: dJ/dX = Y x Z, dJ/dY = Z x X, dJ/dZ = X x Y at each
