@@ -278,7 +278,8 @@ __device__ __forceinline__ void scatter_slice(const R *sl, int T, const C n[3], 
 // (168 registers, 800 bytes of spills) took 5.0 ms, loads of the next field before this field's points 3.36 ms.
 //
 // flags[c]: bit 0, some closed27 J of the state may be below the activation; bit 1, some of the base may be.
-// cell_barrier_kernel evaluates the barrier of those cells; elsewhere it and its change are zero.
+// cell_barrier_kernel evaluates the barrier of those cells; elsewhere it and its change are zero.  A cell with a
+// column that is not finite is flagged too.
 constexpr int kEnergySlots = 45, kDiffSlots = 90;
 template <bool ENERGY, bool DIFF>
 __global__ void __launch_bounds__(CS) cell_soft_kernel(Q1Const q, const double *__restrict__ ua,
@@ -362,6 +363,20 @@ __global__ void __launch_bounds__(CS) cell_soft_kernel(Q1Const q, const double *
         flags[c] = flag;
         if (trial_act) trial_act[c] = 0;
     }
+    // a J that is not finite need not lie below the bound, but leaves no finite sum: then flag the cells it came from
+    // (checked per cell in the loop above, the trial on 256^3 took 3.11 in place of 3.06 ms)
+    if (!finite64(DIFF ? dif[0].hi : acc[0].hi))
+        for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
+             c += (long long)gridDim.x * blockDim.x) {
+            Columns C;
+            load_columns(ub, cell_node0(c, q), q, C);
+            bool finite = finite_columns(C);
+            if (DIFF && finite) {
+                load_columns(ua, cell_node0(c, q), q, C);
+                finite = finite_columns(C);
+            }
+            if (!finite) flags[c] = 3;
+        }
     if (ENERGY) block_reduce_dd<2>(acc, pe);
     if (ENERGY && DIFF) __syncthreads();     // the two reductions share block_reduce_dd's shared array
     if (DIFF) block_reduce_dd<2>(dif, pd);
@@ -489,8 +504,8 @@ __global__ void __launch_bounds__(CS) cell_grad_kernel(Q1Const q, const double *
                 near |= !(J >= low);
                 r[p] = __dsub_rn(J, sJ[p * T]);
             });
-            if (flags) flags[c] = near ? 1 : 0;
             mass27(r);
+            if (flags) flags[c] = near || !finite64(r[0]) ? 1 : 0;     // r[0] has a share of all 27
 #pragma unroll
             for (int p = 0; p < 27; p++) sJ[p * T] = wj * r[p];
         }
@@ -528,10 +543,8 @@ __global__ void __launch_bounds__(BT) cell_grad_barrier_kernel(Q1Const q, const 
         double *sl = smem + threadIdx.x;
         const long long c = mine ? queue[threadIdx.x] : 0;
         Columns C, G;
-        if (mine) {
-            load_columns(u, cell_node0(c, q), q, C);
-            closed_jacobians(C, [&](int p, double J) { sl[p * BT] = J; });
-        }
+        bool some = false;
+        if (mine) some = closed_jacobians(u, cell_node0(c, q), q, C, sl, BT);
         __syncthreads();
         for_block_points(n, [&](int p, int l) {
             const double J = smem[p * BT + l];
@@ -539,11 +552,18 @@ __global__ void __launch_bounds__(BT) cell_grad_barrier_kernel(Q1Const q, const 
         });
         __syncthreads();
         if (mine) {
+            // a cell that is not finite has a gradient only where some point has a slope
+            if (!some)
+                for (int p = 0; p < 27; p++) some |= sl[p * BT] != 0.;
             load_columns(u, cell_node0(c, q), q, C);     // again: 36 columns do not wait in registers
             add_identity(C);
             closed_adjoint(C, G, [&](int p) { return sl[p * BT]; });
             double Lb[8][3];
             columns_to_vertices(G, q, Lb);
+#pragma unroll
+            for (int a = 0; a < 8; a++)
+#pragma unroll
+                for (int r = 0; r < 3; r++) Lb[a][r] = some ? Lb[a][r] : 0.;
 #pragma unroll
             for (int a = 0; a < 8; a++)
 #pragma unroll
@@ -703,13 +723,11 @@ __global__ void __launch_bounds__(CS) cell_ggn_diag_kernel(Q1Const q, const doub
          c += (long long)gridDim.x * blockDim.x) {
         Columns C;
         load_columns(u, cell_node0(c, q), q, C);
-        if (flags) {
-            bool near = false;
+        bool near = false;
+        if (flags)
             closed_points(C, [&](int, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
                 near |= !(det_minus_one(X, Y, Z) >= low);
             });
-            flags[c] = near ? 1 : 0;
-        }
         add_identity(C);
         double out[8][3];
 #pragma unroll
@@ -719,6 +737,8 @@ __global__ void __launch_bounds__(CS) cell_ggn_diag_kernel(Q1Const q, const doub
         ggn_points<false, false>(C, q, [&](int, int ix, int iy, int iz) {
             return root * (iz == 1 ? centre : side) * ((iy == 1 ? centre : side) * (ix == 1 ? centre : side));
         }, out);
+        // a column that is not finite shows in two components of any vertex
+        if (flags) flags[c] = near || !finite64(out[0][0] + out[0][1]) ? 1 : 0;
         store_locals(L, c, q.ncell, out);
     }
 }
@@ -1245,10 +1265,7 @@ __global__ void __launch_bounds__(BT) cell_ggn_barrier_kernel(Q1Const q, const d
         const bool mine = (int)threadIdx.x < n;
         const long long c = mine ? queue[threadIdx.x] : 0;
         Columns C;
-        if (mine) {
-            load_columns(u, cell_node0(c, q), q, C);
-            closed_jacobians(C, [&](int p, double J) { smem[p * BT + threadIdx.x] = J; });
-        }
+        if (mine) closed_jacobians(u, cell_node0(c, q), q, C, smem + threadIdx.x, BT);
         __syncthreads();
         for_block_points(n, [&](int p, int l) {
             const double J = smem[p * BT + l];
@@ -1413,7 +1430,7 @@ __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S,
 // activity mask (trial_act[c] = 1 when some closed27 J is below the activation), and with DIFF its stable change from
 // the base.
 template <bool ENERGY, bool DIFF>
-__global__ void __launch_bounds__(BT) cell_barrier_kernel(Q1Const q, const double *__restrict__ ua,
+__global__ void __launch_bounds__(BT, 3) cell_barrier_kernel(Q1Const q, const double *__restrict__ ua,
                                                           const double *__restrict__ ub,
                                                           const uint8_t *__restrict__ flags, dd *pe, dd *pd,
                                                           unsigned long long *bad,
@@ -1428,12 +1445,8 @@ __global__ void __launch_bounds__(BT) cell_barrier_kernel(Q1Const q, const doubl
         if ((int)threadIdx.x < n) {
             const long long n0 = cell_node0(queue[threadIdx.x], q);
             Columns C;
-            load_columns(ub, n0, q, C);
-            closed_jacobians(C, [&](int p, double J) { sb[p * BT + threadIdx.x] = J; });
-            if (DIFF) {
-                load_columns(ua, n0, q, C);
-                closed_jacobians(C, [&](int p, double J) { sa[p * BT + threadIdx.x] = J; });
-            }
+            closed_jacobians(ub, n0, q, C, sb + threadIdx.x, BT);
+            if (DIFF) closed_jacobians(ua, n0, q, C, sa + threadIdx.x, BT);
         }
         __syncthreads();
         double sum = 0., change = 0.;
@@ -1651,15 +1664,13 @@ __global__ void __launch_bounds__(CS, 6) cell_min_jd_kernel(Q1Const q, const dou
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
          c += (long long)gridDim.x * blockDim.x) {
         Columns C;
-        load_columns(u, cell_node0(c, q), q, C);
-        double mn = __longlong_as_double(0x7FF0000000000000LL);
-        closed_jacobians(C, [&](int p, double j) {
-            J[p * T] = j;
-            mn = fmin(mn, j);
-        });
-        double j[27];
+        closed_jacobians(u, cell_node0(c, q), q, C, J, T);
+        double j[27], mn = __longlong_as_double(0x7FF0000000000000LL);
 #pragma unroll
-        for (int p = 0; p < 27; p++) j[p] = J[p * T];
+        for (int p = 0; p < 27; p++) {
+            j[p] = J[p * T];
+            mn = fmin(mn, j[p]);
+        }
         // exact interior minima of the edge quadratics through t = 0, 1/2, 1 (solvers/jd_affine.py:24)
 #pragma unroll
         for (int e = 0; e < 12; e++) {

@@ -8,13 +8,14 @@
 //    powers that (J - Jr)^2 has) equal the integrals of the interpolating quadratics: diagonal sums in the Legendre
 //    basis, or the tensor product of the 1D mass matrix [4 2 -1; 2 16 2; -1 2 4] / 30;
 //  - the curl penalty is a sum of squares of 18 Hadamard coefficients of edge differences.
-// The localized barrier and the node measure are defined on the closed27 points.  Every sum equals the Gauss27 form's in
-// exact arithmetic.  J is formed in two ways, each where it is the closer one:
+// The localized barrier and the node measure are defined on the closed27 points.  Every sum equals the Gauss27 form's
+// in exact arithmetic.  J is formed in two ways, each where it is the closer one:
 //  - for a residual J - Jr, J - 1 from grad u without adding the identity first: it rounds relative to |grad u| and not
 //    to 1.  Against 80-bit sums the JD penalty and its changes are 1.5 to 9 times closer than the Gauss27 form with F =
 //    I + grad u (which 27 independent point errors average), at 2 of 11 operations per point;
-//  - for J itself, the determinant of F = I + grad u: its products keep a small J's relative accuracy (5e-16 at J = 1e-6,
-//    where 1 + (J - 1) has 6e-11 and the barrier's slope and curvature go like 1/J and 1/J^2), at 9 operations per point.
+//  - for J itself, the determinant of F = I + grad u: its products keep a small J's relative accuracy (5e-16 at J =
+//    1e-6, where 1 + (J - 1) has 6e-11 and the barrier's slope and curvature go like 1/J and 1/J^2), at 9 operations
+//    per point.
 // The operations are explicit round-to-nearest intrinsics: each kernel that evaluates a cell gets the same bits.
 #pragma once
 #include "q1_common.cuh"
@@ -102,13 +103,37 @@ __device__ __forceinline__ double det_columns(const double (&x)[3], const double
                  c2 = __fma_rn(y[0], z[1], -__dmul_rn(y[1], z[0]));
     return __fma_rn(x[2], c2, __fma_rn(x[1], c1, __dmul_rn(x[0], c0)));
 }
-// Turns the columns of grad u into those of F and visits the closed27 J: body(p, J).
-template <class Body>
-__device__ __forceinline__ void closed_jacobians(Columns &C, Body &&body) {
+// every entry finite (the largest exponent seen, on the integer pipe)
+__device__ __forceinline__ bool finite_columns(const Columns &C) {
+    int top = 0;
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            top = max(max(top, __double2hiint(C.X[e][r]) & 0x7FFFFFFF),
+                      max(__double2hiint(C.Y[e][r]) & 0x7FFFFFFF, __double2hiint(C.Z[e][r]) & 0x7FFFFFFF));
+    return top < 0x7FF00000;
+}
+// Where a column is not finite, the general evaluation: it interpolates all four edges of a column at every point, so
+// that a NaN or an infinity reaches also the points where its edge's weight is zero.
+__device__ __forceinline__ void general_jacobians(const double *__restrict__ u, long long n0, const Q1Const &q,
+                                                  double *sl, int T) {
+    double v[8][3], E[3][4][3];
+    load_cell(u, n0, q, v);
+    cell_edges(v, E);
+    sweep<true>(E, q, [&](int p, int, int, int, const double (&V)[3][3]) { sl[p * T] = det_only(V); });
+}
+// The closed27 J of a cell into sl[p T]; C then holds the columns of F.  False where some column is not finite.
+__device__ __forceinline__ bool closed_jacobians(const double *__restrict__ u, long long n0, const Q1Const &q,
+                                                 Columns &C, double *sl, int T) {
+    load_columns(u, n0, q, C);
+    const bool finite = finite_columns(C);
     add_identity(C);
     closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
-        body(p, det_columns(X, Y, Z));
+        sl[p * T] = det_columns(X, Y, Z);
     });
+    if (!finite) general_jacobians(u, n0, q, sl, T);
+    return finite;
 }
 
 // ------------------------------------------------------------------------------------------- JD penalty
