@@ -97,11 +97,11 @@ __device__ __forceinline__ void add_identity(Columns &C) {
         C.Z[e][2] = __dadd_rn(C.Z[e][2], 1.);
     }
 }
-// J = x . (y x z) for the columns of F at a point
+// J for the columns x, y, z of F at a point, expanded along the first row as det_only
 __device__ __forceinline__ double det_columns(const double (&x)[3], const double (&y)[3], const double (&z)[3]) {
-    const double c0 = __fma_rn(y[1], z[2], -__dmul_rn(y[2], z[1])), c1 = __fma_rn(y[2], z[0], -__dmul_rn(y[0], z[2])),
-                 c2 = __fma_rn(y[0], z[1], -__dmul_rn(y[1], z[0]));
-    return __fma_rn(x[2], c2, __fma_rn(x[1], c1, __dmul_rn(x[0], c0)));
+    const double c0 = __fma_rn(y[1], z[2], -__dmul_rn(y[2], z[1])), c1 = __fma_rn(z[1], x[2], -__dmul_rn(z[2], x[1])),
+                 c2 = __fma_rn(x[1], y[2], -__dmul_rn(x[2], y[1]));
+    return __fma_rn(z[0], c2, __fma_rn(y[0], c1, __dmul_rn(x[0], c0)));
 }
 // every entry finite (the largest exponent seen, on the integer pipe)
 __device__ __forceinline__ bool finite_columns(const Columns &C) {
@@ -114,14 +114,24 @@ __device__ __forceinline__ bool finite_columns(const Columns &C) {
                       max(__double2hiint(C.Y[e][r]) & 0x7FFFFFFF, __double2hiint(C.Z[e][r]) & 0x7FFFFFFF));
     return top < 0x7FF00000;
 }
-// Where a column is not finite, the general evaluation: it interpolates all four edges of a column at every point, so
-// that a NaN or an infinity reaches also the points where its edge's weight is zero.
-__device__ __forceinline__ void general_jacobians(const double *__restrict__ u, long long n0, const Q1Const &q,
-                                                  double *sl, int T) {
-    double v[8][3], E[3][4][3];
-    load_cell(u, n0, q, v);
-    cell_edges(v, E);
-    sweep<true>(E, q, [&](int p, int, int, int, const double (&V)[3][3]) { sl[p * T] = det_only(V); });
+// The general evaluation interpolates all four edges of a column at every point, so that an edge that is not finite
+// reaches also the points where its weight is zero (0 times NaN or an infinity).  closed_points leaves it out there: the
+// J of those points become NaN here.  Rolled loops on the field in memory, so that the finite cells' registers stay
+// (the general evaluation itself in its place left 176 bytes of spills in the trial's barrier kernel).
+__device__ __forceinline__ void spread_nonfinite(const double *__restrict__ u, long long n0, const Q1Const &q,
+                                                 double *sl, int T) {
+#pragma unroll 1
+    for (int i = 0; i < 12; i++) {
+        const int j = i >> 2, lo = i & 1, hi = (i >> 1) & 1;
+        const int a = j == 0 ? 2 * lo + 4 * hi : (j == 1 ? lo + 4 * hi : lo + 2 * hi);
+        const double *v0 = u + 3 * vertex_node(n0, a, q), *v1 = u + 3 * vertex_node(n0, a | (1 << j), q);
+        if (finite64(v1[0] - v0[0]) && finite64(v1[1] - v0[1]) && finite64(v1[2] - v0[2])) continue;
+#pragma unroll 1
+        for (int p = 0; p < 27; p++) {
+            const int s = j == 0 ? (p / 3) % 3 : p % 3, t = j == 2 ? (p / 3) % 3 : p / 9;
+            if (s == 2 - 2 * lo || t == 2 - 2 * hi) sl[p * T] = __longlong_as_double(0x7FF8000000000000LL);
+        }
+    }
 }
 // The closed27 J of a cell into sl[p T]; C then holds the columns of F.  False where some column is not finite.
 __device__ __forceinline__ bool closed_jacobians(const double *__restrict__ u, long long n0, const Q1Const &q,
@@ -132,7 +142,7 @@ __device__ __forceinline__ bool closed_jacobians(const double *__restrict__ u, l
     closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
         sl[p * T] = det_columns(X, Y, Z);
     });
-    if (!finite) general_jacobians(u, n0, q, sl, T);
+    if (!finite) spread_nonfinite(u, n0, q, sl, T);
     return finite;
 }
 
