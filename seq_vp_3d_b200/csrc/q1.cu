@@ -1437,7 +1437,9 @@ __global__ void __launch_bounds__(BT, 3) cell_barrier_kernel(Q1Const q, const do
                                                           uint8_t *__restrict__ trial_act) {
     extern __shared__ double smem[];
     __shared__ long long queue[kBlockQueue];
+    __shared__ dd total[ENERGY ? BT : 1];     // barrier sum of the cells of each place in a group
     double *sb = smem, *sa = smem + 27 * BT;
+    if (ENERGY) total[threadIdx.x] = {0., 0.};
     dd acc[1] = {{0., 0.}}, dif[1] = {{0., 0.}};
     unsigned long long nbad = 0;
     const BarrierRule rule = barrier_rule(q);
@@ -1449,28 +1451,50 @@ __global__ void __launch_bounds__(BT, 3) cell_barrier_kernel(Q1Const q, const do
             if (DIFF) closed_jacobians(ua, n0, q, C, sa + threadIdx.x, BT);
         }
         __syncthreads();
-        double sum = 0., change = 0.;
+        double change = 0.;
         bool active = false;
         int cell = 0;
         for_block_points(n, [&](int p, int l) {
             const double jb = sb[p * BT + l];
-            if (ENERGY) {
-                active |= jb < q.act;
-                cell = l;
-                if (!(jb > q.delta)) nbad++;
-                else if (jb < q.act) sum += barrier_value(jb, rule);
-            }
             if (DIFF) {
                 const double ja = sa[p * BT + l];
                 if (ja < q.act || jb < q.act) change += barrier_change(ja, jb, rule);
             }
+            if (ENERGY) {
+                active |= jb < q.act;
+                cell = l;
+                double b = 0.;
+                if (!(jb > q.delta)) nbad++;
+                else if (jb < q.act) b = barrier_value(jb, rule);
+                sb[p * BT + l] = b;
+            }
         });
-        if (ENERGY) {
-            if (trial_act && active) trial_act[queue[cell]] = 1;
-            acc[0] = dd_add_d(acc[0], sum);
-        }
         if (DIFF) dif[0] = dd_add_d(dif[0], q.bw * change);
+        if (ENERGY) {
+            // The sum does not depend on what else is queued (a trial's queue has the base's cells too): each cell's
+            // points in order, then the cells of one place in their groups of BT in the queue's order, warp after warp
+            // and, where a warp has several of one place, lane after lane (0.50 -> 0.54 ms on 256^3).
+            if (trial_act && active) trial_act[queue[cell]] = 1;
+            __syncthreads();
+            const bool mine = (int)threadIdx.x < n;
+            const int lane = threadIdx.x & 31, place = mine ? (int)queue[threadIdx.x] & (BT - 1) : -1;
+            double s[3] = {0., 0., 0.};
+            if (mine)
+#pragma unroll
+                for (int p = 0; p < 27; p++) s[p / 9] += sb[p * BT + threadIdx.x];
+            const double sum = (s[0] + s[1]) + s[2];
+            const int before = __popc(__match_any_sync(0xFFFFFFFFu, place) & ((1u << lane) - 1u));
+            for (int w = 0; 32 * w < n; w++) {
+                if ((int)threadIdx.x >> 5 == w)
+                    for (int r = 0; __any_sync(0xFFFFFFFFu, mine && before >= r); r++) {
+                        if (mine && before == r) total[place] = dd_add_d(total[place], sum);
+                        __syncwarp();
+                    }
+                __syncthreads();
+            }
+        }
     });
+    if (ENERGY) acc[0] = total[threadIdx.x];
     if (ENERGY) block_reduce_dd<1>(acc, pe);
     if (ENERGY && DIFF) __syncthreads();     // the two reductions share block_reduce_dd's shared array
     if (DIFF) block_reduce_dd<1>(dif, pd);
