@@ -229,7 +229,7 @@ def kernel_counts(shape):
 # kernels timed for the profile and the phase split only: their work depends on the state (the certificate stages
 # run on the cells the edge hull leaves unproven, the node-measure extension on candidate cells)
 STATE_DEPENDENT_KERNELS = ("prescreen_kernel", "fallback_grid_kernel", "classify_kernel", "jd_extension_kernel",
-                           "jd_root_kernel", "cell_ggn_hvp_kernel", "cell_trial_barrier_kernel",
+                           "jd_root_kernel", "cell_ggn_hvp_kernel",
                            "cell_grad_barrier32_kernel", "cell_ggn_barrier32_kernel", "cell_grad_barrier_kernel",
                            "cell_ggn_barrier_kernel", "cell_barrier_kernel")
 

@@ -258,22 +258,22 @@ int svp_trial_energy_active(svp_pair *p, const double *base_u, const double *bas
 
 /* svp_trial_energy_active with the JD and curl penalties of the trial and of its differences evaluated in float32
  * (a screen for hosts that take one; the reference screens trial energies in float32 in its default execution,
- * backends/accelerated.py:66-77).  The node terms (image, proximity), the barrier violations and the activity mask
- * are those of svp_trial_energy_active bit for bit, the localized barrier and its difference equal within rounding
- * (a cell with some float32 closed27 J within 1e-3 of the activation takes the float64 closed27 sweep); terms5[2..3]
- * and the JD/curl parts of
- * diff2[0] carry float32 rounding.  band (host) receives an estimate of that error's magnitude: the residuals'
+ * backends/accelerated.py:66-77).  The node terms (image, proximity), the barrier, its violations and the activity
+ * mask are those of svp_trial_energy_active bit for bit (one kernel evaluates both, here in the cells with some float32
+ * closed27 J within 1e-3 of the activation), the barrier's difference equal within rounding (the order of its sum);
+ * terms5[2..3] and the JD/curl parts of diff2[0] carry float32 rounding.  band (host) receives an estimate of that error's magnitude: the residuals'
  * absolute float32 errors (a Gauss-point J: 256 units of 2^-24, a curl component: 32) times the summed residual
  * magnitudes, plus 64 units of relative rounding of both states' squared-residual sums.  The caller resolves a
  * decision that falls within the band with svp_energy_difference_masked (float64) and checks the band against float64
- * evaluations at run time.  diff2[1] (F = image + barrier) is exact as in the float64 call. */
+ * evaluations at run time.  diff2[1] (F = image + barrier) is float64, equal to the
+ * float64 call's within rounding. */
 int svp_trial_energy_screened(svp_pair *p, const double *base_u, const double *base_warped, const double *trial_u,
                               double *trial_warped, double *trial_image_grad, const uint8_t *base_active,
                               uint8_t *trial_active, double *terms5, double *diff2, double *band,
                               int64_t *barrier_violations, void *stream);
 /* The same screen for two evaluated states (energy_comparison.py:135 stable_energy_reductions, as the outer commit
  * compares its start and candidate): diff2 as svp_energy_difference_masked with the JD and curl penalty differences
- * in float32 and the band of diff2[0]; diff2[1] (F) is exact. */
+ * in float32 and the band of diff2[0]; diff2[1] (F) is float64, equal within rounding. */
 int svp_energy_difference_screened(svp_pair *p, const double *base_u, const double *base_warped,
                                    const double *trial_u, const double *trial_warped, const uint8_t *base_active,
                                    double *diff2, double *band, void *stream);

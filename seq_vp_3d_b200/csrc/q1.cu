@@ -1324,18 +1324,6 @@ __device__ __forceinline__ void acc_add(dd &acc, dd t) {
     acc.lo += s.lo + t.lo;
 }
 
-// energy_comparison.py:14-62 localized branch (double precision), unweighted
-__device__ __forceinline__ double barrier_difference(double ja, double jb, double act, double d) {
-    double a = ja < act ? ja : act, b = jb < act ? jb : act;
-    double scale = act - d;
-    double ra = (act - a) / scale, rb = (act - b) / scale;
-    double h = (b - a) / scale;
-    double loga = ra < .5 ? log1p(-ra) : log((a - d) / scale);
-    double x = (b - a) / (a - d);
-    double ratio = x >= -.5 ? log1p(x) : log((b - d) / (a - d));
-    return h * (ra + rb) * loga - rb * rb * ratio;
-}
-
 __global__ void __launch_bounds__(256) node_diff_kernel(Q1Const q, const double *__restrict__ ua,
                                                         const double *__restrict__ wa,
                                                         const double *__restrict__ ub,
@@ -1505,13 +1493,13 @@ __global__ void __launch_bounds__(BT, 3) cell_barrier_kernel(Q1Const q, const do
 }
 
 // ============================================================================================== screened trial
-// The mixed form's line-search trial: the JD and curl penalties at the Gauss points in float32 (reference J and curl
+// A trial for hosts that screen energies: the JD and curl penalties at the Gauss points in float32 (reference J and curl
 // in a float slice, both fields' float edges), their per-cell sums in float and the block sums in double-double; the
-// localized barrier and its difference as cell_trial_kernel forms them in float64 (a cell with some float32 closed27 J
-// within kBarrierGuard of the activation takes the float64 closed27 sweep; elsewhere every J is above the activation
-// in both arithmetics, where the barrier and its difference vanish).  So the violation count and the activity mask
-// are cell_trial_kernel's, the barrier sums equal within rounding, and only the JD/curl sums carry float32 error,
-// which the host screens against a band (the reference's float32 energy screen, backends/accelerated.py:66-77).
+// localized barrier and its difference in float64 by cell_barrier_kernel over the cells with some float32 closed27 J
+// within kBarrierGuard of the activation (elsewhere every J is above the activation in both arithmetics, where the
+// barrier and its difference vanish).  So the violation count and the activity mask are the float64 trial's and the
+// barrier sum and difference its sums, and only the JD/curl sums carry float32 error, which the host screens against a
+// band (the reference's float32 energy screen, backends/accelerated.py:66-77).
 __device__ __forceinline__ void reference_points32(const double *__restrict__ uref, long long n0, const Q1Const &q,
                                                    float *sl, int T) {
     float Er[3][4][3];
@@ -1526,7 +1514,7 @@ __device__ __forceinline__ void reference_points32(const double *__restrict__ ur
     });
 }
 // The soft part of the screened trial (JD and curl penalty sums and differences) in float32; the barrier part runs in
-// cell_trial_barrier_kernel over the cells this kernel flags.  pe, pd: per block, the two soft sums and their two
+// cell_barrier_kernel over the cells this kernel flags.  pe, pd: per block, the two soft sums and their two
 // differences; pb (the screen's error-bound sums): sum w (|ra| + |rb|) of the JD residuals, the same of the curl
 // residual components, sum w ra^2 and sum w |xa|^2 (the base's soft sums), all from the float32 residuals.
 __global__ void __launch_bounds__(CS) cell_trial32_kernel(Q1Const q, const double *__restrict__ ua,
@@ -1576,12 +1564,13 @@ __global__ void __launch_bounds__(CS) cell_trial32_kernel(Q1Const q, const doubl
             aj += w * ja * ja;
             ac += w * ca2;
         });
-        // the closed27 J in float32: a cell with some trial point within the guard (bit 0), or some base point within
-        // the guard where the base may be active (bit 1), is flagged for the float64 barrier kernel; elsewhere every
-        // J is above the activation in both arithmetics (no barrier, no difference, no violation)
+        // the closed27 J in float32: a cell with some trial point within the guard or not finite (bit 0), or some base
+        // point within the guard where the base may be active (bit 1), is flagged for the float64 barrier kernel;
+        // elsewhere every J is above the activation in both arithmetics (no barrier, no difference, no violation)
         bool near_b = false, near_a = false;
         sweep<true, float>(Eb, q, [&](int, int, int, int, const float (&Vb)[3][3]) {
-            near_b |= det_only(Vb) < guard;
+            const float J = det_only(Vb);
+            near_b |= !(J >= guard && J <= 3.402823466e38f);
         });
         if (near_b || !base_act || base_act[c])
             sweep<true, float>(Ea, q, [&](int, int, int, int, const float (&Va)[3][3]) {
@@ -1605,71 +1594,6 @@ __global__ void __launch_bounds__(CS) cell_trial32_kernel(Q1Const q, const doubl
     block_reduce_dd<2>(dif, pd);
     __syncthreads();
     block_reduce_dd<4>(bnd, pb);
-}
-
-// The barrier part of the screened trial in float64 over the flagged cells, exactly as the float64 trial kernel forms
-// it per cell: the trial's closed27 sweep (barrier, violations, the trial's mask bit; its J kept in the thread's
-// shared slice), then the stable barrier differences against the base where the trial is active or the base may be.
-// pe, pd: per block, the barrier sum and the barrier difference sum.
-__global__ void __launch_bounds__(CB) cell_trial_barrier_kernel(Q1Const q, const double *__restrict__ ua,
-                                                                const double *__restrict__ ub,
-                                                                const uint8_t *__restrict__ flags, dd *pe, dd *pd,
-                                                                unsigned long long *bad,
-                                                                uint8_t *__restrict__ trial_act,
-                                                                const uint8_t *__restrict__ base_act) {
-    extern __shared__ double smem[];
-    __shared__ long long queue[CB / 32][64];
-    double *dsl = smem + threadIdx.x;
-    const int T = blockDim.x;
-    dd acc[1] = {{0., 0.}}, dif[1] = {{0., 0.}};
-    unsigned long long nbad = 0;
-    for_flagged_cells(q, flags, queue[threadIdx.x >> 5], [&](long long c, uint8_t flag) {
-        const long long n0 = cell_node0(c, q);
-        const bool near_b = flag & 1;
-        bool active = false;
-        double sb = 0., sbd = 0.;
-        if (near_b) {
-            double E64[3][4][3];
-            load_edges(ub, n0, q, E64);
-            sweep<true>(E64, q, [&](int p, int, int, int, const double (&Vb)[3][3]) {
-                const double jb = det_only(Vb);
-                dsl[p * T] = jb;
-                active |= jb < q.act;
-                if (!(jb > q.delta)) { nbad++; return; }
-                if (jb < q.act) {
-                    double b, b1, b2;
-                    barrier_eval(jb, q.act, q.delta, q.bw, b, b1, b2);
-                    sb += b;
-                }
-            });
-        }
-        if (active || !base_act || base_act[c]) {
-            if (flag & 2) {
-                double E64[3][4][3];
-                load_edges(ua, n0, q, E64);
-                sweep<true>(E64, q, [&](int p, int, int, int, const double (&Va)[3][3]) {
-                    // a trial J above the guard stands for "above the activation": min(J, a) is then a
-                    const double ja = det_only(Va), jb = near_b ? dsl[p * T] : (double)q.act;
-                    if (ja < q.act || jb < q.act) sbd += barrier_difference(ja, jb, q.act, q.delta);
-                });
-            } else if (active) {
-                // the base is above the activation at every point: each difference is psi(jb) - psi(a)
-                for (int p = 0; p < 27; p++) {
-                    const double jb = dsl[p * T];
-                    if (jb < q.act) sbd += barrier_difference((double)q.act, jb, q.act, q.delta);
-                }
-            }
-        }
-        if (trial_act && active) trial_act[c] = 1;
-        acc[0] = dd_add_d(acc[0], sb);
-        acc_add(dif[0], dd{q.bw * sbd, 0.});
-    });
-    dif[0] = two_sum(dif[0].hi, dif[0].lo);
-    block_reduce_dd<1>(acc, pe);
-    __syncthreads();     // the reductions share block_reduce_dd's shared array
-    block_reduce_dd<1>(dif, pd);
-    for (int o = 16; o; o >>= 1) nbad += __shfl_xor_sync(0xFFFFFFFFu, nbad, o);
-    if ((threadIdx.x & 31) == 0 && nbad) atomicAdd(bad, nbad);
 }
 
 // ============================================================================================== node JD measure
@@ -2384,11 +2308,11 @@ extern "C" int svp_energy_difference_screened(svp_pair *p, const double *base_u,
     SVP_REQUIRE(p && base_u && base_warped && trial_u && trial_warped && diff2 && band,
                 "svp_energy_difference_screened: null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = barrier_blocks(p->q);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
     int rc = allow_slices();
     if (rc) return rc;
     dd *pn = p->partial, *pce = pn + (long long)nb * 2, *pcd = pce + (long long)cb * 2, *pcb = pcd + (long long)cb * 2;
-    dd *pbe = pcb + (long long)cb * 4, *pbd = pbe + bb;
+    dd *pbd = pcb + (long long)cb * 4;
     {
         svp::KernelTimer _t("node_diff_kernel", s);
         SVP_LAUNCH(node_diff_kernel<<<nb, 256, 0, s>>>(p->q, base_u, base_warped, trial_u, trial_warped, p->fixed,
@@ -2400,9 +2324,9 @@ extern "C" int svp_energy_difference_screened(svp_pair *p, const double *base_u,
             p->q, base_u, trial_u, p->u_ref, pce, pcd, pcb, p->flags, nullptr, base_active));
     }
     {
-        svp::KernelTimer _t("cell_trial_barrier_kernel", s);
-        SVP_LAUNCH(cell_trial_barrier_kernel<<<bb, CB, sizeof(double) * 27 * CB, s>>>(
-            p->q, base_u, trial_u, p->flags, pbe, pbd, violations(p), nullptr, base_active));
+        svp::KernelTimer _t("cell_barrier_kernel", s);
+        SVP_LAUNCH(cell_barrier_kernel<false, true><<<bb, BT, sizeof(double) * 54 * BT, s>>>(
+            p->q, base_u, trial_u, p->flags, nullptr, pbd, nullptr, nullptr));
     }
     SVP_LAUNCH_CHECK("screened difference kernels");
     ReduceSpec red;
@@ -2411,7 +2335,6 @@ extern "C" int svp_energy_difference_screened(svp_pair *p, const double *base_u,
     red.add(pbd, bb, 1, 8);
     red.add(pce, cb, 2, 10);
     red.add(pcb, cb, 4, 14);
-    red.bad = violations(p);
     if ((rc = reduce_results(p, red, s))) return rc;
     const double *tmp = p->host;
     // E = image + proximity + jd + curl + barrier; F = image + barrier, as svp_energy_difference combines them
@@ -2432,7 +2355,7 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
     SVP_REQUIRE(p && base_u && base_warped && trial_u && trial_warped && terms5 && diff2,
                 "svp_trial_energy: null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = screened ? barrier_blocks(p->q) : flagged_blocks(p->q);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
     int rc = allow_slices();
     if (rc) return rc;
     dd *pne = p->partial, *pnd = pne + (long long)nb * 2, *pce = pnd + (long long)nb * 2, *pcd = pce + (long long)cb * 3;
@@ -2449,20 +2372,15 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
     }
     SVP_LAUNCH_CHECK("warp_trial_kernel");
     if (screened) {
-        {
-            svp::KernelTimer _t("cell_trial32_kernel", s);
-            SVP_LAUNCH(cell_trial32_kernel<<<cb, CS, sizeof(float) * 108 * CS, s>>>(
-                p->q, base_u, trial_u, p->u_ref, pce, pcd, pcb, p->flags, trial_active, base_active));
-        }
-        svp::KernelTimer _t("cell_trial_barrier_kernel", s);
-        SVP_LAUNCH(cell_trial_barrier_kernel<<<bb, CB, sizeof(double) * 27 * CB, s>>>(
-            p->q, base_u, trial_u, p->flags, pbe, pbd, violations(p), trial_active, base_active));
+        svp::KernelTimer _t("cell_trial32_kernel", s);
+        SVP_LAUNCH(cell_trial32_kernel<<<cb, CS, sizeof(float) * 108 * CS, s>>>(
+            p->q, base_u, trial_u, p->u_ref, pce, pcd, pcb, p->flags, trial_active, base_active));
     } else {
-        {
-            svp::KernelTimer _t("cell_trial_kernel", s);
-            SVP_LAUNCH(cell_soft_kernel<true, true><<<cb, CS, slice_bytes(kDiffSlots), s>>>(
-                p->q, base_u, trial_u, p->u_ref, pce, pcd, p->flags, trial_active));
-        }
+        svp::KernelTimer _t("cell_trial_kernel", s);
+        SVP_LAUNCH(cell_soft_kernel<true, true><<<cb, CS, slice_bytes(kDiffSlots), s>>>(
+            p->q, base_u, trial_u, p->u_ref, pce, pcd, p->flags, trial_active));
+    }
+    {
         svp::KernelTimer _t("cell_barrier_kernel", s);
         SVP_LAUNCH(cell_barrier_kernel<true, true><<<bb, BT, sizeof(double) * 54 * BT, s>>>(
             p->q, base_u, trial_u, p->flags, pbe, pbd, violations(p), trial_active));

@@ -105,7 +105,7 @@ class DevicePair:
 
     def energy_difference_screened(self, base_u, base_w, trial_u, trial_w, base_active=None, stream=None):
         """energy_difference with the JD/curl penalty differences in float32 (for hosts that screen): (dE, dF,
-        band), dE within band of the float64 difference, dF the float64 call's value."""
+        band), dE within band of the float64 difference, dF the float64 call's within rounding."""
         d = (ctypes.c_double * 2)()
         band = ctypes.c_double()
         _lib.call("svp_energy_difference_screened", self._h, ptr(base_u), ptr(base_w), ptr(trial_u), ptr(trial_w),
@@ -132,7 +132,8 @@ class DevicePair:
 
     def trial_energy_screened(self, base_u, base_w, trial_u, with_gradient=True, base_active=None, stream=None):
         """trial_energy with the JD/curl penalties in float32 (for hosts that screen energies): the same tuple plus
-        the error estimate of the E difference (the node terms, the barrier and F are the float64 call's bits)."""
+        the error estimate of the E difference (the node terms and the barrier are the float64 call's bits, the
+        F difference equal within rounding)."""
         w = self.node()
         g = self.node(3) if with_gradient else None
         act = self.cell_mask()
