@@ -1416,20 +1416,20 @@ __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S,
 
 // The barrier of the flagged cells (cell_soft_kernel's flags): the state's barrier sum, violations (J <= delta) and
 // activity mask (trial_act[c] = 1 when some closed27 J is below the activation), and with DIFF its stable change from
-// the base.
+// the base.  pe: per block, the barrier sum and the count of violations (an exact sum of whole numbers, so that nothing
+// is carried from one evaluation to the next); pd: the change.
 template <bool ENERGY, bool DIFF>
 __global__ void __launch_bounds__(BT, 3) cell_barrier_kernel(Q1Const q, const double *__restrict__ ua,
                                                           const double *__restrict__ ub,
                                                           const uint8_t *__restrict__ flags, dd *pe, dd *pd,
-                                                          unsigned long long *bad,
                                                           uint8_t *__restrict__ trial_act) {
     extern __shared__ double smem[];
     __shared__ long long queue[kBlockQueue];
     __shared__ dd total[ENERGY ? BT : 1];     // barrier sum of the cells of each place in a group
     double *sb = smem, *sa = smem + 27 * BT;
     if (ENERGY) total[threadIdx.x] = {0., 0.};
-    dd acc[1] = {{0., 0.}}, dif[1] = {{0., 0.}};
-    unsigned long long nbad = 0;
+    dd dif[1] = {{0., 0.}};
+    unsigned nbad = 0;
     const BarrierRule rule = barrier_rule(q);
     for_flagged_blocks(q, flags, queue, [&](int n) {
         if ((int)threadIdx.x < n) {
@@ -1482,14 +1482,12 @@ __global__ void __launch_bounds__(BT, 3) cell_barrier_kernel(Q1Const q, const do
             }
         }
     });
-    if (ENERGY) acc[0] = total[threadIdx.x];
-    if (ENERGY) block_reduce_dd<1>(acc, pe);
+    if (ENERGY) {
+        dd acc[2] = {total[threadIdx.x], {(double)nbad, 0.}};
+        block_reduce_dd<2>(acc, pe);
+    }
     if (ENERGY && DIFF) __syncthreads();     // the two reductions share block_reduce_dd's shared array
     if (DIFF) block_reduce_dd<1>(dif, pd);
-    if (ENERGY) {
-        for (int o = 16; o; o >>= 1) nbad += __shfl_xor_sync(0xFFFFFFFFu, nbad, o);
-        if ((threadIdx.x & 31) == 0 && nbad) atomicAdd(bad, nbad);
-    }
 }
 
 // ============================================================================================== screened trial
@@ -2058,22 +2056,19 @@ __global__ void __launch_bounds__(256) pg_scale_kernel(Q1Const q, const double *
 
 // ============================================================================================== final reduction
 // All block sums of one evaluation in one launch, one block per sum: thread t adds blocks t, t + 256, ... in order, then
-// a fixed tree.  The results go straight to the pair's pinned host buffer, with the violation count (which is zeroed
-// for the next evaluation), so the evaluation ends with a wait and no copy.  A trial took six of these launches, a
+// a fixed tree.  The results go straight to the pair's pinned host buffer, so the evaluation ends with a wait and no copy.  A trial took six of these launches, a
 // memset and two copies to pageable memory: on 48^3 about 60 of its 161 us.
 struct ReduceSpec {
     static constexpr int kMost = 8;
     const dd *src[kMost];
     long long blocks[kMost];
     int K[kMost], out[kMost], n = 0, sums = 0;
-    unsigned long long *bad = nullptr;
     void add(const dd *partial, long long count, int k, int at) {
         src[n] = partial; blocks[n] = count; K[n] = k; out[n] = at;
         n++;
         sums += k;
     }
 };
-constexpr int kBadSlot = 62;      // of the 64 result slots: the violation count's bits
 __global__ void __launch_bounds__(256) reduce_results_kernel(const __grid_constant__ ReduceSpec r, double *out) {
     int i = 0, k = blockIdx.x;
     while (k >= r.K[i]) k -= r.K[i++];
@@ -2083,10 +2078,6 @@ __global__ void __launch_bounds__(256) reduce_results_kernel(const __grid_consta
     if (threadIdx.x == 0) {
         out[r.out[i] + 2 * k] = sum.hi;
         out[r.out[i] + 2 * k + 1] = sum.lo;
-        if (blockIdx.x == 0 && r.bad) {
-            out[kBadSlot] = __longlong_as_double((long long)*r.bad);
-            *r.bad = 0;
-        }
     }
 }
 
@@ -2132,25 +2123,17 @@ int allow_slices() {
 }
 unsigned node_blocks(long long n) { return blocks_for(n, 256, 8); }
 
-// The evaluations' violation counter: its own word, zero between evaluations.
-unsigned long long *violations(svp_pair *p) { return (unsigned long long *)(p->counter + 6); }
 int reduce_results(svp_pair *p, const ReduceSpec &r, cudaStream_t s) {
     SVP_LAUNCH(reduce_results_kernel<<<(unsigned)r.sums, 256, 0, s>>>(r, p->host));
     SVP_CUDA(cudaStreamSynchronize(s));
     return SVP_OK;
-}
-long long violation_count(const svp_pair *p) {
-    long long n;
-    memcpy(&n, &p->host[kBadSlot], sizeof n);
-    return n;
 }
 
 }  // namespace
 
 long long pair_partial_count(const Q1Const &q) {
     const long long nb = node_blocks(q.nnode), cb = slice_blocks(q);
-    const long long bb = barrier_blocks(q) > flagged_blocks(q) ? barrier_blocks(q) : flagged_blocks(q);
-    return nb * 4 + cb * 10 + bb * 2;       // the screened trial's sums
+    return nb * 4 + cb * 10 + flagged_blocks(q) * 3LL;       // the screened trial's sums
 }
 
 int pair_locals(svp_pair *p, int n) {
@@ -2213,18 +2196,16 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
     {
         svp::KernelTimer _t("cell_barrier_kernel", s);
         SVP_LAUNCH(cell_barrier_kernel<true, false><<<bb, BT, sizeof(double) * 27 * BT, s>>>(
-            p->q, nullptr, u, p->flags, pb, nullptr, violations(p), nullptr));
+            p->q, nullptr, u, p->flags, pb, nullptr, nullptr));
     }
     SVP_LAUNCH_CHECK("cell_energy_kernel");
     double node2[2], cell3[3];
     ReduceSpec red;
     red.add(p->partial, nb, 2, 0);
     red.add(pc, cb, 2, 4);
-    red.add(pb, bb, 1, 8);
-    red.bad = violations(p);
+    red.add(pb, bb, 2, 8);
     if ((rc = reduce_results(p, red, s))) return rc;
     const double *tmp = p->host;
-    const long long bad = violation_count(p);
     for (int k = 0; k < 2; k++) node2[k] = tmp[2 * k] + tmp[2 * k + 1];
     for (int k = 0; k < 3; k++) cell3[k] = tmp[4 + 2 * k] + tmp[4 + 2 * k + 1];
     terms5[0] = .5 * node2[0];
@@ -2232,7 +2213,7 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
     terms5[2] = .5 * p->q.mu * cell3[0];
     terms5[3] = .5 * p->q.nu * cell3[1];
     terms5[4] = cell3[2];
-    if (barrier_violations) *barrier_violations = bad;
+    if (barrier_violations) *barrier_violations = (int64_t)(tmp[10] + tmp[11]);
     return SVP_OK;
 }
 
@@ -2259,7 +2240,7 @@ extern "C" int svp_energy_difference_masked(svp_pair *p, const double *base_u, c
     {
         svp::KernelTimer _t("cell_barrier_kernel", s);
         SVP_LAUNCH(cell_barrier_kernel<false, true><<<bb, BT, sizeof(double) * 54 * BT, s>>>(
-            p->q, base_u, trial_u, p->flags, nullptr, pb, nullptr, nullptr));
+            p->q, base_u, trial_u, p->flags, nullptr, pb, nullptr));
     }
     SVP_LAUNCH_CHECK("difference kernels");
     ReduceSpec red;
@@ -2326,7 +2307,7 @@ extern "C" int svp_energy_difference_screened(svp_pair *p, const double *base_u,
     {
         svp::KernelTimer _t("cell_barrier_kernel", s);
         SVP_LAUNCH(cell_barrier_kernel<false, true><<<bb, BT, sizeof(double) * 54 * BT, s>>>(
-            p->q, base_u, trial_u, p->flags, nullptr, pbd, nullptr, nullptr));
+            p->q, base_u, trial_u, p->flags, nullptr, pbd, nullptr));
     }
     SVP_LAUNCH_CHECK("screened difference kernels");
     ReduceSpec red;
@@ -2359,7 +2340,7 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
     int rc = allow_slices();
     if (rc) return rc;
     dd *pne = p->partial, *pnd = pne + (long long)nb * 2, *pce = pnd + (long long)nb * 2, *pcd = pce + (long long)cb * 3;
-    dd *pcb = pcd + (long long)cb * 3, *pbe = pcb + (long long)cb * 4, *pbd = pbe + bb;
+    dd *pcb = pcd + (long long)cb * 3, *pbe = pcb + (long long)cb * 4, *pbd = pbe + (long long)bb * 2;
     SplineRef S = spline_ref(p);
     if (trial_image_grad) {
         svp::KernelTimer _t("warp_trial_kernel_grad", s);
@@ -2383,22 +2364,20 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
     {
         svp::KernelTimer _t("cell_barrier_kernel", s);
         SVP_LAUNCH(cell_barrier_kernel<true, true><<<bb, BT, sizeof(double) * 54 * BT, s>>>(
-            p->q, base_u, trial_u, p->flags, pbe, pbd, violations(p), trial_active));
+            p->q, base_u, trial_u, p->flags, pbe, pbd, trial_active));
     }
     SVP_LAUNCH_CHECK("cell_trial_kernel");
     // soft sums and differences from the soft kernel, the barrier's from the barrier kernel
     ReduceSpec red;
     red.add(pne, nb, 2, 0);
     red.add(pce, cb, 2, 4);
-    red.add(pbe, bb, 1, 8);
-    red.add(pnd, nb, 2, 10);
-    red.add(pcd, cb, 2, 14);
-    red.add(pbd, bb, 1, 18);
-    if (screened) red.add(pcb, cb, 4, 20);
-    red.bad = violations(p);
+    red.add(pbe, bb, 2, 8);
+    red.add(pnd, nb, 2, 12);
+    red.add(pcd, cb, 2, 16);
+    red.add(pbd, bb, 1, 20);
+    if (screened) red.add(pcb, cb, 4, 22);
     if ((rc = reduce_results(p, red, s))) return rc;
     const double *tmp = p->host;
-    const long long bad = violation_count(p);
     // energy terms exactly as svp_energy
     double node2[2], cell3[3];
     for (int k = 0; k < 2; k++) node2[k] = tmp[2 * k] + tmp[2 * k + 1];
@@ -2408,17 +2387,17 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
     terms5[2] = .5 * p->q.mu * cell3[0];
     terms5[3] = .5 * p->q.nu * cell3[1];
     terms5[4] = cell3[2];
-    if (barrier_violations) *barrier_violations = bad;
+    if (barrier_violations) *barrier_violations = (int64_t)(tmp[10] + tmp[11]);
     // differences exactly as svp_energy_difference
-    double img = tmp[10] + tmp[11], prox = tmp[12] + tmp[13];
-    double jd = tmp[14] + tmp[15], curl = tmp[16] + tmp[17], bar = tmp[18] + tmp[19];
+    double img = tmp[12] + tmp[13], prox = tmp[14] + tmp[15];
+    double jd = tmp[16] + tmp[17], curl = tmp[18] + tmp[19], bar = tmp[20] + tmp[21];
     diff2[0] = (((img + prox) + jd) + curl) + bar;
     diff2[1] = img + bar;
     if (band) {
         *band = 0.;
         if (screened) {
-            const double sums[6] = {cell3[0], cell3[1], tmp[20] + tmp[21], tmp[22] + tmp[23], tmp[24] + tmp[25],
-                                    tmp[26] + tmp[27]};
+            const double sums[6] = {cell3[0], cell3[1], tmp[22] + tmp[23], tmp[24] + tmp[25], tmp[26] + tmp[27],
+                                    tmp[28] + tmp[29]};
             *band = screen_band(p, sums);
         }
     }
