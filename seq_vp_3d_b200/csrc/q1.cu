@@ -455,6 +455,9 @@ __device__ __forceinline__ void for_block_points(int n, F &&f) {
     for (int p = threadIdx.x >> shift; p < 27; p += BT >> shift) f(p, l);
 }
 unsigned flagged_blocks(const Q1Const &q) { return blocks_for(q.ncell, BT, 4); }
+// cell_barrier_kernel's 168 registers let three blocks stand on an SM; a fourth ran alone in a second wave (0.54 -> 0.37
+// ms on 256^3, 17 -> 13 us on 48^3).  One grid for its three forms: a sum's order depends on it.
+unsigned cell_barrier_blocks(const Q1Const &q) { return blocks_for(q.ncell, BT, 3); }
 
 // ============================================================================================== cell gradients
 // Vertex values of the soft penalties' gradient (mu_scale, nu_scale: 1 or 0), one cell per thread on its closed27 J
@@ -2133,7 +2136,7 @@ int reduce_results(svp_pair *p, const ReduceSpec &r, cudaStream_t s) {
 
 long long pair_partial_count(const Q1Const &q) {
     const long long nb = node_blocks(q.nnode), cb = slice_blocks(q);
-    return nb * 4 + cb * 10 + flagged_blocks(q) * 3LL;       // the screened trial's sums
+    return nb * 4 + cb * 10 + cell_barrier_blocks(q) * 3LL;       // the screened trial's sums
 }
 
 int pair_locals(svp_pair *p, int n) {
@@ -2182,7 +2185,7 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
                           int64_t *barrier_violations, void *stream) {
     SVP_REQUIRE(p && u && warped && terms5, "svp_energy: null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = cell_barrier_blocks(p->q);
     int rc = allow_slices();
     if (rc) return rc;
     { svp::KernelTimer _t("node_energy_kernel", s); SVP_LAUNCH(node_energy_kernel<<<nb, 256, 0, s>>>(p->q, u, warped, p->fixed, p->u_ref, p->partial)); }
@@ -2226,7 +2229,7 @@ extern "C" int svp_energy_difference_masked(svp_pair *p, const double *base_u, c
     // the cell kernels find the cells near the activation from the J they evaluate, so the masks save nothing here
     (void)base_active;
     (void)trial_active;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = cell_barrier_blocks(p->q);
     int rc = allow_slices();
     if (rc) return rc;
     { svp::KernelTimer _t("node_diff_kernel", s); SVP_LAUNCH(node_diff_kernel<<<nb, 256, 0, s>>>(p->q, base_u, base_warped, trial_u, trial_warped, p->fixed, p->u_ref,
@@ -2289,7 +2292,7 @@ extern "C" int svp_energy_difference_screened(svp_pair *p, const double *base_u,
     SVP_REQUIRE(p && base_u && base_warped && trial_u && trial_warped && diff2 && band,
                 "svp_energy_difference_screened: null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = cell_barrier_blocks(p->q);
     int rc = allow_slices();
     if (rc) return rc;
     dd *pn = p->partial, *pce = pn + (long long)nb * 2, *pcd = pce + (long long)cb * 2, *pcb = pcd + (long long)cb * 2;
@@ -2336,7 +2339,7 @@ static int trial_energy(svp_pair *p, const double *base_u, const double *base_wa
     SVP_REQUIRE(p && base_u && base_warped && trial_u && trial_warped && terms5 && diff2,
                 "svp_trial_energy: null argument");
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = flagged_blocks(p->q);
+    unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = cell_barrier_blocks(p->q);
     int rc = allow_slices();
     if (rc) return rc;
     dd *pne = p->partial, *pnd = pne + (long long)nb * 2, *pce = pnd + (long long)nb * 2, *pcd = pce + (long long)cb * 3;
