@@ -480,7 +480,6 @@ __global__ void __launch_bounds__(CS) cell_grad_kernel(Q1Const q, const double *
     // the mass matrices' 30 per axis and the quadrature's volume
     const double wj = q.mu * mu_scale * q.omega * (1. / 27000.), wc = q.nu * nu_scale * q.omega;
     const double low = near_bound(q.act);
-    const bool soft = mu_scale != 0. || nu_scale != 0.;     // neither: zeros, also where the field is not finite
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
          c += (long long)gridDim.x * blockDim.x) {
         const long long n0 = cell_node0(c, q);
@@ -522,13 +521,23 @@ __global__ void __launch_bounds__(CS) cell_grad_kernel(Q1Const q, const double *
         }
         double L[8][3];
         columns_to_vertices(G, q, L);
-        if (!soft) {
-#pragma unroll
-            for (int a = 0; a < 8; a++)
-#pragma unroll
-                for (int r = 0; r < 3; r++) L[a][r] = 0.;
-        }
         store_locals(L1, c, q.ncell, L);
+    }
+}
+
+// The flags alone, for a gradient without soft penalties.
+__global__ void __launch_bounds__(CS) cell_flag_kernel(Q1Const q, const double *__restrict__ u,
+                                                       uint8_t *__restrict__ flags) {
+    const double low = near_bound(q.act);
+    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
+         c += (long long)gridDim.x * blockDim.x) {
+        Columns C;
+        load_columns(u, cell_node0(c, q), q, C);
+        bool near = !finite_columns(C);
+        closed_points(C, [&](int, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
+            near |= !(det_minus_one(X, Y, Z) >= low);
+        });
+        flags[c] = near ? 1 : 0;
     }
 }
 
@@ -2454,14 +2463,18 @@ static int run_gather(svp_pair *p, const GatherSpec &g, const LT *L1, const LT *
 }
 
 // The plain form's gradient locals: the soft kernel, then the barrier kernel over the flagged cells (the state's mask,
-// or without one the cells the soft kernel flags).  *has2: the cells whose L2 values were written.
+// or without one the cells the soft kernel flags).  Without a soft penalty its values are zeros, also where the field is
+// not finite, and no cell is evaluated for them.  *has2: the cells whose L2 values were written.
 static int grad64(svp_pair *p, const double *u, double mu_scale, double nu_scale, bool barrier, bool split,
                   const uint8_t *active, const uint8_t **has2, cudaStream_t s) {
     int rc = allow_slices();
     if (rc) return rc;
     uint8_t *flags = barrier && !active ? p->flags : nullptr;
     const uint8_t *marked = active ? active : flags;
-    {
+    if (p->q.mu * mu_scale == 0. && p->q.nu * nu_scale == 0.) {
+        SVP_CUDA(cudaMemsetAsync(p->loc1, 0, sizeof(double) * 24 * (size_t)p->q.ncell, s));
+        if (flags) SVP_LAUNCH(cell_flag_kernel<<<slice_blocks(p), CS, 0, s>>>(p->q, u, flags));
+    } else {
         svp::KernelTimer _t("cell_grad_kernel", s);
         SVP_LAUNCH(cell_grad_kernel<<<slice_blocks(p), CS, slice_bytes(45), s>>>(p->q, u, p->u_ref, mu_scale,
                                                                                 nu_scale, p->loc1, flags));

@@ -91,6 +91,20 @@ def test_node_measure(problem):
             assert np.all(np.abs(got[known] - node[known]) <= TOL * node[known])
 
 
+def test_zero_weights(problem):
+    """With neither soft penalty the soft gradient is zero, also where the field is not finite."""
+    from seq_vp_3d_b200.pair import DevicePair
+    P, OP, u, w, g = problem
+    free = DevicePair(P.grid, np.zeros(SHAPE), np.zeros(SHAPE), np.zeros(SHAPE + (3,)), lam=1e-4, mu=0., nu=0.,
+                      kappa=.002)
+    broken = u.copy()
+    broken[NODE + (0,)] = np.nan
+    node = np.ravel_multi_index([i - 1 for i in NODE], [n - 2 for n in SHAPE])      # the broken node's own u enters
+    for term in ("jd", "curl"):
+        got = free.gradient(dev(broken), w, g, term).cpu().numpy().reshape(3, -1)
+        assert not np.delete(got, node, axis=1).any()
+
+
 def test_folded_cells(problem):
     """Cells of negative J: each point with J <= delta is counted, the others form the barrier sum."""
     P, OP, u, w, g = problem
