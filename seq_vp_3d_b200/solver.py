@@ -76,6 +76,7 @@ class State:
     norms: tuple = None                # (GF, GD, GE) when computed with the final gradient
     differences: tuple = None          # ((base eval_id, reference version), (dE, dF)) from the one-pass trial
     active: object = None              # per-cell barrier activity mask (from the state's own trial evaluation)
+    band: float = 0.                   # error estimate of dE in `differences`; 0: float64, as every trial's are
 
     @property
     def total(self):
@@ -216,9 +217,10 @@ class Registration:
             state.norms = (self.gnorm(gF), self.gnorm(gD), self.gnorm(gE))
         return state.norms
 
-    def stable_reductions(self, base, trial):
+    def stable_reductions(self, base, trial, required=None):
         """(E, F) EnergyReduction pairs (actual, resolution) (energy_comparison.py:135): the trial's own differences
-        from its evaluation against this base, or a comparison of the two states."""
+        from its evaluation against this base, or a comparison of the two states.  Both are float64 whatever reduction
+        the decision requires, so `required` (for a caller that passes it) has no effect."""
         cached = trial.differences
         if cached is not None and cached[0] == (base.eval_id, self._reference_version):
             dE, dF = cached[1]
