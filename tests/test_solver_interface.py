@@ -7,7 +7,7 @@ from seq_vp_3d_b200.solver import EPS, Registration, State
 
 
 def evaluated(eval_id, differences=None):
-    return State(theta=None, u=None, warped=None, terms=[1., .5, .25, .125, .0625], certificate=None, eval_id=eval_id,
+    return State(theta=None, u=None, warped=None, energy=[1., .5, .25, .125, .0625], certificate=None, eval_id=eval_id,
                  differences=differences)
 
 
