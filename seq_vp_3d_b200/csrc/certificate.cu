@@ -1846,45 +1846,12 @@ extern "C" int svp_certify_map(svp_certifier *c, const double *u, svp_cert_resul
     out->witness_point[0] = out->witness_point[1] = out->witness_point[2] = nan;
 
     Accum acc;
-    long long n2 = 0;
+    long long n1 = 0, n2 = 0;
     const long long *list2 = nullptr;
     int rc = SVP_OK;
-    bool staged = !hull;
-    if (hull) {
-        SVP_LAUNCH(accum_init_kernel<<<1, 1, 0, s>>>(c->acc));
-        {
-            svp::KernelTimer _t("edge_hull_kernel", s);
-            const unsigned nb = blocks_for(n, 256, 8);
-            if (directed)
-                SVP_LAUNCH(hull_list_kernel<true><<<nb, 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0, c->grid.z0, delta,
-                                                                   c->list1, c->acc));
-            else
-                SVP_LAUNCH(hull_list_kernel<false><<<nb, 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0, c->grid.z0,
-                                                                    delta, c->list1, c->acc));
-        }
-        if (c->cfg.prescreen) {
-            svp::KernelTimer _t("prescreen_kernel", s);
-            if ((rc = launch_prescreen_list(u, c->cg, c->list1, c->pk, delta, c->list2, c->acc, s))) return rc;
-        }
-        if ((rc = read_accum(c, &acc, s))) return rc;
-    } else {
-        SVP_LAUNCH(accum_init_kernel<<<1, 1, 0, s>>>(c->acc));
-        SVP_LAUNCH(precheck_kernel<<<blocks_for(n_nodes(&c->grid), 256, 8), 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0,
-                                                                                      c->grid.z0, c->acc));
-        if ((rc = read_accum(c, &acc, s))) return rc;
-    }
-    // early returns, in certify_map's order (feasibility.py:412-428)
-    if (acc.nonfinite) { out->reason = R_NONFINITE; return SVP_OK; }
-    if (acc.boundary) { out->status = ST_INFEASIBLE; out->reason = R_BOUNDARY; return SVP_OK; }
-    if (acc.invalid) { out->status = ST_INFEASIBLE; out->reason = R_DOMAIN; return SVP_OK; }
-    if (hull && !acc.flagged) {
-        n2 = (long long)(c->cfg.prescreen ? acc.list2 : acc.list1);
-        list2 = c->cfg.prescreen ? c->list2 : c->list1;
-    } else {
-        // The staged form: without the preproof (feasibility.py:447-491) every cell goes to the fallback; with it and
-        // an enclosure that was not finite, every cell of that enclosure's tile does (feasibility.py:650).
-        staged = true;
-        SVP_LAUNCH(accum_init_kernel<<<1, 1, 0, s>>>(c->acc));
+    // The staged form's first stage: without the preproof (feasibility.py:447-491) every cell goes to the fallback; with
+    // it and an enclosure that was not finite, every cell of that enclosure's tile does (feasibility.py:650).
+    auto first_stage = [&]() -> int {
         if ((rc = ensure_staged(c))) return rc;
         SVP_CUDA(cudaMemsetAsync(c->tile_bad, hull ? 0 : 1, sizeof(int) * c->ntiles, s));
         if (hull) {
@@ -1899,9 +1866,46 @@ extern "C" int svp_certify_map(svp_certifier *c, const double *u, svp_cert_resul
         SVP_LAUNCH(hull_stage_kernel<<<blocks_for(n, 256, 8), 256, 0, s>>>(c->margin, c->tile_bad, n, tile, c->sel,
                                                                          c->acc));
         if ((rc = select_flagged<false>(c, nullptr, c->sel, c->list1, c->counts, n, s))) return rc;
-        long long n1 = 0;
         SVP_CUDA(cudaMemcpyAsync(&n1, c->counts, sizeof n1, cudaMemcpyDeviceToHost, s));
-        SVP_CUDA(cudaStreamSynchronize(s));
+        return SVP_OK;
+    };
+    bool staged = !hull;
+    SVP_LAUNCH(accum_init_kernel<<<1, 1, 0, s>>>(c->acc));
+    if (hull) {
+        {
+            svp::KernelTimer _t("edge_hull_kernel", s);
+            const unsigned nb = blocks_for(n, 256, 8);
+            if (directed)
+                SVP_LAUNCH(hull_list_kernel<true><<<nb, 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0, c->grid.z0, delta,
+                                                                   c->list1, c->acc));
+            else
+                SVP_LAUNCH(hull_list_kernel<false><<<nb, 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0, c->grid.z0,
+                                                                    delta, c->list1, c->acc));
+        }
+        if (c->cfg.prescreen) {
+            svp::KernelTimer _t("prescreen_kernel", s);
+            if ((rc = launch_prescreen_list(u, c->cg, c->list1, c->pk, delta, c->list2, c->acc, s))) return rc;
+        }
+    } else {
+        SVP_LAUNCH(precheck_kernel<<<blocks_for(n_nodes(&c->grid), 256, 8), 256, 0, s>>>(u, c->cg, c->grid.x0, c->grid.y0,
+                                                                                      c->grid.z0, c->acc));
+        if ((rc = first_stage())) return rc;
+    }
+    if ((rc = read_accum(c, &acc, s))) return rc;
+    // early returns, in certify_map's order (feasibility.py:412-428)
+    if (acc.nonfinite) { out->reason = R_NONFINITE; return SVP_OK; }
+    if (acc.boundary) { out->status = ST_INFEASIBLE; out->reason = R_BOUNDARY; return SVP_OK; }
+    if (acc.invalid) { out->status = ST_INFEASIBLE; out->reason = R_DOMAIN; return SVP_OK; }
+    if (hull && !acc.flagged) {
+        n2 = (long long)(c->cfg.prescreen ? acc.list2 : acc.list1);
+        list2 = c->cfg.prescreen ? c->list2 : c->list1;
+    } else {
+        if (hull) {
+            staged = true;
+            SVP_LAUNCH(accum_init_kernel<<<1, 1, 0, s>>>(c->acc));
+            if ((rc = first_stage())) return rc;
+            SVP_CUDA(cudaStreamSynchronize(s));
+        }
         n2 = n1;
         list2 = c->list1;
         if (c->cfg.prescreen && n1) {
