@@ -13,13 +13,18 @@ def require_cuda():
         raise RuntimeError("seq_vp_3d_b200 needs a CUDA device (sm_100a); there is no CPU fallback")
 
 
+# torch's raw query of the current stream, which its public interface does not have: 0.3 us where
+# torch.cuda.current_stream() builds a Stream object in 5 us, and a registration step asks about 13 times.  A torch
+# without it is asked through the public call.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def stream_ptr(stream=None):
-    """cudaStream_t of a torch stream (default: the calling thread's current stream on its current device).  The raw
-    query costs 0.3 us where torch.cuda.current_stream() builds a Stream object in 5 us, and a registration step asks
-    about 13 times."""
-    if stream is None:
-        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
-    return ctypes.c_void_p(stream.cuda_stream)
+    """cudaStream_t of a torch stream (default: the calling thread's current stream on its current device)."""
+    if stream is None and _raw_stream is not None and _device is not None:
+        return ctypes.c_void_p(_raw_stream(_device()))
+    return ctypes.c_void_p((torch.cuda.current_stream() if stream is None else stream).cuda_stream)
 
 
 def ptr(t):
