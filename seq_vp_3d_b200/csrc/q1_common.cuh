@@ -379,32 +379,32 @@ __device__ __forceinline__ void barrier_eval(double J, double a, double delta, d
     b2 = w * (-2 * logt + 4 * r / t + rt * rt) / (scale * scale);
 }
 
-// The same barrier's value, slope and stable change (energy_comparison.py:14-62) for the float64 kernels that walk
-// many points: the divisions by the constant scale a - delta are multiplications by its reciprocal (one rounding), so
-// a value has one logarithm, a slope one logarithm and one division, a change two and one.
+// The same barrier's value, slope and stable change (energy_comparison.py:14-62) for the float64 kernels that walk many
+// points, each with what it needs alone.  The scale a - delta divides: its reciprocal is a constant of the pair, so its
+// rounding would be a bias that the sum over the points keeps (2 units of 2^-53 of the sum at a = .5, delta = .001).
 struct BarrierRule {
-    double a, delta, w, inv;      // activation, delta, weight, 1 / (a - delta)
+    double a, delta, w, scale;    // activation, delta, weight, a - delta
 };
 __device__ __forceinline__ BarrierRule barrier_rule(const Q1Const &q) {
-    return {q.act, q.delta, q.bw, 1. / (q.act - q.delta)};
+    return {q.act, q.delta, q.bw, q.act - q.delta};
 }
 // log t, t = (J - delta) / (a - delta) = 1 - r
 __device__ __forceinline__ double barrier_log(double r, double t) { return r < .5 ? log1p(-r) : log(t); }
 __device__ __forceinline__ double barrier_value(double J, const BarrierRule &k) {
-    const double r = (k.a - J) * k.inv, t = (J - k.delta) * k.inv;
+    const double r = (k.a - J) / k.scale, t = (J - k.delta) / k.scale;
     return -k.w * r * r * barrier_log(r, t);
 }
 __device__ __forceinline__ double barrier_slope(double J, const BarrierRule &k) {
-    const double r = (k.a - J) * k.inv, t = (J - k.delta) * k.inv;
-    return k.w * (2. * r * barrier_log(r, t) - r * r / t) * k.inv;
+    const double r = (k.a - J) / k.scale, t = (J - k.delta) / k.scale;
+    return k.w * (2. * r * barrier_log(r, t) - r * r / t) / k.scale;
 }
 // psi(jb) - psi(ja), unweighted
 __device__ __forceinline__ double barrier_change(double ja, double jb, const BarrierRule &k) {
     const double a = ja < k.a ? ja : k.a, b = jb < k.a ? jb : k.a;
-    const double ra = (k.a - a) * k.inv, rb = (k.a - b) * k.inv, h = (b - a) * k.inv;
+    const double ra = (k.a - a) / k.scale, rb = (k.a - b) / k.scale, h = (b - a) / k.scale;
     const double x = (b - a) / (a - k.delta);
     const double ratio = x >= -.5 ? log1p(x) : log((b - k.delta) / (a - k.delta));
-    return h * (ra + rb) * barrier_log(ra, (a - k.delta) * k.inv) - rb * rb * ratio;
+    return h * (ra + rb) * barrier_log(ra, (a - k.delta) / k.scale) - rb * rb * ratio;
 }
 
 }  // namespace svp

@@ -86,3 +86,28 @@ def test_node_measure(problem):
     stats = {}
     got = P.node_min_jd(bd, .25, stats).cpu().numpy()
     assert np.all(got > 0) and np.all(got <= P.node_min_jd(bd).cpu().numpy())
+
+
+@pytest.mark.parametrize("activation,delta", [(.05, 0.), (.5, .001), (.2, .03)])
+def test_barrier_value_has_no_bias(activation, delta):
+    """One J in every cell, exactly known: the barrier sum is 27 values per cell of one point's value.  Over 96 J the
+    relative errors of a value average out: a point's roundings have a deviation of about 1.7 units of 2^-53, so their
+    mean stays below three deviations, 3 * 1.7 / sqrt(96) units."""
+    from seq_vp_3d_b200.grid import grid_from_shape
+    from seq_vp_3d_b200.pair import DevicePair
+    shape = (5, 5, 6)
+    grid = grid_from_shape(shape, (1., 1., 1.))
+    zero = np.zeros(shape)
+    P = DevicePair(grid, zero, zero, np.zeros(shape + (3,)), **W, activation=activation, delta=delta)
+    L = np.longdouble
+    errors = []
+    for J in np.round(np.linspace(delta + .02 * (activation - delta), activation * .9, 96) * 2. ** 16) / 2. ** 16:
+        u = np.zeros(shape + (3,))
+        u[..., 0] = (J - 1) * (np.arange(6) - 2.5)
+        terms, bad = P.energy(torch.from_numpy(u).cuda(), torch.zeros(shape, dtype=torch.float64, device="cuda"))
+        a, d = L(activation), L(delta)
+        r = (a - L(J)) / (a - d)
+        exact = -27 * grid.n_cells * L(np.float64(W["kappa"]) / 27) * r * r * np.log1p(-r)
+        assert bad == 0
+        errors.append(float((L(terms[4]) - exact) / exact))
+    assert abs(np.mean(errors)) <= 3 * 1.7 / np.sqrt(96) * 2. ** -53
