@@ -243,10 +243,10 @@ __device__ __forceinline__ uint2 fold_half(TI v) {
 // Row strides of the returned tile: [line][column] (left passes; a lane writes two columns at once) and
 // [row][position] (x pass).
 template <class TC> constexpr int kTileCol = kQC<TC> + 4;
-inline __host__ __device__ int tile_row(int mt) { return 32 * mt + 1; }
+inline constexpr __host__ __device__ int tile_row(int mt) { return 32 * mt + 1; }
 template <class TC> constexpr int kStep = 4 * (kQC<TC> + 2) + 1;   // cells of one staged mma step, see dst_pass_kernel
 template <class TC>
-size_t dst_smem(bool x, int mt) {
+constexpr size_t dst_smem(bool x, int mt) {
     const size_t stage = sizeof(uint4) * 2 * 2 * 2 * kStep<TC>;
     const size_t tile = sizeof(TC) * (x ? (size_t)kQC<TC> * tile_row(mt) : (size_t)32 * mt * kTileCol<TC>);
     return stage > tile ? stage : tile;
@@ -458,23 +458,10 @@ __global__ void __launch_bounds__(DT, 512 / DT) dst_pass_kernel(DstFrag D, const
     }
 }
 
-// the passes' shared memory may lie above the 48 KB default: set once per kernel and device (see allow_slices in q1.cu)
 template <bool XP, bool PRE, int MW, int EPI, class TC, class TI, class TO>
 int launch_dst(const DstFrag &F, const TI *in, long long ncol, int W, long long bs, TO *out, const double *pre,
                const double *den, const double *post, double sign, cudaStream_t s) {
-    static std::mutex mu;
-    static bool done[64] = {};
-    int dev = 0;
-    SVP_CUDA(cudaGetDevice(&dev));
-    SVP_REQUIRE(dev >= 0 && dev < 64, "launch_dst: device ordinal out of range");
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!done[dev]) {
-            SVP_CUDA(cudaFuncSetAttribute(dst_pass_kernel<XP, PRE, MW, EPI, TC, TI, TO>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dst_smem<TC>(XP, 2 * MW)));
-            done[dev] = true;
-        }
-    }
+    static_assert(dst_smem<TC>(XP, 2 * MW) <= 48 * 1024, "a pass needs no more than the default shared memory");
     const long long blocks = div_up(ncol, kQC<TC>) * F.tiles;
     SVP_REQUIRE(blocks <= 0x7fffffffLL && ncol <= 0xffffffffLL, "dst pass: grid too large");
     SVP_LAUNCH((dst_pass_kernel<XP, PRE, MW, EPI, TC, TI, TO><<<(unsigned)blocks, DT, dst_smem<TC>(XP, F.mt), s>>>(
@@ -579,7 +566,7 @@ static int dst_pass(const svp_pair *p, int axis, const TI *in, TO *out, const do
     return SVP_OK;
 }
 
-// Folded half matrices of the orthonormal DST-I (see HalfDst): H_g[a][k] = S[2a + g][k], k < ceil(n/2) (g = 0) or
+// Folded half matrices of the orthonormal DST-I (see dst_pass_kernel): H_g[a][k] = S[2a + g][k], k < ceil(n/2) (g = 0) or
 // floor(n/2) (g = 1).
 std::vector<double> dst1_half(int n) {
     std::vector<double> S = dst1_matrix(n);

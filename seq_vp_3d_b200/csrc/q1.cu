@@ -2111,8 +2111,10 @@ unsigned slice_blocks(const Q1Const &q) { return blocks_for(q.ncell, CS, 2 * CEL
 unsigned slice_blocks(const svp_pair *p) { return slice_blocks(p->q); }
 // dynamic shared memory of the slice kernels: k doubles per thread
 constexpr size_t slice_bytes(int k) { return sizeof(double) * (size_t)k * CS; }
+// the cell kernels' slices, beside block_reduce_dd's 1 KB, fit the default
+static_assert(slice_bytes(kDiffSlots) + 1024 <= 48 * 1024, "a cell kernel's slice is above the default shared memory");
 int allow_slices() {
-    // large slices are above the 48 KB default.  The attribute belongs to the device's context (the primary
+    // the two-field barrier kernels' J (54 KB) are above the 48 KB default.  The attribute belongs to the device's context (the primary
     // context torch and this library share), so it is set on the first call per device, not on every launch: a
     // cudaFuncSetAttribute costs host time that the GPU then spends idle.
     static std::mutex mu;
@@ -2122,10 +2124,6 @@ int allow_slices() {
     SVP_REQUIRE(dev >= 0 && dev < 64, "allow_slices: device ordinal out of range");
     std::lock_guard<std::mutex> lock(mu);
     if (done[dev]) return SVP_OK;
-    SVP_CUDA(cudaFuncSetAttribute(cell_soft_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)slice_bytes(kDiffSlots)));
-    SVP_CUDA(cudaFuncSetAttribute(cell_soft_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)slice_bytes(kDiffSlots)));
     SVP_CUDA(cudaFuncSetAttribute(cell_barrier_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)(sizeof(double) * 54 * BT)));
     SVP_CUDA(cudaFuncSetAttribute(cell_barrier_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2195,8 +2193,6 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
     SVP_REQUIRE(p && u && warped && terms5, "svp_energy: null argument");
     cudaStream_t s = (cudaStream_t)stream;
     unsigned nb = node_blocks(p->q.nnode), cb = slice_blocks(p), bb = cell_barrier_blocks(p->q);
-    int rc = allow_slices();
-    if (rc) return rc;
     { svp::KernelTimer _t("node_energy_kernel", s); SVP_LAUNCH(node_energy_kernel<<<nb, 256, 0, s>>>(p->q, u, warped, p->fixed, p->u_ref, p->partial)); }
     SVP_LAUNCH_CHECK("node_energy_kernel");
     dd *pc = p->partial + (long long)nb * 2, *pb = pc + (long long)cb * 2;
@@ -2216,7 +2212,8 @@ extern "C" int svp_energy(svp_pair *p, const double *u, const double *warped, do
     red.add(p->partial, nb, 2, 0);
     red.add(pc, cb, 2, 4);
     red.add(pb, bb, 2, 8);
-    if ((rc = reduce_results(p, red, s))) return rc;
+    const int rc = reduce_results(p, red, s);
+    if (rc) return rc;
     const double *tmp = p->host;
     for (int k = 0; k < 2; k++) node2[k] = tmp[2 * k] + tmp[2 * k + 1];
     for (int k = 0; k < 3; k++) cell3[k] = tmp[4 + 2 * k] + tmp[4 + 2 * k + 1];
@@ -2467,8 +2464,6 @@ static int run_gather(svp_pair *p, const GatherSpec &g, const LT *L1, const LT *
 // not finite, and no cell is evaluated for them.  *has2: the cells whose L2 values were written.
 static int grad64(svp_pair *p, const double *u, double mu_scale, double nu_scale, bool barrier, bool split,
                   const uint8_t *active, const uint8_t **has2, cudaStream_t s) {
-    int rc = allow_slices();
-    if (rc) return rc;
     uint8_t *flags = barrier && !active ? p->flags : nullptr;
     const uint8_t *marked = active ? active : flags;
     if (p->q.mu * mu_scale == 0. && p->q.nu * nu_scale == 0.) {
