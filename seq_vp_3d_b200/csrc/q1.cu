@@ -230,7 +230,7 @@ __device__ __forceinline__ void add_flux(R *sl, int T, int ix, int iy, int iz, c
         sl[(54 + (ix * 3 + iy) * 3 + r) * T] += f[r][2];
     }
 }
-// adjoint of the edge interpolation (scatter_edges) reading S from the slice
+// adjoint of the edge interpolation: adds the fluxes S (add_flux) from the slice to the vertex values L
 template <class R, class C>
 __device__ __forceinline__ void scatter_slice(const R *sl, int T, const C n[3], const C m[3], const C ih[3],
                                               R L[8][3]) {

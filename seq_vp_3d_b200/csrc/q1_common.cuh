@@ -170,27 +170,8 @@ __device__ __forceinline__ void cell_edges(const T v[8][3], T E[3][4][3]) {
     }
 }
 
-// Derivative tables at a 3-point rule per axis: G[j][s][t][r] = d u_r / d x_j at the point whose two other
-// coordinates take nodes s (the lower-numbered other axis) and t (the higher); n[] nodes, m[] = 1 - nodes.
-template <class T>
-__device__ __forceinline__ void point_derivatives(const T E[3][4][3], const T n[3], const T m[3], const T ih[3],
-                                                  T G[3][3][3][3]) {
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-#pragma unroll
-        for (int s = 0; s < 3; s++)
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                // interpolate along the lower other axis first (edges e = b0 + 2 b1)
-                T l0 = m[s] * E[j][0][r] + n[s] * E[j][1][r];
-                T l1 = m[s] * E[j][2][r] + n[s] * E[j][3][r];
-#pragma unroll
-                for (int t = 0; t < 3; t++) G[j][s][t][r] = (m[t] * l0 + n[t] * l1) * ih[j];
-            }
-}
-
-// Column j of grad u at one point, straight from the edges (the same operation sequence as point_derivatives, so
-// the values are bitwise those of the tables): s indexes the lower-numbered other axis, t the higher.
+// Column j of grad u at one point, straight from the edges: first along the lower-numbered other axis (node s), then
+// along the higher (t); n nodes, m = 1 - nodes.
 template <int J, class T>
 __device__ __forceinline__ void column(const T E[3][4][3], T ms, T ns, T mt, T nt, T ih, T out[3]) {
 #pragma unroll
@@ -280,17 +261,6 @@ __device__ __forceinline__ void sweep2(const R E[3][4][3], const R E2[3][4][3], 
     }
 }
 
-// V[r][j] at point (ix, iy, iz) from the tables
-template <class T>
-__device__ __forceinline__ void grad_at(const T G[3][3][3][3], int ix, int iy, int iz, T V[3][3]) {
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-        V[r][0] = G[0][iy][iz][r];
-        V[r][1] = G[1][ix][iz][r];
-        V[r][2] = G[2][ix][iy][r];
-    }
-}
-
 // Cofactor rows (cross products of cyclic rows of F = I + V) and J = F0 . A0 (geometry.py:11 cofactor, :26 determinant).
 template <class T>
 __device__ __forceinline__ void cofactor_det(const T V[3][3], T A[3][3], T &J) {
@@ -327,40 +297,6 @@ __device__ __forceinline__ void curl_of(const T V[3][3], T C[3]) {
     C[0] = V[2][1] - V[1][2];
     C[1] = V[0][2] - V[2][0];
     C[2] = V[1][0] - V[0][1];
-}
-
-// Adjoint of point_derivatives: accumulate vertex values L[a][r] from per-point fluxes summed over the free axis,
-// S[j][s][t][r] (same indexing as G).
-template <class T>
-__device__ __forceinline__ void scatter_edges(const T S[3][3][3][3], const T n[3], const T m[3], const T ih[3],
-                                              T L[8][3]) {
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-            T e[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll
-            for (int s = 0; s < 3; s++) {
-                T t0 = T(0), t1 = T(0);
-#pragma unroll
-                for (int t = 0; t < 3; t++) {
-                    T v = S[j][s][t][r] * ih[j];
-                    t0 += m[t] * v;
-                    t1 += n[t] * v;
-                }
-                e[0] += m[s] * t0;
-                e[1] += n[s] * t0;
-                e[2] += m[s] * t1;
-                e[3] += n[s] * t1;
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                int lo = k & 1, hi = k >> 1;
-                int a = j == 0 ? 2 * lo + 4 * hi : (j == 1 ? lo + 4 * hi : lo + 2 * hi);
-                L[a | (1 << j)][r] += e[k];
-                L[a][r] -= e[k];
-            }
-        }
 }
 
 // ------------------------------------------------------------------------------------------- localized barrier
