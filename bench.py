@@ -158,8 +158,9 @@ FLOP_PER_CELL = {
     "cell_grad_kernel": 3213,
     # edges 84 + columns 27 x 14 + 27 x (3 rows x (9 + 3 + 8 + 4 + 16 + 16) + 4) + the state-independent curl term 24
     "cell_ggn_diag_kernel": 5130,
-    # one field 678 + 12 edge quadratics 120 + Bernstein 27 x 4 + minima 54
-    "cell_min_jd_kernel": 960,
+    # one field: edges 72, averages 120, identity 12, determinants 27 x 14; 12 edge quadratics 120 + Bernstein 27 x 4 +
+    # minima 54
+    "cell_min_jd_kernel": 864,
 }
 FP64_PEAK_TFLOPS = 148 * 64 * 2 * 1.965e9 / 1e12     # nominal: 148 SMs x 64 FP64 FMA/clk x 2 x 1965 MHz
 # float32 operations per cell of the mixed form's cell kernels (the float64 barrier of the flagged cells runs in its
@@ -176,11 +177,11 @@ FLOP32_PER_CELL = {
     "cell_ggn_diag32_kernel": 8835,
 }
 FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12    # nominal: 148 SMs x 128 FP32 FMA/clk x 2 x 1965 MHz
-# DRAM bytes (read + write) per cell measured by ncu on a 160^3 grid (4,019,679 cells; profiles/
-# trial_certify_gradient_dst_160.md); scaled to a launch by the cells it processes (traffic grows with the cell count:
-# every launch streams its fields once, plus neighbour re-reads of the same order)
+# DRAM bytes (read + write) per cell measured by ncu on a 160^3 grid (4,019,679 cells); scaled to a launch by the cells it
+# processes (traffic grows with the cell count: every launch streams its fields once, plus neighbour re-reads of the
+# same order)
 TRAFFIC_PER_CELL = {"cell_trial_kernel": (481246976 + 7654144) / 4019679,
-                    # 160x192x224 (6,772,287 cells; profiles/cell_kernels_head_pair_160x192x224.md)
+                    # 160x192x224 (6,772,287 cells)
                     "cell_trial32_kernel": (813766656 + 19263232) / 6772287,
                     "cell_grad32_kernel": (325485312 + 340621568) / 4019679,
                     "edge_hull_kernel": (106352896 + 8323072) / 4019679,
@@ -210,7 +211,8 @@ def kernel_counts(shape):
         # mixed form: the same float64 inputs, float32 locals out
         "cell_grad32_kernel": (2 * 24 * nn + 96 * nc, None),
         "cell_ggn_diag32_kernel": (24 * nn + 96 * nc, None),
-        "edge_hull_kernel": (24 * nn + 9 * nc, None),
+        # the first stage of certify_map; 8 bytes more per cell that it lists, which depends on the state
+        "edge_hull_kernel": (24 * nn, None),
         # trial u, base u, base warped, fixed, u_ref in; warped (+ gradient) out; coefficients cache resident
         "warp_trial_kernel_grad": ((24 + 24 + 8 + 8 + 24 + 8 + 24) * nn, None),
         "warp_trial_kernel": ((24 + 24 + 8 + 8 + 24 + 8) * nn, None),
@@ -221,7 +223,6 @@ def kernel_counts(shape):
         "dst_right_kernel": (2 * 3 * 8 * nf, dst[0]),
         "node_diff_kernel": (2 * (24 + 8) * nn + 8 * nn + 24 * nn, None),
         "node_energy_kernel": ((24 + 8 + 8 + 24) * nn, None),
-        "precheck_kernel": (24 * nn, None),
         "cell_min_jd_kernel": (24 * nn + 8 * nc, c("cell_min_jd_kernel")),
     }
 

@@ -237,20 +237,17 @@ int svp_trial_energy(svp_pair *p, const double *base_u, const double *base_warpe
                      int64_t *barrier_violations, void *stream);
 
 /* The same two evaluations with per-cell barrier activity masks (uint8, one per cell: 1 where some closed27 J of
- * the cell is below the barrier activation).  trial_active (optional) receives the trial's mask;
- * svp_energy_difference_masked, given both states' masks, skips the closed27 sweep of cells inactive in both
- * fields.  The results are bitwise those of svp_trial_energy / svp_energy_difference (the skipped points contribute
- * nothing). */
+ * the cell is below the barrier activation).  trial_active (optional) receives the trial's mask.  Masks that
+ * svp_energy_difference_masked is given are not read: the cells near the activation are found from the J that it
+ * evaluates.  The results are bitwise those of svp_trial_energy / svp_energy_difference. */
 int svp_trial_energy_masked(svp_pair *p, const double *base_u, const double *base_warped, const double *trial_u,
                             double *trial_warped, double *trial_image_grad, uint8_t *trial_active, double *terms5,
                             double *diff2, int64_t *barrier_violations, void *stream);
 int svp_energy_difference_masked(svp_pair *p, const double *base_u, const double *base_warped, const double *trial_u,
                                  const double *trial_warped, const uint8_t *base_active, const uint8_t *trial_active,
                                  double *diff2, void *stream);
-/* svp_trial_energy_masked given also the base's mask (base_active: the mask its own evaluation returned, or NULL):
- * the base's closed27 sweep then runs only in cells where some point of the base or of the trial is below the
- * activation, the only cells whose barrier difference is not zero.  Values bitwise those of
- * svp_trial_energy_masked. */
+/* svp_trial_energy_masked given also the base's mask (base_active: the mask its own evaluation returned, or NULL), which
+ * is not read, as above.  Values bitwise those of svp_trial_energy_masked. */
 int svp_trial_energy_active(svp_pair *p, const double *base_u, const double *base_warped, const double *trial_u,
                             double *trial_warped, double *trial_image_grad, const uint8_t *base_active,
                             uint8_t *trial_active, double *terms5, double *diff2, int64_t *barrier_violations,

@@ -1,9 +1,11 @@
 // Fused per-cell Q1 kernels of the certified-registration energy (FP64 plain form):
-//   warp_kernel        cubic B-spline value (+ gradient) at X + u, image and proximity energy sums
-//   cell_energy_kernel Gauss27 JD/curl penalties against u_ref, closed27 localized barrier
-//   cell_grad_kernel   per-cell vertex gradients (soft penalties, barrier) -> SoA locals
-//   gather_kernel      atomic-free node gather in fixed vertex order, plus the node terms
-//   ggn kernels, stable-difference kernels, node JD measure, global closed27 cubic root
+//   warp_kernel          cubic B-spline value (+ gradient) at X + u, image and proximity energy sums
+//   cell_soft_kernel     JD/curl penalties against u_ref and their stable changes, from the closed27 J
+//   cell_barrier_kernel  localized barrier, its change and violations of the cells near the activation
+//   cell_grad_kernel     per-cell vertex gradients of the soft penalties -> SoA locals; cell_grad_barrier_kernel adds
+//                        the barrier's
+//   gather_kernel        atomic-free node gather in fixed vertex order, plus the node terms
+//   ggn kernels, node JD measure, global closed27 cubic root; the mixed form's float32 cell kernels
 // Reference: jd_curl/three_d/{residuals.py, linearization.py, energy_comparison.py, interpolation.py,
 // solvers/jd_affine.py, solvers/global_jd_step.py}.
 #include <cmath>
@@ -206,8 +208,8 @@ __global__ void __launch_bounds__(256) sample_points_kernel(SplineRef S, const d
 
 // ============================================================================================== cell helpers
 // Kernels with 27-point tables keep them in a per-thread slice of dynamic shared memory (slice k at
-// smem[k * blockDim.x + threadIdx.x]: bank-conflict free); the edges of the fields stay in registers and the
-// point loops stay rolled, so no kernel touches local memory.
+// smem[k * blockDim.x + threadIdx.x]: bank-conflict free); the edges of the fields stay in registers.  Local memory
+// is touched by cell_grad_kernel (64 bytes of spills) and cell_ggn_hvp_kernel (148).
 constexpr int CS = 64;     // threads per block of the shared-memory cell kernels
 
 __device__ __forceinline__ void load_edges(const double *__restrict__ u, long long n0, const Q1Const &q,
@@ -1370,7 +1372,7 @@ __global__ void __launch_bounds__(256) node_diff_kernel(Q1Const q, const double 
 // Bound by the latency of its scattered loads (16 warps per SM at 128 registers; 85 registers spill and lose) and the
 // float64 work between them.  At 256^3: 1441 us; 1401 with a plane of coefficients fetched ahead, 1329 with the L1
 // prefetches, 1240 with 6 reciprocals per axis read as pairs in place of 14 single ones, 1211 with the differences
-// accumulated in 8 operations for 20, 1136 with the weights' roots from a table.  Its 16 doubles a node at 6.55 TB/s
+// accumulated in 8 operations for 26, 1136 with the weights' roots from a table.  Its 16 doubles a node at 6.55 TB/s
 // would take 328 us.
 template <bool GRAD>
 __global__ void __launch_bounds__(256) warp_trial_kernel(Q1Const q, SplineRef S, const double *__restrict__ ua,

@@ -56,10 +56,9 @@ __device__ __forceinline__ dd dd_shfl_xor(dd a, int o) {
 }
 
 // Sums of K double-doubles over a warp, lanes 16, 8, 4, 2, 1 apart.  While a lane holds several values it keeps half of
-// them and sends the others to its partner, so 6 values take 8 additions per lane in place of 30 (each is 20 float64
+// them and sends the others to its partner, so 6 values take 8 additions per lane in place of 30 (each is 26 float64
 // operations: at one element per thread they are the kernel).  dd_add is symmetric, so every value has the bits of
-// adding it in all lanes.  Value `first` is in acc[0] of the one lane that returns
-// true for it.
+// adding it in all lanes.  Value `first` is in acc[0] of the one lane that returns true for it.
 template <int K>
 __device__ __forceinline__ bool warp_reduce_dd(dd (&acc)[K], int &first) {
     const int lane = threadIdx.x & 31;

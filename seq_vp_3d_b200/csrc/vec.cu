@@ -9,8 +9,10 @@ namespace svp {
 namespace {
 
 // acc += a b, product and sum with their errors (the dot product of Ogita, Rump and Oishi, "Accurate sum and dot
-// product", 2005: as accurate as twice the precision, rounded once): 11 operations, where a double-double addition of the
-// exact product takes 22 and made step_dots_kernel float64-bound (287 us at 20 M elements).  dot_end: as a double-double.
+// product", 2005: as accurate as twice the precision, rounded once): 10 operations, where a double-double addition of the
+// exact product takes 28 and made step_dots_kernel float64-bound (287 us at 20 M elements, now 180).  The low word rounds
+// once more per element than a normalised sum's: 80-element sums of random products, added up, give the same double up to
+// a condition number of 1e14 and differ in the last bit at 1e16.  dot_end: as a double-double.
 __device__ __forceinline__ void dot_add(dd &acc, double a, double b) {
     const dd p = two_prod(a, b), s = two_sum(acc.hi, p.hi);
     acc.hi = s.hi;

@@ -96,8 +96,8 @@ class DevicePair:
         return np.array(t[:]), int(bad.value)
 
     def energy_difference(self, base_u, base_w, trial_u, trial_w, base_active=None, trial_active=None, stream=None):
-        """(E(trial) - E(base), F(trial) - F(base)), cancellation-free; the optional barrier activity masks of the
-        two states only skip work (same values)."""
+        """(E(trial) - E(base), F(trial) - F(base)), cancellation-free.  The barrier activity masks of the two states
+        are accepted and not used: the cells near the activation are found from the J evaluated here."""
         d = (ctypes.c_double * 2)()
         _lib.call("svp_energy_difference_masked", self._h, ptr(base_u), ptr(base_w), ptr(trial_u), ptr(trial_w),
                   ptr(base_active), ptr(trial_active), d, stream_ptr(stream))
@@ -118,8 +118,8 @@ class DevicePair:
     def trial_energy(self, base_u, base_w, trial_u, with_gradient=True, base_active=None, stream=None):
         """Warp and evaluate a trial against its base in one pass: (warped, image_grad or None, terms[5],
         barrier violations, (E(trial) - E(base), F(trial) - F(base)), the trial's barrier activity mask).
-        base_active (the base's own mask) limits the base's barrier sweep to the cells where it can contribute;
-        the values are the same bits."""
+        base_active (the base's own mask) is accepted and not used: the cells near the activation are found from the
+        J evaluated here."""
         w = self.node()
         g = self.node(3) if with_gradient else None
         act = self.cell_mask()

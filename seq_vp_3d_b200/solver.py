@@ -137,7 +137,8 @@ class Registration:
         self.certifier = cert_mod.certifier(grid, self.config, directed=precision == "mixed")
         # Trial energies and the outer comparison are float64 in both forms: the closed27 cell kernels evaluate a
         # trial against its base in 1.24 ms on 160x192x224 where the float32 screen (svp_trial_energy_screened, still
-        # an entry point for hosts that screen) takes 1.86 ms, so nothing is screened here.
+        # an entry point for hosts that screen) takes 1.86 ms, so nothing is screened here.  The record of a
+        # screen stays among a result's counts, always off, for readers of results.
         self.screen = dict(on=False, evaluations=0, checks=0, band_hits=0, violations=0, max_error_over_band=0.)
         self.q_sum = grid.node_weight_total()
         self.length = float(np.linalg.norm([a[-1] - a[0] for a in grid.axes]))
