@@ -254,8 +254,9 @@ int svp_trial_energy_active(svp_pair *p, const double *base_u, const double *bas
                             void *stream);
 
 /* svp_trial_energy_active with the JD and curl penalties of the trial and of its differences evaluated in float32
- * (a screen for hosts that take one; the reference screens trial energies in float32 in its default execution,
- * backends/accelerated.py:66-77).  The node terms (image, proximity), the barrier, its violations and the activity
+ * (a screen for hosts written for one, as the reference screens trial energies in float32 in its default execution,
+ * backends/accelerated.py:66-77; on B200 the float64 call is the faster one, 1.24 against 1.86 ms for the soft cell
+ * kernel at 160x192x224).  The node terms (image, proximity), the barrier, its violations and the activity
  * mask are those of svp_trial_energy_active bit for bit (one kernel evaluates both, here in the cells with some float32
  * closed27 J within 1e-3 of the activation), the barrier's difference equal within rounding (the order of its sum);
  * terms5[2..3] and the JD/curl parts of diff2[0] carry float32 rounding.  band (host) receives an estimate of that error's magnitude: the residuals'
