@@ -282,7 +282,7 @@ __device__ __forceinline__ void scatter_slice(const R *sl, int T, const C n[3], 
 // flags[c]: bit 0, some closed27 J of the state may be below the activation; bit 1, some of the base may be.
 // cell_barrier_kernel evaluates the barrier of those cells; elsewhere it and its change are zero.  A cell with a
 // column that is not finite is flagged too.
-constexpr int kEnergySlots = 45, kDiffSlots = 90;
+constexpr int kEnergySlots = 27, kDiffSlots = 72;
 template <bool ENERGY, bool DIFF>
 __global__ void __launch_bounds__(CS) cell_soft_kernel(Q1Const q, const double *__restrict__ ua,
                                                        const double *__restrict__ ub,
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(CS) cell_soft_kernel(Q1Const q, const double *
     extern __shared__ double smem[];
     double *sJ = smem + threadIdx.x;
     const int T = blockDim.x;
-    double *sC = sJ + 27 * T, *sR = sJ + 45 * T, *sX = sJ + 72 * T;
+    double *sR = sJ + 27 * T, *sX = sJ + 54 * T;
     dd acc[2] = {{0., 0.}, {0., 0.}}, dif[2] = {{0., 0.}, {0., 0.}};
     const double wj = .5 * q.mu * q.omega, wc = .5 * q.nu * q.omega, low = near_bound(q.act);
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < q.ncell;
@@ -300,28 +300,25 @@ __global__ void __launch_bounds__(CS) cell_soft_kernel(Q1Const q, const double *
         const long long n0 = cell_node0(c, q);
         Columns C;
         {
-            load_columns(uref, n0, q, C);
-            double k[18];
-            curl_coefficients(C, k);
+            double v[8][3], w[8][3], k[18];
+            load_cell(ub, n0, q, v);
+            load_cell(uref, n0, q, w);
+            curl_difference(v, w, q, k);
+            if (ENERGY)
+                acc[1] = dd_add_d(acc[1], __dmul_rn(q.omega, curl_sum([&](int i, double &a) {
+                                                        a = __fma_rn(k[i], k[i], a);
+                                                    })));
+            if (DIFF)
 #pragma unroll
-            for (int i = 0; i < 18; i++) sC[i * T] = k[i];
+                for (int i = 0; i < 18; i++) sX[i * T] = k[i];
+            vertex_columns(w, q, C);
             closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
                                  const double (&Z)[3]) { sJ[p * T] = det_minus_one(X, Y, Z); });
         }
         unsigned char flag = 0;
         {
             load_columns(ub, n0, q, C);
-            double k[18], r[27];
-            curl_coefficients(C, k);
-            const double s = curl_sum([&](int i, double &a) {
-                const double x = __dsub_rn(k[i], sC[i * T]);
-                a = __fma_rn(x, x, a);
-                if (DIFF) {
-                    sC[i * T] = k[i];
-                    sX[i * T] = x;
-                }
-            });
-            if (ENERGY) acc[1] = dd_add_d(acc[1], __dmul_rn(q.omega, s));
+            double r[27];
             bool near = false;
             closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
                                  const double (&Z)[3]) {
@@ -341,14 +338,14 @@ __global__ void __launch_bounds__(CS) cell_soft_kernel(Q1Const q, const double *
                 for (int i = 0; i < 27; i++) sR[i * T] = r[i];
         }
         if (DIFF) {
-            load_columns(ua, n0, q, C);
-            double k[18], d[27];
-            curl_coefficients(C, k);
-            const double s = curl_sum([&](int i, double &a) {
-                const double x = __dsub_rn(sC[i * T], k[i]);
-                a = __fma_rn(x, __fma_rn(2., sX[i * T], -x), a);
-            });
-            dif[1] = dd_add_d(dif[1], __dmul_rn(wc, s));
+            double v[8][3], w[8][3], k[18], d[27];
+            load_cell(ub, n0, q, v);
+            load_cell(ua, n0, q, w);
+            curl_difference(v, w, q, k);
+            dif[1] = dd_add_d(dif[1], __dmul_rn(wc, curl_sum([&](int i, double &a) {
+                                                    a = __fma_rn(k[i], __fma_rn(2., sX[i * T], -k[i]), a);
+                                                })));
+            vertex_columns(w, q, C);
             bool near = false;
             closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
                                  const double (&Z)[3]) {
@@ -487,20 +484,19 @@ __global__ void __launch_bounds__(CS) cell_grad_kernel(Q1Const q, const double *
         const long long n0 = cell_node0(c, q);
         Columns C, G;
         {
-            load_columns(uref, n0, q, C);
-            double k[18];
-            curl_coefficients(C, k);
+            double v[8][3], w[8][3], k[18];
+            load_cell(u, n0, q, v);
+            load_cell(uref, n0, q, w);
+            curl_difference(v, w, q, k);
 #pragma unroll
             for (int i = 0; i < 18; i++) sC[i * T] = k[i];
+            vertex_columns(w, q, C);
             closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
                                  const double (&Z)[3]) { sJ[p * T] = det_minus_one(X, Y, Z); });
         }
         load_columns(u, n0, q, C);
         {
-            double k[18], r[27];
-            curl_coefficients(C, k);
-#pragma unroll
-            for (int i = 0; i < 18; i++) sC[i * T] = __dsub_rn(k[i], sC[i * T]);
+            double r[27];
             bool near = false;
             closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3],
                                  const double (&Z)[3]) {

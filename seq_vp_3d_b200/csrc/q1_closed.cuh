@@ -243,6 +243,20 @@ __device__ __forceinline__ void curl_coefficients(const Columns &C, double (&c)[
     c[6] = A0.D2; c[7] = B0.D2; c[8] = A1.D1; c[9] = B1.D2; c[10] = A2.D1; c[11] = B2.D1;
     c[12] = A0.D12; c[13] = B0.D12; c[14] = A1.D12; c[15] = B1.D12; c[16] = A2.D12; c[17] = B2.D12;
 }
+// The same of a - b, from the fields' vertices.  The curl is linear, and the difference of two close states is small and
+// formed almost without rounding, so its coefficients round relative to themselves, where the difference of the two
+// fields' coefficients carries the rounding of both.
+__device__ __forceinline__ void curl_difference(const double (&a)[8][3], const double (&b)[8][3], const Q1Const &q,
+                                                double (&c)[18]) {
+    double d[8][3];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int r = 0; r < 3; r++) d[i][r] = __dsub_rn(a[i][r], b[i][r]);
+    Columns D;
+    vertex_columns(d, q, D);
+    curl_coefficients(D, c);
+}
 __device__ constexpr double curl_weight(int k) { return k < 3 ? 1. / 16 : (k < 12 ? 1. / 48 : 1. / 144); }
 template <class F>
 __device__ __forceinline__ double curl_sum(F &&f) {
