@@ -148,14 +148,15 @@ def peaks():
 # (3 components x (2 bilinear lerps of 3 + final lerp and 1/h of 4)); det = 17; cofactor+det = 35; curl = 3.
 # Barrier-active points add a few hundred more (not counted).
 FLOP_PER_CELL = {
-    # three fields x 732 + two residuals (subtract 27, transform 162, sums 100) + the curl sums 130
-    "cell_trial_kernel": 2904,
-    "cell_diff_kernel": 2850,
-    # two fields x 732 + one residual 289 + the curl sum 54
-    "cell_energy_kernel": 1807,
-    # two fields x 732 + residuals 27 + mass matrices 270 + adjoint pass 27 x (6 + 36) + its averages 120 + scatter 108
+    # three fields x 678 + two differences' curls (24 + edges 48 + 54) + two residuals (subtract 27, transform 162, sums
+    # 100) + the curl sums 130
+    "cell_trial_kernel": 2994,
+    "cell_diff_kernel": 2940,
+    # two fields x 678 + one difference's curl 126 + one residual 289 + the curl sum 54
+    "cell_energy_kernel": 1825,
+    # two fields x 678 + the difference's curl 126 + residuals 27 + mass matrices 270 + adjoint pass 27 x (6 + 36) + its averages 120 + scatter 108
     # + curl adjoint 90
-    "cell_grad_kernel": 3213,
+    "cell_grad_kernel": 3231,
     # edges 84 + columns 27 x 14 + 27 x (3 rows x (9 + 3 + 8 + 4 + 16 + 16) + 4) + the state-independent curl term 24
     "cell_ggn_diag_kernel": 5130,
     # one field: edges 72, averages 120, identity 12, determinants 27 x 14; 12 edge quadratics 120 + Bernstein 27 x 4 +

@@ -274,9 +274,9 @@ __device__ __forceinline__ void scatter_slice(const R *sl, int T, const C n[3], 
 //
 // Bound: FP64 issue.  About 2,000 FP64 instructions per cell with both parts (J of three fields at 27 points each 11
 // operations, edges and averages 162, two Legendre transforms 108); the Gauss27 form took 6,200.  The 27 J - 1, the
-// curl coefficients and the residual coefficients wait in the thread's shared slice (90 doubles: one access costs as
-// much as four FP64 instructions, so tables that are used at once stay in registers).  Trial on 256^3: 11.20 -> 3.04
-// ms per launch, FP64 pipe 64% busy; two warps per scheduler (255 registers) leave its dependency stalls.  Three warps
+// residual's coefficients and its curl's wait in the thread's shared slice (72 doubles: one access costs as much as four
+// FP64 instructions, so tables that are used at once stay in registers).  Trial on 256^3: 11.20 -> 3.04 ms per launch,
+// 2.96 with the curl taken from differences of the fields; FP64 pipe 64% busy; two warps per scheduler (255 registers) leave its dependency stalls.  Three warps
 // (168 registers, 800 bytes of spills) took 5.0 ms, loads of the next field before this field's points 3.36 ms.
 //
 // flags[c]: bit 0, some closed27 J of the state may be below the activation; bit 1, some of the base may be.
@@ -565,8 +565,7 @@ __global__ void __launch_bounds__(BT) cell_grad_barrier_kernel(Q1Const q, const 
             // a cell that is not finite has a gradient only where some point has a slope
             if (!some)
                 for (int p = 0; p < 27; p++) some |= sl[p * BT] != 0.;
-            load_columns(u, cell_node0(c, q), q, C);     // again: 36 columns do not wait in registers
-            add_identity(C);
+            load_columns<true>(u, cell_node0(c, q), q, C);     // again: 36 columns do not wait in registers
             closed_adjoint(C, G, [&](int p) { return sl[p * BT]; });
             double Lb[8][3];
             columns_to_vertices(G, q, Lb);

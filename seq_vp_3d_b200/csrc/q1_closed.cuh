@@ -29,24 +29,31 @@ struct Columns {
 
 __device__ __forceinline__ double mean2(double a, double b) { return __dmul_rn(.5, __dadd_rn(a, b)); }
 
+// ID: the columns of F = I + grad u, the identity added in one rounding (of F, which a compression makes small, and not
+// of grad u).
+template <bool ID = false>
 __device__ __forceinline__ void vertex_columns(const double (&v)[8][3], const Q1Const &q, Columns &C) {
+    auto entry = [](double difference, double ih, bool diagonal) {
+        return ID && diagonal ? __fma_rn(difference, ih, 1.) : __dmul_rn(difference, ih);
+    };
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         const int lo = e & 1, hi = e >> 1;
         const int ax = 2 * lo + 4 * hi, ay = lo + 4 * hi, az = lo + 2 * hi;
 #pragma unroll
         for (int r = 0; r < 3; r++) {
-            C.X[e][r] = __dmul_rn(__dsub_rn(v[ax | 1][r], v[ax][r]), q.ih[0]);
-            C.Y[e][r] = __dmul_rn(__dsub_rn(v[ay | 2][r], v[ay][r]), q.ih[1]);
-            C.Z[e][r] = __dmul_rn(__dsub_rn(v[az | 4][r], v[az][r]), q.ih[2]);
+            C.X[e][r] = entry(__dsub_rn(v[ax | 1][r], v[ax][r]), q.ih[0], r == 0);
+            C.Y[e][r] = entry(__dsub_rn(v[ay | 2][r], v[ay][r]), q.ih[1], r == 1);
+            C.Z[e][r] = entry(__dsub_rn(v[az | 4][r], v[az][r]), q.ih[2], r == 2);
         }
     }
 }
+template <bool ID = false>
 __device__ __forceinline__ void load_columns(const double *__restrict__ u, long long n0, const Q1Const &q,
                                              Columns &C) {
     double v[8][3];
     load_cell(u, n0, q, v);
-    vertex_columns(v, q, C);
+    vertex_columns<ID>(v, q, C);
 }
 
 // The column values of one plane t (0, 1, 2) of its higher other coordinate: P[s][r], s the lower other coordinate.
@@ -136,9 +143,8 @@ __device__ __forceinline__ void spread_nonfinite(const double *__restrict__ u, l
 // The closed27 J of a cell into sl[p T]; C then holds the columns of F.  False where some column is not finite.
 __device__ __forceinline__ bool closed_jacobians(const double *__restrict__ u, long long n0, const Q1Const &q,
                                                  Columns &C, double *sl, int T) {
-    load_columns(u, n0, q, C);
+    load_columns<true>(u, n0, q, C);
     const bool finite = finite_columns(C);
-    add_identity(C);
     closed_points(C, [&](int p, int, int, int, const double (&X)[3], const double (&Y)[3], const double (&Z)[3]) {
         sl[p * T] = det_columns(X, Y, Z);
     });
