@@ -181,7 +181,7 @@ FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12    # nominal: 148 SMs x 128 FP
 # DRAM bytes (read + write) per cell measured by ncu on a 160^3 grid (4,019,679 cells); scaled to a launch by the cells it
 # processes (traffic grows with the cell count: every launch streams its fields once, plus neighbour re-reads of the
 # same order)
-TRAFFIC_PER_CELL = {"cell_trial_kernel": (481246976 + 7654144) / 4019679,
+TRAFFIC_PER_CELL = {"cell_trial_kernel": (474183424 + 10150912) / 4019679,
                     # 160x192x224 (6,772,287 cells)
                     "cell_trial32_kernel": (813766656 + 19263232) / 6772287,
                     "cell_grad32_kernel": (325485312 + 340621568) / 4019679,
