@@ -23,7 +23,7 @@ struct svp_pair {
     double *host = nullptr;                   // pinned results that kernels write (64 doubles)
     long long *counter = nullptr;             // small device counters (8)
     long long *cand = nullptr;                // candidate cells of the T69/T73 node JD extension (ncell)
-    uint8_t *flags = nullptr;                 // (ncell) cells the float32 cell kernels hand to the float64 barrier
+    uint8_t *flags = nullptr;                 // (ncell) cells the soft cell kernels hand to the barrier kernels
     // DST-I Poisson metric
     // folded orthonormal DST-I half matrices, x, y, z, zero-padded and in the mma's fragment order (DstFrag)
     double *dst_f64[3] = {nullptr, nullptr, nullptr};
